@@ -249,6 +249,9 @@ struct dnsmc_solver {
     int slab_len = 0, slab_klen = 0;
     DevBuf<int2> d_posT;   // per cell (ti, ft) for T-only tables
     DevBuf<int4> d_posTX;  // per cell (ti*(nX-1)+xi, ft, fx, ti)
+    DevBuf<float> d_posG;  // per cell T^4 (grey model)
+    int posG_na = 0, posG_nb = 0;  // the padded extents d_posG was written for (0: not written)
+    int last_pna = 0, last_pnb = 0;  // those of the last solve's d_posT / d_posTX
     bool tables_dirty = true;
 
     // fields
@@ -845,6 +848,39 @@ void tiling(const dnsmc_solver *s, int *ta, int *tb, int *npa, int *npb, int *np
     *npw = ni;
 }
 
+// The padded extents of the march's field: the periodic axes continue past
+// their end by the packet's extent (the gas march on the fine grid), so that
+// a lane's cells lie at fixed offsets from the packet's corner; rows of a
+// multiple of 8 values keep their alignment.
+void padded_extents(const dnsmc_solver *s, bool pad, int *pna, int *pnb) {
+    const dnsmc_config &c = s->cfg;
+    *pna = c.jmax;
+    *pnb = c.kmax;
+    if (!pad) return;
+    int ta, tb, npa, npb, npw;
+    tiling(s, &ta, &tb, &npa, &npb, &npw);
+    *pna = march_extent_row(c.jmax, ta);
+    *pnb = march_extent(c.kmax, tb);
+}
+
+// T^4 of the resident fields for the grey march (after new fields; again
+// when the packet's extent has changed).
+int grey_positions(dnsmc_solver *s) {
+    const dnsmc_config &c = s->cfg;
+    int pna, pnb;
+    padded_extents(s, true, &pna, &pnb);
+    if (s->posG_na == pna && s->posG_nb == pnb) return DNSMC_OK;
+    TRY(s->d_posG.ensure((size_t)s->nfields * c.imax * pna * pnb));
+    FieldPos q{};
+    q.fT = s->d_fieldT.p; q.outG = s->d_posG.p;
+    q.nfields = s->nfields; q.nw = c.imax; q.na = c.jmax; q.nb = c.kmax; q.pna = pna; q.pnb = pnb;
+    if (const int rc = launch_field_pos(q, s->stream))
+        return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rc));
+    s->posG_na = pna;
+    s->posG_nb = pnb;
+    return DNSMC_OK;
+}
+
 int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, int tmax_steps,
                   int *d_trace_rec, int *d_trace_n, unsigned int *d_trace_rng) {
     dnsmc_config &c = s->cfg;
@@ -922,7 +958,9 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     P.n_tbins = s->n_tbins_used;
     P.sampler = c.sampler;
     P.nbatch = c.nvar;
-    P.kappa = c.kappa;
+    P.kappa = t.grey_bands && mode != MODE_GREY ? t.gb_kappa : c.kappa;
+    P.uni = t.grey_bands && mode != MODE_GREY ? 1 : 0;
+    P.rda = 1.0f / P.da; P.rdb = 1.0f / P.db;
     P.Wgrey = (float)(4.0 * c.kappa * kSigma);
     P.Tw4[0] = c.T_west * c.T_west * c.T_west * c.T_west;
     P.Tw4[1] = c.T_east * c.T_east * c.T_east * c.T_east;
@@ -980,11 +1018,21 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
                          P.n_groups);
         P.rays_gstride = P.n_packets;
     }
-    const long long ncell = (long long)s->nfields * P.field_stride;
-    if (mode == MODE_TX && !trace) TRY(s->d_posTX.ensure((size_t)ncell));
-    if (mode == MODE_T && !trace) TRY(s->d_posT.ensure((size_t)ncell));
+    padded_extents(s, !mg && !gen, &P.pna, &P.pnb);
+    P.pstride = (long long)c.imax * P.pna * P.pnb;
+    const long long npos = (long long)s->nfields * P.pstride;
+    if (mode == MODE_TX) TRY(s->d_posTX.ensure((size_t)npos));
+    if (mode == MODE_T) TRY(s->d_posT.ensure((size_t)npos));
+    if (mode == MODE_GREY && !mg && !gen) TRY(grey_positions(s));
     P.fieldP = s->d_posT.p;
     P.fieldPX = s->d_posTX.p;
+    P.fieldG = s->d_posG.p;
+    FieldPos fp{};  // table coordinates of the field for this table (once per solve)
+    fp.fT = mode == MODE_TX ? nullptr : s->d_fieldT.p;
+    fp.fTX = mode == MODE_TX ? s->d_fieldTX.p : nullptr;
+    fp.outP = s->d_posT.p; fp.outPX = s->d_posTX.p;
+    fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
+    fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
     TRY(s->d_misc.ensure(4));
     TRY(s->d_counters.ensure(2));
     P.queue = s->d_misc.p;
@@ -996,9 +1044,11 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         int smax = 0;
         if (cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device) != cudaSuccess)
             smax = 48 * 1024;
-        const size_t stat = 1024;  // the march kernels' static shared memory (barriers), at most
-        if (march_smem(P, threads, kLaneCells) + stat > (size_t)smax) threads = 128;
-        if (march_smem(P, threads, kLaneCells) + stat > (size_t)smax)
+        const bool pair = !mg && !gen;
+        const size_t stat = pair ? kPairStaticSmem : 1024;  // the march kernels' static shared memory, at most
+        auto need = [&](int th) { return (pair ? march_pair_smem(P, th) : march_smem(P, th, kLaneCells)) + stat; };
+        if (need(threads) > (size_t)smax) threads = 128;
+        if (need(threads) > (size_t)smax)
             return fail(DNSMC_ERR_TABLE, "a spectral sample's table slab (%d bytes) exceeds the shared memory of the march",
                         P.slab_len * 8);
     }
@@ -1019,6 +1069,13 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.trace_f = tf; P.trace_g = tg; P.trace_p = tp; P.trace_r = tr; P.trace_max = tmax_steps;
         P.trace_rec = d_trace_rec; P.trace_n = d_trace_n; P.trace_rng = d_trace_rng;
         P.tally = nullptr;
+        if (mode != MODE_GREY && (P.pna != s->last_pna || P.pnb != s->last_pnb || P.nfields != s->last.nfields)) {
+            // the coordinates of the last solve are not for this packet shape
+            const int rcp = launch_field_pos(fp, s->stream);
+            if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
+            s->last_pna = P.pna;
+            s->last_pnb = P.pnb;
+        }
         const int rc = mg ? launch_march_mg(mode, P, 1, 32, s->stream, true)
                           : launch_march_ex(mode, P, 1, 32, s->stream, true, cv, false, gen);
         if (rc) return fail(DNSMC_ERR_CUDA, "trace launch: %s", cudaGetErrorString((cudaError_t)rc));
@@ -1098,8 +1155,9 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.item_order = s->d_order.p;
     }
     const int sms = device_sm_count();
-    const size_t smem = march_smem(P, threads, mg ? 1 : kLaneCells);
-    const int occ = mg ? march_mg_occupancy(mode, threads, smem) : march_occupancy_ex(mode, threads, cv, mom, gen, smem);
+    const size_t smem = mg ? march_smem(P, threads, 1) : (gen ? march_smem(P, threads, kLaneCells) : march_pair_smem(P, threads));
+    const int occ = mg ? march_mg_occupancy(mode, threads, smem)
+                       : march_occupancy_ex(mode, P.uni != 0, threads, cv, mom, gen, smem);
     const int blocks = std::max(1, sms * occ);
 
     FinalizeParams F;
@@ -1141,12 +1199,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     // ---- the kernel sequence of a solve (stream-ordered; capturable) -------
     auto kernels = [&](bool events) -> int {
         if (mode != MODE_GREY) {
-            // table coordinates of the field for this table (once per solve)
-            const int rcp = mode == MODE_TX
-                                ? launch_field_pos(nullptr, s->d_fieldTX.p, nullptr, s->d_posTX.p, ncell, P.T0,
-                                                   P.invdT, P.nT, P.X0, P.invdX, P.nX, s->stream)
-                                : launch_field_pos(s->d_fieldT.p, nullptr, s->d_posT.p, nullptr, ncell, P.T0, P.invdT,
-                                                   P.nT, P.X0, P.invdX, P.nX, s->stream);
+            const int rcp = launch_field_pos(fp, s->stream);
             if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
         }
         if (cv) {
@@ -1231,6 +1284,8 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     s->last = P;
     s->lastF = F;
+    s->last_pna = P.pna;
+    s->last_pnb = P.pnb;
     CUDA_TRY(cudaEventRecord(s->ev_done, s->stream));
     s->in_flight = true;
     s->solved = true;
@@ -1414,6 +1469,8 @@ int upload_fields_host(dnsmc_solver *s, int nfields, const float *T, const float
     if (c.grid_num > 1)
         TRY(upload_coarse(s, nfields, want_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, want_x ? 2 : 1));
     s->nfields = nfields;
+    s->posG_na = 0;
+    if (c.model == DNSMC_MODEL_GREY && c.grid_num == 1 && !want_x) TRY(grey_positions(s));
     s->have_x = want_x;
     s->tmax_fields = (float)st[0];
     s->tmin_fields = (float)st[1];
@@ -1597,7 +1654,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     s->d_fw.release(); s->d_k.release(); s->d_ib.release(); s->d_ibw.release();
-    s->d_slab.release(); s->d_posT.release(); s->d_posTX.release();
+    s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posTX.release();
     s->d_cv_grp.release(); s->d_cv_sid.release(); s->d_cv_C.release(); s->d_layer.release();
     s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_Jf.release(); s->d_cv_Cf.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();
@@ -1843,6 +1900,8 @@ int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const
     if (c.grid_num > 1)
         TRY(upload_coarse(s, nfields, dx ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, dx ? 2 : 1));
     s->nfields = nfields;
+    s->posG_na = 0;
+    if (c.model == DNSMC_MODEL_GREY && c.grid_num == 1 && !dx) TRY(grey_positions(s));
     s->have_x = dx != nullptr;
     s->tmax_fields = (float)st[0];
     s->tmin_fields = (float)st[1];

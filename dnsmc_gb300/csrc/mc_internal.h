@@ -54,8 +54,17 @@ struct MarchParams {
     int nfields;
     long long field_stride;   // cells per field (nw*na*nb)
     const float  *fieldT;     // MODE_GREY: temperature
-    const int2   *fieldP;     // MODE_T: (ti, ft) table temperature cell and fraction
-    const int4   *fieldPX;    // MODE_TX: (ti*(nX-1)+xi | ti<<16 ... see CellPos) per cell
+    // MODE_T: (ti, ft) table temperature cell and fraction; MODE_TX:
+    // (ti*(nX-1)+xi, ft, fx, ti); MODE_GREY: T^4, the sign bit set where T is
+    // not positive.  Rows of pna values (j), pnb rows a plane (k), pstride
+    // values a field: na, nb and field_stride, or (the gas march on the fine
+    // grid) the periodic axes continued past their end by the packet's extent
+    const int2   *fieldP;
+    const int4   *fieldPX;
+    const float  *fieldG;
+    int pna, pnb;
+    long long pstride;
+    float rda, rdb;           // 1/da, 1/db (estimates of crossing counts only)
     // spectral tables
     int nbands, nT, nX;
     float T0, invdT, X0, invdX;
@@ -76,7 +85,8 @@ struct MarchParams {
     int n_groups;
     int n_tbins;              // 1: one table (at Tmax); nT: per table temperature
     // grey model
-    float kappa;              // absorption coefficient
+    float kappa;              // absorption coefficient (grey model; uni)
+    int uni;                  // 1: tables of one absorption coefficient, kappa (grey band tables)
     float Wgrey;              // 4 * kappa * sigma
     float Tw4[2];             // wall T^4 (west, east), grey model
     // rays
@@ -251,7 +261,7 @@ long long launch_count();
 // launchers (mc_kernels.cu); all stream-ordered
 int launch_march_ex(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace, bool cv,
                     bool mom, bool gen);
-int march_occupancy_ex(int mode, int threads, bool cv, bool mom, bool gen, size_t smem);
+int march_occupancy_ex(int mode, bool uni, int threads, bool cv, bool mom, bool gen, size_t smem);
 int launch_march_mg(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace);
 int march_mg_occupancy(int mode, int threads, size_t smem);
 // dynamic shared memory of a march launch with `cells` cells per lane: each
@@ -259,6 +269,13 @@ int march_mg_occupancy(int mode, int threads, size_t smem);
 // sums of the item (float pairs, 8 bytes), then per thread the RQMC replicate's shift (uint4)
 inline size_t march_smem(const MarchParams &p, int threads, int cells) {
     return (size_t)((threads + 31) / 32) * (size_t)p.slab_len * 8u + (size_t)threads * (24u * (size_t)cells + 16u);
+}
+// of a launch of the gas march: each warp's slab and walk buffer, then per
+// thread the sums of its two cells; kPairStaticSmem at most beside it
+constexpr int kWalkWords = 176;  // words of a warp's walk buffer (mc_march_pair.cuh)
+constexpr size_t kPairStaticSmem = 256;
+inline size_t march_pair_smem(const MarchParams &p, int threads) {
+    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u) + (size_t)threads * 24u * kLaneCells;
 }
 int launch_march_gen(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace, bool cv,
                      bool mom);                                      // mc_march_gen.cu
@@ -268,17 +285,37 @@ int upload_sobol_dirs_gen(const uint32_t dirs[4][32]);               // mc_march
 // (launch_march_gen: the same march with the general medium)
 int launch_march_pair(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace, bool cv,
                       bool mom);
-int march_pair_occupancy(int mode, int threads, bool cv, bool mom, size_t smem);
+int march_pair_occupancy(int mode, bool uni, int threads, bool cv, bool mom, size_t smem);
 int upload_sobol_dirs_pair(const uint32_t dirs[4][32]);
 int launch_march(int mode, const MarchParams &p, int blocks, int threads,
                  void *stream, bool trace);
 int launch_finalize(const FinalizeParams &p, void *stream);
-int launch_field_pos(const float *fT, const float2 *fTX, int2 *outP, int4 *outPX, long long n, float T0,
-                     float invdT, int nT, float X0, float invdX, int nX, void *stream);
+// Table coordinates (outP or outPX), or T^4 (outG), of every cell of nfields
+// packed fields [f][i][k][j], into rows of pna values and pnb rows a plane
+// (na <= pna < 2 na, nb <= pnb < 2 nb: continued periodically)
+inline int march_extent(int n, int tile) { return n + (tile < n ? tile : n) - 1; }  // n cells, packets of tile
+inline int march_extent_row(int n, int tile) {  // of j: a multiple of 8 keeps the rows' alignment
+    const int r = (march_extent(n, tile) + 7) / 8 * 8;
+    return r < 2 * n ? r : march_extent(n, tile);
+}
+struct FieldPos {
+    const float *fT;
+    const float2 *fTX;
+    int2 *outP;
+    int4 *outPX;
+    float *outG;
+    int nfields, nw, na, nb, pna, pnb;
+    float T0, invdT, X0, invdX;
+    int nT, nX;
+};
+int launch_field_pos(const FieldPos &q, void *stream);
 // src element (i, j, k) at src[base + i*si + j*sj + k*sk]; writes dst[f] layout
 int launch_pack_T(const float *src, float *dst, int nw, int na, int nb,
                   long long si, long long sj, long long sk, long long base,
                   void *stream);
+// T^4 (sign bit set where T is not positive) of a dense field, i fastest, into
+// rows of pna values and pnb rows a plane (as FieldPos::outG)
+int launch_pack_T4(const float *src, float *dst, int nw, int na, int nb, int pna, int pnb, void *stream);
 int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
                    int na, int nb, long long si, long long sj, long long sk,
                    long long base, void *stream);
@@ -287,7 +324,6 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
 int launch_field_stats(const float *fT, const float2 *fTX, long long n,
                        double *partials, double *out, void *stream);
 int field_stats_partials();   // doubles needed in `partials`
-int march_occupancy(int mode, int threads);  // resident blocks per SM
 
 // Control-variate preparation (all stream-ordered).
 struct CvParams {

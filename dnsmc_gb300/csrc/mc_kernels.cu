@@ -44,27 +44,36 @@ namespace dnsmc {
 
 // Table coordinates of the field for the march: p = clamp((T - T0)/dT, 0,
 // nT-1) (and the same for x_H2O), computed once per solve with the same FP32
-// operations the march used to apply per step.
-__global__ void field_pos_kernel(const float *fT, const float2 *fTX, int2 *outP, int4 *outPX, long long n,
-                                 float T0, float invdT, int nT, float X0, float invdX, int nX) {
+// operations the march used to apply per step; or T^4 for the grey model.
+// Row by row of the output, a thread per j.
+__global__ void field_pos_kernel(const FieldPos q) {
+    const long long rows = (long long)q.nfields * q.nw * q.pnb, n = rows * q.pna;
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / q.pna, fw = r / q.pnb;
+        int a = (int)(i - r * q.pna), b = (int)(r - fw * q.pnb);
+        a = a >= q.na ? a - q.na : a;
+        b = b >= q.nb ? b - q.nb : b;
+        const long long src = (fw * q.nb + b) * q.na + a;
         int ti, xi;
         float ft, fx;
-        if (fTX) {
-            const float2 v = fTX[i];
-            float pt = (v.x - T0) * invdT;
-            pt = fminf(fmaxf(pt, 0.0f), (float)(nT - 1));
-            float px = (v.y - X0) * invdX;
-            px = fminf(fmaxf(px, 0.0f), (float)(nX - 1));
-            pos_split(pt, nT, &ti, &ft);
-            pos_split(px, nX, &xi, &fx);
-            outPX[i] = make_int4(ti * (nX - 1) + xi, __float_as_int(ft), __float_as_int(fx), ti);
+        if (q.outG) {
+            const float T = q.fT[src], t2 = T * T, v = t2 * t2;
+            q.outG[i] = T > 0.0f ? v : -v;
+        } else if (q.fTX) {
+            const float2 v = q.fTX[src];
+            float pt = (v.x - q.T0) * q.invdT;
+            pt = fminf(fmaxf(pt, 0.0f), (float)(q.nT - 1));
+            float px = (v.y - q.X0) * q.invdX;
+            px = fminf(fmaxf(px, 0.0f), (float)(q.nX - 1));
+            pos_split(pt, q.nT, &ti, &ft);
+            pos_split(px, q.nX, &xi, &fx);
+            q.outPX[i] = make_int4(ti * (q.nX - 1) + xi, __float_as_int(ft), __float_as_int(fx), ti);
         } else {
-            float pt = (fT[i] - T0) * invdT;
-            pt = fminf(fmaxf(pt, 0.0f), (float)(nT - 1));
-            pos_split(pt, nT, &ti, &ft);
-            outP[i] = make_int2(ti, __float_as_int(ft));
+            float pt = (q.fT[src] - q.T0) * q.invdT;
+            pt = fminf(fmaxf(pt, 0.0f), (float)(q.nT - 1));
+            pos_split(pt, q.nT, &ti, &ft);
+            q.outP[i] = make_int2(ti, __float_as_int(ft));
         }
     }
 }
@@ -185,6 +194,19 @@ __global__ void pack_T_kernel(const float *src, float *dst, int nw, int na, int 
     }
 }
 
+__global__ void pack_T4_kernel(const float *src, float *dst, int nw, int na, int nb, int pna, int pnb) {
+    const long long n = (long long)nw * pnb * pna;
+    for (long long d = blockIdx.x * (long long)blockDim.x + threadIdx.x; d < n; d += (long long)gridDim.x * blockDim.x) {
+        const long long r = d / pna;
+        int a = (int)(d - r * pna), b = (int)(r % pnb);
+        const int w = (int)(r / pnb);
+        a = a >= na ? a - na : a;
+        b = b >= nb ? b - nb : b;
+        const float T = src[w + (long long)nw * (a + (long long)na * b)], t2 = T * T, v = t2 * t2;
+        dst[d] = T > 0.0f ? v : -v;
+    }
+}
+
 __global__ void pack_TX_kernel(const float *srcT, const float *srcX, float2 *dst, int nw, int na,
                                int nb, long long si, long long sj, long long sk, long long base) {
     const long long n = (long long)nw * na * nb;
@@ -259,9 +281,9 @@ int launch_march_ex(int mode, const MarchParams &p, int blocks, int threads, voi
     return launch_march_pair(mode, p, blocks, threads, stream, trace, cv, mom);
 }
 
-int march_occupancy_ex(int mode, int threads, bool cv, bool mom, bool gen, size_t smem) {
+int march_occupancy_ex(int mode, bool uni, int threads, bool cv, bool mom, bool gen, size_t smem) {
     if (gen) return march_gen_occupancy(mode, threads, cv, mom, smem);
-    return march_pair_occupancy(mode, threads, cv, mom, smem);
+    return march_pair_occupancy(mode, uni, threads, cv, mom, smem);
 }
 
 // Multigrid march (reference tables or grey model; no control variate, no
@@ -928,13 +950,10 @@ int launch_cv_mean(const CvParams &c, void *stream) {
     return (int)cudaGetLastError();
 }
 
-int march_occupancy(int mode, int threads) { return march_occupancy_ex(mode, threads, false, false, false, 0); }
-
-int launch_field_pos(const float *fT, const float2 *fTX, int2 *outP, int4 *outPX, long long n, float T0,
-                     float invdT, int nT, float X0, float invdX, int nX, void *stream) {
+int launch_field_pos(const FieldPos &q, void *stream) {
+    const long long n = (long long)q.nfields * q.nw * q.pnb * q.pna;
     dnsmc::note_launch();
-    field_pos_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(fT, fTX, outP, outPX, n, T0, invdT, nT,
-                                                                        X0, invdX, nX);
+    field_pos_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(q);
     return (int)cudaGetLastError();
 }
 
@@ -1033,6 +1052,13 @@ int launch_pack_T(const float *src, float *dst, int nw, int na, int nb, long lon
     const long long n = (long long)nw * na * nb;
     dnsmc::note_launch();
     pack_T_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(src, dst, nw, na, nb, si, sj, sk, base);
+    return (int)cudaGetLastError();
+}
+
+int launch_pack_T4(const float *src, float *dst, int nw, int na, int nb, int pna, int pnb, void *stream) {
+    const long long n = (long long)nw * pna * pnb;
+    dnsmc::note_launch();
+    pack_T4_kernel<<<grid_for(n, 256), 256, 0, (cudaStream_t)stream>>>(src, dst, nw, na, nb, pna, pnb);
     return (int)cudaGetLastError();
 }
 

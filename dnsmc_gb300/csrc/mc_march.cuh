@@ -358,8 +358,9 @@ __device__ __forceinline__ bool slab_bar_wait(const uint64_t *bar, uint32_t pari
 
 // The sample's slab (k, then Ib of its band; slab_len * 8 bytes, a multiple
 // of 16 at a 16-byte aligned address on both sides) into this warp's shared
-// copy.  The previous ray's lookups are done first (the warp converges, and
-// the async proxy is ordered after the generic one).  *phase is the warp's
+// copy: slab_issue starts the copy once the previous ray's lookups are done
+// (the warp converges, and the async proxy is ordered after the generic
+// one), slab_wait waits for it, load_slab does both.  *phase is the warp's
 // barrier parity, flipped per completed copy.  The first wait polls
 // P.slab_polls0 times (kSlabWaitPolls; fewer only in tests of this path).
 // A wait that runs out sets DNSMC_STATUS_COPY_TIMEOUT (the host reports the
@@ -367,8 +368,7 @@ __device__ __forceinline__ bool slab_bar_wait(const uint64_t *bar, uint32_t pari
 // returns false with the phase unchanged: the warp then takes no further
 // copies or items and calls slab_drain before it exits.  The outcome is
 // the same in every lane of the warp.
-__device__ __forceinline__ bool load_slab(const MarchParams &P, int sid, float2 *slk, int lane, uint64_t *bar,
-                                          uint32_t *phase, unsigned int *flags) {
+__device__ __forceinline__ void slab_issue(const MarchParams &P, int sid, float2 *slk, int lane, uint64_t *bar) {
     __syncwarp();
     if (lane == 0) {
         const uint32_t bytes = (uint32_t)P.slab_len * 8u;
@@ -381,12 +381,21 @@ __device__ __forceinline__ bool load_slab(const MarchParams &P, int sid, float2 
                      "l"(src), "r"(bytes), "r"(smem_addr(bar))
                      : "memory");
     }
+}
+
+__device__ __forceinline__ bool slab_wait(const MarchParams &P, uint64_t *bar, uint32_t *phase, unsigned int *flags) {
     if (!__all_sync(0xffffffffu, slab_bar_wait(bar, *phase, P.slab_polls0))) {
         *flags |= DNSMC_STATUS_COPY_TIMEOUT;
         if (!__all_sync(0xffffffffu, slab_bar_wait(bar, *phase, kSlabWaitPolls))) return false;
     }
     *phase ^= 1u;
     return true;
+}
+
+__device__ __forceinline__ bool load_slab(const MarchParams &P, int sid, float2 *slk, int lane, uint64_t *bar,
+                                          uint32_t *phase, unsigned int *flags) {
+    slab_issue(P, sid, slk, lane, bar);
+    return slab_wait(P, bar, phase, flags);
 }
 
 // Before a warp whose copy did not arrive exits: one more bounded wait for

@@ -12,7 +12,7 @@ int launch_march_gen(int mode, const MarchParams &p, int blocks, int threads, vo
 }
 
 int march_gen_occupancy(int mode, int threads, bool cv, bool mom, size_t smem) {
-    return march_cells_occupancy<true>(mode, threads, cv, mom, smem);
+    return march_cells_occupancy<true>(mode, false, threads, cv, mom, smem);
 }
 
 int upload_sobol_dirs_gen(const uint32_t dirs[4][32]) {

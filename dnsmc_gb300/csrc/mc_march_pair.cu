@@ -11,8 +11,8 @@ int launch_march_pair(int mode, const MarchParams &p, int blocks, int threads, v
     return launch_march_cells<false>(mode, p, blocks, threads, stream, trace, cv, mom);
 }
 
-int march_pair_occupancy(int mode, int threads, bool cv, bool mom, size_t smem) {
-    return march_cells_occupancy<false>(mode, threads, cv, mom, smem);
+int march_pair_occupancy(int mode, bool uni, int threads, bool cv, bool mom, size_t smem) {
+    return march_cells_occupancy<false>(mode, uni, threads, cv, mom, smem);
 }
 
 int upload_sobol_dirs_pair(const uint32_t dirs[4][32]) {

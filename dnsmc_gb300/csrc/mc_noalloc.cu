@@ -11,7 +11,7 @@
 // size that each GPU loading this library holds until the process exits.
 //
 // The kernels are the same persistent march and finalize kernels the handle
-// API launches (launch_march / launch_finalize / launch_pack_T in
+// API launches (launch_march / launch_finalize / launch_pack_T4 in
 // mc_kernels.cu); only the location of their scratch differs.
 #include <cuda_runtime.h>
 
@@ -32,7 +32,11 @@ constexpr long long kMaxCells = DNSMC_NOALLOC_MAX_CELLS;
 constexpr int kMaxFaces = DNSMC_NOALLOC_MAX_IMAX + 1;
 constexpr size_t kTallyOff = 0;                                      // double2 per cell
 constexpr size_t kFieldOff = kTallyOff + (size_t)kMaxCells * 16;     // float per cell
-constexpr size_t kFacesOff = kFieldOff + (size_t)kMaxCells * 4;      // wall-normal faces
+// T^4 with the periodic axes continued by the packet's extent
+// (march_extent): the most values that any allowed grid and packet shape
+// needs (34 x 8 x 963 cells, 8 x 8 packets)
+constexpr long long kMaxPadded = 693360;
+constexpr size_t kFacesOff = kFieldOff + (size_t)kMaxPadded * 4;     // wall-normal faces
 constexpr size_t kMiscOff = kFacesOff + (((size_t)kMaxFaces * 4 + 255) / 256) * 256;
 constexpr size_t kMiscBytes = 256;  // [0] queue, [1] status, [2] group flag (uint32); [2..3] counters (u64)
 constexpr size_t kScratchBytes = kMiscOff + kMiscBytes;
@@ -117,14 +121,15 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     cudaError_t e = cudaMemsetAsync(misc, 0, kMiscBytes, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(faces, xu, (size_t)(c.imax + 1) * sizeof(float), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString(e));
-    int rc = launch_pack_T(dT, field, c.imax, c.jmax, c.kmax, 1, c.imax, (long long)c.imax * c.jmax, 0, st);
-    if (rc) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString((cudaError_t)rc));
-
     // the grey black-wall march runs kLaneCells cells per lane
     // the handle API's automatic packet shape (8 x 8, or 16 x 4 / 32 x 2 for
     // fewer than 8 / 4 cells along k)
     const int ta = c.tile_a ? c.tile_a : (c.kmax >= 8 ? 8 : (c.kmax >= 4 ? 16 : 32));
     const int tb = 32 / ta * kLaneCells;
+    const int pna = march_extent_row(c.jmax, ta), pnb = march_extent(c.kmax, tb);
+    if ((long long)c.imax * pna * pnb > kMaxPadded) return report_error(DNSMC_ERR_ARG, "grid beyond the allocation-free limit");
+    int rc = launch_pack_T4(dT, field, c.imax, c.jmax, c.kmax, pna, pnb, st);
+    if (rc) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString((cudaError_t)rc));
     MarchParams P{};
     P.nw = c.imax; P.na = c.jmax; P.nb = c.kmax;
     P.da = c.Ly / (float)c.jmax; P.db = c.Lz / (float)c.kmax;
@@ -135,7 +140,10 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     P.n_packets = P.npa * P.npb * P.npw;
     P.nfields = 1;
     P.field_stride = ncell;
-    P.fieldT = field;
+    P.fieldG = field;
+    P.pna = pna; P.pnb = pnb;
+    P.pstride = (long long)c.imax * pna * pnb;
+    P.rda = 1.0f / P.da; P.rdb = 1.0f / P.db;
     P.n_groups = 1;
     P.n_tbins = 1;
     P.kappa = c.kappa;
@@ -159,8 +167,8 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     P.tally = tally;
     const int threads = c.block_threads ? c.block_threads : 256;
     // persistent grid: resident blocks at the launch's dynamic shared memory
-    const size_t smem = march_smem(P, threads, kLaneCells);
-    const int blocks = device_sm_count() * march_occupancy_ex(MODE_GREY, threads, false, false, false, smem);
+    const size_t smem = march_pair_smem(P, threads);
+    const int blocks = device_sm_count() * march_occupancy_ex(MODE_GREY, false, threads, false, false, false, smem);
     rc = launch_march(MODE_GREY, P, blocks > 0 ? blocks : 1, threads, st, false);
     if (rc) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString((cudaError_t)rc));
 
