@@ -339,7 +339,8 @@ struct dnsmc_solver {
     double sig_scale = 1.0;
     DevBuf<float> d_Qf, d_sigf;
     PinBuf<float> h_Qf, h_sigf;
-    DevBuf<unsigned int> d_misc;  // [0] queue, [1] status
+    DevBuf<unsigned int> d_misc;  // [0] queue, [1] status, [4 ...] finished units per item (split items)
+    DevBuf<float> d_rayx;         // every ray's contribution (split items), at most kRayxBytes
     DevBuf<unsigned long long> d_counters;
     unsigned long long h_counters[2] = {0, 0};
     unsigned int h_status = 0;
@@ -1033,6 +1034,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     fp.outP = s->d_posT.p; fp.outPX = s->d_posTX.p;
     fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
     fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
+    P.parts = 1;
     TRY(s->d_misc.ensure(4));
     TRY(s->d_counters.ensure(2));
     P.queue = s->d_misc.p;
@@ -1159,6 +1161,17 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     const int occ = mg ? march_mg_occupancy(mode, threads, smem)
                        : march_occupancy_ex(mode, P.uni != 0, threads, cv, mom, gen, smem);
     const int blocks = std::max(1, sms * occ);
+    if (!mg && !gen && !mom && !P.rays_per_packet) {  // few items: their rays in several units
+        P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes);
+        if (P.parts > 1) {
+            TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * 64)));
+            TRY(s->d_misc.ensure((size_t)(4 + P.n_items)));
+            P.rayx = s->d_rayx.p;
+            P.queue = s->d_misc.p;
+            P.status = s->d_misc.p + 1;
+            P.parts_done = s->d_misc.p + 4;
+        }
+    }
 
     FinalizeParams F;
     memset(&F, 0, sizeof F);
@@ -1207,7 +1220,10 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             if (rc == 0) rc = launch_cv_mean(cp, s->stream);
             if (rc) return fail(DNSMC_ERR_CUDA, "control-variate launch: %s", cudaGetErrorString((cudaError_t)rc));
         }
-        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, 4 * sizeof(unsigned int), s->stream));
+        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, (4 + (P.parts > 1 ? (size_t)P.n_items : 0)) * sizeof(unsigned int),
+                                 s->stream));
+        if (P.parts > 1 && P.item_steps)
+            CUDA_TRY(cudaMemsetAsync(P.item_steps, 0, (size_t)P.n_items * sizeof(unsigned long long), s->stream));
         CUDA_TRY(cudaMemsetAsync(s->d_counters.p, 0, 2 * sizeof(unsigned long long), s->stream));
         if (P.item_order) {
             const int rco = launch_item_order(P.rays_per_packet, P.rays_gstride, P.n_packets, P.n_groups, P.n_items,
@@ -1664,7 +1680,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_part.release(); s->d_fieldV.release(); s->d_layerV.release();
     s->d_entries.release(); s->d_group_start.release(); s->d_group_empty.release();
     s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_sig.release(); s->h_sig.release(); s->d_Qg.release(); s->d_varg.release();
-    s->h_Q.release(); s->d_misc.release(); s->d_counters.release();
+    s->h_Q.release(); s->d_misc.release(); s->d_rayx.release(); s->d_counters.release();
     s->d_Qf.release(); s->d_sigf.release(); s->h_Qf.release(); s->h_sigf.release();
     if (s->ev_march0) cudaEventDestroy(s->ev_march0);
     if (s->ev_march1) cudaEventDestroy(s->ev_march1);

@@ -119,8 +119,15 @@ struct MarchParams {
     float Ly, Lz;
     int max_steps;
     // work queue and outputs
-    unsigned int *queue;      // atomic item counter (zeroed per launch)
+    unsigned int *queue;      // atomic counter of queue units (zeroed per launch)
     long long n_items;
+    // few items (march_parts): an item's rays in `parts` queue units, unit u
+    // of item u / parts; every ray's contribution goes to rayx[item][ray][64
+    // cells], and the warp that finishes an item's last unit (parts_done,
+    // zeroed per launch) sums them in ray order
+    int parts;                // 1: an item is one unit and is summed as it goes
+    float *rayx;
+    unsigned int *parts_done; // [item]
     double2 *tally;           // see layout above
     long long region_cells;   // (ew1-ew0)*(ea1-ea0)*(eb1-eb0)
     unsigned int *status;     // DNSMC_STATUS_* bits
@@ -276,6 +283,22 @@ constexpr int kWalkWords = 176;  // words of a warp's walk buffer (mc_march_pair
 constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {
     return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u) + (size_t)threads * 24u * kLaneCells;
+}
+// Queue units per item: an item is one warp's serial work over its rays, so
+// with few items the chip idles; units of at least one ray, about 16 per
+// resident warp.  warps: resident warps of the launch; cap_bytes: the most
+// that the rays' contributions may take.
+// 16 per warp leaves the last wave under a tenth of the launch.  Grey 8 x 32 x 4
+// at 32 rays (32 items): march 79 -> 18 us; grey 64^3 at 256 rays (4096
+// items, 1.7 waves of warps): 4.85 -> 4.36 ms.  From 16 items a warp on, one
+// unit per item: the sums stay in shared memory (128^3 with 8 band groups:
+// 262144 items, unchanged).
+constexpr long long kRayxBytes = 1LL << 30;
+inline int march_parts(long long n_items, int rays, long long warps, long long cap_bytes) {
+    if (n_items < 1 || rays < 2 || n_items >= 16 * warps) return 1;
+    if (n_items * rays > cap_bytes / (64 * (long long)sizeof(float))) return 1;
+    const long long want = (16 * warps + n_items - 1) / n_items;
+    return (int)(want < rays ? want : rays);
 }
 int launch_march_gen(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace, bool cv,
                      bool mom);                                      // mc_march_gen.cu

@@ -453,6 +453,46 @@ __device__ __forceinline__ void tally_ray(const MarchParams &P, float X, int m, 
     }
 }
 
+// Rays [rbeg, rend) of a unit: part `part` of an item of N rays.
+__device__ __forceinline__ void unit_rays(const MarchParams &P, int part, int N, int *rbeg, int *rend) {
+    const int per = (N + P.parts - 1) / P.parts;
+    *rbeg = min(part * per, N);
+    *rend = min(*rbeg + per, N);
+}
+
+// A warp has stored a unit's contributions (rayx): whether it was the item's
+// last unit.  The result is the same in every lane.
+__device__ __forceinline__ bool unit_done(const MarchParams &P, long long item, int lane) {
+    __threadfence();
+    __syncwarp();
+    unsigned int n = 0;
+    if (lane == 0) n = atomicAdd(P.parts_done + item, 1u);
+    n = __shfl_sync(0xffffffffu, n, 0);
+    __threadfence();
+    return n == (unsigned int)P.parts - 1u;
+}
+
+// Sums of one cell of an item over its N rays in ray order (x: the cell's
+// first contribution, 64 values a ray), as tally_ray adds them.
+__device__ __forceinline__ double2 sum_rays(const MarchParams &P, const float *x, int N, int M) {
+    float2 sum = make_float2(0.0f, 0.0f), sq = sum, rep = sum;
+    int m = 0;
+    for (int r0 = 0; r0 < N; r0 += 8) {
+        float v[8];
+        const int n = min(8, N - r0);
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = q < n ? __ldcg(x + (long long)(r0 + q) * 64) : 0.0f;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            if (q < n) {
+                tally_ray(P, v[q], m, M, &sum, &sq, &rep);
+                m = P.sampler && m == M - 1 ? 0 : m + 1;
+            }
+        }
+    }
+    return make_double2(ff_value(sum), ff_value(sq));
+}
+
 // ---------------------------------------------------------------------------
 // The multigrid march (grid_num > 1; the reference's grid switch,
 // code/mc_gpu.cu:193-207), one cell per lane, 32-cell packets: the absorbing

@@ -66,12 +66,18 @@ static_assert(kWalkState + 7 <= kWalkWords && kWalkWords % 4 == 0, "a warp's wal
 // the float after a non-negative float
 __device__ __forceinline__ float next_up(float v) { return __uint_as_float(__float_as_uint(v) + 1u); }
 
-// crossings of a periodic axis before time tau: the n with (n + off) dt < tau
-// (r: an estimate of 1 / dt)
+// crossings of a periodic axis before time tau: the n with (n + off) dt < tau.
+// r is an estimate of 1 / dt: its error (a few 2^-24) moves the count by less
+// than one up to 2^20 crossings, which one comparison each way mends; more
+// crossings are stepped.
 __device__ __forceinline__ float crossings_before(float tau, float r, float dt, float off) {
     float g = fmaxf(floorf(fmaf(tau, r, 1.0f - off)), 0.0f);
-    while (g > 0.0f && !((g - 1.0f + off) * dt < tau)) g -= 1.0f;
-    while ((g + off) * dt < tau) g += 1.0f;
+    if (g >= 1048576.0f) {
+        while ((g - 1.0f + off) * dt >= tau) g -= 1.0f;
+        while ((g + off) * dt < tau) g += 1.0f;
+    }
+    g = (g - 1.0f + off) * dt >= tau ? g - 1.0f : g;
+    g = (g + off) * dt < tau ? g + 1.0f : g;
     return g;
 }
 
@@ -221,8 +227,9 @@ __device__ __forceinline__ const typename FieldT<MODE>::type *field_base(const M
 // UNI: the absorption coefficient is the same everywhere (grey model, grey
 // band tables), so are a step's attenuation and the packet's transmissivity:
 // the warp computes expm1 of a chunk's steps side by side, a cell-step is one
-// gather, one difference and one fused multiply-add.
-template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM>
+// gather, one difference and one fused multiply-add.  SPLIT: items in
+// several queue units (MarchParams::parts).
+template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT>
 __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const MarchParams P) {
     typedef typename FieldT<MODE>::type VT;
     constexpr int C = kLaneCells;  // cells per lane
@@ -260,6 +267,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const 
 
     for (;;) {
         long long item;
+        int part = 0;
         if (TRACE) {
             if (threadIdx.x >= 32) return;
             item = ((long long)P.trace_f * P.n_groups + P.trace_g) * P.n_packets + P.trace_p;
@@ -267,7 +275,11 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const 
             unsigned int it = 0;
             if (lane == 0) it = atomicAdd(P.queue, 1u);
             it = __shfl_sync(FULL, it, 0);
-            if ((long long)it >= P.n_items) break;
+            if ((long long)it >= (SPLIT ? P.n_items * P.parts : P.n_items)) break;
+            if (SPLIT) {
+                part = (int)(it % (unsigned)P.parts);
+                it /= (unsigned)P.parts;
+            }
             item = P.item_order ? (long long)__ldg(P.item_order + it) : (long long)it;
         }
         const int p = (int)(item % P.n_packets);
@@ -325,6 +337,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const 
 #pragma unroll
                 for (int q = 0; q < 9; ++q) mo[k][q] = 0.0;
         const int M = P.sampler ? max(1, N / max(1, P.nbatch)) : 1;
+        if (!SPLIT)
 #pragma unroll
         for (int k = 0; k < C; ++k) {
             *acc(0, k) = make_float2(0.0f, 0.0f); *acc(1, k) = make_float2(0.0f, 0.0f); *acc(2, k) = make_float2(0.0f, 0.0f);
@@ -332,8 +345,10 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const 
         unsigned long long isteps = 0;
         unsigned int lsteps = 0;  // this lane's active cell-steps in the item
         int bcur = -1;
-        const int rbeg = TRACE ? P.trace_r : 0;
-        const int rend = TRACE ? P.trace_r + 1 : ((K > 0) ? N : 0);
+        int rbeg = TRACE ? P.trace_r : 0;
+        int rend = TRACE ? P.trace_r + 1 : ((K > 0) ? N : 0);
+        float *const rayx = SPLIT ? P.rayx + item * N * 64 + lane : nullptr;
+        if (SPLIT) unit_rays(P, part, rend, &rbeg, &rend);
         for (int r = rbeg; r < rend; ++r) {
             int m;
             const uint4 x = ray_words(P, r, M, p, ctr2, &bcur, &s_shift[warp], &m);
@@ -563,13 +578,23 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const 
                 if (active[k]) {
                     ++my_rays;
                     if (!isfinite(X)) flags |= DNSMC_STATUS_NONFINITE;
-                    tally_ray(P, X, m, M, acc(0, k), acc(1, k), acc(2, k));
+                    if (SPLIT) rayx[(long long)r * 64 + 32 * k] = X;
+                    else tally_ray(P, X, m, M, acc(0, k), acc(1, k), acc(2, k));
                 }
             }
         }
         if (dead) break;  // the item's sums are incomplete; the solve fails
         my_steps += lsteps;
         if (TRACE) return;
+        if (SPLIT) {
+            if (P.item_steps && lane == 0) atomicAdd(P.item_steps + item, isteps);
+            if (unit_done(P, item, lane)) {
+#pragma unroll
+                for (int k = 0; k < C; ++k)
+                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays(P, rayx + 32 * k, K > 0 ? N : 0, M);
+            }
+            continue;
+        }
         if (P.item_steps && lane == 0) P.item_steps[item] = isteps;
 #pragma unroll
         for (int k = 0; k < C; ++k) {
@@ -1079,10 +1104,10 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
 // The two-cell march of a medium: the absorbing gas (march_pair_kernel; UNI:
 // of the same absorption coefficient everywhere) or the general medium
 // (march_gen_kernel).
-template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool GEN> struct march_cells_kernel {
-    static constexpr void (*fn)(const MarchParams) = march_pair_kernel<MODE, UNI, TRACE, CV, MOM>;
+template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT, bool GEN> struct march_cells_kernel {
+    static constexpr void (*fn)(const MarchParams) = march_pair_kernel<MODE, UNI, TRACE, CV, MOM, SPLIT>;
 };
-template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM> struct march_cells_kernel<MODE, UNI, TRACE, CV, MOM, true> {
+template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT> struct march_cells_kernel<MODE, UNI, TRACE, CV, MOM, SPLIT, true> {
     static constexpr void (*fn)(const MarchParams) = march_gen_kernel<MODE, TRACE, CV, MOM>;
 };
 
@@ -1092,12 +1117,15 @@ int launch_march_cells(int mode, const MarchParams &p, int blocks, int threads, 
     cudaStream_t st = (cudaStream_t)stream;
     if (trace) { blocks = 1; threads = 32; mom = false; }
     const size_t smem = GEN ? march_smem(p, threads, kLaneCells) : march_pair_smem(p, threads);
-#define DNSMC_L(M, U, T, CV_, O) \
-    return march_launch_one(march_cells_kernel<M, U, T, CV_, O, GEN>::fn, blocks, threads, smem, st, p)
-#define DNSMC_MODE(M, U)                                                                               \
-    if (trace) { if (cv) DNSMC_L(M, U, true, true, false); else DNSMC_L(M, U, true, false, false); }   \
-    else if (cv) { if (mom) DNSMC_L(M, U, false, true, true); else DNSMC_L(M, U, false, true, false); } \
-    else DNSMC_L(M, U, false, false, false);
+#define DNSMC_L(M, U, T, CV_, O, S) \
+    return march_launch_one(march_cells_kernel<M, U, T, CV_, O, S, GEN>::fn, blocks, threads, smem, st, p)
+#define DNSMC_MODE(M, U)                                                                                \
+    if (trace) { if (cv) DNSMC_L(M, U, true, true, false, false); else DNSMC_L(M, U, true, false, false, false); } \
+    else if (cv && mom) DNSMC_L(M, U, false, true, true, false);                                        \
+    else if (!GEN && p.parts > 1) {                                                                     \
+        if (cv) DNSMC_L(M, U, false, true, false, !GEN); else DNSMC_L(M, U, false, false, false, !GEN); \
+    } else if (cv) DNSMC_L(M, U, false, true, false, false);                                            \
+    else DNSMC_L(M, U, false, false, false, false);
     switch (mode) {
         case MODE_GREY: DNSMC_MODE(MODE_GREY, !GEN) break;
         case MODE_T:
@@ -1117,9 +1145,9 @@ template <bool GEN>
 int march_cells_occupancy(int mode, bool uni, int threads, bool cv, bool mom, size_t smem) {
     int nb = 0;
 #define DNSMC_O(M, U)                                                                                     \
-    nb = cv ? (mom ? march_occupancy_one(march_cells_kernel<M, U, false, true, true, GEN>::fn, threads, smem)     \
-                   : march_occupancy_one(march_cells_kernel<M, U, false, true, false, GEN>::fn, threads, smem))   \
-            : march_occupancy_one(march_cells_kernel<M, U, false, false, false, GEN>::fn, threads, smem)
+    nb = cv ? (mom ? march_occupancy_one(march_cells_kernel<M, U, false, true, true, false, GEN>::fn, threads, smem)     \
+                   : march_occupancy_one(march_cells_kernel<M, U, false, true, false, false, GEN>::fn, threads, smem))   \
+            : march_occupancy_one(march_cells_kernel<M, U, false, false, false, false, GEN>::fn, threads, smem)
     if (mode == MODE_GREY) DNSMC_O(MODE_GREY, !GEN);
     if (mode == MODE_T) {
         if (!GEN && uni) DNSMC_O(MODE_T, !GEN);

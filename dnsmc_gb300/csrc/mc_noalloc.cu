@@ -164,6 +164,7 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     P.counters = counters;
     P.region_cells = ncell;
     P.n_items = P.n_packets;
+    P.parts = 1;  // splitting items would need more scratch
     P.tally = tally;
     const int threads = c.block_threads ? c.block_threads : 256;
     // persistent grid: resident blocks at the launch's dynamic shared memory

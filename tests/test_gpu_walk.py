@@ -89,3 +89,28 @@ def test_traces_of_several_chunks_match_the_replay():
             longest = max(longest, n)
         assert longest > 64
     s.close()
+
+
+@pytest.mark.parametrize("size,groups,rays,sampler", [
+    ((5, 9, 8), 1, 37, D.SAMPLER_IID),       # a unit per ray
+    ((40, 24, 24), 2, 50, D.SAMPLER_RQMC),   # 720 items: uneven units
+    ((64, 64, 40), 1, 26, D.SAMPLER_RQMC),   # 2560 items: units of several rays
+    ((96, 72, 64), 8, 2, D.SAMPLER_RQMC),    # 55296 items: a unit per item
+])
+def test_split_items_match_the_replay(size, groups, rays, sampler):
+    """Items of few-item solves are split over queue units by rays: the sums
+    are the replay's bit for bit."""
+    ni, nj, nk = size
+    t = synth.ck_table(nbands=8, nq=4, nT=24, nX=4, seed=9)
+    s = D.Solver(D.default_config(model=D.MODEL_TABLE, imax=ni, jmax=nj, kmax=nk, Lx=1.0, Ly=2.0, Lz=2.0, stretched_x=0,
+                                  T_west=500.0, T_east=600.0, seed=5, sampler=sampler, nvar=2, n_groups=groups,
+                                  local_sampling=1))
+    s.set_table(t["k"] * 0.05, t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"], X0=t["X0"], dX=t["dX"])
+    T = smooth_field(ni, nj, nk, 600, 1500, 3)
+    x = np.full(T.shape, 0.1, np.float32)
+    s.set_fields(T, x)
+    s.set_rays(rays)
+    assert_bitexact(s, T, x)
+    c = s.counters()
+    assert c.rays == ni * nj * nk * groups * rays
+    s.close()
