@@ -224,13 +224,23 @@ __device__ __forceinline__ const typename FieldT<MODE>::type *field_base(const M
     else return P.fieldG;
 }
 
+// Resident 256-thread blocks per SM.  Tables: 2 (128 registers: the values of
+// four steps of two cells; 3 spill, 66.2 -> 70.1 ms on the 128^3 channel).
+// UNI: 3 (grey) and 4 (band tables): its steps are short, so the walk's
+// generation and the gathers need more warps to hide behind -- grey 64^3
+// 4.32 (2) / 3.51 (3) / 3.62 ms (4), grey bands through the drop-in pair 9.43 /
+// 9.12 / 8.65 ms.  Moments (18 FP64 sums a lane): 2.
+__host__ __device__ constexpr int pair_min_blocks(int mode, bool uni, bool mom) {
+    return uni && !mom ? (mode == MODE_GREY ? 3 : 4) : DNSMC_PAIR_MINB;
+}
+
 // UNI: the absorption coefficient is the same everywhere (grey model, grey
 // band tables), so are a step's attenuation and the packet's transmissivity:
 // the warp computes expm1 of a chunk's steps side by side, a cell-step is one
 // gather, one difference and one fused multiply-add.  SPLIT: items in
 // several queue units (MarchParams::parts).
 template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT>
-__global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_pair_kernel(const MarchParams P) {
+__global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pair_kernel(const MarchParams P) {
     typedef typename FieldT<MODE>::type VT;
     constexpr int C = kLaneCells;  // cells per lane
     static_assert(C == 2, "the attenuation goes through a cell pair");
