@@ -1050,7 +1050,10 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         const size_t stat = pair ? kPairStaticSmem : 1024;  // the march kernels' static shared memory, at most
         auto need = [&](int th) { return (pair ? march_pair_smem(P, th) : march_smem(P, th, kLaneCells)) + stat; };
         if (need(threads) > (size_t)smax) threads = 128;
-        if (need(threads) > (size_t)smax)
+        // the largest slab is what four warps of the general march hold; the
+        // gas march, which keeps more beside it, then takes fewer warps
+        while (pair && threads > 32 && need(threads) > (size_t)smax) threads /= 2;
+        if (march_smem(P, 128, kLaneCells) + 1024 > (size_t)smax)
             return fail(DNSMC_ERR_TABLE, "a spectral sample's table slab (%d bytes) exceeds the shared memory of the march",
                         P.slab_len * 8);
     }

@@ -277,12 +277,13 @@ int march_mg_occupancy(int mode, int threads, size_t smem);
 inline size_t march_smem(const MarchParams &p, int threads, int cells) {
     return (size_t)((threads + 31) / 32) * (size_t)p.slab_len * 8u + (size_t)threads * (24u * (size_t)cells + 16u);
 }
-// of a launch of the gas march: each warp's slab and walk buffer, then per
+// of a launch of the gas march: each warp's slab, walk buffer and ray batch, then per
 // thread the sums of its two cells; kPairStaticSmem at most beside it
 constexpr int kWalkWords = 176;  // words of a warp's walk buffer (mc_march_pair.cuh)
+constexpr size_t kBatchBytes = 1536;  // a warp's ray batch
 constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {
-    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u) + (size_t)threads * 24u * kLaneCells;
+    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u + kBatchBytes) + (size_t)threads * 24u * kLaneCells;
 }
 // Queue units per item: an item is one warp's serial work over its rays, so
 // with few items the chip idles; units of at least one ray, about 16 per
