@@ -309,15 +309,12 @@ struct dnsmc_solver {
     std::vector<double> Ccoef;               // [band*nq+g] target coefficients
     std::vector<int> cv_grp, cv_sid;
     std::vector<double> cv_C;
-    std::vector<float> cv_Cf;
     DevBuf<int> d_cv_grp, d_cv_sid;
     DevBuf<double> d_cv_C;
     DevBuf<float2> d_layer, d_sur;
     DevBuf<double2> d_Jhat, d_muY;
     DevBuf<double> d_cvnodes;                // node sums of E[Y] (float pairs, 8 bytes each)
-    DevBuf<float4> d_Jf;
     DevBuf<float4> d_surtab;                 // tabulated surrogate [f][sample][nw][2][kSurBins]
-    DevBuf<float> d_cv_Cf;
     DevBuf<float2> d_beta;
     DevBuf<double> d_moments;
     bool beta_set = false;
@@ -1097,7 +1094,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         TRY(s->d_sur.ensure(nsur));
         TRY(s->d_surtab.ensure(nsur * 2 * kSurBins));
         TRY(s->d_Jhat.ensure(nsur));
-        TRY(s->d_Jf.ensure(nsur));
         TRY(s->d_muY.ensure((size_t)s->nfields * P.n_groups * P.region_cells));
         if (mode != MODE_GREY && !s->cv_uploaded) {
             TRY(s->d_cv_grp.ensure(s->cv_grp.size()));
@@ -1106,9 +1102,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             CUDA_TRY(cudaMemcpyAsync(s->d_cv_grp.p, s->cv_grp.data(), s->cv_grp.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
             CUDA_TRY(cudaMemcpyAsync(s->d_cv_sid.p, s->cv_sid.data(), s->cv_sid.size() * sizeof(int), cudaMemcpyHostToDevice, s->stream));
             CUDA_TRY(cudaMemcpyAsync(s->d_cv_C.p, s->cv_C.data(), s->cv_C.size() * sizeof(double), cudaMemcpyHostToDevice, s->stream));
-            s->cv_Cf.assign(s->cv_C.begin(), s->cv_C.end());
-            TRY(s->d_cv_Cf.ensure(std::max<size_t>(1, s->cv_Cf.size())));
-            CUDA_TRY(cudaMemcpyAsync(s->d_cv_Cf.p, s->cv_Cf.data(), s->cv_Cf.size() * sizeof(float), cudaMemcpyHostToDevice, s->stream));
             s->cv_uploaded = true;
         }
         cp.nfields = s->nfields; cp.nw = c.imax; cp.na = c.jmax; cp.nb = c.kmax;
@@ -1123,8 +1116,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         cp.n_samples = S; cp.sur = s->d_sur.p; cp.fw = s->d_fw.p; cp.toll = c.toll; cp.dtoll = P.dtoll;
         cp.surtab = s->d_surtab.p;
         cp.Jhat = s->d_Jhat.p;
-        cp.Jf = s->d_Jf.p;
-        cp.samp_Cf = s->d_cv_Cf.p;
         cp.n_groups = P.n_groups;
         cp.grp_start = s->d_cv_grp.p; cp.samp_id = s->d_cv_sid.p; cp.samp_C = s->d_cv_C.p;
         cp.Wgrey = 4.0 * c.kappa * kSigma;
@@ -1137,8 +1128,8 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             cp.part = s->d_part.p;
             cp.layerV = s->d_layerV.p;
         }
-        // E[Y] from node sums for tables without particles
-        if (mode != MODE_GREY && !have_part) {
+        // E[Y] from node sums for tables
+        if (mode != MODE_GREY) {
             TRY(s->d_cvnodes.ensure((size_t)cv_node_count(cp)));
             cp.nodes = s->d_cvnodes.p;
         }
@@ -1675,7 +1666,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_fw.release(); s->d_k.release(); s->d_ib.release(); s->d_ibw.release();
     s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posTX.release();
     s->d_cv_grp.release(); s->d_cv_sid.release(); s->d_cv_C.release(); s->d_layer.release();
-    s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_Jf.release(); s->d_cv_Cf.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
+    s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();
     s->d_stat_part.release(); s->d_stat_out.release(); s->d_rays_pp.release(); s->d_rays_rcp.release(); s->d_item_steps.release(); s->d_kP.release();
     s->d_order.release(); s->d_order_hist.release();

@@ -373,13 +373,11 @@ struct CvParams {
     float4 *surtab;
     double2 *Jhat;            // [f][sample][nw] (Jhat, Ahat): exact means of J and A over the
                               // isotropic directions (mu uniform on [-1, 1])
-    float4 *Jf;               // [f][sample][nw] (Jhat hi, Jhat lo, Ahat, layer-mean Ib) for the mean
     // mean of Y per (field, group, cell) in tally layout
     int n_groups;
     const int *grp_start;     // n_groups+1 into samp_id / samp_C
     const int *samp_id;
     const double *samp_C;
-    const float *samp_Cf;     // samp_C rounded to float
     double Wgrey;
     int ew0, ew1, ea0, ea1, eb0, eb1;
     long long region_cells;
@@ -389,8 +387,8 @@ struct CvParams {
     const float *fieldV;      // [f][i][k][j] volume fraction, or null
     const float2 *part;       // [band] (absorption, scattering) per unit volume fraction
     float *layerV;            // [f][nw] layer-mean volume fraction
-    // node sums of E[Y] (tables without particles): per (field, group,
-    // region layer) and table cell the sums over the group's samples, as
+    // node sums of E[Y] (tables): per (field, group, region layer) and table
+    // cell the sums over the group's samples, as
     // float pairs (hi, lo) of 8 bytes each; cv_node_count() of them
     double *nodes;
 };

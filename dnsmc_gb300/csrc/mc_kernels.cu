@@ -520,34 +520,15 @@ __global__ void __launch_bounds__(kTableThreads) cv_table_kernel(const CvParams 
     for (int l = t; l < nw; l += kTableThreads) {
         const double2 a = s_mean[2 * l], b = s_mean[2 * l + 1];
         const double J = (a.x + b.x) * sc, A = (a.y + b.y) * sc;
-        const float Jhi = (float)J;
         const long long idx = fs * nw + l;
         c.Jhat[idx] = make_double2(J, A);
-        c.Jf[idx] = make_float4(Jhi, (float)(J - (double)Jhi), (float)A, s_sur[l].y);
     }
 }
 
-// Compensated FP32 accumulation (Kahan): sum - comp carries the exact sum to
-// about 2^-44 relative; the file is compiled without FMA contraction, so the
-// compensation is not folded away.
-struct KahanF {
-    float s = 0.0f, comp = 0.0f;
-    __device__ __forceinline__ void add(float v) {
-        const float y = v - comp;
-        const float t = s + y;
-        comp = (t - s) - y;
-        s = t;
-    }
-    __device__ __forceinline__ double value() const { return (double)s - (double)comp; }
-};
-
-// E[Y] per (field, group, cell of the region), tally layout [f][g][i][k][j]:
-//   E[Y_a] = sum_s C_s k_s(T_i, x_i) (Ib_s(T_i) - Jhat_s(layer)),
-//   E[Y_b] = sum_s C_s k_s(T_i, x_i) (Ib_s(T_i) - Ibar_s(layer)) Ahat_s(layer),
-// over the group's spectral samples, in FP32 with compensated sums (the
-// device's FP64 rate is a small fraction of its FP32 rate); Jhat enters as a
-// double-float pair so Ib - Jhat keeps its digits where they cancel.
-__global__ void cv_mean_kernel(const CvParams c) {
+// E[Y] of the grey model per (field, cell of the region), tally layout:
+//   E[Y_a] = W (T^4 - Jhat(layer)),  E[Y_b] = W (T^4 - Ibar(layer)) Ahat(layer),
+// W the march's weight 4 sigma (kappa + fv a).
+__global__ void cv_mean_grey_kernel(const CvParams c) {
     const int njR = c.ea1 - c.ea0, nkR = c.eb1 - c.eb0;
     const long long n = (long long)c.nfields * c.region_cells;
     const long long plane = (long long)c.na * c.nb;
@@ -558,61 +539,20 @@ __global__ void cv_mean_kernel(const CvParams c) {
         const int jR = (int)(tc % njR);
         const long long r = tc / njR;
         const int kR = (int)(r % nkR);
-        const int iR = (int)(r / nkR);
-        const int w = c.ew0 + iR;
-        const long long cell = (long long)f * c.nw * plane + (long long)w * plane + (long long)(c.eb0 + kR) * c.na + (c.ea0 + jR);
-        float T, x = 0.f;
-        if (c.mode == MODE_TX) { const float2 v = c.fieldTX[cell]; T = v.x; x = v.y; }
-        else T = c.fieldT[cell];
+        const int w = c.ew0 + (int)(r / nkR);
+        const long long cell = ((long long)f * c.nw + w) * plane + (long long)(c.eb0 + kR) * c.na + (c.ea0 + jR);
+        const float T = c.fieldT[cell], t2 = T * T;
         const long long sbase = (long long)f * c.n_samples * c.nw + w;
-        const float fv = c.fieldV ? c.fieldV[cell] : 0.0f;
-        if (c.mode == MODE_GREY) {
-            const float t2 = T * T;
-            const double2 jh = c.Jhat[sbase];
-            // the march's own FP32 weight 4 sigma (kappa + fv a) when particles are present
-            const double Wk = c.part ? (double)((float)(4.0 * 5.670373e-08) * fmaf(fv, c.part[0].x, c.kappa)) : c.Wgrey;
-            const double acc = Wk * ((double)(t2 * t2) - jh.x);
-            const double accB = Wk * ((double)(t2 * t2) - (double)c.sur[sbase].y) * jh.y;
-            c.muY[(long long)f * c.n_groups * c.region_cells + tc] = make_double2(acc, accB);
-            continue;
-        }
-        int ti, xi = 0;
-        float ft, fx = 0.f;
-        grid_pos(T, c.T0, c.invdT, c.nT, &ti, &ft);
-        if (c.mode == MODE_TX) grid_pos(x, c.X0, c.invdX, c.nX, &xi, &fx);
-        for (int g = 0; g < c.n_groups; ++g) {
-            KahanF sa, sb;
-            for (int q = c.grp_start[g]; q < c.grp_start[g + 1]; ++q) {
-                const int sid = c.samp_id[q];
-                float k;
-                if (c.mode == MODE_TX) {
-                    const float *s = c.ktab + (long long)sid * c.nT * c.nX + ti * c.nX + xi;
-                    const float k00 = __ldg(s), k01 = __ldg(s + 1);
-                    const float k10 = __ldg(s + c.nX), k11 = __ldg(s + c.nX + 1);
-                    const float k0 = fmaf(fx, k01 - k00, k00);
-                    const float k1 = fmaf(fx, k11 - k10, k10);
-                    k = fmaf(ft, k1 - k0, k0);
-                } else {
-                    const float *s = c.ktab + (long long)sid * c.nT + ti;
-                    const float k0 = __ldg(s), k1 = __ldg(s + 1);
-                    k = fmaf(ft, k1 - k0, k0);
-                }
-                if (c.part) k = fmaf(fv, __ldg(&c.part[sid / c.nq].x), k);
-                const float *ib = c.ibtab + (sid / c.nq) * c.nT + ti;
-                const float i0 = __ldg(ib), i1 = __ldg(ib + 1);
-                const float Ib = fmaf(ft, i1 - i0, i0);
-                const float4 J = __ldg(c.Jf + sbase + (long long)sid * c.nw);
-                const float ck = __ldg(c.samp_Cf + q) * k;
-                sa.add(ck * ((Ib - J.x) - J.y));
-                sb.add(ck * (Ib - J.w) * J.z);
-            }
-            c.muY[((long long)f * c.n_groups + g) * c.region_cells + tc] = make_double2(sa.value(), sb.value());
-        }
+        const double2 jh = c.Jhat[sbase];
+        // the march's own FP32 weight when particles are present
+        const double Wk = c.part ? (double)((float)(4.0 * 5.670373e-08) * fmaf(c.fieldV[cell], c.part[0].x, c.kappa)) : c.Wgrey;
+        c.muY[(long long)f * c.n_groups * c.region_cells + tc] =
+            make_double2(Wk * ((double)(t2 * t2) - jh.x), Wk * ((double)(t2 * t2) - (double)c.sur[sbase].y) * jh.y);
     }
 }
 
 // ---------------------------------------------------------------------------
-// E[Y] through node sums (tables without particles).  With k_s(T, x) the
+// E[Y] through node sums (tables).  With k_s(T, x) the
 // bilinear and Ib_s(T) the linear interpolant of the tables at the cell's
 // table coordinates (weights wt_a in T, wx_b in x; sum_a' wt_a' = 1),
 //   E[Y_a] = sum_s C_s k_s (Ib_s - Jhat_s(w))
@@ -624,19 +564,27 @@ __global__ void cv_mean_kernel(const CvParams c) {
 //   Db[t][x][a][a'] = sum_s C_s Ahat_s k_s[t+a][x] (Ib_s[t+a'] - Ibar_s):
 // a cell needs 16 node sums per group instead of a pass over the group's
 // samples, and the differences Ib - Jhat, where optically thick samples
-// cancel, are formed per sample before any sum.  Arithmetic in float pairs
+// cancel, are formed per sample before any sum.  Particles add fv a_s to k_s:
+// four more sums per table temperature, with a_s for the k of the node,
+//   Pa[t][a'] = sum_s C_s a_s (Ib_s[t+a'] - Jhat_s),  Pb alike,
+// of which a cell takes fv sum_a' wt_a' P[t][a'] (96^3 cells, 8 groups of 128
+// samples: 4.19 ms a pass over the samples, 0.63 ms both kernels of the sums).  Arithmetic in float pairs
 // (hi + lo, about 48 bits: error-free products by fma and error-free sums;
 // this file is compiled without FMA contraction), at FP32 rates -- this
 // GPU's FP64 rate is a small fraction of them.  The cell's weights are
 // formed in FP64 and its 16-term combination summed in pairs.
 // ---------------------------------------------------------------------------
 struct NodeLayout {
-    int nTc, per;  // table cells (t, x), pairs per (field, group, layer): Da then Db, 4 each per cell
+    // table cells (t, x), work units (one per cell, with particles one more
+    // per temperature), pairs per (field, group, layer): Da then Db, 4 each
+    // per cell, then (Pa, Pb), 2 each per temperature
+    int nTc, units, per;
 };
 __host__ __device__ inline NodeLayout node_layout(const CvParams &c) {
     NodeLayout L;
     L.nTc = (c.nT - 1) * c.nX;
-    L.per = L.nTc * 8;
+    L.units = L.nTc + (c.part ? c.nT - 1 : 0);
+    L.per = L.nTc * 8 + (L.units - L.nTc) * 4;
     return L;
 }
 
@@ -672,7 +620,7 @@ __global__ void __launch_bounds__(256) cv_nodes_kernel(const CvParams c) {
     __shared__ int s_ib[256];      // band * nT
     __shared__ int s_koff[256];    // sample * nT * nX
     __shared__ float2 s_C[256], s_CA[256], s_J[256];  // C, C Ahat, Jhat as pairs
-    __shared__ float s_Ibar[256];
+    __shared__ float s_Ibar[256], s_part[256];
     const NodeLayout L = node_layout(c);
     const int niR = c.ew1 - c.ew0;
     const long long b = blockIdx.x;
@@ -683,9 +631,10 @@ __global__ void __launch_bounds__(256) cv_nodes_kernel(const CvParams c) {
     const int w = c.ew0 + wR;
     float2 *out = reinterpret_cast<float2 *>(c.nodes) + b * L.per;
     const int q0 = c.grp_start[g], q1 = c.grp_start[g + 1];
-    for (int u0 = 0; u0 < L.nTc; u0 += blockDim.x) {
+    for (int u0 = 0; u0 < L.units; u0 += blockDim.x) {
         const int u = u0 + threadIdx.x;
-        const int t = u / c.nX, x = u - t * c.nX;
+        const bool particles = u >= L.nTc;
+        const int t = particles ? u - L.nTc : u / c.nX, x = particles ? 0 : u - t * c.nX;
         float2 acc[8];
 #pragma unroll
         for (int r = 0; r < 8; ++r) acc[r] = make_float2(0.0f, 0.0f);
@@ -704,13 +653,14 @@ __global__ void __launch_bounds__(256) cv_nodes_kernel(const CvParams c) {
                 s_CA[threadIdx.x] = ff_of(C * jh.y);
                 s_J[threadIdx.x] = ff_of(jh.x);
                 s_Ibar[threadIdx.x] = c.sur[o].y;
+                s_part[threadIdx.x] = c.part ? c.part[sid / c.nq].x : 0.0f;
             }
             __syncthreads();
-            if (u >= L.nTc) continue;
+            if (u >= L.units) continue;
             for (int j = 0; j < nq; ++j) {
                 const float *kk = c.ktab + s_koff[j] + t * c.nX + x;
                 const float *ib = c.ibtab + s_ib[j] + t;
-                const float k0 = __ldg(kk), k1 = __ldg(kk + c.nX);
+                const float k0 = particles ? s_part[j] : __ldg(kk), k1 = __ldg(kk + c.nX);
                 const float i0 = __ldg(ib), i1 = __ldg(ib + 1);
                 const float2 J = s_J[j];
                 const float Ibar = s_Ibar[j];
@@ -734,6 +684,9 @@ __global__ void __launch_bounds__(256) cv_nodes_kernel(const CvParams c) {
                 out[(long long)u * 4 + r] = acc[r];
                 out[(long long)L.nTc * 4 + (long long)u * 4 + r] = acc[4 + r];
             }
+        } else if (particles && u < L.units) {
+            float2 *o = out + (long long)L.nTc * 8 + (long long)t * 4;
+            o[0] = acc[0]; o[1] = acc[1]; o[2] = acc[4]; o[3] = acc[5];
         }
     }
 }
@@ -772,6 +725,12 @@ __global__ void cv_mean_nodes_kernel(const CvParams c) {
         for (int bx = 0; bx < nb; ++bx)
             for (int a = 0; a < 2; ++a)
                 for (int a2 = 0; a2 < 2; ++a2) w4[bx][a * 2 + a2] = ff_of(wx[bx] * wt[a] * wt[a2]);
+        float2 wp[2];
+        if (c.part) {
+            const double fv = c.fieldV[cell];
+            wp[0] = ff_of(fv * wt[0]);
+            wp[1] = ff_of(fv * wt[1]);
+        }
         for (int g = 0; g < c.n_groups; ++g) {
             const float2 *lay = reinterpret_cast<const float2 *>(c.nodes) +
                                 (((long long)f * c.n_groups + g) * niR + iR) * L.per;
@@ -782,6 +741,14 @@ __global__ void cv_mean_nodes_kernel(const CvParams c) {
                 for (int q = 0; q < 4; ++q) {
                     ea = ff_add(ea, ff_mulff(w4[bx][q], __ldg(lay + o + q)));
                     eb = ff_add(eb, ff_mulff(w4[bx][q], __ldg(lay + (long long)L.nTc * 4 + o + q)));
+                }
+            }
+            if (c.part) {
+                const float2 *o = lay + (long long)L.nTc * 8 + (long long)ti * 4;
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    ea = ff_add(ea, ff_mulff(wp[q], __ldg(o + q)));
+                    eb = ff_add(eb, ff_mulff(wp[q], __ldg(o + 2 + q)));
                 }
             }
             c.muY[((long long)f * c.n_groups + g) * c.region_cells + tc] =
@@ -937,7 +904,7 @@ int cv_table_allow_smem() {
 int launch_cv_mean(const CvParams &c, void *stream) {
     const long long n = (long long)c.nfields * c.region_cells;
     cudaStream_t st = (cudaStream_t)stream;
-    if (c.nodes) {  // tables without particles: node sums, then the cells
+    if (c.nodes) {  // tables: node sums, then the cells
         const long long blocks = (long long)c.nfields * c.n_groups * (c.ew1 - c.ew0);
         dnsmc::note_launch();
         cv_nodes_kernel<<<(unsigned)blocks, 256, 0, st>>>(c);
@@ -945,7 +912,7 @@ int launch_cv_mean(const CvParams &c, void *stream) {
         cv_mean_nodes_kernel<<<grid_for(n, 256), 256, 0, st>>>(c);
     } else {
         dnsmc::note_launch();
-        cv_mean_kernel<<<grid_for(n, 256), 256, 0, st>>>(c);
+        cv_mean_grey_kernel<<<grid_for(n, 256), 256, 0, st>>>(c);
     }
     return (int)cudaGetLastError();
 }
