@@ -250,8 +250,8 @@ struct dnsmc_solver {
     DevBuf<int2> d_posT;   // per cell (ti, ft) for T-only tables
     DevBuf<int4> d_posTX;  // per cell (ti*(nX-1)+xi, ft, fx, ti)
     DevBuf<float> d_posG;  // per cell T^4 (grey model)
+    DevBuf<float2> d_posVG;  // general medium: (T^4, fv); tables use d_posTX
     int posG_na = 0, posG_nb = 0;  // the padded extents d_posG was written for (0: not written)
-    int last_pna = 0, last_pnb = 0;  // those of the last solve's d_posT / d_posTX
     bool tables_dirty = true;
 
     // fields
@@ -967,7 +967,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     if (have_part && s->fv_fields != s->nfields)
         return fail(DNSMC_ERR_STATE, "particles set: set the particle field of the %d resident snapshots", s->nfields);
     const bool gen = have_part || c.eps_west < 1.0f || c.eps_east < 1.0f;
-    P.fieldV = have_part ? s->d_fieldV.p : nullptr;
     P.part = have_part ? s->d_part.p : nullptr;
     P.fv_max = have_part ? s->fv_max : 0.0f;
     P.hg_g = s->hg_g;
@@ -1016,19 +1015,28 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
                          P.n_groups);
         P.rays_gstride = P.n_packets;
     }
-    padded_extents(s, !mg && !gen, &P.pna, &P.pnb);
+    padded_extents(s, !mg, &P.pna, &P.pnb);
     P.pstride = (long long)c.imax * P.pna * P.pnb;
     const long long npos = (long long)s->nfields * P.pstride;
-    if (mode == MODE_TX) TRY(s->d_posTX.ensure((size_t)npos));
-    if (mode == MODE_T) TRY(s->d_posT.ensure((size_t)npos));
+    if (mode == MODE_TX || (mode == MODE_T && gen)) TRY(s->d_posTX.ensure((size_t)npos));
+    if (mode == MODE_T && !gen) TRY(s->d_posT.ensure((size_t)npos));
+    if (mode == MODE_GREY && gen) TRY(s->d_posVG.ensure((size_t)npos));
     if (mode == MODE_GREY && !mg && !gen) TRY(grey_positions(s));
     P.fieldP = s->d_posT.p;
     P.fieldPX = s->d_posTX.p;
     P.fieldG = s->d_posG.p;
+    P.fieldVX = s->d_posTX.p;
+    P.fieldVG = s->d_posVG.p;
     FieldPos fp{};  // table coordinates of the field for this table (once per solve)
     fp.fT = mode == MODE_TX ? nullptr : s->d_fieldT.p;
     fp.fTX = mode == MODE_TX ? s->d_fieldTX.p : nullptr;
-    fp.outP = s->d_posT.p; fp.outPX = s->d_posTX.p;
+    if (gen) {
+        fp.fV = have_part ? s->d_fieldV.p : nullptr;
+        if (mode == MODE_GREY) fp.outVG = s->d_posVG.p;
+        else fp.outVX = s->d_posTX.p;
+    } else {
+        fp.outP = s->d_posT.p; fp.outPX = s->d_posTX.p;
+    }
     fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
     fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
     P.parts = 1;
@@ -1043,12 +1051,13 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         int smax = 0;
         if (cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device) != cudaSuccess)
             smax = 48 * 1024;
-        const bool pair = !mg && !gen;
+        const bool pair = !mg;
         const size_t stat = pair ? kPairStaticSmem : 1024;  // the march kernels' static shared memory, at most
         auto need = [&](int th) { return (pair ? march_pair_smem(P, th) : march_smem(P, th, kLaneCells)) + stat; };
         if (need(threads) > (size_t)smax) threads = 128;
-        // the largest slab is what four warps of the general march hold; the
-        // gas march, which keeps more beside it, then takes fewer warps
+        // the largest slab is what four warps hold with 64 bytes a thread
+        // beside it; the marches on the fine grid, which keep more, then
+        // take fewer warps
         while (pair && threads > 32 && need(threads) > (size_t)smax) threads /= 2;
         if (march_smem(P, 128, kLaneCells) + 1024 > (size_t)smax)
             return fail(DNSMC_ERR_TABLE, "a spectral sample's table slab (%d bytes) exceeds the shared memory of the march",
@@ -1071,12 +1080,9 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.trace_f = tf; P.trace_g = tg; P.trace_p = tp; P.trace_r = tr; P.trace_max = tmax_steps;
         P.trace_rec = d_trace_rec; P.trace_n = d_trace_n; P.trace_rng = d_trace_rng;
         P.tally = nullptr;
-        if (mode != MODE_GREY && (P.pna != s->last_pna || P.pnb != s->last_pnb || P.nfields != s->last.nfields)) {
-            // the coordinates of the last solve are not for this packet shape
+        if (mode != MODE_GREY || gen) {  // for the present packet shape
             const int rcp = launch_field_pos(fp, s->stream);
             if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
-            s->last_pna = P.pna;
-            s->last_pnb = P.pnb;
         }
         const int rc = mg ? launch_march_mg(mode, P, 1, 32, s->stream, true)
                           : launch_march_ex(mode, P, 1, 32, s->stream, true, cv, false, gen);
@@ -1151,11 +1157,11 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.item_order = s->d_order.p;
     }
     const int sms = device_sm_count();
-    const size_t smem = mg ? march_smem(P, threads, 1) : (gen ? march_smem(P, threads, kLaneCells) : march_pair_smem(P, threads));
+    const size_t smem = mg ? march_smem(P, threads, 1) : march_pair_smem(P, threads);
     const int occ = mg ? march_mg_occupancy(mode, threads, smem)
                        : march_occupancy_ex(mode, P.uni != 0, threads, cv, mom, gen, smem);
     const int blocks = std::max(1, sms * occ);
-    if (!mg && !gen && !mom && !P.rays_per_packet) {  // few items: their rays in several units
+    if (!mg && !mom && !P.rays_per_packet) {  // few items: their rays in several units
         P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes);
         if (P.parts > 1) {
             TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * 64)));
@@ -1205,7 +1211,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
 
     // ---- the kernel sequence of a solve (stream-ordered; capturable) -------
     auto kernels = [&](bool events) -> int {
-        if (mode != MODE_GREY) {
+        if (mode != MODE_GREY || gen) {
             const int rcp = launch_field_pos(fp, s->stream);
             if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
         }
@@ -1294,8 +1300,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     s->last = P;
     s->lastF = F;
-    s->last_pna = P.pna;
-    s->last_pnb = P.pnb;
     CUDA_TRY(cudaEventRecord(s->ev_done, s->stream));
     s->in_flight = true;
     s->solved = true;

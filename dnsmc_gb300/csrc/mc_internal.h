@@ -57,11 +57,15 @@ struct MarchParams {
     // MODE_T: (ti, ft) table temperature cell and fraction; MODE_TX:
     // (ti*(nX-1)+xi, ft, fx, ti); MODE_GREY: T^4, the sign bit set where T is
     // not positive.  Rows of pna values (j), pnb rows a plane (k), pstride
-    // values a field: na, nb and field_stride, or (the gas march on the fine
-    // grid) the periodic axes continued past their end by the packet's extent
+    // values a field: na, nb and field_stride (multigrid), or (the marches on
+    // the fine grid) the periodic axes continued past their end by the packet's extent
     const int2   *fieldP;
     const int4   *fieldPX;
     const float  *fieldG;
+    // the general medium's, with the particle volume fraction: tables
+    // (ti*(nX-1)+xi | ti << 16, ft, fx, fv), grey (T^4, fv)
+    const int4   *fieldVX;
+    const float2 *fieldVG;
     int pna, pnb;
     long long pstride;
     float rda, rdb;           // 1/da, 1/db (estimates of crossing counts only)
@@ -102,7 +106,6 @@ struct MarchParams {
     float toll;
     float dtoll;              // ln(1/toll): optical-depth cut-off of the surrogate walk
     // general medium (GEN march): particles and grey walls
-    const float *fieldV;      // [f][i][k][j] particle volume fraction, or null
     const float2 *part;       // [band] (absorption, scattering) per unit volume fraction [1/m], or null
     float fv_max;             // largest volume fraction of the fields (collision majorant)
     float hg_g;               // Henyey-Greenstein asymmetry factor
@@ -314,7 +317,7 @@ int upload_sobol_dirs_pair(const uint32_t dirs[4][32]);
 int launch_march(int mode, const MarchParams &p, int blocks, int threads,
                  void *stream, bool trace);
 int launch_finalize(const FinalizeParams &p, void *stream);
-// Table coordinates (outP or outPX), or T^4 (outG), of every cell of nfields
+// Table coordinates (outP, outPX or outVX), or T^4 (outG or outVG), of every cell of nfields
 // packed fields [f][i][k][j], into rows of pna values and pnb rows a plane
 // (na <= pna < 2 na, nb <= pnb < 2 nb: continued periodically)
 inline int march_extent(int n, int tile) { return n + (tile < n ? tile : n) - 1; }  // n cells, packets of tile
@@ -328,6 +331,9 @@ struct FieldPos {
     int2 *outP;
     int4 *outPX;
     float *outG;
+    const float *fV;          // volume fraction (null: 0) for outVX and outVG
+    int4 *outVX;
+    float2 *outVG;
     int nfields, nw, na, nb, pna, pnb;
     float T0, invdT, X0, invdX;
     int nT, nX;

@@ -57,9 +57,11 @@ __global__ void field_pos_kernel(const FieldPos q) {
         const long long src = (fw * q.nb + b) * q.na + a;
         int ti, xi;
         float ft, fx;
-        if (q.outG) {
+        const float fv = q.fV ? q.fV[src] : 0.0f;
+        if (q.outG || q.outVG) {
             const float T = q.fT[src], t2 = T * T, v = t2 * t2;
-            q.outG[i] = T > 0.0f ? v : -v;
+            if (q.outG) q.outG[i] = T > 0.0f ? v : -v;
+            else q.outVG[i] = make_float2(T > 0.0f ? v : -v, fv);
         } else if (q.fTX) {
             const float2 v = q.fTX[src];
             float pt = (v.x - q.T0) * q.invdT;
@@ -68,12 +70,15 @@ __global__ void field_pos_kernel(const FieldPos q) {
             px = fminf(fmaxf(px, 0.0f), (float)(q.nX - 1));
             pos_split(pt, q.nT, &ti, &ft);
             pos_split(px, q.nX, &xi, &fx);
-            q.outPX[i] = make_int4(ti * (q.nX - 1) + xi, __float_as_int(ft), __float_as_int(fx), ti);
+            const int kx = ti * (q.nX - 1) + xi;  // below 2^16, as ti: the march's slab fits shared memory
+            if (q.outVX) q.outVX[i] = make_int4(kx | ti << 16, __float_as_int(ft), __float_as_int(fx), __float_as_int(fv));
+            else q.outPX[i] = make_int4(kx, __float_as_int(ft), __float_as_int(fx), ti);
         } else {
             float pt = (q.fT[src] - q.T0) * q.invdT;
             pt = fminf(fmaxf(pt, 0.0f), (float)(q.nT - 1));
             pos_split(pt, q.nT, &ti, &ft);
-            q.outP[i] = make_int2(ti, __float_as_int(ft));
+            if (q.outVX) q.outVX[i] = make_int4(ti | ti << 16, __float_as_int(ft), 0, __float_as_int(fv));
+            else q.outP[i] = make_int2(ti, __float_as_int(ft));
         }
     }
 }

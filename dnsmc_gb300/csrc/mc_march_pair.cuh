@@ -68,13 +68,14 @@ __device__ __forceinline__ float next_up(float v) { return __uint_as_float(__flo
 
 // crossings of a periodic axis before time tau: the n with (n + off) dt < tau.
 // r is an estimate of 1 / dt: its error (a few 2^-24) moves the count by less
-// than one up to 2^20 crossings, which one comparison each way mends; more
-// crossings are stepped.
+// than one up to 2^20 crossings, which one comparison each way mends; larger
+// counts (a ray has at most 2^22 steps) are stepped, a bounded number of times
+// whatever the inputs.
 __device__ __forceinline__ float crossings_before(float tau, float r, float dt, float off) {
-    float g = fmaxf(floorf(fmaf(tau, r, 1.0f - off)), 0.0f);
+    float g = fminf(fmaxf(floorf(fmaf(tau, r, 1.0f - off)), 0.0f), 8388608.0f);
     if (g >= 1048576.0f) {
-        while ((g - 1.0f + off) * dt >= tau) g -= 1.0f;
-        while ((g + off) * dt < tau) g += 1.0f;
+        for (int i = 0; i < 16 && (g - 1.0f + off) * dt >= tau; ++i) g -= 1.0f;
+        for (int i = 0; i < 16 && (g + off) * dt < tau; ++i) g += 1.0f;
     }
     g = (g - 1.0f + off) * dt >= tau ? g - 1.0f : g;
     g = (g + off) * dt < tau ? g + 1.0f : g;
@@ -105,12 +106,32 @@ struct Walk {
     int cw, ca, cb;
 };
 
+// The ray's direction in the walk, which then starts at time 0 from its
+// (oW, offA, offB) offsets.
+__device__ __forceinline__ void walk_direction(const MarchParams &P, Walk &w, float sW, float sA, float sB) {
+    const float aW = fabsf(sW), aA = fabsf(sA), aB = fabsf(sB);
+    const float invW = 1.0f / aW, invA = 1.0f / aA, invB = 1.0f / aB;
+    w.dW = sW > 0.f ? 1 : -1; w.dA = sA > 0.f ? 1 : -1; w.dB = sB > 0.f ? 1 : -1;
+    // crossing time of a wall-normal face: (fw[c + 1] - o) / s going up,
+    // (o - fw[c]) / |s| = (fw[c] - o) * (-1/|s|) going down (exact negation)
+    w.sinvW = w.dW > 0 ? invW : -invW;
+    w.dtA = P.da * invA; w.dtB = P.db * invB;
+    w.rA = aA * P.rda; w.rB = aB * P.rdb;
+    w.t = 0.0f; w.nA = 0.0f; w.nB = 0.0f;
+}
+
+// How a chunk ends: the walk goes on, its last step reaches a wall, or (COL)
+// the tentative collision at time tcol comes next.
+enum WalkEnd { WALK_ON = 0, WALK_WALL = 1, WALK_COL = 2 };
+
 // Generate the next chunk (at most cap steps, cap <= kWalkCap; about `aim` of
-// them).  Returns the steps generated; *wall: the last of them reaches a wall.
-// The state is advanced (in shared memory, walk_state reads it back).
-template <bool TRACE>
-__device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, float aim, int cap, float *buf, int lane,
-                                          bool *wall, int step0) {
+// them; none after tcol).  Returns the steps generated (at least one, but
+// before a collision and for unusable faces), *end how the chunk ends.  The
+// state is advanced in shared memory (walk_state reads it back; not written
+// when there are no steps).
+template <bool TRACE, bool COL>
+__device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, float aim, int cap, float tcol, float *buf,
+                                          int lane, int *end, int step0) {
     const unsigned FULL = 0xffffffffu;
     const float INF = __int_as_float(0x7f800000);
     const int dW = w.dW, dA = w.dA, dB = w.dB;
@@ -125,7 +146,10 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     tw[lane] = twl;
     const int nv = __popc(__ballot_sync(FULL, in));          // >= 1: the cell is in the grid
     const float tw0 = __shfl_sync(FULL, twl, 0), twe = __shfl_sync(FULL, twl, nv - 1);
-    if (lane == 0) tw[32] = INF;
+    if (lane == 0) {
+        tw[32] = INF;
+        buf[kWalkState + 6] = 0.0f;  // (int) 0 steps, unless a lane makes the last one
+    }
     // the window: about `aim` crossings at the present rates, no more than
     // the listed wall-normal ones, at least the next crossing
     const float rW = twe < INF ? __fdividef((float)(nv - 1), fmaxf(twe - tw0, 1e-30f)) : 0.0f;
@@ -133,6 +157,12 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     te = fminf(te, nv < 32 ? (twe < INF ? next_up(twe) : INF) : twe);
     const float tmin = fminf(tw0, fminf((w.nA + w.offA) * dtA, (w.nB + w.offB) * dtB));
     te = fmaxf(te, next_up(tmin));
+    bool col = false;
+    if (COL && tcol < INF) {
+        const float tc = next_up(tcol);
+        col = tc <= te;
+        te = fminf(te, tc);
+    }
     const float dt = (te - w.t) * (1.0f / 31.0f);
     const float tau = lane == 31 ? te : fminf(fmaf((float)lane, dt, w.t), te);
     // crossing counts at this lane's slice start
@@ -153,7 +183,8 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     const int n0 = min(total, cap);
     bool hit = false;
     if (lane < 31 && e < eend) {
-        int cw = w.cw + dW * k, ca = wrap_move(w.ca, dA * mA, P.na), cb = wrap_move(w.cb, dB * mB, P.nb);
+        // (the bounds hold by themselves for faces in ascending order)
+        int cw = min(max(w.cw + dW * k, 0), P.nw - 1), ca = wrap_move(w.ca, dA * mA, P.na), cb = wrap_move(w.cb, dB * mB, P.nb);
         float tA = (nA + w.offA) * dtA, tB = (nB + w.offB) * dtB, tW = tw[k];
         // the time of the crossing before the slice
         float t = fmaxf(w.t, fmaxf((nA - 1.0f + w.offA) * dtA, (nB - 1.0f + w.offB) * dtB));
@@ -172,7 +203,7 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
             t = tn;
             if (bW) {
                 hit = (unsigned)(cw + dW) >= (unsigned)P.nw;
-                if (!hit) { cw += dW; ++k; tW = tw[k]; }
+                if (!hit) { cw += dW; k = min(k + 1, 32); tW = tw[k]; }
             } else if (bA) {
                 nA += 1.0f;
                 tA = (nA + w.offA) * dtA;
@@ -198,7 +229,8 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
             buf[5 + 2 * e] = __int_as_float(off);
         }
     }
-    *wall = __any_sync(FULL, hit);
+    hit = __any_sync(FULL, hit);
+    *end = hit ? WALK_WALL : (col && total <= cap ? WALK_COL : WALK_ON);
     __syncwarp();
     return __float_as_int(buf[kWalkState + 6]);
 }
@@ -215,13 +247,14 @@ __device__ __forceinline__ void walk_state(const float *buf, Walk &w) {
 // Every lane setting up every ray took 250 of its ~3000 instructions: 128^3
 // channel 66.1 -> 62.3 ms, 4 x 96^3 batch 130.1 -> 119.6 ms.
 struct RayBatch {
-    float4 walk[32];    // sinvW, dtA and dtB (signed like the direction), the sample's weight factor
+    float4 walk[32];    // sinvW, dtA and dtB (signed like the direction; general medium: the
+                        // direction itself), the sample's weight factor
     float4 rates[32];   // rA, rB, band and spectral sample (as int bits)
     float4 sur[32];     // surrogate: collected intensity, own-layer absorptance, own-layer intensity
 };
 static_assert(sizeof(RayBatch) == kBatchBytes, "march_pair_smem");
 
-template <int MODE, bool TRACE, bool CV>
+template <int MODE, bool TRACE, bool CV, bool GEN>
 __device__ __forceinline__ void ray_batch(const MarchParams &P, RayBatch *B, int r, int M, int p, uint32_t ctr2, int gs,
                                          int K, int f, int w0, int lane) {
     uint4 x;
@@ -238,11 +271,8 @@ __device__ __forceinline__ void ray_batch(const MarchParams &P, RayBatch *B, int
     }
     float sW, sA, sB;
     ray_direction(x, &sW, &sA, &sB);
-    const float aW = fabsf(sW), aA = fabsf(sA), aB = fabsf(sB);
-    const float invW = 1.0f / aW, invA = 1.0f / aA, invB = 1.0f / aB;
-    // crossing time of a wall-normal face: (fw[c + 1] - o) / s going up,
-    // (o - fw[c]) / |s| = (fw[c] - o) * (-1/|s|) going down (exact negation)
-    const float dtA = P.da * invA, dtB = P.db * invB;
+    Walk w;
+    walk_direction(P, w, sW, sA, sB);
     float eW = P.Wgrey;
     int nbnd = 0, sid = 0;
     if constexpr (MODE != MODE_GREY) {
@@ -253,8 +283,9 @@ __device__ __forceinline__ void ray_batch(const MarchParams &P, RayBatch *B, int
         sid = e.koff;
         eW = e.W;
     }
-    B->walk[lane] = make_float4(sW > 0.f ? invW : -invW, sA > 0.f ? dtA : -dtA, sB > 0.f ? dtB : -dtB, eW);
-    B->rates[lane] = make_float4(aA * P.rda, aB * P.rdb, __int_as_float(nbnd), __int_as_float(sid));
+    B->walk[lane] = GEN ? make_float4(sW, sA, sB, eW)
+                        : make_float4(w.sinvW, w.dA > 0 ? w.dtA : -w.dtA, w.dB > 0 ? w.dtB : -w.dtB, eW);
+    B->rates[lane] = make_float4(w.rA, w.rB, __int_as_float(nbnd), __int_as_float(sid));
     if (CV) {
         // the ray's straight flight through the layer-mean medium, the same
         // for all cells (same layer)
@@ -415,7 +446,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
             const int rb = (r - rbeg) & 31;
             if (rb == 0) {
                 __syncwarp();
-                if (r + lane < rend) ray_batch<MODE, TRACE, CV>(P, batch, r + lane, M, p, ctr2, gs, K, f, w0, lane);
+                if (r + lane < rend) ray_batch<MODE, TRACE, CV, false>(P, batch, r + lane, M, p, ctr2, gs, K, f, w0, lane);
                 __syncwarp();
             }
             // the ray's table slab is on its way while the walk's first chunk
@@ -445,17 +476,17 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
             int steps = 0;
             bool first = true;
             for (;;) {  // chunks of the walk
-                bool wall;
+                int end;
                 // a short first chunk where this item's rays have been short
-                const int n = walk_chunk<TRACE>(P, w, first && est < 20 ? 28.0f : (float)(kWalkCap - 4),
-                                                min(kWalkCap, P.max_steps - steps), wbuf, lane, &wall, steps);
+                const int n = walk_chunk<TRACE, false>(P, w, first && est < 20 ? 28.0f : (float)(kWalkCap - 4),
+                                                       min(kWalkCap, P.max_steps - steps), 0.0f, wbuf, lane, &end, steps);
                 if constexpr (UNI) {
                     // e = expm1(k (t - tn)) of the chunk's steps, a lane each
                     for (int q = lane; q < n; q += 32) wbuf[4 + 2 * q] = mc_expm1(P.kappa * wbuf[4 + 2 * q]);
                     __syncwarp();
                 }
                 {
-                    const unsigned c1 = __float_as_uint(wbuf[3]);
+                    const unsigned c1 = n ? __float_as_uint(wbuf[3]) : corner;
 #pragma unroll
                     for (int k = 0; k < C; ++k) vb[k] = __ldg(fp[k] + c1);
                 }
@@ -477,6 +508,10 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
                             wk[k] = bw.w * ki;
                         }
                     }
+                }
+                if (n == 0) {  // no walk through these faces (not in ascending order, or not finite)
+                    flags |= DNSMC_STATUS_STEP_CAP;
+                    break;
                 }
                 const float4 *wp = reinterpret_cast<const float4 *>(wbuf + 4);
                 bool done = false;
@@ -573,7 +608,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
                 }
                 if (done) { steps += n; break; }
                 steps += n;
-                if (wall) {
+                if (end == WALK_WALL) {
 #pragma unroll
                     for (int k = 0; k < C; ++k) {
                         const int side = w.dW > 0 ? 1 : 0;
@@ -676,45 +711,53 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
 
 // ---------------------------------------------------------------------------
 // The same march for the general medium (GEN): particles with scattering and
-// grey diffuse walls; restarts of the walk at every scattering and wall
-// reflection, so the crossing counts are integers with the restart offsets.
+// grey diffuse walls.  The walk restarts at every scattering and wall
+// reflection; its chunks end at the ray's next tentative collision, which is a
+// step of its own.
+// As the gas march it is bound by the L1 gathers and issue; a cell's volume
+// fraction rides in its 16-byte coordinates.  96^3 gas with particles, 8 rays:
+// 19.8 ms with the walk in every lane, 11.6 ms.
 // ---------------------------------------------------------------------------
-template <int MODE, bool TRACE, bool CV, bool MOM>
+template <int MODE> struct GenFieldT { typedef int4 type; };
+template <> struct GenFieldT<MODE_GREY> { typedef float2 type; };
+__device__ __forceinline__ float gen_fraction(const int4 &v) { return __int_as_float(v.w); }
+__device__ __forceinline__ float gen_fraction(const float2 &v) { return v.y; }
+
+template <int MODE, bool TRACE, bool CV, bool MOM, bool SPLIT>
 __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const MarchParams P) {
-    typedef typename FieldT<MODE>::type VT;
+    typedef typename GenFieldT<MODE>::type VT;
     const float INF = __int_as_float(0x7f800000);
     constexpr int C = kLaneCells;  // cells per lane
-    static_assert(C % 2 == 0, "the attenuation goes through cell pairs");
+    static_assert(C == 2, "the attenuation goes through a cell pair");
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int tid = threadIdx.x;
     const int la = lane % P.tile_a, lb = lane / P.tile_a;
     const int hb = 32 / P.tile_a;  // k rows between a lane's two cells
     const int njR = P.ea1 - P.ea0, nkR = P.eb1 - P.eb0;
-    const int plane = P.na * P.nb;
     unsigned long long my_rays = 0, my_steps = 0;
     unsigned int flags = 0;
-    // dynamic shared memory (march_smem): this warp's copy of the current
-    // ray's table slab (tabulated models); per-cell sums of the item as
-    // float pairs (ray sum, sum of squares or of squared replicate means,
-    // current replicate sum) [3][C][threads] and the replicate's shift [threads] --
-    // shared memory, so registers hold the march's own working set
+    // dynamic shared memory as the gas march's (march_pair_smem)
     extern __shared__ float4 s_dyn[];
     const int nthr = blockDim.x;
-    float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + (threadIdx.x >> 5) * P.slab_len;
+    const int warp = threadIdx.x >> 5, nwarp = (nthr + 31) >> 5;
+    float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + warp * P.slab_len;
     const float2 *const sli = slk + P.slab_klen;
-    double *const s_acc = reinterpret_cast<double *>(reinterpret_cast<float2 *>(s_dyn) + ((nthr + 31) >> 5) * P.slab_len);
-    uint4 *const s_shift = reinterpret_cast<uint4 *>(s_acc + 3 * C * nthr);
+    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * kWalkWords;
+    RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
+                                                        nwarp * kWalkWords) + warp;
+    float2 *const s_acc = reinterpret_cast<float2 *>(batch - warp + nwarp);
     auto acc = [&](int q, int k) { return s_acc + (q * C + k) * nthr + tid; };
     // each warp's transaction barrier of its slab copies, and its parity
     __shared__ uint64_t s_bar[8];
-    uint64_t *const sbar = &s_bar[threadIdx.x >> 5];
+    uint64_t *const sbar = &s_bar[warp];
     uint32_t sphase = 0;
     slab_bar_init(sbar, lane);
     bool dead = false;  // a slab copy did not arrive: this warp stops marching
 
     for (;;) {
         long long item;
+        int part = 0;
         if (TRACE) {
             if (threadIdx.x >= 32) return;
             item = ((long long)P.trace_f * P.n_groups + P.trace_g) * P.n_packets + P.trace_p;
@@ -722,7 +765,11 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
             unsigned int it = 0;
             if (lane == 0) it = atomicAdd(P.queue, 1u);
             it = __shfl_sync(FULL, it, 0);
-            if ((long long)it >= P.n_items) break;
+            if ((long long)it >= (SPLIT ? P.n_items * P.parts : P.n_items)) break;
+            if (SPLIT) {
+                part = (int)(it % (unsigned)P.parts);
+                it /= (unsigned)P.parts;
+            }
             item = P.item_order ? (long long)__ldg(P.item_order + it) : (long long)it;
         }
         const int p = (int)(item % P.n_packets);
@@ -734,38 +781,37 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
         const int pb = rest % P.npb;
         const int pw = rest / P.npb;
         const int w0 = P.ew0 + pw;
-        const int a0 = P.ea0 + pa * P.tile_a + la;
-        const bool act_a = a0 < P.ea1;
-        const int acl = act_a ? a0 : P.ea0;  // cells outside the region march a valid cell, untallied
+        const int ac = P.ea0 + pa * P.tile_a, bc = P.eb0 + pb * P.tile_b;  // the packet's corner
         bool active[C];
-        int bcl[C], tcell[C];
+        int tcell[C];
+        const VT *fp[C];  // the lane's cells as offsets from the corner (cells outside the region: the corner)
 #pragma unroll
         for (int k = 0; k < C; ++k) {
-            const int b0 = P.eb0 + pb * P.tile_b + lb + k * hb;
-            active[k] = act_a && b0 < P.eb1;
-            bcl[k] = active[k] ? b0 : P.eb0;
-            tcell[k] = ((w0 - P.ew0) * nkR + (bcl[k] - P.eb0)) * njR + (acl - P.ea0);
+            active[k] = ac + la < P.ea1 && bc + lb + k * hb < P.eb1;
+            const int a = active[k] ? la : 0, b = active[k] ? lb + k * hb : 0;
+            tcell[k] = (pw * nkR + pb * P.tile_b + b) * njR + pa * P.tile_a + a;
+            const long long o = (long long)f * P.pstride + b * P.pna + a;
+            if constexpr (MODE == MODE_GREY) fp[k] = P.fieldVG + o;
+            else fp[k] = P.fieldVX + o;
         }
+        const unsigned corner = ((unsigned)w0 * P.pnb + bc) * P.pna + ac;
         const int N = P.rays_per_packet ? P.rays_per_packet[G * P.rays_gstride + p] : P.rays;
-        const long long fbase = (long long)f * P.field_stride;
-        const int rowW0 = w0 * plane;
         const float oW = (__ldg(P.fw + w0) + __ldg(P.fw + w0 + 1)) * 0.5f;
         // alias table of this packet: band group G of the temperature bin
         // nearest to the temperature of the packet's first cell
         int gs = 0, K = 1;
         if constexpr (MODE == MODE_GREY) {
+            // T^4 with the sign set where the temperature is not positive
 #pragma unroll
             for (int k = 0; k < C; ++k) {
-                const float Ti = load_field<MODE>(P, fbase, rowW0 + bcl[k] * P.na + acl);
-                if (!(Ti > 0.0f) && active[k]) flags |= DNSMC_STATUS_BAD_FIELD;
+                const float v = __ldg(fp[k] + corner).x;
+                if (active[k] && (__float_as_int(v) < 0 || v != v)) flags |= DNSMC_STATUS_BAD_FIELD;
             }
         } else {
             int boff = 0;
             if (P.n_tbins > 1) {
-                int kx, ti;
-                float ft, fx;
-                cell_coords<MODE>(load_field<MODE>(P, fbase, rowW0 + bcl[0] * P.na + acl), &kx, &ti, &ft, &fx);
-                const float tp0 = __shfl_sync(FULL, (float)ti + ft, 0);
+                const int4 v = __ldg(fp[0] + corner);
+                const float tp0 = __shfl_sync(FULL, (float)(v.x >> 16) + __int_as_float(v.y), 0);
                 int bin = __float2int_rn(tp0);
                 bin = min(max(bin, 0), P.n_tbins - 1);
                 boff = bin * P.n_groups;
@@ -781,268 +827,236 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
 #pragma unroll
                 for (int q = 0; q < 9; ++q) mo[k][q] = 0.0;
         const int M = P.sampler ? max(1, N / max(1, P.nbatch)) : 1;
+        if (!SPLIT)
 #pragma unroll
-        for (int k = 0; k < C; ++k) { *acc(0, k) = 0.0; *acc(1, k) = 0.0; *acc(2, k) = 0.0; }
+        for (int k = 0; k < C; ++k) {
+            *acc(0, k) = make_float2(0.0f, 0.0f); *acc(1, k) = make_float2(0.0f, 0.0f); *acc(2, k) = make_float2(0.0f, 0.0f);
+        }
         unsigned long long isteps = 0;
         unsigned int lsteps = 0;  // this lane's active cell-steps in the item
-        int bcur = -1;
-        const int rbeg = TRACE ? P.trace_r : 0;
-        const int rend = TRACE ? P.trace_r + 1 : ((K > 0) ? N : 0);
+        int rbeg = TRACE ? P.trace_r : 0;
+        int rend = TRACE ? P.trace_r + 1 : ((K > 0) ? N : 0);
+        float *const rayx = SPLIT ? P.rayx + item * N * 64 + lane : nullptr;
+        if (SPLIT) unit_rays(P, part, rend, &rbeg, &rend);
+        int m = P.sampler ? rbeg % M : 0;  // the ray's index in its replicate
         for (int r = rbeg; r < rend; ++r) {
-            int m;
-            const uint4 x = ray_words(P, r, M, p, ctr2, &bcur, &s_shift[tid], &m);
-            if (TRACE && lane == 0) {
-                P.trace_rng[0] = x.x; P.trace_rng[1] = x.y; P.trace_rng[2] = x.z; P.trace_rng[3] = x.w;
+            const int rb = (r - rbeg) & 31;
+            if (rb == 0) {
+                __syncwarp();
+                if (r + lane < rend) ray_batch<MODE, TRACE, CV, true>(P, batch, r + lane, M, p, ctr2, gs, K, f, w0, lane);
+                __syncwarp();
             }
-            float sW_e, sA_e, sB_e;  // the emission direction
-            ray_direction(x, &sW_e, &sA_e, &sB_e);
-
-            // spectral sample, each cell's own k, Ib and weight wk
-            int nbnd = 0, sid = 0;
-            float wk[C], Ii[C];
-            VT vcur[C];
-            float fvcur[C];  // the particle volume fraction of the current cells
+            // the ray's table slab is on its way while the walk's first chunk
+            // is generated
+            float sW, sA, sB;
+            int nbnd;
+            {
+                const float4 bw = batch->walk[rb], br = batch->rates[rb];
+                sW = bw.x; sA = bw.y; sB = bw.z;
+                nbnd = __float_as_int(br.z);
+                if constexpr (MODE != MODE_GREY) slab_issue(P, __float_as_int(br.w), slk, lane, sbar);
+            }
             float pab = 0.0f, psc = 0.0f;  // particle absorption / scattering per unit volume fraction
-#pragma unroll
-            for (int k = 0; k < C; ++k) {
-                vcur[k] = load_field<MODE>(P, fbase, rowW0 + bcl[k] * P.na + acl);
-                fvcur[k] = P.fieldV ? __ldg(P.fieldV + fbase + rowW0 + bcl[k] * P.na + acl) : 0.0f;
-            }
-            if constexpr (MODE == MODE_GREY) {
-                if (P.part) { const float2 pp = __ldg(P.part); pab = pp.x; psc = pp.y; }
-#pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    const float Ti = vcur[k];
-                    const float t2 = Ti * Ti;
-                    Ii[k] = t2 * t2;
-                    wk[k] = P.W4sig * fmaf(fvcur[k], pab, P.kappa);
-                }
-            } else {
-                const int j = (int)__umulhi(x.z, (uint32_t)K);
-                SpecEntry e = P.entries[gs + j];
-                if (!(u24(x.w) < e.prob)) e = P.entries[gs + (int)(e.alias_nb & 0xFFFFu)];
-                nbnd = (int)(e.alias_nb >> 16);
-                sid = e.koff;
-                if (!load_slab(P, sid, slk, lane, sbar, &sphase, &flags)) { dead = true; break; }
-                if (P.part) { const float2 pp = __ldg(P.part + nbnd); pab = pp.x; psc = pp.y; }
-#pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    int kx, ti;
-                    float ft, fx;
-                    cell_coords<MODE>(vcur[k], &kx, &ti, &ft, &fx);
-                    float ki = lookup_k<MODE>(slk, kx, ft, fx);
-                    ki = fmaf(fvcur[k], pab, ki);
-                    Ii[k] = lookup_ib(sli, ti, ft);
-                    wk[k] = e.W * ki;
-                }
-            }
-
-            // warp-uniform DDA from (pw0, fa0, fb0): the wall-normal coordinate
-            // and the fractional offsets inside the current periodic cells (the
+            if (P.part) { const float2 pp = __ldg(P.part + nbnd); pab = pp.x; psc = pp.y; }
+            // the walk from (w.oW, fa0, fb0): the wall-normal coordinate and
+            // the fractional offsets inside the current periodic cells (the
             // cell centres at emission, restarted at every scattering and wall
             // reflection)
-            float sW = sW_e, sA = sA_e, sB = sB_e;
-            float pw0 = oW, fa0 = 0.5f, fb0 = 0.5f, offA = 0.5f, offB = 0.5f;
-            float invW, invA, invB, sinvW, tW, dtA, dtB, tA, tB;
-            int dW, dA, dB, nA = 0, nB = 0;
-            // per direction: the exit face (fw[c + 1] - o)/s going up, (fw[c] - o)
-            // * (-1/|s|) going down (the values of (o - fw[c])/|s|: negation is
-            // exact), the index beyond the wall, the one-compare periodic wraps
-            const float *fwn;
-            int wallW, dRowW, wrapA, resetA, wrapB, resetB;
-            int cw = w0;
-            auto dda_init = [&]() {
-                invW = 1.0f / fabsf(sW); invA = 1.0f / fabsf(sA); invB = 1.0f / fabsf(sB);
-                dW = sW > 0.f ? 1 : -1; dA = sA > 0.f ? 1 : -1; dB = sB > 0.f ? 1 : -1;
-                fwn = P.fw + (dW > 0 ? 1 : 0);
-                sinvW = dW > 0 ? invW : -invW;
-                wallW = dW > 0 ? P.nw : -1;
-                dRowW = dW * plane;
-                wrapA = dA > 0 ? P.na : -1; resetA = dA > 0 ? 0 : P.na - 1;
-                wrapB = dB > 0 ? P.nb : -1; resetB = dB > 0 ? 0 : P.nb - 1;
-                tW = (__ldg(fwn + cw) - pw0) * sinvW;
-                dtA = P.da * invA; dtB = P.db * invB;
-                offA = dA > 0 ? 1.0f - fa0 : fa0;
-                offB = dB > 0 ? 1.0f - fb0 : fb0;
-                tA = offA * dtA; tB = offB * dtB;
-                nA = 0; nB = 0;
+            Walk w;
+            float fa0 = 0.5f, fb0 = 0.5f;
+            w.oW = oW;
+            w.cw = w0; w.ca = ac; w.cb = bc;
+            auto restart = [&]() {
+                walk_direction(P, w, sW, sA, sB);
+                // (an axis the ray does not move along is never crossed,
+                // wherever the ray is in its cell)
+                w.offA = w.dtA < INF ? (w.dA > 0 ? 1.0f - fa0 : fa0) : 0.5f;
+                w.offB = w.dtB < INF ? (w.dB > 0 ? 1.0f - fb0 : fb0) : 0.5f;
             };
-            dda_init();
-            int ca = acl, rowW = rowW0;
-            int cb[C], rowB[C];
-            float tau[C], D[C];
+            restart();
+            VT va[C], vb[C], vc[C], vd[C];  // field values of two steps and of the two after
+#pragma unroll
+            for (int k = 0; k < C; ++k) va[k] = __ldg(fp[k] + corner);
+            float wk[C], Ii[C], tau[C], D[C];
+            int life[C];  // steps each cell was live for (while it is: 2^30)
 #pragma unroll
             for (int k = 0; k < C; ++k) {
-                cb[k] = bcl[k];
-                rowB[k] = bcl[k] * P.na;
                 tau[k] = active[k] ? 1.0f : 0.0f;
                 D[k] = 0.0f;
+                life[k] = active[k] ? 1 << 30 : 0;
             }
-            float t = 0.0f;
             int steps = 0;
             // scattering events: one Philox word quadruple per event
             uint32_t ev = 0;
             uint4 evx = make_uint4(0u, 0u, 0u, 0u);
-            float sigbar = 0.0f, tcol = INF;
             auto draw = [&]() {
                 evx = philox4x32_10(make_uint4((uint32_t)r, (uint32_t)p, ctr2, 0x5CA70000u + ev), P.key0, P.key1);
                 ++ev;
             };
-            sigbar = P.fv_max * psc;
+            const float sigbar = P.fv_max * psc;
+            float tcol = INF;
             if (sigbar > 0.0f) { draw(); tcol = mc_neglog(u24o(evx.x)) / sigbar; }
-            // unrolled by two: the current / next field values alternate
-            // registers instead of being copied every step
-#pragma unroll 2
-            for (;;) {
-                const bool sW_ = tW <= tA && tW <= tB;
-                const bool sA_ = !sW_ && tA <= tB;
-                int axis = sW_ ? 0 : (sA_ ? 1 : 2);
-                float tn = sW_ ? tW : (sA_ ? tA : tB);
-                {  // a tentative collision first
-                    const bool col = tcol < tn;
-                    axis = col ? 3 : axis;
-                    tn = col ? tcol : tn;
+            // One step of both cells, the same paired update as the gas
+            // march's: e = expm1(k * (t - tn)) = -alpha, nta = tau e = -ta,
+            // D += nta (-g), tau += nta; a cell already dumped (tau 0) adds
+            // exactly nothing.
+            auto step = [&](const VT (&v)[C], float nds, int s) {
+                float kj[C], ngj[C];
+#pragma unroll
+                for (int h = 0; h < C; ++h) {
+                    float fv;
+                    if constexpr (MODE == MODE_GREY) {
+                        ngj[h] = v[h].x - Ii[h];
+                        kj[h] = P.kappa;
+                        fv = v[h].y;
+                    } else {
+                        const float ft = __int_as_float(v[h].y);
+                        kj[h] = lookup_k<MODE>(slk, v[h].x & 0xffff, ft, __int_as_float(v[h].z));
+                        ngj[h] = lookup_ib(sli, v[h].x >> 16, ft) - Ii[h];
+                        fv = __int_as_float(v[h].w);
+                    }
+                    kj[h] = fmaf(fv, pab, kj[h]);
                 }
-                const float ds = tn - t;
-                const float nds = t - tn;  // minus the segment length (exact negation)
-                // next cell of the walk, and its field values fetched now; the
-                // axis is the same in every lane, but selects cost fewer
-                // instructions here than branches the compiler must treat as
-                // divergent
-                int ncw, nca, nrowW;
-                int ncb[C], nrowB[C];
-                const bool aW = axis == 0, aA = axis == 1, aB = axis == 2;
-                ncw = aW ? cw + dW : cw;
-                nrowW = aW ? rowW + dRowW : rowW;
+                const float2 e = mc_expm1_x2(__fmul2_rn(make_float2(kj[0], kj[1]), make_float2(nds, nds)));
+                const float2 nta = __fmul2_rn(make_float2(tau[0], tau[1]), e);
+                const float2 d2 = __ffma2_rn(nta, make_float2(ngj[0], ngj[1]), make_float2(D[0], D[1]));
+                const float2 t2 = __fadd2_rn(make_float2(tau[0], tau[1]), nta);
+                D[0] = d2.x; D[1] = d2.y;
+                tau[0] = t2.x; tau[1] = t2.y;
+#pragma unroll
+                for (int h = 0; h < C; ++h) {
+                    if (tau[h] < P.toll) {
+                        D[h] = fmaf(-tau[h], ngj[h], D[h]);
+                        tau[h] = 0.0f;
+                        life[h] = min(life[h], s + 1);
+                    }
+                }
+                if (TRACE && lane == 0 && s < P.trace_max) P.trace_rec[6 * s + 5] = __float_as_int(tau[0]);
+            };
+            bool first = true;
+            for (;;) {  // chunks of the walk
+                int end;
+                const int n = walk_chunk<TRACE, true>(P, w, (float)(kWalkCap - 4), min(kWalkCap, P.max_steps - steps), tcol,
+                                                      wbuf, lane, &end, steps);
                 {
-                    int u = ca + dA;
-                    u = u == wrapA ? resetA : u;
-                    nca = aA ? u : ca;
+                    const unsigned c1 = n ? __float_as_uint(wbuf[3]) : corner;
+#pragma unroll
+                    for (int k = 0; k < C; ++k) vb[k] = __ldg(fp[k] + c1);
                 }
+                if (first) {
+                    first = false;
+                    if constexpr (MODE != MODE_GREY)
+                        if (!slab_wait(P, sbar, &sphase, &flags)) { dead = true; break; }
 #pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    int u = cb[k] + dB;
-                    u = u == wrapB ? resetB : u;
-                    ncb[k] = aB ? u : cb[k];
-                    nrowB[k] = aB ? u * P.na : rowB[k];
-                }
-                const bool wall = aW && ncw == wallW;
-                // fetched for every cell, live or not (a dumped cell's value
-                // is never used); a collision keeps the cell, so the address
-                // is the current one, and at a wall the row stays inside the
-                // grid and the walk restarts or ends
-                const int lrowW = wall ? rowW : nrowW;
-                VT vnext[C];
-                float fvnext[C];
-#pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    vnext[k] = load_field<MODE>(P, fbase, lrowW + nrowB[k] + nca);
-                    fvnext[k] = P.fieldV ? __ldg(P.fieldV + fbase + lrowW + nrowB[k] + nca) : fvcur[k];
-                }
-                // attenuation and collected intensity of this segment; a cell
-                // already dumped (tau 0) adds exactly nothing.  The same
-                // paired update as the gas march: e = expm1(k * (t - tn)) =
-                // -alpha, nta = tau e = -ta, D += nta (-g), tau += nta.
-#pragma unroll
-                for (int k = 0; k < C; k += 2) {
-                    float kj[2], ngj[2];
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        lsteps += tau[k + h] > 0.0f ? 1u : 0u;
+                    for (int k = 0; k < C; ++k) {
                         if constexpr (MODE == MODE_GREY) {
-                            const float t2 = vcur[k + h] * vcur[k + h];
-                            ngj[h] = t2 * t2 - Ii[k + h];
-                            kj[h] = P.kappa;
+                            Ii[k] = va[k].x;
+                            wk[k] = P.W4sig * fmaf(va[k].y, pab, P.kappa);
                         } else {
-                            int kx, tj;
-                            float ftj, fxj;
-                            cell_coords<MODE>(vcur[k + h], &kx, &tj, &ftj, &fxj);
-                            kj[h] = lookup_k<MODE>(slk, kx, ftj, fxj);
-                            const float Ibj = lookup_ib(sli, tj, ftj);
-                            ngj[h] = Ibj - Ii[k + h];
-                        }
-                        kj[h] = fmaf(fvcur[k + h], pab, kj[h]);
-                    }
-                    const float2 e = mc_expm1_x2(__fmul2_rn(make_float2(kj[0], kj[1]), make_float2(nds, nds)));
-                    const float2 nta = __fmul2_rn(make_float2(tau[k], tau[k + 1]), e);
-                    const float2 d2 = __ffma2_rn(nta, make_float2(ngj[0], ngj[1]), make_float2(D[k], D[k + 1]));
-                    const float2 t2 = __fadd2_rn(make_float2(tau[k], tau[k + 1]), nta);
-                    D[k] = d2.x; D[k + 1] = d2.y;
-                    tau[k] = t2.x; tau[k + 1] = t2.y;
-#pragma unroll
-                    for (int h = 0; h < 2; ++h)
-                        if (tau[k + h] < P.toll) { D[k + h] = fmaf(-tau[k + h], ngj[h], D[k + h]); tau[k + h] = 0.0f; }
-                }
-                if (TRACE && lane == 0 && steps < P.trace_max) {
-                    int *rec = P.trace_rec + 6 * steps;
-                    rec[0] = cw; rec[1] = dA * nA; rec[2] = dB * nB; rec[3] = axis;
-                    rec[4] = __float_as_int(ds); rec[5] = __float_as_int(tau[0]);
-                }
-                t = tn;
-                ++steps;
-                {
-                    if (wall) {
-                        const int side = ncw < 0 ? 0 : 1;
-                        const float Iw = (MODE == MODE_GREY) ? P.Tw4[side] : __ldg(P.ibw + side * P.nbands + nbnd);
-                        {
-                            // grey wall: it takes eps of the throughput at its
-                            // own intensity and reflects the rest diffusely
-                            const float eps = P.eps[side];
-                            bool live = false;
-#pragma unroll
-                            for (int k = 0; k < C; ++k) {
-                                if (tau[k] > 0.0f) {
-                                    const float gw = Ii[k] - Iw;
-                                    D[k] = fmaf(tau[k] * eps, gw, D[k]);
-                                    tau[k] = eps >= 1.0f ? 0.0f : tau[k] * (1.0f - eps);
-                                    if (tau[k] > 0.0f && tau[k] < P.toll) { D[k] = fmaf(tau[k], gw, D[k]); tau[k] = 0.0f; }
-                                }
-                                live = live || tau[k] > 0.0f;
-                            }
-                            if (!__any_sync(FULL, live)) break;
-                            // diffuse reflection from the wall point
-                            const float ta_ = t / dtA, tb_ = t / dtB;
-                            fa0 = dA > 0 ? fa0 + (ta_ - (float)nA) : fa0 - (ta_ - (float)nA);
-                            fb0 = dB > 0 ? fb0 + (tb_ - (float)nB) : fb0 - (tb_ - (float)nB);
-                            fa0 = fminf(fmaxf(fa0, 0.0f), 1.0f);
-                            fb0 = fminf(fmaxf(fb0, 0.0f), 1.0f);
-                            pw0 = side == 0 ? __ldg(P.fw) : __ldg(P.fw + P.nw);
-                            draw();  // this event's words: the reflected direction only
-                            const float cmu = sqrtf(u24(evx.z));
-                            const float smu = sqrtf(fmaxf(0.0f, 1.0f - cmu * cmu));
-                            float cp, sp;
-                            mc_sincos_turn(evx.w >> 8, &cp, &sp);
-                            sW = side == 0 ? cmu : -cmu;
-                            sA = smu * cp;
-                            sB = smu * sp;
-                            dda_init();
-                            t = 0.0f;
-                            if (sigbar > 0.0f) { draw(); tcol = mc_neglog(u24o(evx.x)) / sigbar; }
-                            if (steps >= P.max_steps) {
-                                if (live) flags |= DNSMC_STATUS_STEP_CAP;
-                                break;
-                            }
-                            continue;
+                            const float ft = __int_as_float(va[k].y);
+                            float ki = lookup_k<MODE>(slk, va[k].x & 0xffff, ft, __int_as_float(va[k].z));
+                            ki = fmaf(__int_as_float(va[k].w), pab, ki);
+                            Ii[k] = lookup_ib(sli, va[k].x >> 16, ft);
+                            wk[k] = batch->walk[rb].w * ki;
                         }
                     }
-                    cw = ncw;
-                    rowW = nrowW;
-                    if (aW) tW = (__ldg(fwn + cw) - pw0) * sinvW;
-                    ca = nca;
-#pragma unroll
-                    for (int k = 0; k < C; ++k) { cb[k] = ncb[k]; rowB[k] = nrowB[k]; }
-                    nA += aA ? 1 : 0;
-                    tA = aA ? ((float)nA + offA) * dtA : tA;
-                    nB += aB ? 1 : 0;
-                    tB = aB ? ((float)nB + offB) * dtB : tB;
                 }
-                if (axis == 3) {
-                    // tentative collision: shared decision, per-cell weights
+                bool done = false;
+                if (n) {
+                    // two steps on v0, v1 while the two after are fetched into
+                    // v2, v3; the exit vote after the second
+                    const float4 *wp = reinterpret_cast<const float4 *>(wbuf + 4);
+                    float4 wc = wp[0];
+                    int s = 0;
+                    auto pair = [&](const VT (&v0)[C], const VT (&v1)[C], VT (&v2)[C], VT (&v3)[C]) {
+                        const unsigned o2 = __float_as_uint(wc.y), o3 = __float_as_uint(wc.w);
+#pragma unroll
+                        for (int k = 0; k < C; ++k) v2[k] = __ldg(fp[k] + o2);
+#pragma unroll
+                        for (int k = 0; k < C; ++k) v3[k] = __ldg(fp[k] + o3);
+                        const float d0 = wc.x, d1 = wc.z;
+                        wc = *++wp;
+                        step(v0, d0, steps + s);
+                        step(v1, d1, steps + s + 1);
+                        done = !__any_sync(FULL, tau[0] > 0.0f || tau[1] > 0.0f);
+                        s += 2;
+                    };
+                    for (;;) {
+                        pair(va, vb, vc, vd);
+                        if (done || s >= n) break;
+                        pair(vc, vd, va, vb);
+                        if (done || s >= n) break;
+                    }
+                    steps += n;
+                    walk_state(wbuf, w);
+                }
+                if (done) break;  // every cell dumped
+                if (end == WALK_WALL) {
+                    const int side = w.dW > 0 ? 1 : 0;
+                    const float Iw = (MODE == MODE_GREY) ? P.Tw4[side] : __ldg(P.ibw + side * P.nbands + nbnd);
+                    // grey wall: it takes eps of the throughput at its
+                    // own intensity and reflects the rest diffusely
+                    const float eps = P.eps[side];
+                    bool live = false;
+#pragma unroll
+                    for (int k = 0; k < C; ++k) {
+                        if (tau[k] > 0.0f) {
+                            const float gw = Ii[k] - Iw;
+                            D[k] = fmaf(tau[k] * eps, gw, D[k]);
+                            tau[k] = eps >= 1.0f ? 0.0f : tau[k] * (1.0f - eps);
+                            if (tau[k] > 0.0f && tau[k] < P.toll) { D[k] = fmaf(tau[k], gw, D[k]); tau[k] = 0.0f; }
+                            if (!(tau[k] > 0.0f)) life[k] = min(life[k], steps);
+                        }
+                        live = live || tau[k] > 0.0f;
+                    }
+                    if (!__any_sync(FULL, live)) break;
+                    // diffuse reflection from the wall point
+                    const float ta_ = w.t / w.dtA, tb_ = w.t / w.dtB;
+                    fa0 = w.dA > 0 ? fa0 + (ta_ - w.nA) : fa0 - (ta_ - w.nA);
+                    fb0 = w.dB > 0 ? fb0 + (tb_ - w.nB) : fb0 - (tb_ - w.nB);
+                    fa0 = fminf(fmaxf(fa0, 0.0f), 1.0f);
+                    fb0 = fminf(fmaxf(fb0, 0.0f), 1.0f);
+                    w.oW = side == 0 ? __ldg(P.fw) : __ldg(P.fw + P.nw);
+                    draw();  // this event's words: the reflected direction only
+                    const float cmu = sqrtf(u24(evx.z));
+                    const float smu = sqrtf(fmaxf(0.0f, 1.0f - cmu * cmu));
+                    float cp, sp;
+                    mc_sincos_turn(evx.w >> 8, &cp, &sp);
+                    sW = side == 0 ? cmu : -cmu;
+                    sA = smu * cp;
+                    sB = smu * sp;
+                    restart();
+                    if (sigbar > 0.0f) { draw(); tcol = mc_neglog(u24o(evx.x)) / sigbar; }
+                    if (steps >= P.max_steps) {
+                        if (live) flags |= DNSMC_STATUS_STEP_CAP;
+                        break;
+                    }
+                } else if (steps >= P.max_steps || (n == 0 && end != WALK_COL)) {
+                    // the step cap, or no walk through these faces
+                    if (tau[0] > 0.0f || tau[1] > 0.0f) flags |= DNSMC_STATUS_STEP_CAP;
+                    break;
+                }
+                // the cell the walk is in now
+                const unsigned c0 = ((unsigned)w.cw * P.pnb + w.cb) * P.pna + w.ca;
+#pragma unroll
+                for (int k = 0; k < C; ++k) va[k] = __ldg(fp[k] + c0);
+                if (end == WALK_COL) {
+                    // tentative collision: a step to it, then the shared
+                    // decision with per-cell weights
+                    if (TRACE && lane == 0 && steps < P.trace_max) {
+                        int *rec = P.trace_rec + 6 * steps;
+                        rec[0] = w.cw; rec[1] = w.dA * (int)w.nA; rec[2] = w.dB * (int)w.nB; rec[3] = 3;
+                        rec[4] = __float_as_int(tcol - w.t);
+                    }
+                    step(va, w.t - tcol, steps);
+                    w.t = tcol;
+                    ++steps;
                     float pl[C];
                     float ps = 0.0f, pc = 0.0f;
 #pragma unroll
                     for (int k = 0; k < C; ++k) {
-                        pl[k] = tau[k] > 0.0f ? fminf(1.0f, fvcur[k] * psc / sigbar) : 0.0f;
+                        const float fv = gen_fraction(va[k]);
+                        pl[k] = tau[k] > 0.0f ? fminf(1.0f, fv * psc / sigbar) : 0.0f;
                         ps = k == 0 ? pl[k] : ps + pl[k];
                         pc = k == 0 ? (tau[k] > 0.0f ? 1.0f : 0.0f) : pc + (tau[k] > 0.0f ? 1.0f : 0.0f);
                     }
@@ -1051,58 +1065,49 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                         pc += __shfl_xor_sync(FULL, pc, o);
                     }
                     const float q = pc > 0.0f ? ps / pc : 0.0f;
-                    if (u24(evx.y) < q) {
+                    const bool scatter = u24(evx.y) < q;
 #pragma unroll
-                        for (int k = 0; k < C; ++k)
-                            if (tau[k] > 0.0f) tau[k] = tau[k] * (pl[k] / q);
-                        const float ta_ = t / dtA, tb_ = t / dtB;
-                        fa0 = dA > 0 ? fa0 + (ta_ - (float)nA) : fa0 - (ta_ - (float)nA);
-                        fb0 = dB > 0 ? fb0 + (tb_ - (float)nB) : fb0 - (tb_ - (float)nB);
+                    for (int k = 0; k < C; ++k)
+                        if (tau[k] > 0.0f) {
+                            tau[k] = tau[k] * (scatter ? pl[k] / q : (1.0f - pl[k]) / (1.0f - q));
+                            if (!(tau[k] > 0.0f)) life[k] = min(life[k], steps);
+                        }
+                    float t0 = w.t;  // the next collision's time counts from here
+                    if (scatter) {
+                        const float ta_ = w.t / w.dtA, tb_ = w.t / w.dtB;
+                        fa0 = w.dA > 0 ? fa0 + (ta_ - w.nA) : fa0 - (ta_ - w.nA);
+                        fb0 = w.dB > 0 ? fb0 + (tb_ - w.nB) : fb0 - (tb_ - w.nB);
                         fa0 = fminf(fmaxf(fa0, 0.0f), 1.0f);
                         fb0 = fminf(fmaxf(fb0, 0.0f), 1.0f);
-                        pw0 = fminf(fmaxf(fmaf(sW, t, pw0), __ldg(P.fw + cw)), __ldg(P.fw + cw + 1));
+                        w.oW = fminf(fmaxf(fmaf(sW, w.t, w.oW), __ldg(P.fw + w.cw)), __ldg(P.fw + w.cw + 1));
                         hg_scatter(P.hg_g, evx.z, evx.w, &sW, &sA, &sB);
-                        dda_init();
-                        t = 0.0f;
-                    } else {
-#pragma unroll
-                        for (int k = 0; k < C; ++k)
-                            if (tau[k] > 0.0f) tau[k] = tau[k] * ((1.0f - pl[k]) / (1.0f - q));
+                        restart();
+                        t0 = 0.0f;
                     }
                     draw();
-                    tcol = t + mc_neglog(u24o(evx.x)) / sigbar;
-                }
-#pragma unroll
-                for (int k = 0; k < C; ++k) {
-                    vcur[k] = vnext[k];
-                    fvcur[k] = fvnext[k];
-                }
-                bool alive = false;
-#pragma unroll
-                for (int k = 0; k < C; ++k) alive = alive || tau[k] > 0.0f;
-                if (!__any_sync(FULL, alive)) break;
-                if (steps >= P.max_steps) {
-                    if (alive) flags |= DNSMC_STATUS_STEP_CAP;
-                    break;
+                    tcol = t0 + mc_neglog(u24o(evx.x)) / sigbar;
+                    if (!__any_sync(FULL, tau[0] > 0.0f || tau[1] > 0.0f)) break;
+                    if (steps >= P.max_steps) {
+                        if (tau[0] > 0.0f || tau[1] > 0.0f) flags |= DNSMC_STATUS_STEP_CAP;
+                        break;
+                    }
                 }
             }
+            if (dead) break;
+            // the walk's length: the steps of the cell that lived longest
+            steps = min(steps, __reduce_max_sync(FULL, max(life[0], life[1])));
             if (TRACE && lane == 0) *P.trace_n = steps;
+#pragma unroll
+            for (int k = 0; k < C; ++k) lsteps += active[k] ? (unsigned)min(life[k], steps) : 0u;
             isteps += (unsigned long long)steps;
-            // control variate: the ray's straight flight through the
-            // layer-mean medium, the same for both cells (same layer)
-            float Jbar = 0.0f, Aown = 0.0f, I0 = 0.0f;
-            if (CV) {
-                const long long srow = ((long long)f * P.n_samples + sid) * P.nw + w0;
-                I0 = __ldg(P.sur + srow).y;
-                surrogate_lookup(P.surtab + srow * (2 * kSurBins), sW_e, &Jbar, &Aown);
-            }
+            const float4 sur = CV ? batch->sur[rb] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
             for (int k = 0; k < C; ++k) {
                 float X = wk[k] * D[k];
                 if (CV) {
                     // Y_a: the ray through the layer-mean medium; Y_b: its own-layer part
-                    const float Ya = wk[k] * (Ii[k] - Jbar);
-                    const float Yb = wk[k] * (Aown * (Ii[k] - I0));
+                    const float Ya = wk[k] * (Ii[k] - sur.x);
+                    const float Yb = wk[k] * (sur.y * (Ii[k] - sur.z));
                     if (MOM && active[k]) {
                         const double xd = X, ya = Ya, yb = Yb;
                         mo[k][0] += xd; mo[k][1] += ya; mo[k][2] += yb;
@@ -1117,21 +1122,30 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                 if (active[k]) {
                     ++my_rays;
                     if (!isfinite(X)) flags |= DNSMC_STATUS_NONFINITE;
-                    tally_ray(P, X, m, M, reinterpret_cast<float2 *>(acc(0, k)), reinterpret_cast<float2 *>(acc(1, k)),
-                              reinterpret_cast<float2 *>(acc(2, k)));
+                    if (SPLIT) rayx[(long long)r * 64 + 32 * k] = X;
+                    else tally_ray(P, X, m, M, acc(0, k), acc(1, k), acc(2, k));
                 }
             }
+            m = P.sampler && m == M - 1 ? 0 : m + 1;
         }
         if (dead) break;  // the item's sums are incomplete; the solve fails
         my_steps += lsteps;
         if (TRACE) return;
+        if (SPLIT) {
+            if (P.item_steps && lane == 0) atomicAdd(P.item_steps + item, isteps);
+            if (unit_done(P, item, lane)) {
+#pragma unroll
+                for (int k = 0; k < C; ++k)
+                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays(P, rayx + 32 * k, K > 0 ? N : 0, M);
+            }
+            continue;
+        }
         if (P.item_steps && lane == 0) P.item_steps[item] = isteps;
 #pragma unroll
         for (int k = 0; k < C; ++k) {
             if (!active[k]) continue;
             const long long o = fg * P.region_cells + tcell[k];
-            P.tally[o] = make_double2(ff_value(*reinterpret_cast<const float2 *>(acc(0, k))),
-                                      ff_value(*reinterpret_cast<const float2 *>(acc(1, k))));
+            P.tally[o] = make_double2(ff_value(*acc(0, k)), ff_value(*acc(1, k)));
             if (MOM) {
                 double *out = P.moments + o * 9;
 #pragma unroll
@@ -1160,7 +1174,7 @@ template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT, bool GE
     static constexpr void (*fn)(const MarchParams) = march_pair_kernel<MODE, UNI, TRACE, CV, MOM, SPLIT>;
 };
 template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT> struct march_cells_kernel<MODE, UNI, TRACE, CV, MOM, SPLIT, true> {
-    static constexpr void (*fn)(const MarchParams) = march_gen_kernel<MODE, TRACE, CV, MOM>;
+    static constexpr void (*fn)(const MarchParams) = march_gen_kernel<MODE, TRACE, CV, MOM, SPLIT>;
 };
 
 template <bool GEN>
@@ -1168,14 +1182,14 @@ int launch_march_cells(int mode, const MarchParams &p, int blocks, int threads, 
                        bool mom) {
     cudaStream_t st = (cudaStream_t)stream;
     if (trace) { blocks = 1; threads = 32; mom = false; }
-    const size_t smem = GEN ? march_smem(p, threads, kLaneCells) : march_pair_smem(p, threads);
+    const size_t smem = march_pair_smem(p, threads);
 #define DNSMC_L(M, U, T, CV_, O, S) \
     return march_launch_one(march_cells_kernel<M, U, T, CV_, O, S, GEN>::fn, blocks, threads, smem, st, p)
 #define DNSMC_MODE(M, U)                                                                                \
     if (trace) { if (cv) DNSMC_L(M, U, true, true, false, false); else DNSMC_L(M, U, true, false, false, false); } \
     else if (cv && mom) DNSMC_L(M, U, false, true, true, false);                                        \
-    else if (!GEN && p.parts > 1) {                                                                     \
-        if (cv) DNSMC_L(M, U, false, true, false, !GEN); else DNSMC_L(M, U, false, false, false, !GEN); \
+    else if (p.parts > 1) {                                                                             \
+        if (cv) DNSMC_L(M, U, false, true, false, true); else DNSMC_L(M, U, false, false, false, true); \
     } else if (cv) DNSMC_L(M, U, false, true, false, false);                                            \
     else DNSMC_L(M, U, false, false, false, false);
     switch (mode) {

@@ -114,3 +114,51 @@ def test_split_items_match_the_replay(size, groups, rays, sampler):
     c = s.counters()
     assert c.rays == ni * nj * nk * groups * rays
     s.close()
+
+
+# kind, (ni, nj, nk), albedo scale of the particles, overrides, region
+GEN_CASES = [
+    ("grey", (9, 3, 2), 1.0, dict(kappa=0.05, eps_east=0.3), None),
+    ("grey", (40, 5, 11), 0.1, dict(kappa=0.02, max_steps=65), None),
+    ("grey", (60, 8, 8), 0.0, dict(kappa=0.05, eps_west=0.2, eps_east=0.2), None),       # no scattering: reflections only
+    ("T", (17, 33, 9), 5.0, dict(eps_west=0.9, tile_a=16, max_steps=40), (1, 16, 3, 31, 0, 9)),
+    ("TX", (70, 6, 9), 0.3, dict(toll=1e-5), None),
+    ("TX", (13, 26, 19), 1.0, dict(stretched_x=1, n_groups=2, local_sampling=1, control_variate=1, cv_moments=1), None),
+    ("TX", (48, 64, 40), 1.0, dict(n_groups=8, eps_west=0.8), None),                     # a unit per item
+]
+
+
+@pytest.mark.parametrize("kind,size,albedo,kw,region", GEN_CASES)
+def test_general_medium_walks_match_the_replay(kind, size, albedo, kw, region):
+    """Chunks that end at collisions, walls and caps; restarts from any point of
+    a cell; packed fields with the volume fraction; split and whole items."""
+    from test_gpu_scatter import check_bitexact, particle_table
+    ni, nj, nk = size
+    cfg = dict(model=D.MODEL_GREY if kind == "grey" else D.MODEL_TABLE, imax=ni, jmax=nj, kmax=nk, Lx=1.5, Ly=2.0, Lz=0.7,
+               stretched_x=0, T_west=500.0, T_east=700.0, seed=77, sampler=D.SAMPLER_RQMC, nvar=2)
+    cfg.update(kw)
+    s = D.Solver(D.default_config(**cfg))
+    T, x, nb = smooth_field(ni, nj, nk, 600, 1500, 3), None, 1
+    rng = np.random.default_rng(5)
+    if kind != "grey":
+        t = synth.ck_table(nbands=8, nq=4, nT=24, nX=4, seed=5)
+        nb = 8
+        if kind == "T":
+            s.set_table(t["k"][..., 2] * 0.05, t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"])
+        else:
+            s.set_table(t["k"] * 0.05, t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"], X0=t["X0"], dX=t["dX"])
+            x = (0.12 + 0.05 * rng.uniform(-1, 1, T.shape)).astype(np.float32)
+    s.set_fields(T, x)
+    a, sc = particle_table(nb)
+    fv = rng.uniform(0.0, 2e-5, T.shape).astype(np.float32)
+    s.set_particles(a, sc * albedo, -0.3)
+    s.set_particle_field(fv)
+    if region:
+        s.set_region(*region)
+    s.set_rays(2 if ni * nj * nk > 1e5 else 10)
+    status = s.status
+    if "max_steps" in kw:
+        s.status = lambda: status() & ~D.STATUS_STEP_CAP
+    check_bitexact(s, T[None], None if x is None else x[None], fv[None])
+    assert status() == (D.STATUS_STEP_CAP if "max_steps" in kw else 0)
+    s.close()
