@@ -21,11 +21,10 @@
 // with GELU (tanh form), BF16 weights and activations, FP32 accumulation on
 // the fifth-generation tensor cores (tcgen05.mma, accumulators in tensor
 // memory; mc_cvnet_tc.cuh): the forward pass (inference with the features
-// and the coefficient epilogue fused in; training with its saves) and the
-// backward GEMMs.  Training: a loss kernel writes dL/dout; the backward pass
-// runs dW = dZ^T H (split over the batch with a deterministic reduction) and
-// dH = dZ W with the GELU derivative fused, and Adam updates FP32 master
-// weights.
+// and the coefficient epilogue fused in) and the training step
+// (mc_cvnet_train.cuh: forward, loss and input gradients of a tile in one
+// kernel; dW = dZ^T H split over the batch with a deterministic reduction;
+// Adam on FP32 master weights).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -186,151 +185,7 @@ __global__ void features_kernel(const FeatParams P) {
     }
 }
 
-struct GemmParams {
-    int M, N, K, klen;        // klen: K range per split
-    const bf16 *A;
-    long long a_sm, a_sk;
-    const bf16 *B;
-    long long b_sk, b_sn;
-    float *C;                 // partials [split][M][N]
-    const float *Z;           // [M][N] pre-activation for the fused GELU' epilogue
-    bf16 *D;                  // [M][N]
-};
-
-// grad[off + e] = sum over splits of partials (fixed order)
-__global__ void reduce_splits_kernel(const float *part, int splits, long long n, float *grad) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        for (int z = 0; z < splits; ++z) s += part[z * n + e];
-        grad[e] = s;
-    }
-}
-
-// db[n] = sum over rows of dZ[row][n]; one block per column, fixed tree order
-__global__ void colsum_kernel(const bf16 *dZ, long long rows, int ncol, float *db) {
-    __shared__ float red[256];
-    const int n = blockIdx.x;
-    float s = 0.0f;
-    for (long long r = threadIdx.x; r < rows; r += blockDim.x) s += __bfloat162float(dZ[r * ncol + n]);
-    red[threadIdx.x] = s;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) db[n] = red[0];
-}
-
-// ---------------------------------------------------------------------------
-// Loss: per row and band-group slot g < G
-//   beta loss  (V(beta) + ridge (Caa da^2 + Cbb db^2)) / S_beta
-//   var loss   (v / S_v) exp(-o_v) + o_v     (minimiser: o_v = log E[v / S_v])
-//   cost loss  (c / S_c) exp(-o_c) + o_c
-// mean over rows; dOut = d(mean)/d out, written as bf16.
-// ---------------------------------------------------------------------------
-struct LossParams {
-    long long rows, nvalid;
-    int G;
-    const float *out;         // [rows][NOUT]
-    const float *lab;         // [*][G][NLAB]
-    const int *idx;           // row r -> label row idx[r]
-    float Sbeta, Sv, Sc, ridge;
-    bf16 *dout;               // [rows][NOUT]
-    double *part;             // per block: beta, var, cost loss sums
-};
-
 __device__ __forceinline__ float clampo(float o) { return fminf(fmaxf(o, -15.0f), 15.0f); }
-
-__global__ void loss_kernel(const LossParams L) {
-    __shared__ double red[3][256];
-    double lb = 0.0, lv = 0.0, lc = 0.0;
-    const float inv = 1.0f / (float)max(1LL, L.nvalid);
-    for (long long r = blockIdx.x * (long long)blockDim.x + threadIdx.x; r < L.rows;
-         r += (long long)gridDim.x * blockDim.x) {
-        float d[NOUT];
-#pragma unroll
-        for (int q = 0; q < NOUT; ++q) d[q] = 0.0f;
-        if (r < L.nvalid) {
-            const long long lr = L.idx ? (long long)L.idx[r] : r;
-            for (int g = 0; g < L.G; ++g) {
-                const float *y = L.lab + (lr * L.G + g) * NLAB;
-                const float *o = L.out + r * NOUT + 4 * g;
-                const float Cxx = y[0], Caa = y[1], Cbb = y[2], Cxa = y[3], Cxb = y[4], Cab = y[5];
-                const float da = o[0], db = o[1];
-                const float ba = 1.0f + da, bb = -1.0f + db;
-                const float V = Cxx - 2.0f * ba * Cxa - 2.0f * bb * Cxb + ba * ba * Caa + 2.0f * ba * bb * Cab +
-                                bb * bb * Cbb;
-                lb += (double)((V + L.ridge * (Caa * da * da + Cbb * db * db)) / L.Sbeta);
-                d[4 * g + 0] = (2.0f * (ba * Caa + bb * Cab - Cxa) + 2.0f * L.ridge * Caa * da) / L.Sbeta * inv;
-                d[4 * g + 1] = (2.0f * (bb * Cbb + ba * Cab - Cxb) + 2.0f * L.ridge * Cbb * db) / L.Sbeta * inv;
-                if (y[6] > 0.0f) {
-                    const float ov = clampo(o[2]), e = y[6] / L.Sv * expf(-ov);
-                    lv += (double)(e + ov);
-                    d[4 * g + 2] = (1.0f - e) * inv;
-                }
-                if (y[7] > 0.0f) {
-                    const float oc = clampo(o[3]), e = y[7] / L.Sc * expf(-oc);
-                    lc += (double)(e + oc);
-                    d[4 * g + 3] = (1.0f - e) * inv;
-                }
-            }
-        }
-        uint32_t *dst = reinterpret_cast<uint32_t *>(L.dout + r * NOUT);
-#pragma unroll
-        for (int q = 0; q < NOUT / 2; ++q) dst[q] = pack_bf16(d[2 * q], d[2 * q + 1]);
-    }
-    red[0][threadIdx.x] = lb; red[1][threadIdx.x] = lv; red[2][threadIdx.x] = lc;
-    __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w)
-            for (int q = 0; q < 3; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0)
-        for (int q = 0; q < 3; ++q) L.part[blockIdx.x * 3 + q] = red[q][0];
-}
-
-// Adam on the FP32 master copy; bf16 copy of the weights.
-__global__ void adam_kernel(float *p, const float *grad, float *m, float *v, bf16 *w, long long n, float lr, float b1,
-                            float b2, float eps, float c1, float c2) {
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        const float gr = grad[e];
-        const float mm = b1 * m[e] + (1.0f - b1) * gr;
-        const float vv = b2 * v[e] + (1.0f - b2) * gr * gr;
-        m[e] = mm;
-        v[e] = vv;
-        const float upd = lr * (mm / c1) / (sqrtf(vv / c2) + eps);
-        p[e] -= upd;
-    }
-}
-
-// bf16 copies of the weight blocks of the master array: w[0, NWEIGHT) row
-// major per matrix ([out][in], the warp-level kernels), w[NWEIGHT, 2 NWEIGHT)
-// in the tensor-core order [in/8][out][8] of the tcgen05 forward (the same
-// block offsets)
-__host__ __device__ __forceinline__ long long tc_order(long long e) {
-    long long off, rows, cols;
-    if (e < WOFF_2) { off = WOFF_1; rows = HID; cols = K0; }
-    else if (e < WOFF_3) { off = WOFF_2; rows = HID; cols = HID; }
-    else if (e < WOFF_4) { off = WOFF_3; rows = HID; cols = HID; }
-    else { off = WOFF_4; rows = NOUT; cols = HID; }
-    const long long q = e - off, n = q / cols, k = q % cols;
-    return off + (k >> 3) * rows * 8 + n * 8 + (k & 7);
-}
-
-__global__ void weights_to_bf16_kernel(const float *p, bf16 *w) {
-    const long long n = NWEIGHT;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x) {
-        long long src;
-        if (e < WOFF_2) src = OFF_W1 + e;
-        else if (e < WOFF_3) src = OFF_W2 + (e - WOFF_2);
-        else if (e < WOFF_4) src = OFF_W3 + (e - WOFF_3);
-        else src = OFF_W4 + (e - WOFF_4);
-        const bf16 v = __float2bfloat16(p[src]);
-        w[e] = v;
-        w[NWEIGHT + tc_order(e)] = v;
-    }
-}
 
 // ---------------------------------------------------------------------------
 // Training labels from a solve with per-ray moments: per (row = region cell in
@@ -403,6 +258,7 @@ struct ApplyParams {
 
 }  // namespace
 #include "mc_cvnet_tc.cuh"
+#include "mc_cvnet_train.cuh"
 namespace {
 
 struct AllocParams {
@@ -553,7 +409,7 @@ struct dnsmc_cvnet {
     long long cap_rows = 0;
     NBuf<int> idx;
     NBuf<bf16> H0, H1, H2, H3, dO, dZ3, dZ2, dZ1;
-    NBuf<float> Z1, Z2, Z3, out, part;
+    NBuf<float> part;
     NBuf<double> lpart;
     // inference
     NBuf<bf16> iX;
@@ -567,7 +423,7 @@ struct dnsmc_cvnet {
     ~dnsmc_cvnet() {
         P.release(); grad.release(); m.release(); v.release(); W.release(); dX.release(); dlab.release();
         idx.release(); H0.release(); H1.release(); H2.release(); H3.release(); dO.release(); dZ3.release();
-        dZ2.release(); dZ1.release(); Z1.release(); Z2.release(); Z3.release(); out.release(); part.release();
+        dZ2.release(); dZ1.release(); part.release();
         lpart.release(); iX.release(); iout.release(); vc.release(); wgt.release(); cost.release(); lam.release();
         lam_part.release(); lam_done.release();
         status.release();
@@ -594,7 +450,7 @@ int launch_forward_tc(TcParams &F, dnsmc_cvnet *n, cudaStream_t st) {
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int blocks = (int)std::max(1LL, std::min((long long)sms, (tiles + TC_WG - 1) / TC_WG));
-    F.Wtc = n->W.p + NWEIGHT;
+    F.Wtc = n->W.p;
     F.P = n->P.p;
     F.status = n->status.p;
     dnsmc::note_launch();
@@ -605,107 +461,58 @@ int launch_forward_tc(TcParams &F, dnsmc_cvnet *n, cudaStream_t st) {
 
 int ensure_work(dnsmc_cvnet *n, long long rows) {
     if (rows <= n->cap_rows) return DNSMC_OK;
-    RTRY(n->idx.ensure(rows)); RTRY(n->H0.ensure(rows * K0));
+    RTRY(n->H0.ensure(rows * K0));
     RTRY(n->H1.ensure(rows * HID)); RTRY(n->H2.ensure(rows * HID)); RTRY(n->H3.ensure(rows * HID));
-    RTRY(n->Z1.ensure(rows * HID)); RTRY(n->Z2.ensure(rows * HID)); RTRY(n->Z3.ensure(rows * HID));
     RTRY(n->dZ1.ensure(rows * HID)); RTRY(n->dZ2.ensure(rows * HID)); RTRY(n->dZ3.ensure(rows * HID));
-    RTRY(n->out.ensure(rows * NOUT)); RTRY(n->dO.ensure(rows * NOUT));
+    RTRY(n->dO.ensure(rows * NOUT));
     n->cap_rows = rows;
     return DNSMC_OK;
 }
 
-// dW (M=nout x N=nin) = dZ^T H over rows, split over the rows; db = colsum(dZ)
-int launch_gemm_tc(const GemmParams &G, dim3 grid, dnsmc_cvnet *n) {
-    static int attr = 0;
-    if (!attr) {
-        CK(cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GT_SMEM));
-        attr = 1;
-    }
-    dnsmc::note_launch();
-    gemm_tc_kernel<<<grid, 128, GT_SMEM, n->stream>>>(G, n->status.p);
-    CK(cudaGetLastError());
-    return DNSMC_OK;
-}
-
-int weight_grad(dnsmc_cvnet *n, const bf16 *dZ, int nout, const bf16 *H, int nin, long long rows, long long offW,
-                long long offB) {
-    const int splits = (int)std::min<long long>(64, std::max<long long>(1, rows / 256));
-    const int klen = (int)(((rows + splits - 1) / splits + GT_K - 1) / GT_K * GT_K);
-    RTRY(n->part.ensure((size_t)splits * nout * nin));
-    GemmParams G{};
-    G.M = nout; G.N = nin; G.K = (int)rows; G.klen = klen;
-    G.A = dZ; G.a_sm = 1; G.a_sk = nout;
-    G.B = H; G.b_sk = nin; G.b_sn = 1;
-    G.C = n->part.p;
-    RTRY(launch_gemm_tc(G, dim3((nout + 127) / 128, (nin + 127) / 128, splits), n));
-    dnsmc::note_launch();
-    reduce_splits_kernel<<<grid1((long long)nout * nin, 256), 256, 0, n->stream>>>(n->part.p, splits,
-                                                                                   (long long)nout * nin,
-                                                                                   n->grad.p + offW);
-    CK(cudaGetLastError());
-    dnsmc::note_launch();
-    colsum_kernel<<<nout, 256, 0, n->stream>>>(dZ, rows, nout, n->grad.p + offB);
-    CK(cudaGetLastError());
-    return DNSMC_OK;
-}
-
-// dZprev (rows x nin) = (dZ W) * gelu'(Zprev)
-int input_grad(dnsmc_cvnet *n, const bf16 *dZ, int nout, long long woff, int nin, long long rows, const float *Zprev,
-               bf16 *dZprev) {
-    GemmParams G{};
-    G.M = (int)rows; G.N = nin; G.K = nout; G.klen = nout;
-    G.A = dZ; G.a_sm = nout; G.a_sk = 1;
-    G.B = n->W.p + woff; G.b_sk = nin; G.b_sn = 1;
-    G.Z = Zprev; G.D = dZprev;
-    return launch_gemm_tc(G, dim3((unsigned)((rows + 127) / 128), (nin + 127) / 128, 1), n);
-}
-
-// forward + loss + backward on `rows` rows (nvalid real) of X/lab through idx
-int fwd_bwd(dnsmc_cvnet *n, const bf16 *X, const float *lab, int G, const int *idx, long long rows, long long nvalid,
-            double loss[3]) {
+// Forward, loss, backward (and with `adam` the update) on `rows` rows (a
+// multiple of 128, nvalid real) of X/lab through idx; the tiles' loss sums go
+// to `loss` ([rows / 128][3], device).
+int train_step(dnsmc_cvnet *n, const bf16 *X, const float *lab, int G, const int *idx, long long rows, long long nvalid,
+               double *loss, bool adam) {
     RTRY(ensure_work(n, rows));
-    TcParams F{};
-    F.rows = rows; F.X = X; F.idx = idx; F.nvalid = nvalid; F.out = n->out.p;
-    F.H0 = n->H0.p; F.Z1 = n->Z1.p; F.Z2 = n->Z2.p; F.Z3 = n->Z3.p; F.H1 = n->H1.p; F.H2 = n->H2.p; F.H3 = n->H3.p;
-    RTRY(launch_forward_tc(F, n, n->stream));
-    LossParams L{};
-    L.rows = rows; L.nvalid = nvalid; L.G = G; L.out = n->out.p; L.lab = lab; L.idx = idx;
-    L.Sbeta = n->Sbeta; L.Sv = n->Sv; L.Sc = n->Sc; L.ridge = n->cfg.ridge; L.dout = n->dO.p;
-    const int lblocks = grid1(rows, 256);
-    RTRY(n->lpart.ensure((size_t)lblocks * 3));
-    L.part = n->lpart.p;
+    TrainParams F{};
+    F.rows = rows; F.nvalid = nvalid; F.X = X; F.lab = lab; F.idx = idx; F.G = G;
+    F.Sbeta = n->Sbeta; F.Sv = n->Sv; F.Sc = n->Sc; F.ridge = n->cfg.ridge;
+    F.W = n->W.p; F.P = n->P.p;
+    F.H0 = n->H0.p; F.H1 = n->H1.p; F.H2 = n->H2.p; F.H3 = n->H3.p;
+    F.dO = n->dO.p; F.dZ3 = n->dZ3.p; F.dZ2 = n->dZ2.p; F.dZ1 = n->dZ1.p;
+    F.part = loss; F.status = n->status.p;
+    int sms = 152;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device);
+    CK(cudaFuncSetAttribute(train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
     dnsmc::note_launch();
-    loss_kernel<<<lblocks, 256, 0, n->stream>>>(L);
+    train_tile_kernel<<<(unsigned)std::min<long long>(rows / TC_TILE, sms), TR_THREADS, TR_SMEM, n->stream>>>(F);
     CK(cudaGetLastError());
-    RTRY(weight_grad(n, n->dO.p, NOUT, n->H3.p, HID, rows, OFF_W4, OFF_B4));
-    RTRY(input_grad(n, n->dO.p, NOUT, WOFF_4, HID, rows, n->Z3.p, n->dZ3.p));
-    RTRY(weight_grad(n, n->dZ3.p, HID, n->H2.p, HID, rows, OFF_W3, OFF_B3));
-    RTRY(input_grad(n, n->dZ3.p, HID, WOFF_3, HID, rows, n->Z2.p, n->dZ2.p));
-    RTRY(weight_grad(n, n->dZ2.p, HID, n->H1.p, HID, rows, OFF_W2, OFF_B2));
-    RTRY(input_grad(n, n->dZ2.p, HID, WOFF_2, HID, rows, n->Z1.p, n->dZ1.p));
-    RTRY(weight_grad(n, n->dZ1.p, HID, n->H0.p, K0, rows, OFF_W1, OFF_B1));
-    if (loss) {
-        std::vector<double> h((size_t)lblocks * 3);
-        CK(cudaMemcpyAsync(h.data(), n->lpart.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, n->stream));
-        CK(cudaStreamSynchronize(n->stream));
-        loss[0] = loss[1] = loss[2] = 0.0;
-        for (int b = 0; b < lblocks; ++b)
-            for (int q = 0; q < 3; ++q) loss[q] += h[(size_t)b * 3 + q];
+    WgradParams Wp{};
+    Wp.rows = rows;
+    Wp.splits = (int)std::min<long long>(64, std::max<long long>(1, rows / 256));
+    Wp.klen = (int)(((rows + Wp.splits - 1) / Wp.splits + 63) / 64 * 64);
+    RTRY(n->part.ensure((size_t)wg_part(3, Wp.splits) + (size_t)Wp.splits * NOUT * HID));
+    Wp.part = n->part.p;
+    const bf16 *dZ[4] = {n->dZ1.p, n->dZ2.p, n->dZ3.p, n->dO.p}, *H[4] = {n->H0.p, n->H1.p, n->H2.p, n->H3.p};
+    for (int l = 0; l < 4; ++l) { Wp.dZ[l] = dZ[l]; Wp.H[l] = H[l]; }
+    CK(cudaFuncSetAttribute(train_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM));
+    dnsmc::note_launch();
+    train_wgrad_kernel<<<dim3((unsigned)Wp.splits, 4), WG_THREADS, WG_SMEM, n->stream>>>(Wp, n->status.p);
+    CK(cudaGetLastError());
+    UpdateParams U{};
+    U.part = n->part.p; U.splits = Wp.splits; U.rows = rows;
+    for (int l = 0; l < 4; ++l) U.dZ[l] = dZ[l];
+    U.grad = n->grad.p; U.adam = adam ? 1 : 0;
+    U.p = n->P.p; U.m = n->m.p; U.v = n->v.p; U.w = n->W.p;
+    if (adam) {
+        n->step += 1;
+        U.lr = n->cfg.lr; U.b1 = n->cfg.adam_beta1; U.b2 = n->cfg.adam_beta2; U.eps = n->cfg.adam_eps;
+        U.c1 = 1.0f - powf(n->cfg.adam_beta1, (float)n->step);
+        U.c2 = 1.0f - powf(n->cfg.adam_beta2, (float)n->step);
     }
-    return DNSMC_OK;
-}
-
-int adam_step(dnsmc_cvnet *n) {
-    n->step += 1;
-    const float c1 = 1.0f - powf(n->cfg.adam_beta1, (float)n->step);
-    const float c2 = 1.0f - powf(n->cfg.adam_beta2, (float)n->step);
     dnsmc::note_launch();
-    adam_kernel<<<grid1(NPARAM, 256), 256, 0, n->stream>>>(n->P.p, n->grad.p, n->m.p, n->v.p, n->W.p, NPARAM,
-                                                            n->cfg.lr, n->cfg.adam_beta1, n->cfg.adam_beta2,
-                                                            n->cfg.adam_eps, c1, c2);
-    CK(cudaGetLastError());
-    dnsmc::note_launch();
-    weights_to_bf16_kernel<<<grid1(NWEIGHT, 256), 256, 0, n->stream>>>(n->P.p, n->W.p);
+    train_update_kernel<<<WU_WBLOCKS + WU_BBLOCKS, WU_THREADS, 0, n->stream>>>(U);
     CK(cudaGetLastError());
     return DNSMC_OK;
 }
@@ -804,7 +611,7 @@ int dnsmc_cvnet_create(const dnsmc_cvnet_config *cfg, dnsmc_cvnet **out) {
     if (!rc) rc = n->grad.ensure(NPARAM);
     if (!rc) rc = n->m.ensure(NPARAM);
     if (!rc) rc = n->v.ensure(NPARAM);
-    if (!rc) rc = n->W.ensure(2 * NWEIGHT);  // row-major and tensor-core order
+    if (!rc) rc = n->W.ensure(NWEIGHT_ALL);  // tensor-core order, then the transposes
     if (!rc) rc = n->status.ensure(1);
     if (!rc && (e = cudaMemset(n->status.p, 0, sizeof(unsigned int))) != cudaSuccess) rc = cuda_fail("cudaMemset", e);
     if (!rc) rc = init_params(n);
@@ -984,30 +791,28 @@ int dnsmc_cvnet_train(dnsmc_cvnet *n, int epochs, double *loss) {
     if (epochs < 1) return arg_fail("epochs must be >= 1");
     if (n->nrows < 1) return state_fail("no training data");
     RTRY(set_dev(n));
-    const long long B = n->cfg.batch;
+    const long long B = n->cfg.batch, steps = (n->nrows + B - 1) / B, tiles = B / TC_TILE;
     RTRY(ensure_work(n, B));
+    RTRY(n->idx.ensure((size_t)n->nrows));
+    RTRY(n->lpart.ensure((size_t)(steps * tiles * 3)));
     std::vector<int> perm((size_t)n->nrows);
-    double acc[3] = {0, 0, 0};
-    long long nb = 0;
     for (int ep = 0; ep < epochs; ++ep) {
         for (long long i = 0; i < n->nrows; ++i) perm[(size_t)i] = (int)i;
         std::shuffle(perm.begin(), perm.end(), n->rng);
-        for (long long b0 = 0; b0 < n->nrows; b0 += B) {
-            const long long nv = std::min(B, n->nrows - b0);
-            CK(cudaMemcpyAsync(n->idx.p, perm.data() + b0, nv * sizeof(int), cudaMemcpyHostToDevice, n->stream));
-            double l[3];
-            const bool last = (ep == epochs - 1);
-            RTRY(fwd_bwd(n, n->dX.p, n->dlab.p, n->dG, n->idx.p, B, nv, last ? l : nullptr));
-            RTRY(adam_step(n));
-            if (last) {
-                for (int q = 0; q < 3; ++q) acc[q] += l[q];
-                nb += nv;
-            }
-        }
+        // the whole pass is enqueued at once; the loss sums of its steps are
+        // read at the end (those of the last pass)
+        CK(cudaMemcpyAsync(n->idx.p, perm.data(), (size_t)n->nrows * sizeof(int), cudaMemcpyHostToDevice, n->stream));
+        for (long long q = 0; q < steps; ++q)
+            RTRY(train_step(n, n->dX.p, n->dlab.p, n->dG, n->idx.p + q * B, B, std::min(B, n->nrows - q * B),
+                            n->lpart.p + q * tiles * 3, true));
     }
+    std::vector<double> h((size_t)(steps * tiles * 3));
+    CK(cudaMemcpyAsync(h.data(), n->lpart.p, h.size() * sizeof(double), cudaMemcpyDeviceToHost, n->stream));
     CK(cudaStreamSynchronize(n->stream));
     if (loss) {
-        for (int q = 0; q < 3; ++q) loss[q + 1] = nb ? acc[q] / nb : 0.0;
+        double acc[3] = {0, 0, 0};
+        for (size_t e = 0; e < h.size(); ++e) acc[e % 3] += h[e];
+        for (int q = 0; q < 3; ++q) loss[q + 1] = acc[q] / n->nrows;
         loss[0] = loss[1] + loss[2] + loss[3];
     }
     return DNSMC_OK;
@@ -1024,7 +829,7 @@ int dnsmc_cvnet_eval(dnsmc_cvnet *n, const float *features, long long rows, floa
     RTRY(n->iout.ensure((size_t)rows * NOUT));
     CK(cudaMemcpyAsync(n->iX.p, h.data(), h.size() * sizeof(bf16), cudaMemcpyHostToDevice, n->stream));
     TcParams F{};
-    F.rows = rows; F.X = n->iX.p; F.nvalid = rows; F.out = n->iout.p;
+    F.rows = rows; F.X = n->iX.p; F.out = n->iout.p;
     RTRY(launch_forward_tc(F, n, n->stream));
     CK(cudaMemcpyAsync(out, n->iout.p, (size_t)rows * NOUT * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     unsigned int st = 0;
@@ -1050,11 +855,17 @@ int dnsmc_cvnet_gradient(dnsmc_cvnet *n, const float *features, const float *lab
     RTRY(lab.ensure((size_t)rows * n_groups * NLAB));
     CK(cudaMemcpy(x.p, h.data(), h.size() * sizeof(bf16), cudaMemcpyHostToDevice));
     CK(cudaMemcpy(lab.p, labels, (size_t)rows * n_groups * NLAB * sizeof(float), cudaMemcpyHostToDevice));
-    double l[3];
-    int rc = fwd_bwd(n, x.p, lab.p, n_groups, nullptr, R, rows, l);
+    double l[3] = {0, 0, 0};
+    const long long tiles = R / TC_TILE;
+    int rc = n->lpart.ensure((size_t)(tiles * 3));
+    if (!rc) rc = train_step(n, x.p, lab.p, n_groups, nullptr, R, rows, n->lpart.p, false);
     if (!rc) {
-        cudaError_t e = cudaMemcpy(grad, n->grad.p, NPARAM * sizeof(float), cudaMemcpyDeviceToHost);
+        std::vector<double> hl((size_t)(tiles * 3));
+        cudaError_t e = cudaStreamSynchronize(n->stream);
+        if (e == cudaSuccess) e = cudaMemcpy(grad, n->grad.p, NPARAM * sizeof(float), cudaMemcpyDeviceToHost);
+        if (e == cudaSuccess) e = cudaMemcpy(hl.data(), n->lpart.p, hl.size() * sizeof(double), cudaMemcpyDeviceToHost);
         if (e != cudaSuccess) rc = cuda_fail("cudaMemcpy", e);
+        for (size_t q = 0; q < hl.size(); ++q) l[q % 3] += hl[q];
     }
     x.release();
     lab.release();
