@@ -54,3 +54,25 @@ def test_generated_table_drives_a_solve():
     Q, S = s.solve(timeout_s=120)
     assert np.isfinite(Q).all() and np.abs(Q).max() > 0 and s.status() == 0
     s.close()
+
+
+@pytest.mark.parametrize("n_pwrk", [2, 3, 777, 10000, 50000])
+def test_bins_of_awkward_spectra(n_pwrk):
+    """Points are binned in FP32 where that decides the bin: bands that are flat
+    to 1e-13, that span sixty decades, hold zeros and subnormals, two points,
+    or lie beyond FP32's range, against the oracle (bounds as above)."""
+    rng = np.random.default_rng(4)
+    n = 4001
+    smooth = np.exp(3.0 * np.sin(np.linspace(0, 40, n)))
+    rows = [smooth, 0.3 * (1 + 1e-13 * rng.integers(0, 9, n)), 10.0 ** rng.uniform(-30, 30, n),
+            np.where(rng.random(n) < 0.2, 0.0, smooth), smooth * 1e-35, smooth * 1e-310, smooth * 1e60,
+            1.0 + 1e-5 * smooth, np.full(n, 2.5)]
+    k = np.stack(rows)[:, None, :]
+    spec = dict(kappa=k, wv0=1000.0, dwv=0.01, first=np.array([0, 1500, 3999], np.int64),
+                count=np.array([1501, 2500, 2], np.int32), wv_left=np.array([1000.0, 1015.0, 1039.99]),
+                wv_right=np.array([1015.0, 1040.0, 1040.0]))
+    gq, _ = synth.gauss_legendre_half(16)
+    kq, kavg = D.ck_from_lbl(spec, gq, n_pwrk=n_pwrk)
+    ko, ao = O.ck_from_lbl(spec, gq, n_pwrk=n_pwrk)
+    np.testing.assert_allclose(kq, ko, rtol=1e-5)
+    np.testing.assert_allclose(kavg, ao, rtol=1e-9)
