@@ -1432,7 +1432,10 @@ int field_stats_checked(dnsmc_solver *s, int nfields, bool with_x, double st[4])
     const dnsmc_config &c = s->cfg;
     const long long ncell = (long long)c.imax * c.jmax * c.kmax;
     TRY(s->d_stat_part.ensure(field_stats_partials()));
-    TRY(s->d_stat_out.ensure(4));
+    if (!s->d_stat_out.p) {
+        TRY(s->d_stat_out.ensure(5));
+        CUDA_TRY(cudaMemsetAsync(s->d_stat_out.p, 0, 5 * sizeof(double), s->stream));
+    }
     const int rc = launch_field_stats(with_x ? nullptr : s->d_fieldT.p, with_x ? s->d_fieldTX.p : nullptr,
                                       nfields * ncell, s->d_stat_part.p, s->d_stat_out.p, s->stream);
     if (rc) return fail(DNSMC_ERR_CUDA, "stats launch: %s", cudaGetErrorString((cudaError_t)rc));

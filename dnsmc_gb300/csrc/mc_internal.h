@@ -350,7 +350,8 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
                    int na, int nb, long long si, long long sj, long long sk,
                    long long base, void *stream);
 // max T, min T, sum x and the count of non-positive or non-finite T over n
-// cells into out[0..3] (device), deterministic
+// cells into out[0..3] (device), deterministic; out[4] is the kernel's counter
+// of finished blocks, zero before the first launch
 int launch_field_stats(const float *fT, const float2 *fTX, long long n,
                        double *partials, double *out, void *stream);
 int field_stats_partials();   // doubles needed in `partials`
