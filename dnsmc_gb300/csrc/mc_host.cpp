@@ -152,11 +152,11 @@ void coarse_faces(int im0, int l, float L, int stretched, std::vector<float> &xu
     for (int i = 0; i <= im; ++i) xu[i] = f[(size_t)i * im0 / im];
 }
 
-// centres c[1..n] of faces u[0..n] (1-based, as the splines below)
+// centres c[0..n-1] of faces u[0..n]
 void centres(const std::vector<float> &u, std::vector<float> &c) {
     const int n = (int)u.size() - 1;
-    c.assign(n + 2, 0.0f);
-    for (int i = 1; i <= n; ++i) c[i] = (u[i - 1] + u[i]) * 0.5f;
+    c.resize(n);
+    for (int i = 0; i < n; ++i) c[i] = (u[i] + u[i + 1]) * 0.5f;
 }
 
 void uniform_faces(int n, float L, std::vector<float> &u) {
@@ -280,7 +280,9 @@ struct dnsmc_solver {
 
     // multigrid: spline-coarsened temperatures of levels 1..grid_num-1
     DevBuf<float> d_mgT, d_mgfw;
-    DevBuf<float> d_mgpos, d_mgtmp;          // spline positions; coarsening passes' scratch
+    DevBuf<unsigned char> d_mgtab;           // splines: coefficients, brackets, positions
+    DevBuf<float> d_mgtmp;                   // coarsening passes' intermediate fields
+    DevBuf<double> d_mgwork;                 // lines too long for shared memory
     long long mg_off[kMaxLevels] = {0};
     int mg_fwoff[kMaxLevels] = {0};
     int mg_fields = 0;
@@ -1333,94 +1335,145 @@ int wait_done(dnsmc_solver *s, double timeout_s) {
     return DNSMC_OK;
 }
 
+// What the splines along one axis take from its positions alone (0-based; the
+// recurrence of code/spline.cpp:119-170 up to the values, and the bisection
+// for each coarse position).
+void spline_coefs(const std::vector<float> &x, SplineCoef *k) {
+    const int n = (int)x.size();
+    float y2 = 0.0f;
+    for (int e = 0; e < n; ++e) {
+        k[e] = SplineCoef{1.0, 1.0, 0.0f, 0.0f};
+        if (e == 0 || e == n - 1) continue;
+        const float sig = (x[e] - x[e - 1]) / (x[e + 1] - x[e - 1]);
+        const float p = sig * y2 + 2.0f;
+        y2 = (sig - 1.0f) / p;
+        k[e] = SplineCoef{1.0 / (double)p, (double)p, sig, y2};
+    }
+}
+void spline_brackets(const std::vector<float> &x, const std::vector<float> &v, SplineAt *at) {
+    for (size_t c = 0; c < v.size(); ++c) {
+        int lo = 0, hi = (int)x.size() - 1;
+        while (hi - lo > 1) {
+            const int k = (hi + lo + 2) / 2 - 1;  // the 1-based bisection's midpoint
+            if (x[k] > v[c]) hi = k; else lo = k;
+        }
+        const float h = x[hi] - x[lo];
+        at[c] = SplineAt{lo, (x[hi] - v[c]) / h, (v[c] - x[lo]) / h, h * h};
+    }
+}
+
 // Coarse temperatures of every field for the multigrid march: the spline
 // coarsening (interp3D) on the device from the packed fine temperatures
-// (src: [f][i][k][j], T every src_step floats), three passes per level and
-// field on the solver's stream; the coarse wall-normal faces of every level.
+// (src: [f][i][k][j], T every src_step floats), three passes for all levels
+// and as many fields as the scratch holds, on the solver's stream; the coarse
+// wall-normal faces of every level.
 int upload_coarse(dnsmc_solver *s, int nfields, const float *src, int src_step) {
     const dnsmc_config &c = s->cfg;
     const int G = c.grid_num;
     const int I = c.imax, J = c.jmax, K = c.kmax;
     const long long ncell = (long long)I * J * K;
-    long long off = 0;
+    long long off = 0, ntx = 0, ntxy = 0;
+    long long ox[kMaxLevels] = {}, oxy[kMaxLevels] = {};
     for (int l = 1; l < G; ++l) {
         s->mg_off[l] = off;
         off += (long long)nfields * (I >> l) * (J >> l) * (K >> l);
+        ox[l] = ntx; oxy[l] = ntxy;
+        ntx += (long long)(I >> l) * J * K;
+        ntxy += (long long)(I >> l) * (J >> l) * K;
     }
-    // cell-centre positions, 1-based: fine x, y, z, then per level coarse x, y, z
-    std::vector<float> xu, yu, zu, pos, cen;
-    make_faces(I, c.Lx, c.stretched_x, xu);
-    uniform_faces(J, c.Ly, yu);
-    uniform_faces(K, c.Lz, zu);
-    long long po[kMaxLevels][3] = {}, pf[3];
-    auto put = [&](const std::vector<float> &u) {
-        centres(u, cen);
-        const long long o = (long long)pos.size();
-        pos.insert(pos.end(), cen.begin(), cen.end());
-        return o;
-    };
-    pf[0] = put(xu); pf[1] = put(yu); pf[2] = put(zu);
-    std::vector<float> faces;
-    int fo = 0;
-    for (int l = 1; l < G; ++l) {
-        std::vector<float> cxu, cyu, czu;
-        coarse_faces(I, l, c.Lx, c.stretched_x, cxu);
-        uniform_faces(J >> l, c.Ly, cyu);
-        uniform_faces(K >> l, c.Lz, czu);
-        po[l][0] = put(cxu); po[l][1] = put(cyu); po[l][2] = put(czu);
-        s->mg_fwoff[l] = fo;
-        faces.insert(faces.end(), cxu.begin(), cxu.end());
-        fo += (int)cxu.size();
+    // tables of the three axes in one buffer: coefficients, brackets of every
+    // level, positions (16-byte parts first)
+    std::vector<float> u[3], cu;
+    make_faces(I, c.Lx, c.stretched_x, u[0]);
+    uniform_faces(J, c.Ly, u[1]);
+    uniform_faces(K, c.Lz, u[2]);
+    const int n[3] = {I, J, K};
+    size_t nco = 0, nat = 0, npos = 0, oco[3], opos[3], oat[kMaxLevels][3] = {};
+    for (int d = 0; d < 3; ++d) {
+        oco[d] = nco; nco += n[d];
+        opos[d] = npos; npos += n[d];
+        for (int l = 1; l < G; ++l) { oat[l][d] = nat; nat += n[d] >> l; }
     }
-    const int im1 = I >> 1, jm1 = J >> 1;
-    const long long ntmp = (long long)im1 * J * K + (long long)im1 * jm1 * K;  // level 1 is the largest
-    const long long nwork = 3 * std::max({(long long)(I + 2) * J * K, (long long)(J + 2) * im1 * K,
-                                          (long long)(K + 2) * im1 * jm1});
+    const size_t bat = nco * sizeof(SplineCoef), bpos = bat + nat * sizeof(SplineAt);
+    std::vector<unsigned char> tab(bpos + npos * sizeof(float));
+    std::vector<float> faces, fc, cc;
+    for (int d = 0; d < 3; ++d) {
+        centres(u[d], fc);
+        spline_coefs(fc, reinterpret_cast<SplineCoef *>(tab.data()) + oco[d]);
+        std::copy(fc.begin(), fc.end(), reinterpret_cast<float *>(tab.data() + bpos) + opos[d]);
+        for (int l = 1; l < G; ++l) {
+            if (d == 0) {
+                coarse_faces(I, l, c.Lx, c.stretched_x, cu);
+                s->mg_fwoff[l] = (int)faces.size();
+                faces.insert(faces.end(), cu.begin(), cu.end());
+            } else {
+                uniform_faces(n[d] >> l, d == 1 ? c.Ly : c.Lz, cu);
+            }
+            centres(cu, cc);
+            spline_brackets(fc, cc, reinterpret_cast<SplineAt *>(tab.data() + bat) + oat[l][d]);
+        }
+    }
+    // fields per pass: all, within 256 MB of intermediate values
+    const long long ntmp = ntx + ntxy;
+    const int chunk = (int)std::min<long long>(nfields, std::max<long long>(1, (256ll << 20) / (4 * ntmp)));
+    size_t nwork = 0;
+    for (int p = 0; p < 3; ++p) {
+        long long nl = 0;
+        for (int l = 1; l < G; ++l) nl += p == 1 ? (long long)(I >> l) * K : (long long)(I >> l) * (J >> l);
+        nwork = std::max(nwork, spline_work_doubles(n[p], p == 0 ? (long long)J * K : nl));
+    }
     TRY(s->d_mgT.ensure((size_t)std::max(1LL, off)));
     TRY(s->d_mgfw.ensure(faces.size()));
-    TRY(s->d_mgpos.ensure(pos.size()));
-    TRY(s->d_mgtmp.ensure((size_t)(ntmp + nwork)));
+    TRY(s->d_mgtab.ensure(tab.size()));
+    TRY(s->d_mgtmp.ensure((size_t)(ntmp * chunk)));
+    TRY(s->d_mgwork.ensure(nwork));
     CUDA_TRY(cudaMemcpyAsync(s->d_mgfw.p, faces.data(), faces.size() * sizeof(float), cudaMemcpyHostToDevice,
                              s->stream));
-    CUDA_TRY(cudaMemcpyAsync(s->d_mgpos.p, pos.data(), pos.size() * sizeof(float), cudaMemcpyHostToDevice,
-                             s->stream));
-    const float *P = s->d_mgpos.p;
-    float *tx = s->d_mgtmp.p;
-    float *work = tx + ntmp;
-    for (int f = 0; f < nfields; ++f)
-        for (int l = 1; l < G; ++l) {
-            const int im = I >> l, jm = J >> l, km = K >> l;
-            float *txy = tx + (long long)im * J * K;
+    CUDA_TRY(cudaMemcpyAsync(s->d_mgtab.p, tab.data(), tab.size(), cudaMemcpyHostToDevice, s->stream));
+    float *tx = s->d_mgtmp.p, *txy = tx + ntx * chunk;
+    for (int f0 = 0; f0 < nfields; f0 += chunk) {
+        const int nf = std::min(chunk, nfields - f0);
+        for (int p = 0; p < 3; ++p) {
             SplinePass q{};
-            q.work = work;
-            // along x: fine [i][k][j] -> tx [ic][k][j], lines (j, k)
-            q.src = src + (long long)f * ncell * src_step; q.src_step = src_step;
-            q.s_a = 1; q.s_b = J; q.s_e = (long long)J * K;
-            q.dst = tx; q.d_a = 1; q.d_b = J; q.d_e = (long long)J * K;
-            q.na = J; q.nlines = (long long)J * K; q.n = I; q.m = im;
-            q.xf = P + pf[0]; q.xc = P + po[l][0];
-            int rc = launch_spline_pass(q, s->stream);
-            // along y: tx [ic][k][j] -> txy [ic][k][jc], lines (ic, k)
-            if (!rc) {
-                q.src = tx; q.src_step = 1;
-                q.s_a = (long long)K * J; q.s_b = J; q.s_e = 1;
-                q.dst = txy; q.d_a = (long long)K * jm; q.d_b = jm; q.d_e = 1;
-                q.na = im; q.nlines = (long long)im * K; q.n = J; q.m = jm;
-                q.xf = P + pf[1]; q.xc = P + po[l][1];
-                rc = launch_spline_pass(q, s->stream);
+            q.nfields = nf; q.n = n[p]; q.src_step = p == 0 ? src_step : 1;
+            q.coef = reinterpret_cast<const SplineCoef *>(s->d_mgtab.p) + oco[p];
+            q.x = reinterpret_cast<const float *>(s->d_mgtab.p + bpos) + opos[p];
+            q.work = s->d_mgwork.p;
+            q.njobs = p == 0 ? 1 : G - 1;
+            for (int l = 1; l < G; ++l) {
+                const int im = I >> l, jm = J >> l, km = K >> l;
+                SplineOut &o = q.out[l - 1];
+                SplineJob &b = q.job[p == 0 ? 0 : l - 1];
+                o.at = reinterpret_cast<const SplineAt *>(s->d_mgtab.p + bat) + oat[l][p];
+                b.out0 = p == 0 ? 0 : l - 1;
+                b.nout = p == 0 ? G - 1 : 1;
+                if (p == 0) {
+                    // fine [i][k][j] -> tx [ic][k][j], lines (j, k)
+                    b.src = src + f0 * ncell * src_step;
+                    b.s_a = 1; b.s_b = J; b.s_e = (long long)J * K; b.s_f = ncell * src_step;
+                    b.na = (unsigned)J; b.nlines = (long long)J * K;
+                    o.dst = tx + ox[l] * chunk; o.m = im;
+                    o.d_a = 1; o.d_b = J; o.d_e = (long long)J * K; o.d_f = (long long)im * J * K;
+                } else if (p == 1) {
+                    // tx [ic][k][j] -> txy [ic][k][jc], lines (k, ic)
+                    b.src = tx + ox[l] * chunk;
+                    b.s_a = J; b.s_b = (long long)K * J; b.s_e = 1; b.s_f = (long long)im * J * K;
+                    b.na = (unsigned)K; b.nlines = (long long)im * K;
+                    o.dst = txy + oxy[l] * chunk; o.m = jm;
+                    o.d_a = jm; o.d_b = (long long)K * jm; o.d_e = 1; o.d_f = (long long)im * jm * K;
+                } else {
+                    // txy [ic][k][jc] -> the march layout [ic][kc][jc], lines (jc, ic)
+                    b.src = txy + oxy[l] * chunk;
+                    b.s_a = 1; b.s_b = (long long)K * jm; b.s_e = jm; b.s_f = (long long)im * jm * K;
+                    b.na = (unsigned)jm; b.nlines = (long long)jm * im;
+                    o.dst = s->d_mgT.p + s->mg_off[l] + (long long)f0 * im * jm * km; o.m = km;
+                    o.d_a = 1; o.d_b = (long long)km * jm; o.d_e = jm; o.d_f = (long long)im * jm * km;
+                }
             }
-            // along z: txy [ic][k][jc] -> the march layout [ic][kc][jc], lines (jc, ic)
-            if (!rc) {
-                q.src = txy;
-                q.s_a = 1; q.s_b = (long long)K * jm; q.s_e = jm;
-                q.dst = s->d_mgT.p + s->mg_off[l] + (long long)f * im * jm * km;
-                q.d_a = 1; q.d_b = (long long)km * jm; q.d_e = jm;
-                q.na = jm; q.nlines = (long long)jm * im; q.n = K; q.m = km;
-                q.xf = P + pf[2]; q.xc = P + po[l][2];
-                rc = launch_spline_pass(q, s->stream);
-            }
+            const int rc = launch_spline_pass(q, s->stream);
             if (rc) return fail(DNSMC_ERR_CUDA, "spline coarsening launch: %s", cudaGetErrorString((cudaError_t)rc));
         }
+    }
     s->mg_fields = nfields;
     return DNSMC_OK;
 }
@@ -1677,7 +1730,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();
     s->d_stat_part.release(); s->d_stat_out.release(); s->d_rays_pp.release(); s->d_rays_rcp.release(); s->d_item_steps.release(); s->d_kP.release();
     s->d_order.release(); s->d_order_hist.release();
-    s->d_mgT.release(); s->d_mgfw.release(); s->d_mgpos.release(); s->d_mgtmp.release();
+    s->d_mgT.release(); s->d_mgfw.release(); s->d_mgtab.release(); s->d_mgtmp.release(); s->d_mgwork.release();
     s->d_part.release(); s->d_fieldV.release(); s->d_layerV.release();
     s->d_entries.release(); s->d_group_start.release(); s->d_group_empty.release();
     s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_sig.release(); s->h_sig.release(); s->d_Qg.release(); s->d_varg.release();

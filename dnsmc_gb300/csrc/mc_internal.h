@@ -246,22 +246,54 @@ int launch_item_order(const int *rays, int gstride, int n_packets, int n_groups,
                       unsigned int *hist, unsigned int *order, void *stream);
 
 // One pass of the spline coarsening (interp3D, code/spline.cpp:35-116) over
-// nlines = na * nb lines: line (la, lb) reads n fine values at
-// src[(la*s_a + lb*s_b + (i-1)*s_e) * src_step] (positions xf[1..n]) and
-// writes m coarse values at dst[la*d_a + lb*d_b + (c-1)*d_e] (positions
-// xc[1..m]); work holds 3 * (n + 2) * nlines floats.
-struct SplinePass {
-    const float *src;
-    long long s_a, s_b, s_e;
-    int src_step;             // floats per source element (2: T of a (T, x) pair)
-    float *dst;
-    long long d_a, d_b, d_e;
-    long long na, nlines;
-    int n, m;
-    const float *xf, *xc;     // 1-based device arrays of n + 2 and m + 2 floats
-    float *work;
+// lines of n fine values along one axis.  Line L of a job is (la, lb) =
+// (L % na, L / na); its value e of field f is src[(la*s_a + lb*s_b + e*s_e) *
+// src_step + f*s_f], and its coarse value c goes to dst[la*d_a + lb*d_b +
+// c*d_e + f*d_f] of each of the job's outputs.  Device arrays of the axis: the
+// fine positions x[n], the recurrence's coefficients and per output the
+// brackets of the coarse positions.
+struct SplineCoef {
+    double rp, p;             // 1 / p, p
+    float sig, c;             // c = (sig - 1) / p; 0 at the ends
 };
-int launch_spline_pass(const SplinePass &q, void *stream);
+struct SplineAt {
+    int lo;                   // the bracket is [lo, lo + 1], h wide
+    float aa, bb, h2;         // (x[lo+1] - v) / h, (v - x[lo]) / h, h^2
+};
+struct SplineOut {
+    float *dst;
+    long long d_a, d_b, d_e, d_f;
+    int m;
+    const SplineAt *at;
+};
+struct SplineJob {
+    const float *src;
+    long long s_a, s_b, s_e, s_f;
+    unsigned na;
+    long long nlines;         // < 2^31
+    int out0, nout;           // its outputs
+    int block0;               // its first block (set by the launch)
+};
+struct SplinePass {
+    SplineJob job[kMaxLevels];
+    SplineOut out[kMaxLevels];
+    int njobs, nfields, n;
+    int src_step;             // floats per source element (2: T of a (T, x) pair)
+    int lines;                // of a block (set by the launch)
+    const float *x;
+    const SplineCoef *coef;
+    double *work;             // spline_work_doubles() when that is not 0
+};
+// of a block of W lines of n values: right sides (double) and values (float),
+// a column of padding against bank conflicts
+__host__ __device__ inline size_t spline_line_doubles(int n, int W) { return ((size_t)n * (W + 1) * 3 + 1) / 2; }
+// The spline's scratch in global memory for lines that do not fit in a block's
+// shared memory (200 KB, one line a block), else 0.
+inline size_t spline_work_doubles(int n, long long nlines) {
+    const size_t one = spline_line_doubles(n, 1);
+    return one * sizeof(double) > 200u * 1024u ? one * (size_t)nlines : 0;
+}
+int launch_spline_pass(SplinePass &q, void *stream);
 
 // Kernels this library has launched in this process (every launch site
 // calls note_launch; a CUDA-graph replay adds the kernel nodes of its graph).

@@ -976,61 +976,125 @@ int launch_finalize(const FinalizeParams &p, void *stream) {
 // Spline coarsening of the temperature for the multigrid march: the
 // reference's interp3D (code/spline.cpp:35-116), a separable natural cubic
 // spline through the fine cell centres along x, then y, then z, evaluated at
-// the coarse cell centres.  One thread per spline line; each pass is one
-// launch.  The arithmetic is the Numerical Recipes spline / splint of
-// code/spline.cpp:119-170 written as the oracle restates it (float with the
-// same double sub-expressions; this translation unit is compiled with
-// -fmad=false), so the coarse fields are bit-identical to the oracle's.
+// the coarse cell centres.  The arithmetic is the Numerical Recipes spline /
+// splint of code/spline.cpp:119-170 written as the oracle restates it (float
+// with the same double sub-expressions; this translation unit is compiled
+// with -fmad=false), so the coarse fields are bit-identical to the oracle's.
+//
+// What bounds it is the tridiagonal recurrence of a line, n dependent steps
+// in FP64.  Everything that is not in that chain is taken out of it: the
+// coefficients that depend on positions alone come from the host, the right
+// sides and the evaluation are spread over the block, and the chain's
+// division by p is q0 = a * r, q = fma(fma(-q0, p, a), r, q0) with r = RN(1/p)
+// (Markstein 1990).  q is the correctly rounded a / p here: a - q0 p is exact
+// (p has 24 bits), so before its rounding q differs from a / p by 2^-52 of an
+// ulp at most, while a quotient by a 24-bit p keeps 2^-25 of an ulp from every
+// midpoint of doubles.  All levels and fields share a launch, and the pass
+// along x one recurrence for all levels: three launches.  64^3, four coarse
+// levels: 99 us (twelve launches, a thread per line with its chain in
+// global memory: 1250 us).
 // ---------------------------------------------------------------------------
-__global__ void spline_pass_kernel(SplinePass q) {
-    for (long long L = blockIdx.x * (long long)blockDim.x + threadIdx.x; L < q.nlines;
-         L += (long long)gridDim.x * blockDim.x) {
-        const long long la = L % q.na, lb = L / q.na;
-        const float *src = q.src + (la * q.s_a + lb * q.s_b) * q.src_step;
-        float *dst = q.dst + la * q.d_a + lb * q.d_b;
-        // this line's work arrays, interleaved across lines (1-based, n + 2)
-        float *a = q.work + L;
-        float *y2 = a + (long long)(q.n + 2) * q.nlines;
-        float *u = y2 + (long long)(q.n + 2) * q.nlines;
-        const long long w = q.nlines;
-        const float *x = q.xf;
-        const int n = q.n;
-        for (int i = 1; i <= n; ++i) a[i * w] = src[(long long)(i - 1) * q.s_e * q.src_step];
-        // second derivatives (natural end conditions)
-        y2[1 * w] = 0.0f;
-        u[1 * w] = 0.0f;
-        for (int i = 2; i <= n - 1; ++i) {
-            const float sig = (x[i] - x[i - 1]) / (x[i + 1] - x[i - 1]);
-            const float p = sig * y2[(i - 1) * w] + 2.0f;
-            y2[i * w] = (sig - 1.0f) / p;
-            const float ui = (a[(i + 1) * w] - a[i * w]) / (x[i + 1] - x[i]) -
-                             (a[i * w] - a[(i - 1) * w]) / (x[i] - x[i - 1]);
-            u[i * w] = (float)((6.0 * ui / (x[i + 1] - x[i - 1]) - sig * u[(i - 1) * w]) / p);
+template <bool WORK>
+__global__ void __launch_bounds__(256) spline_pass_kernel(const SplinePass q) {
+    extern __shared__ double s_line[];
+    const int W = q.lines, W1 = W + 1, n = q.n;
+    int j = 0;
+    while (j + 1 < q.njobs && (int)blockIdx.x >= q.job[j + 1].block0) ++j;
+    const SplineJob &b = q.job[j];
+    const long long L0 = (long long)((int)blockIdx.x - b.block0) * W;
+    const int nl = (int)min((long long)W, b.nlines - L0);  // this block's lines
+    // [element][line]: right side, then u, then the second derivative; value
+    double *t = WORK ? q.work + (size_t)(blockIdx.y * (size_t)gridDim.x + blockIdx.x) * spline_line_doubles(n, W) : s_line;
+    float *a = reinterpret_cast<float *>(t + (size_t)n * W1);
+    auto slot = [&](int e, int l) { return reinterpret_cast<float *>(t + (size_t)e * W1 + l); };
+    for (int f = blockIdx.y; f < q.nfields; f += gridDim.y) {
+        const float *src = b.src + f * b.s_f;
+        for (int k = threadIdx.x; k < n * nl; k += blockDim.x) {
+            int e, l;
+            if (b.s_e == 1) { l = k / n; e = k - l * n; } else { e = k / nl; l = k - e * nl; }
+            const unsigned lb = (unsigned)(L0 + l) / b.na, la = (unsigned)(L0 + l) - lb * b.na;
+            a[(size_t)e * W1 + l] = src[(la * b.s_a + lb * b.s_b + e * b.s_e) * q.src_step];
         }
-        y2[n * w] = 0.0f;
-        for (int k = n - 1; k >= 1; --k) y2[k * w] = y2[k * w] * y2[(k + 1) * w] + u[k * w];
-        // values at the coarse centres (bisection for the bracket)
-        for (int c = 1; c <= q.m; ++c) {
-            const float v = q.xc[c];
-            int lo = 1, hi = n;
-            while (hi - lo > 1) {
-                const int k = (hi + lo) >> 1;
-                if (x[k] > v) hi = k; else lo = k;
+        __syncthreads();
+        for (int k = threadIdx.x; k < (n - 2) * nl; k += blockDim.x) {
+            const int e = k / nl + 1, l = k - (e - 1) * nl;
+            const float *v = a + (size_t)e * W1 + l;
+            const float ui = (v[W1] - v[0]) / (q.x[e + 1] - q.x[e]) - (v[0] - v[-W1]) / (q.x[e] - q.x[e - 1]);
+            t[(size_t)e * W1 + l] = 6.0 * ui / (q.x[e + 1] - q.x[e - 1]);
+        }
+        __syncthreads();
+        if ((int)threadIdx.x < nl) {
+            const int l = threadIdx.x;
+            float u = 0.0f;
+            *slot(0, l) = 0.0f;
+#pragma unroll 4
+            for (int e = 1; e < n - 1; ++e) {
+                const SplineCoef k = q.coef[e];
+                const double num = t[(size_t)e * W1 + l] - k.sig * u;
+                const double q0 = num * k.rp;
+                const double q1 = fma(fma(-q0, k.p, num), k.rp, q0);
+                const bool fin = (__double2hiint(num) & 0x7ff00000) != 0x7ff00000;
+                u = (float)(fin ? q1 : num);  // p > 0: an infinity stays one
+                *slot(e, l) = u;
             }
-            const float h = x[hi] - x[lo];
-            const float aa = (x[hi] - v) / h, bb = (v - x[lo]) / h;
-            const float ylo = a[lo * w], yhi = a[hi * w];
-            dst[(long long)(c - 1) * q.d_e] =
-                (float)(aa * ylo + bb * yhi +
-                        ((aa * aa * aa - aa) * y2[lo * w] + (bb * bb * bb - bb) * y2[hi * w]) * (h * h) / 6.0);
+            float y2 = 0.0f;
+            *slot(n - 1, l) = 0.0f;
+#pragma unroll 4
+            for (int e = n - 2; e >= 0; --e) {
+                y2 = q.coef[e].c * y2 + *slot(e, l);
+                *slot(e, l) = y2;
+            }
         }
+        __syncthreads();
+        for (int o = b.out0; o < b.out0 + b.nout; ++o) {
+            const SplineOut &w = q.out[o];
+            float *dst = w.dst + f * w.d_f;
+            for (int k = threadIdx.x; k < w.m * nl; k += blockDim.x) {
+                int c, l;
+                if (w.d_e == 1) { l = k / w.m; c = k - l * w.m; } else { c = k / nl; l = k - c * nl; }
+                const SplineAt p = w.at[c];
+                const float *v = a + (size_t)p.lo * W1 + l;
+                const float y2lo = *slot(p.lo, l), y2hi = *slot(p.lo + 1, l);
+                const unsigned lb = (unsigned)(L0 + l) / b.na, la = (unsigned)(L0 + l) - lb * b.na;
+                dst[la * w.d_a + lb * w.d_b + c * w.d_e] =
+                    (float)(p.aa * v[0] + p.bb * v[W1] +
+                            ((p.aa * p.aa * p.aa - p.aa) * y2lo + (p.bb * p.bb * p.bb - p.bb) * y2hi) * p.h2 / 6.0);
+            }
+        }
+        __syncthreads();
     }
 }
 
-int launch_spline_pass(const SplinePass &q, void *stream) {
-    if (q.nlines <= 0) return 0;
+// Lines of a block: 32, fewer where that leaves SMs without a block (the
+// chain's time does not depend on it) or the lines do not fit in shared
+// memory; lines too long for it even so stay in q.work.
+int launch_spline_pass(SplinePass &q, void *stream) {
+    const size_t limit = 200u * 1024u;
+    long long lines = 0;
+    for (int j = 0; j < q.njobs; ++j) lines += q.job[j].nlines;
+    q.lines = 32;
+    while (q.lines > 8 && lines * q.nfields < 152ll * q.lines) q.lines /= 2;
+    while (q.lines > 1 && spline_line_doubles(q.n, q.lines) * sizeof(double) > limit) q.lines /= 2;
+    const size_t smem = spline_line_doubles(q.n, q.lines) * sizeof(double);
+    const bool work = smem > limit;
+    long long blocks = 0;
+    for (int j = 0; j < q.njobs; ++j) {
+        q.job[j].block0 = (int)blocks;
+        blocks += (q.job[j].nlines + q.lines - 1) / q.lines;
+    }
+    if (blocks <= 0 || q.nfields <= 0) return 0;
+    const dim3 grid((unsigned)blocks, (unsigned)(work ? 1 : std::min(q.nfields, 65535)));
     dnsmc::note_launch();
-    spline_pass_kernel<<<grid_for(q.nlines, 128), 128, 0, (cudaStream_t)stream>>>(q);
+    if (work) {
+        if (!q.work) return (int)cudaErrorInvalidValue;
+        spline_pass_kernel<true><<<grid, 256, 0, (cudaStream_t)stream>>>(q);
+    } else {
+        if (smem > 48u * 1024u) {
+            const cudaError_t e = cudaFuncSetAttribute(spline_pass_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+            if (e != cudaSuccess) return (int)e;
+        }
+        spline_pass_kernel<false><<<grid, 256, smem, (cudaStream_t)stream>>>(q);
+    }
     return (int)cudaGetLastError();
 }
 

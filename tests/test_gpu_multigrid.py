@@ -40,6 +40,28 @@ def test_coarse_fields_match_the_oracle(stretched):
     s.close()
 
 
+@pytest.mark.parametrize("shape,levels,nf", [
+    ((2, 2, 2), 2, 1),           # no inner point on any line
+    ((6, 10, 34), 2, 3),         # partial blocks of lines on every axis
+    ((4, 1040, 4), 3, 2),        # long lines, fewer of them to a block
+    ((128, 64, 96), 6, 1),       # all levels, full blocks
+    ((8600, 2, 2), 2, 2),        # lines that do not fit in shared memory
+])
+def test_coarse_fields_of_odd_sizes_match_the_oracle(shape, levels, nf):
+    ni, nj, nk = shape
+    s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=ni, jmax=nj, kmax=nk, Lx=2.0, Ly=6.28, Lz=3.14,
+                                  stretched_x=0, grid_num=levels, kappa=1.0, T_west=300, T_east=300))
+    T = np.random.default_rng(ni + nj).uniform(300, 1500, (nf, nk, nj, ni)).astype(np.float32)
+    s.set_fields(T)
+    for f in range(nf):
+        Tf = np.zeros((nk + 2, nj + 2, ni + 2), np.float32)
+        Tf[1:-1, 1:-1, 1:-1] = T[f]
+        for lv in range(1, levels):
+            ref = O.coarsen(Tf.ravel(), ni, nj, nk, 2.0, 6.28, 3.14, 0, levels, lv)[1:-1, 1:-1, 1:-1]
+            np.testing.assert_array_equal(s.coarse_field(f, lv), ref)
+    s.close()
+
+
 def test_coarse_fields_from_device_inputs_and_with_x():
     """The coarsening reads the packed device field: fields given as device
     arrays, and fields carrying x_H2O (the T of each (T, x) pair), give the
