@@ -6,8 +6,8 @@
 // allocation after initialisation so their memory footprint stays fixed.
 // dnsmc_solve_grey_noalloc serves them: the caller passes device input and
 // output arrays, and every intermediate buffer of the solve (packed field,
-// wall-normal faces, per-cell tallies, work-queue counter, status and counter
-// words) lives in g_noalloc_scratch, one file-scope __device__ array of fixed
+// wall-normal faces, per-cell tallies, rays' contributions, work-queue counter,
+// status and counter words) lives in g_noalloc_scratch, one file-scope __device__ array of fixed
 // size that each GPU loading this library holds until the process exits.
 //
 // The kernels are the same persistent march and finalize kernels the handle
@@ -39,7 +39,16 @@ constexpr long long kMaxPadded = 693360;
 constexpr size_t kFacesOff = kFieldOff + (size_t)kMaxPadded * 4;     // wall-normal faces
 constexpr size_t kMiscOff = kFacesOff + (((size_t)kMaxFaces * 4 + 255) / 256) * 256;
 constexpr size_t kMiscBytes = 256;  // [0] queue, [1] status, [2] group flag (uint32); [2..3] counters (u64)
-constexpr size_t kScratchBytes = kMiscOff + kMiscBytes;
+// items split by rays (march_parts): finished units per item and every ray's
+// contribution, as many as the array holds (all that 32^3 cells need up to
+// 256 rays).  One warp per item leaves most of the GPU idle on the grids this
+// entry point serves (32^3 is 512 items for about 3600 resident warps): 32^3 at
+// 60 rays 366 us unsplit, 129 us split.
+constexpr long long kMaxSplitItems = 16384;
+constexpr size_t kDoneOff = kMiscOff + kMiscBytes;
+constexpr size_t kRayxOff = kDoneOff + (size_t)kMaxSplitItems * 4;
+constexpr size_t kRayxRoom = 32u << 20;
+constexpr size_t kScratchBytes = kRayxOff + kRayxRoom;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kScratchBytes];
 
@@ -116,9 +125,9 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     double2 *tally = (double2 *)(base + kTallyOff);
 
     // Scratch keeps the previous call's contents: the queue, status, group
-    // flag and counters must start at zero; faces, field and tallies are
-    // fully overwritten below before they are read.
-    cudaError_t e = cudaMemsetAsync(misc, 0, kMiscBytes, st);
+    // flag, counters and finished-unit counts must start at zero; faces, field,
+    // contributions and tallies are fully overwritten below before they are read.
+    cudaError_t e = cudaMemsetAsync(misc, 0, kMiscBytes + (size_t)kMaxSplitItems * 4, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(faces, xu, (size_t)(c.imax + 1) * sizeof(float), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString(e));
     // the grey black-wall march runs kLaneCells cells per lane
@@ -164,12 +173,16 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     P.counters = counters;
     P.region_cells = ncell;
     P.n_items = P.n_packets;
-    P.parts = 1;  // splitting items would need more scratch
     P.tally = tally;
     const int threads = c.block_threads ? c.block_threads : 256;
     // persistent grid: resident blocks at the launch's dynamic shared memory
     const size_t smem = march_pair_smem(P, threads);
     const int blocks = device_sm_count() * march_occupancy_ex(MODE_GREY, false, threads, false, false, false, smem);
+    P.parts = P.n_items > kMaxSplitItems ? 1 : march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxRoom);
+    if (P.parts > 1) {
+        P.parts_done = (unsigned int *)(base + kDoneOff);
+        P.rayx = (float *)(base + kRayxOff);
+    }
     rc = launch_march(MODE_GREY, P, blocks > 0 ? blocks : 1, threads, st, false);
     if (rc) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString((cudaError_t)rc));
 

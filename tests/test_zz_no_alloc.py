@@ -84,6 +84,30 @@ def test_noalloc_grey_matches_handle_api_twice(ni, nj, nk):
 
 
 @GPU
+@pytest.mark.parametrize("ni,nj,nk,rays", [(5, 9, 1, 3),          # fewer rays than units asked for
+                                           (32, 32, 32, 256),     # the contributions fill the fixed array
+                                           (32, 32, 32, 257),     # one ray more: an item is one unit
+                                           (6, 64, 40, 77)])      # units of unequal length
+def test_noalloc_split_items_match_the_handle_api(ni, nj, nk, rays):
+    torch = _torch_cuda()
+    cfg = D.default_config(model=D.MODEL_GREY, imax=ni, jmax=nj, kmax=nk, Lx=2.0, Ly=6.2831853, Lz=3.1415927,
+                           stretched_x=1, T_west=300.0, T_east=420.0, kappa=1.3, nvar=1, photmax=rays, seed=11)
+    lib = _lib.load()
+    T = field(ni, nj, nk, 5)
+    s = D.Solver(cfg)
+    s.set_fields(T)
+    s.set_rays(rays)
+    Qref, Sref = s.solve(timeout_s=120)
+    xu, _, _ = s.geometry()
+    s.close()
+    for _ in range(2):
+        Q, V, status = _noalloc(lib, torch, cfg, xu, T)
+        assert status == 0
+        np.testing.assert_array_equal(Q, Qref[0])
+        np.testing.assert_array_equal(np.sqrt(V), Sref[0])
+
+
+@GPU
 def test_noalloc_reports_bad_temperature_then_recovers():
     """A temperature of 0 sets DNSMC_STATUS_BAD_FIELD in the caller's status
     word; the next call on a good field reports 0 again (the shared status
