@@ -472,7 +472,7 @@ int  dnsmc_cvnet_apply(dnsmc_cvnet *net, dnsmc_solver *s, int flags,
  * initialisation.  It solves a grey medium (cfg->model == DNSMC_MODEL_GREY,
  * IID sampler, nvar*photmax rays per cell, the whole grid) and calls no
  * cudaMalloc/cudaFree or allocating library routine: its intermediate buffers
- * live in one fixed file-scope device array of about 7 MB that every GPU
+ * live in one fixed file-scope device array of about 41 MB that every GPU
  * loading the library holds until the process exits.
  *   xu   : host, imax+1 wall-normal face coordinates [m] (e.g. from
  *          dnsmc_get_geometry or the caller's own grid), copied to the
