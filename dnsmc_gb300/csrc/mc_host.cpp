@@ -53,6 +53,8 @@ int fail(int code, const char *fmt, ...) {
     } while (0)
 
 constexpr double kSigma = 5.670373e-08;  // code/param.h:70
+constexpr size_t kMiscWords = 8;       // queue, status and counters of a solve (dnsmc_solver::d_misc)
+constexpr double kSpinSeconds = 5e-3;  // wait_done: polled without sleeping
 constexpr double kPi = 3.14159265358979323846;
 
 // Band-centre Planck intensity per unit wavenumber [W/(m^2 sr m^-1)], nu in
@@ -338,9 +340,11 @@ struct dnsmc_solver {
     double sig_scale = 1.0;
     DevBuf<float> d_Qf, d_sigf;
     PinBuf<float> h_Qf, h_sigf;
-    DevBuf<unsigned int> d_misc;  // [0] queue, [1] status, [4 ...] finished units per item (split items)
+    // [0] queue, [1] status, [4..7] the two 64-bit counters, [8 ...] finished
+    // units per item (split items); the first 8 words come back with the results
+    DevBuf<unsigned int> d_misc;
+    PinBuf<unsigned int> h_misc;
     DevBuf<float> d_rayx;         // every ray's contribution (split items), at most kRayxBytes
-    DevBuf<unsigned long long> d_counters;
     unsigned long long h_counters[2] = {0, 0};
     unsigned int h_status = 0;
     float march_ms = 0.f, solve_ms = 0.f;
@@ -1042,11 +1046,11 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
     fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
     P.parts = 1;
-    TRY(s->d_misc.ensure(4));
-    TRY(s->d_counters.ensure(2));
+    TRY(s->d_misc.ensure(kMiscWords));
+    TRY(s->h_misc.ensure(kMiscWords));
     P.queue = s->d_misc.p;
     P.status = s->d_misc.p + 1;
-    P.counters = s->d_counters.p;
+    P.counters = reinterpret_cast<unsigned long long *>(s->d_misc.p + 4);
     int threads = c.block_threads ? c.block_threads : 256;
     {
         // every warp holds its ray's table slab in shared memory
@@ -1167,11 +1171,12 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes);
         if (P.parts > 1) {
             TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * 64)));
-            TRY(s->d_misc.ensure((size_t)(4 + P.n_items)));
+            TRY(s->d_misc.ensure((size_t)(kMiscWords + P.n_items)));
             P.rayx = s->d_rayx.p;
             P.queue = s->d_misc.p;
             P.status = s->d_misc.p + 1;
-            P.parts_done = s->d_misc.p + 4;
+            P.counters = reinterpret_cast<unsigned long long *>(s->d_misc.p + 4);
+            P.parts_done = s->d_misc.p + kMiscWords;
         }
     }
 
@@ -1222,11 +1227,10 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             if (rc == 0) rc = launch_cv_mean(cp, s->stream);
             if (rc) return fail(DNSMC_ERR_CUDA, "control-variate launch: %s", cudaGetErrorString((cudaError_t)rc));
         }
-        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, (4 + (P.parts > 1 ? (size_t)P.n_items : 0)) * sizeof(unsigned int),
+        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, (kMiscWords + (P.parts > 1 ? (size_t)P.n_items : 0)) * sizeof(unsigned int),
                                  s->stream));
         if (P.parts > 1 && P.item_steps)
             CUDA_TRY(cudaMemsetAsync(P.item_steps, 0, (size_t)P.n_items * sizeof(unsigned long long), s->stream));
-        CUDA_TRY(cudaMemsetAsync(s->d_counters.p, 0, 2 * sizeof(unsigned long long), s->stream));
         if (P.item_order) {
             const int rco = launch_item_order(P.rays_per_packet, P.rays_gstride, P.n_packets, P.n_groups, P.n_items,
                                               std::max(1, c.sampler == DNSMC_SAMPLER_RQMC ? c.nvar : 1),
@@ -1249,6 +1253,8 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             CUDA_TRY(cudaMemcpyAsync(s->h_sig.p, s->d_sig.p, nout * sizeof(double), cudaMemcpyDeviceToHost,
                                      s->stream));
         }
+        CUDA_TRY(cudaMemcpyAsync(s->h_misc.p, s->d_misc.p, kMiscWords * sizeof(unsigned int), cudaMemcpyDeviceToHost,
+                                 s->stream));
         return DNSMC_OK;
     };
 
@@ -1309,6 +1315,10 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     return DNSMC_OK;
 }
 
+// Wait for the solve in flight.  Polls without sleeping for kSpinSeconds, then
+// every 50 us: a sleep of 50 us takes about twice that, as long as a small
+// solve itself.  With status and counters arriving with the results instead of
+// by two blocking copies: grey 8 x 32 x 4 call 206 -> 101 us.
 int wait_done(dnsmc_solver *s, double timeout_s) {
     if (!s->in_flight) return DNSMC_OK;
     TRY(set_device(s));
@@ -1317,19 +1327,16 @@ int wait_done(dnsmc_solver *s, double timeout_s) {
         cudaError_t e = cudaEventQuery(s->ev_done);
         if (e == cudaSuccess) break;
         if (e != cudaErrorNotReady) return fail(DNSMC_ERR_CUDA, "solve failed: %s", cudaGetErrorString(e));
-        if (timeout_s > 0) {
-            const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-            if (el > timeout_s) return fail(DNSMC_ERR_TIMEOUT, "solve still running after %.3f s", timeout_s);
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(50));
+        const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+        if (timeout_s > 0 && el > timeout_s) return fail(DNSMC_ERR_TIMEOUT, "solve still running after %.3f s", timeout_s);
+        if (el > kSpinSeconds) std::this_thread::sleep_for(std::chrono::microseconds(50));
+        else std::this_thread::yield();
     }
     s->in_flight = false;
     CUDA_TRY(cudaEventElapsedTime(&s->march_ms, s->ev_march0, s->ev_march1));
     CUDA_TRY(cudaEventElapsedTime(&s->solve_ms, s->ev_solve0, s->ev_done));
-    unsigned int misc[4];
-    CUDA_TRY(cudaMemcpy(misc, s->d_misc.p, sizeof misc, cudaMemcpyDeviceToHost));
-    CUDA_TRY(cudaMemcpy(s->h_counters, s->d_counters.p, sizeof s->h_counters, cudaMemcpyDeviceToHost));
-    s->h_status = misc[1];
+    memcpy(s->h_counters, s->h_misc.p + 4, sizeof s->h_counters);
+    s->h_status = s->h_misc.p[1];
     if (s->h_status & DNSMC_STATUS_COPY_TIMEOUT)
         return fail(DNSMC_ERR_TIMEOUT, "solve failed: a march's table copy did not arrive within its bounded wait");
     return DNSMC_OK;
@@ -1478,22 +1485,27 @@ int upload_coarse(dnsmc_solver *s, int nfields, const float *src, int src_step) 
     return DNSMC_OK;
 }
 
-// Tmax / Tmin / sum x over the packed resident fields (code/mc_gpu.cu:470-486),
-// on the device; fails (and drops the fields) when a temperature is not
-// positive and finite.
-int field_stats_checked(dnsmc_solver *s, int nfields, bool with_x, double st[4]) {
-    const dnsmc_config &c = s->cfg;
-    const long long ncell = (long long)c.imax * c.jmax * c.kmax;
+// launch_field_stats of n resident values, its results read back
+int field_stats(dnsmc_solver *s, int kind, const float *v, long long n, double st[4]) {
     TRY(s->d_stat_part.ensure(field_stats_partials()));
     if (!s->d_stat_out.p) {
         TRY(s->d_stat_out.ensure(5));
         CUDA_TRY(cudaMemsetAsync(s->d_stat_out.p, 0, 5 * sizeof(double), s->stream));
     }
-    const int rc = launch_field_stats(with_x ? nullptr : s->d_fieldT.p, with_x ? s->d_fieldTX.p : nullptr,
-                                      nfields * ncell, s->d_stat_part.p, s->d_stat_out.p, s->stream);
+    const int rc = launch_field_stats(kind, v, n, s->d_stat_part.p, s->d_stat_out.p, s->stream);
     if (rc) return fail(DNSMC_ERR_CUDA, "stats launch: %s", cudaGetErrorString((cudaError_t)rc));
     CUDA_TRY(cudaMemcpyAsync(st, s->d_stat_out.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return DNSMC_OK;
+}
+
+// Tmax / Tmin / sum x over the packed resident fields (code/mc_gpu.cu:470-486),
+// on the device; fails (and drops the fields) when a temperature is not
+// positive and finite.
+int field_stats_checked(dnsmc_solver *s, int nfields, bool with_x, double st[4]) {
+    const dnsmc_config &c = s->cfg;
+    TRY(field_stats(s, with_x ? STATS_TX : STATS_T, with_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p,
+                    (long long)nfields * c.imax * c.jmax * c.kmax, st));
     if (st[3] > 0.0 || !(st[1] > 0.0) || !std::isfinite(st[0])) {
         s->nfields = 0;
         return fail(DNSMC_ERR_ARG, "temperature field has non-positive or non-finite values");
@@ -1734,7 +1746,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_part.release(); s->d_fieldV.release(); s->d_layerV.release();
     s->d_entries.release(); s->d_group_start.release(); s->d_group_empty.release();
     s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_sig.release(); s->h_sig.release(); s->d_Qg.release(); s->d_varg.release();
-    s->h_Q.release(); s->d_misc.release(); s->d_rayx.release(); s->d_counters.release();
+    s->h_Q.release(); s->d_misc.release(); s->d_rayx.release(); s->h_misc.release();
     s->d_Qf.release(); s->d_sigf.release(); s->h_Qf.release(); s->h_sigf.release();
     if (s->ev_march0) cudaEventDestroy(s->ev_march0);
     if (s->ev_march1) cudaEventDestroy(s->ev_march1);
@@ -2024,30 +2036,26 @@ int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
     } else {
         return fail(DNSMC_ERR_ARG, "unknown layout %d", layout);
     }
-    float vmax = 0.0f;
-    double vsum = 0.0;
-    for (int f = 0; f < s->nfields; ++f)
-        for (int k = 0; k < c.kmax; ++k)
-            for (int j = 0; j < c.jmax; ++j) {
-                const long long o = f * nsrc + base + j * sj + k * sk;
-                for (int i = 0; i < c.imax; ++i) {
-                    const float v = fv[o + i];
-                    if (!(v >= 0.0f) || !std::isfinite(v)) return fail(DNSMC_ERR_ARG, "volume fractions must be finite and >= 0");
-                    vmax = std::max(vmax, v);
-                    vsum += v;
-                }
-            }
     TRY(set_device(s));
     TRY(wait_done(s, 0));
-    TRY(s->d_raw.ensure((size_t)nsrc));
-    TRY(s->d_fieldV.ensure((size_t)s->nfields * ncell));
+    // packed beside the raw values first: a field that is refused leaves the
+    // resident one as it was
+    const size_t nv = (size_t)s->nfields * ncell;
+    TRY(s->d_raw.ensure((size_t)nsrc + nv));
+    TRY(s->d_fieldV.ensure(nv));
+    float *const packed = s->d_raw.p + nsrc;
     for (int f = 0; f < s->nfields; ++f) {
         CUDA_TRY(cudaMemcpyAsync(s->d_raw.p, fv + f * nsrc, nsrc * sizeof(float), cudaMemcpyHostToDevice, s->stream));
-        const int rc = launch_pack_T(s->d_raw.p, s->d_fieldV.p + f * ncell, c.imax, c.jmax, c.kmax, 1, sj, sk, base,
-                                     s->stream);
+        const int rc = launch_pack_T(s->d_raw.p, packed + f * ncell, c.imax, c.jmax, c.kmax, 1, sj, sk, base, s->stream);
         if (rc) return fail(DNSMC_ERR_CUDA, "pack launch: %s", cudaGetErrorString((cudaError_t)rc));
     }
+    double st[4];
+    TRY(field_stats(s, STATS_V, packed, (long long)nv, st));
+    if (st[3] > 0.0) return fail(DNSMC_ERR_ARG, "volume fractions must be finite and >= 0");
+    CUDA_TRY(cudaMemcpyAsync(s->d_fieldV.p, packed, nv * sizeof(float), cudaMemcpyDeviceToDevice, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
+    const float vmax = (float)st[0];
+    const double vsum = st[2];
     s->fv_fields = s->nfields;
     s->fv_max = vmax;
     s->fv_mean = vsum / ((double)s->nfields * ncell);
@@ -2295,29 +2303,57 @@ int dnsmc_wait(dnsmc_solver *s, double timeout_s) {
     return wait_done(s, timeout_s);
 }
 
-// Host copy of a large result array on several threads: the caller's array
-// is often freshly allocated, and its first-touch page faults dominate a
-// single-threaded copy.
-static void parallel_copy(void *dst, const void *src, size_t bytes) {
-    const size_t chunk = (size_t)2 << 20;
-    const unsigned nt = (unsigned)std::min<size_t>(8, (bytes + chunk - 1) / chunk);
-    if (nt <= 1) { memcpy(dst, src, bytes); return; }
+// Make the pages of a caller's array present before the copy engine writes
+// them (its own faults on pages never touched cost 10 ms for 16 MB): one write
+// a page, on a thread for every 4 MB, 4 at most.  The copy overwrites it all.
+static void touch_pages(void *dst, size_t bytes) {
+    const size_t page = 4096, nt = std::min<size_t>(4, std::max<size_t>(1, bytes >> 22));
+    const size_t per = (bytes / nt + page) / page * page;
+    auto part = [=](size_t a) {
+        const size_t e = std::min(bytes, a + per);
+        for (size_t o = a; o < e; o += page) static_cast<volatile char *>(dst)[o] = 0;
+        if (a < e) static_cast<volatile char *>(dst)[e - 1] = 0;
+    };
     std::vector<std::thread> th;
-    const size_t per = (bytes / nt + 4095) & ~(size_t)4095;
-    for (unsigned t = 0; t < nt; ++t) {
-        const size_t o = (size_t)t * per;
-        if (o >= bytes) break;
-        const size_t len = std::min(per, bytes - o);
-        th.emplace_back([=] { memcpy((char *)dst + o, (const char *)src + o, len); });
+    for (size_t t = 1; t < nt; ++t) {
+        try {
+            th.emplace_back(part, t * per);
+        } catch (...) {
+            part(t * per);
+        }
     }
+    part(0);
     for (auto &x : th) x.join();
 }
 
+// The last solve's results into the caller's arrays, from the device: the copy
+// engine writes present pages of the coherent host as fast as pinned memory (8
+// MB into pages in use 54 us, into new ones 440 us; a host copy from the
+// solve's pinned buffers 257 and 534 us, a thread 45 us to start).  Below 512
+// KB the host copy from those (hQ, hsigma) is shorter than two copies' launch.
+static int results_out(dnsmc_solver *s, void *Q, void *sigma, const void *hQ, const void *hsigma, const void *dQ,
+                       const void *dsigma, size_t bytes) {
+    if (bytes < ((size_t)512 << 10)) {
+        if (Q) memcpy(Q, hQ, bytes);
+        if (sigma) memcpy(sigma, hsigma, bytes);
+        return DNSMC_OK;
+    }
+    TRY(set_device(s));
+    if (Q) touch_pages(Q, bytes);
+    if (Q) CUDA_TRY(cudaMemcpyAsync(Q, dQ, bytes, cudaMemcpyDeviceToHost, s->stream));
+    if (sigma) touch_pages(sigma, bytes);
+    if (sigma) CUDA_TRY(cudaMemcpyAsync(sigma, dsigma, bytes, cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return DNSMC_OK;
+}
+
 // Rows of imax floats of a dense (imax, jl, kmax) block into the interior
-// of a Fortran array (0:imax+1, 0:jl+1, 0:kmax+1), several threads over k.
+// of a Fortran array (0:imax+1, 0:jl+1, 0:kmax+1): a thread for every 4 MB
+// (over k), since starting one costs as much as copying 1 MB.
 static void scatter_fortran(float *dst, const float *src, int imax, int jl, int kmax) {
     if (!dst) return;
-    const unsigned nt = (unsigned)std::max(1, std::min(8, kmax / 8));
+    const size_t bytes = (size_t)imax * jl * kmax * sizeof(float);
+    const unsigned nt = (unsigned)std::max<size_t>(1, std::min<size_t>(std::min(8, kmax), bytes >> 22));
     auto part = [=](int k0, int k1) {
         for (int k = k0; k < k1; ++k)
             for (int j = 0; j < jl; ++j)
@@ -2336,10 +2372,8 @@ int dnsmc_get_results(dnsmc_solver *s, double *Q, double *sigma) {
     TRY(wait_done(s, 0));
     if (s->solved_result_type != DNSMC_RESULT_F64)
         return fail(DNSMC_ERR_STATE, "the last solve returned float results: use dnsmc_get_results_float");
-    const size_t n = (size_t)s->nfields * s->last.region_cells;
-    if (Q) parallel_copy(Q, s->h_Q.p, n * sizeof(double));
-    if (sigma) parallel_copy(sigma, s->h_sig.p, n * sizeof(double));
-    return DNSMC_OK;
+    const size_t n = (size_t)std::min(s->nfields, s->last.nfields) * s->last.region_cells;
+    return results_out(s, Q, sigma, s->h_Q.p, s->h_sig.p, s->d_Q.p, s->d_sig.p, n * sizeof(double));
 }
 
 int dnsmc_set_result_type(dnsmc_solver *s, int type) {
@@ -2354,10 +2388,9 @@ int dnsmc_get_results_float(dnsmc_solver *s, float *Q, float *sigma) {
     if (!s) return fail(DNSMC_ERR_ARG, "null solver");
     if (!s->solved) return fail(DNSMC_ERR_STATE, "no solve has been run");
     TRY(wait_done(s, 0));
-    const size_t n = (size_t)s->nfields * s->last.region_cells;
+    const size_t n = (size_t)std::min(s->nfields, s->last.nfields) * s->last.region_cells;
     if (s->solved_result_type == DNSMC_RESULT_F32) {
-        if (Q) parallel_copy(Q, s->h_Qf.p, n * sizeof(float));
-        if (sigma) parallel_copy(sigma, s->h_sigf.p, n * sizeof(float));
+        return results_out(s, Q, sigma, s->h_Qf.p, s->h_sigf.p, s->d_Qf.p, s->d_sigf.p, n * sizeof(float));
     } else {
         for (size_t i = 0; i < n; ++i) {
             if (Q) Q[i] = (float)s->h_Q.p[i];

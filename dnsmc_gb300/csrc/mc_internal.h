@@ -381,11 +381,14 @@ int launch_pack_T4(const float *src, float *dst, int nw, int na, int nb, int pna
 int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
                    int na, int nb, long long si, long long sj, long long sk,
                    long long base, void *stream);
-// max T, min T, sum x and the count of non-positive or non-finite T over n
-// cells into out[0..3] (device), deterministic; out[4] is the kernel's counter
-// of finished blocks, zero before the first launch
-int launch_field_stats(const float *fT, const float2 *fTX, long long n,
-                       double *partials, double *out, void *stream);
+// Over n cells into out[0..3] (device), deterministic: the largest and
+// smallest value, a sum and a count of refused values -- of temperatures T
+// (STATS_T; not positive or not finite), of (T, x) pairs (STATS_TX; T as
+// before, the sum of x), of volume fractions (STATS_V; negative or not finite,
+// their sum).  out[4] is the kernel's counter of finished blocks, zero before
+// the first launch.
+enum { STATS_T, STATS_TX, STATS_V };
+int launch_field_stats(int kind, const float *v, long long n, double *partials, double *out, void *stream);
 int field_stats_partials();   // doubles needed in `partials`
 
 // Control-variate preparation (all stream-ordered).

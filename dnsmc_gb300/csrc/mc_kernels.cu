@@ -226,8 +226,8 @@ __global__ void pack_TX_kernel(const float *srcT, const float *srcX, float2 *dst
     }
 }
 
-// Tmax, Tmin, sum of x and the count of temperatures that are not positive
-// and finite, over n cells, in a fixed order (deterministic): a grid-strided
+// Extremes, sum and count of refused values of n cells (launch_field_stats) in
+// a fixed order (deterministic): a grid-strided
 // share per block, then the block that finishes last reduces the blocks' parts
 // as the threads' were: 9 us at 64^3 and 5 us at 8 x 32 x 4 (two launches, the
 // second one thread reading 256 parts in turn: 71 us).
@@ -248,8 +248,8 @@ __device__ __forceinline__ FieldStats stats_block(FieldStats v, FieldStats *s) {
     }
     return s[0];
 }
-__global__ void __launch_bounds__(kStatThreads) field_stats_kernel(const float *fT, const float2 *fTX, long long n,
-                                                                  FieldStats *part, double *out) {
+template <int KIND>
+__global__ void __launch_bounds__(kStatThreads) field_stats_kernel(const float *v, long long n, FieldStats *part, double *out) {
     __shared__ FieldStats s[kStatThreads];
     __shared__ bool last;
     // FP32 extremes and FP64 sums of this thread's share (few FP64
@@ -259,8 +259,9 @@ __global__ void __launch_bounds__(kStatThreads) field_stats_kernel(const float *
     int bad = 0;
     for (long long i = blockIdx.x * (long long)kStatThreads + threadIdx.x; i < n; i += (long long)gridDim.x * kStatThreads) {
         float T;
-        if (fTX) { const float2 v = fTX[i]; T = v.x; sm += v.y; } else { T = fT[i]; }
-        if (!(T > 0.0f) || !isfinite(T)) ++bad;
+        if (KIND == STATS_TX) { const float2 tx = reinterpret_cast<const float2 *>(v)[i]; T = tx.x; sm += tx.y; } else { T = v[i]; }
+        if (KIND == STATS_V) sm += T;
+        if (!(KIND == STATS_V ? T >= 0.0f : T > 0.0f) || !isfinite(T)) ++bad;
         mx = fmaxf(mx, T); mn = fminf(mn, T);
     }
     const FieldStats b = stats_block({(double)mx, (double)mn, sm, (double)bad}, s);
@@ -1121,11 +1122,13 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw, in
     return (int)cudaGetLastError();
 }
 
-int launch_field_stats(const float *fT, const float2 *fTX, long long n, double *partials, double *out,
-                       void *stream) {
+int launch_field_stats(int kind, const float *v, long long n, double *partials, double *out, void *stream) {
     cudaStream_t st = (cudaStream_t)stream;
     dnsmc::note_launch();
-    field_stats_kernel<<<kStatBlocks, kStatThreads, 0, st>>>(fT, fTX, n, reinterpret_cast<FieldStats *>(partials), out);
+    FieldStats *part = reinterpret_cast<FieldStats *>(partials);
+    if (kind == STATS_T) field_stats_kernel<STATS_T><<<kStatBlocks, kStatThreads, 0, st>>>(v, n, part, out);
+    else if (kind == STATS_TX) field_stats_kernel<STATS_TX><<<kStatBlocks, kStatThreads, 0, st>>>(v, n, part, out);
+    else field_stats_kernel<STATS_V><<<kStatBlocks, kStatThreads, 0, st>>>(v, n, part, out);
     return (int)cudaGetLastError();
 }
 

@@ -105,6 +105,37 @@ def test_bitexact_particles_scattering_grey_walls(cv):
     s.close()
 
 
+@pytest.mark.parametrize("bad", [-1e-9, math.nan, math.inf])
+def test_refused_volume_fractions_leave_the_resident_field(bad):
+    """The check runs on the device over the interior cells only: ghost cells
+    of the Fortran layout are not looked at, and a refused field changes
+    nothing."""
+    s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=12, jmax=32, kmax=5, Lx=2.0, Ly=6.28, Lz=3.14,
+                                  stretched_x=0, T_west=300, T_east=600, kappa=0.4, seed=3))
+    T = smooth_field(12, 32, 5, 400, 1200, 2)
+    s.set_fields(T)
+    s.set_particles(np.array([0.5e5], np.float32), np.array([1.0e5], np.float32), 0.3)
+    fv = np.zeros((5, 32, 12), np.float32)
+    fv[1:4] = 1e-5
+    s.set_particle_field(fv)
+    s.set_rays(8)
+    Q0, S0 = s.solve(timeout_s=60)
+    for at in ((0, 0, 0), (2, 17, 5), (4, 31, 11)):
+        v = fv.copy()
+        v[at] = bad
+        with pytest.raises(RuntimeError, match="volume fractions"):
+            s.set_particle_field(v)
+    Q1, S1 = s.solve(timeout_s=60)
+    np.testing.assert_array_equal(Q0, Q1)
+    np.testing.assert_array_equal(S0, S1)
+    f = np.full((7, 34, 14), bad, np.float32)
+    f[1:-1, 1:-1, 1:-1] = fv
+    s.set_particle_field(f, layout=D.LAYOUT_FORTRAN)
+    Q2, S2 = s.solve(timeout_s=60)
+    np.testing.assert_array_equal(Q0, Q2)
+    s.close()
+
+
 def test_equilibrium_is_exactly_zero():
     s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=16, jmax=32, kmax=4, Lx=2.0, Ly=6.28, Lz=3.14,
                                   stretched_x=0, T_west=900, T_east=900, eps_west=0.5, eps_east=0.3, kappa=0.7,
