@@ -285,6 +285,8 @@ struct dnsmc_solver {
     DevBuf<unsigned char> d_mgtab;           // splines: coefficients, brackets, positions
     DevBuf<float> d_mgtmp;                   // coarsening passes' intermediate fields
     DevBuf<double> d_mgwork;                 // lines too long for shared memory
+    DevBuf<int2> d_mgP;                      // their table coordinates (T tables)
+    long long mg_total = 0;                  // values of all levels and fields
     long long mg_off[kMaxLevels] = {0};
     int mg_fwoff[kMaxLevels] = {0};
     int mg_fields = 0;
@@ -988,6 +990,8 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.mg_levels = c.grid_num;
         P.mg_steps = c.mg_steps;
         P.mgT = s->d_mgT.p;
+        if (mode == MODE_T) TRY(s->d_mgP.ensure((size_t)s->mg_total));
+        P.mgP = s->d_mgP.p;
         P.mgfw = s->d_mgfw.p;
         for (int l = 1; l < c.grid_num; ++l) {
             P.mg_off[l] = s->mg_off[l];
@@ -1045,6 +1049,22 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
     fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
+    // the coarse levels' coordinates, all in one row
+    auto field_positions = [&]() -> int {
+        if (mode != MODE_GREY || gen) {
+            const int rc = launch_field_pos(fp, s->stream);
+            if (rc) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rc));
+        }
+        for (long long o = 0; mg && mode == MODE_T && o < s->mg_total; o += 1LL << 30) {
+            FieldPos q = fp;
+            q.fT = s->d_mgT.p + o; q.outP = s->d_mgP.p + o;
+            q.nfields = q.nw = q.nb = q.pnb = 1;
+            q.na = q.pna = (int)std::min(1LL << 30, s->mg_total - o);
+            const int rc = launch_field_pos(q, s->stream);
+            if (rc) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rc));
+        }
+        return DNSMC_OK;
+    };
     P.parts = 1;
     TRY(s->d_misc.ensure(kMiscWords));
     TRY(s->h_misc.ensure(kMiscWords));
@@ -1086,10 +1106,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.trace_f = tf; P.trace_g = tg; P.trace_p = tp; P.trace_r = tr; P.trace_max = tmax_steps;
         P.trace_rec = d_trace_rec; P.trace_n = d_trace_n; P.trace_rng = d_trace_rng;
         P.tally = nullptr;
-        if (mode != MODE_GREY || gen) {  // for the present packet shape
-            const int rcp = launch_field_pos(fp, s->stream);
-            if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
-        }
+        TRY(field_positions());  // for the present packet shape
         const int rc = mg ? launch_march_mg(mode, P, 1, 32, s->stream, true)
                           : launch_march_ex(mode, P, 1, 32, s->stream, true, cv, false, gen);
         if (rc) return fail(DNSMC_ERR_CUDA, "trace launch: %s", cudaGetErrorString((cudaError_t)rc));
@@ -1163,14 +1180,15 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.item_order = s->d_order.p;
     }
     const int sms = device_sm_count();
-    const size_t smem = mg ? march_smem(P, threads, 1) : march_pair_smem(P, threads);
-    const int occ = mg ? march_mg_occupancy(mode, threads, smem)
+    const size_t smem = mg ? march_mg_smem(P, threads) : march_pair_smem(P, threads);
+    const int occ = mg ? march_mg_occupancy(mode, P.uni != 0, threads, smem)
                        : march_occupancy_ex(mode, P.uni != 0, threads, cv, mom, gen, smem);
     const int blocks = std::max(1, sms * occ);
-    if (!mg && !mom && !P.rays_per_packet) {  // few items: their rays in several units
-        P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes);
+    if (!mom && !P.rays_per_packet) {  // few items: their rays in several units
+        const int cells = 32 * lane_cells(s);
+        P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes, cells);
         if (P.parts > 1) {
-            TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * 64)));
+            TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * cells)));
             TRY(s->d_misc.ensure((size_t)(kMiscWords + P.n_items)));
             P.rayx = s->d_rayx.p;
             P.queue = s->d_misc.p;
@@ -1218,10 +1236,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
 
     // ---- the kernel sequence of a solve (stream-ordered; capturable) -------
     auto kernels = [&](bool events) -> int {
-        if (mode != MODE_GREY || gen) {
-            const int rcp = launch_field_pos(fp, s->stream);
-            if (rcp) return fail(DNSMC_ERR_CUDA, "coordinate launch: %s", cudaGetErrorString((cudaError_t)rcp));
-        }
+        TRY(field_positions());
         if (cv) {
             int rc = launch_cv_prepare(cp, s->stream);
             if (rc == 0) rc = launch_cv_mean(cp, s->stream);
@@ -1482,6 +1497,7 @@ int upload_coarse(dnsmc_solver *s, int nfields, const float *src, int src_step) 
         }
     }
     s->mg_fields = nfields;
+    s->mg_total = off;
     return DNSMC_OK;
 }
 
@@ -1742,7 +1758,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();
     s->d_stat_part.release(); s->d_stat_out.release(); s->d_rays_pp.release(); s->d_rays_rcp.release(); s->d_item_steps.release(); s->d_kP.release();
     s->d_order.release(); s->d_order_hist.release();
-    s->d_mgT.release(); s->d_mgfw.release(); s->d_mgtab.release(); s->d_mgtmp.release(); s->d_mgwork.release();
+    s->d_mgT.release(); s->d_mgfw.release(); s->d_mgP.release(); s->d_mgtab.release(); s->d_mgtmp.release(); s->d_mgwork.release();
     s->d_part.release(); s->d_fieldV.release(); s->d_layerV.release();
     s->d_entries.release(); s->d_group_start.release(); s->d_group_empty.release();
     s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_sig.release(); s->h_sig.release(); s->d_Qg.release(); s->d_varg.release();

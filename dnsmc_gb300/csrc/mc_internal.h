@@ -115,6 +115,7 @@ struct MarchParams {
     // grid, 2x coarser per axis; level l has (nw, na, nb) >> l cells
     int mg_levels, mg_steps;
     const float *mgT;                  // coarse temperatures, level l at mg_off[l]: [f][i][k][j]
+    const int2 *mgP;                   // their table coordinates (T tables)
     const float *mgfw;                 // coarse wall-normal faces, level l at mg_fwoff[l]
     long long mg_off[kMaxLevels];
     int mg_fwoff[kMaxLevels];
@@ -305,7 +306,7 @@ int launch_march_ex(int mode, const MarchParams &p, int blocks, int threads, voi
                     bool mom, bool gen);
 int march_occupancy_ex(int mode, bool uni, int threads, bool cv, bool mom, bool gen, size_t smem);
 int launch_march_mg(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace);
-int march_mg_occupancy(int mode, int threads, size_t smem);
+int march_mg_occupancy(int mode, bool uni, int threads, size_t smem);
 // dynamic shared memory of a march launch with `cells` cells per lane: each
 // warp's table slab (slab_len float2), then per thread and cell the three
 // sums of the item (float pairs, 8 bytes), then per thread the RQMC replicate's shift (uint4)
@@ -320,6 +321,11 @@ constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {
     return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u + kBatchBytes) + (size_t)threads * 24u * kLaneCells;
 }
+// ... of the multigrid march: each warp's slab and ray batch, then a thread's sums
+constexpr size_t kMgBatchBytes = 1024;
+inline size_t march_mg_smem(const MarchParams &p, int threads) {
+    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kMgBatchBytes) + (size_t)threads * 24u;
+}
 // Queue units per item: an item is one warp's serial work over its rays, so
 // with few items the chip idles; units of at least one ray, about 16 per
 // resident warp.  warps: resident warps of the launch; cap_bytes: the most
@@ -330,9 +336,9 @@ inline size_t march_pair_smem(const MarchParams &p, int threads) {
 // unit per item: the sums stay in shared memory (128^3 with 8 band groups:
 // 262144 items, unchanged).
 constexpr long long kRayxBytes = 1LL << 30;
-inline int march_parts(long long n_items, int rays, long long warps, long long cap_bytes) {
+inline int march_parts(long long n_items, int rays, long long warps, long long cap_bytes, int cells = 64) {
     if (n_items < 1 || rays < 2 || n_items >= 16 * warps) return 1;
-    if (n_items * rays > cap_bytes / (64 * (long long)sizeof(float))) return 1;
+    if (n_items * rays > cap_bytes / (cells * (long long)sizeof(float))) return 1;
     const long long want = (16 * warps + n_items - 1) / n_items;
     return (int)(want < rays ? want : rays);
 }

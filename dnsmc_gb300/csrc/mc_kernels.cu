@@ -38,7 +38,7 @@
 // the same reason.  Tallies (sum X, sum X^2) are FP64.
 #include <atomic>
 
-#include "mc_march.cuh"
+#include "mc_march_mg.cuh"
 
 namespace dnsmc {
 
@@ -312,26 +312,13 @@ int march_occupancy_ex(int mode, bool uni, int threads, bool cv, bool mom, bool 
 int launch_march_mg(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace) {
     cudaStream_t st = (cudaStream_t)stream;
     if (trace) { blocks = 1; threads = 32; }
-    const size_t smem = march_smem(p, threads, 1);
-    if (mode == MODE_GREY) {
-        if (trace) return march_launch_one(march_mg_kernel<MODE_GREY, true>, blocks, threads,
-                                           smem, st, p);
-        return march_launch_one(march_mg_kernel<MODE_GREY, false>, blocks, threads, smem, st,
-                                p);
-    }
-    if (mode == MODE_T) {
-        if (trace) return march_launch_one(march_mg_kernel<MODE_T, true>, blocks, threads,
-                                           smem, st, p);
-        return march_launch_one(march_mg_kernel<MODE_T, false>, blocks, threads, smem, st, p);
-    }
-    return (int)cudaErrorInvalidValue;
+    const auto k = march_mg_fn(mode, p.uni != 0, p.parts > 1, trace);
+    return k ? march_launch_one(k, blocks, threads, march_mg_smem(p, threads), st, p) : (int)cudaErrorInvalidValue;
 }
 
-int march_mg_occupancy(int mode, int threads, size_t smem) {
-    int nb = 0;
-    if (mode == MODE_GREY)
-        nb = march_occupancy_one(march_mg_kernel<MODE_GREY, false>, threads, smem);
-    if (mode == MODE_T) nb = march_occupancy_one(march_mg_kernel<MODE_T, false>, threads, smem);
+int march_mg_occupancy(int mode, bool uni, int threads, size_t smem) {
+    const auto k = march_mg_fn(mode, uni, false, false);
+    const int nb = k ? march_occupancy_one(k, threads, smem) : 0;
     return nb > 0 ? nb : 1;
 }
 

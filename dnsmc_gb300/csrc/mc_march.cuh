@@ -1,9 +1,8 @@
 // mc_march.cuh -- the device helpers of the marches (Philox, Sobol', the
 // attenuation and trigonometric polynomials, table lookups, the control
-// variate's straight flight, the ray's words, direction, slab and tally),
-// the multigrid march (march_mg_kernel, instantiated in mc_kernels.cu) and
-// the launch helpers; the fine-grid two-cell marches are in
-// mc_march_pair.cuh.  The march translation units are compiled with
+// variate's straight flight, the ray's direction, slab and tally) and the
+// launch helpers; the fine-grid two-cell marches are in mc_march_pair.cuh, the
+// multigrid march in mc_march_mg.cuh.  The march translation units are compiled with
 // -fmad=false: the arithmetic is written with explicit fmaf so the host
 // replay (oracle/mc_oracle.cpp) reproduces every ray bit for bit; exp, log,
 // sin and cos are the project's own polynomial kernels for the same reason.
@@ -281,31 +280,8 @@ __device__ __forceinline__ void surrogate_lookup(const float4 *row, float sW, fl
 }
 
 // ---------------------------------------------------------------------------
-// Pieces shared by the marches (the multigrid march below and the two-cell
-// marches of mc_march_pair.cuh): the words of a packet-ray, its direction,
-// the copy of its spectral sample's table slab, one ray's tally.
+// Pieces shared by the marches: a packet-ray's direction, the copy of its spectral sample's table slab, one ray's tally.
 // ---------------------------------------------------------------------------
-
-// The ray's four uniform words.  RQMC: point m of replicate b = r / M of a
-// Sobol' net, XOR-shifted by the replicate's Philox word (kept in *shift and
-// recomputed when the replicate changes, *bcur); iid: one Philox call.
-__device__ __forceinline__ uint4 ray_words(const MarchParams &P, int r, int M, int p, uint32_t ctr2, int *bcur,
-                                          uint4 *shift, int *m_out) {
-    if (P.sampler) {
-        const int b = r / M;
-        const int m = r - b * M;
-        if (b != *bcur) {
-            *shift = philox4x32_10(make_uint4((uint32_t)b, (uint32_t)p, ctr2, 0x50B01u), P.key0, P.key1);
-            *bcur = b;
-        }
-        const uint4 sh = *shift;
-        const uint4 sb = sobol4((uint32_t)m);
-        *m_out = m;
-        return make_uint4(sb.x ^ sh.x, sb.y ^ sh.y, sb.z ^ sh.z, sb.w ^ sh.w);
-    }
-    *m_out = 0;
-    return philox4x32_10(make_uint4((uint32_t)r, (uint32_t)p, ctr2, 0u), P.key0, P.key1);
-}
 
 // Isotropic direction (the reference's emiss_ang, code/mc_gpu.cu:813-820):
 // cos(theta) = 1 - 2u from the top 24 bits of x.y, phi = 2 pi u' from x.x.
@@ -360,7 +336,7 @@ __device__ __forceinline__ bool slab_bar_wait(const uint64_t *bar, uint32_t pari
 // of 16 at a 16-byte aligned address on both sides) into this warp's shared
 // copy: slab_issue starts the copy once the previous ray's lookups are done
 // (the warp converges, and the async proxy is ordered after the generic
-// one), slab_wait waits for it, load_slab does both.  *phase is the warp's
+// one), slab_wait waits for it.  *phase is the warp's
 // barrier parity, flipped per completed copy.  The first wait polls
 // P.slab_polls0 times (kSlabWaitPolls; fewer only in tests of this path).
 // A wait that runs out sets DNSMC_STATUS_COPY_TIMEOUT (the host reports the
@@ -390,12 +366,6 @@ __device__ __forceinline__ bool slab_wait(const MarchParams &P, uint64_t *bar, u
     }
     *phase ^= 1u;
     return true;
-}
-
-__device__ __forceinline__ bool load_slab(const MarchParams &P, int sid, float2 *slk, int lane, uint64_t *bar,
-                                          uint32_t *phase, unsigned int *flags) {
-    slab_issue(P, sid, slk, lane, bar);
-    return slab_wait(P, bar, phase, flags);
 }
 
 // Before a warp whose copy did not arrive exits: one more bounded wait for
@@ -473,7 +443,8 @@ __device__ __forceinline__ bool unit_done(const MarchParams &P, long long item, 
 }
 
 // Sums of one cell of an item over its N rays in ray order (x: the cell's
-// first contribution, 64 values a ray), as tally_ray adds them.
+// first contribution, CELLS values a ray), as tally_ray adds them.
+template <int CELLS>
 __device__ __forceinline__ double2 sum_rays(const MarchParams &P, const float *x, int N, int M) {
     float2 sum = make_float2(0.0f, 0.0f), sq = sum, rep = sum;
     int m = 0;
@@ -481,7 +452,7 @@ __device__ __forceinline__ double2 sum_rays(const MarchParams &P, const float *x
         float v[8];
         const int n = min(8, N - r0);
 #pragma unroll
-        for (int q = 0; q < 8; ++q) v[q] = q < n ? __ldcg(x + (long long)(r0 + q) * 64) : 0.0f;
+        for (int q = 0; q < 8; ++q) v[q] = q < n ? __ldcg(x + (long long)(r0 + q) * CELLS) : 0.0f;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
             if (q < n) {
@@ -491,361 +462,6 @@ __device__ __forceinline__ double2 sum_rays(const MarchParams &P, const float *x
         }
     }
     return make_double2(ff_value(sum), ff_value(sq));
-}
-
-// ---------------------------------------------------------------------------
-// The multigrid march (grid_num > 1; the reference's grid switch,
-// code/mc_gpu.cu:193-207), one cell per lane, 32-cell packets: the absorbing
-// gas with black walls, grey or T tables, no control variate.  Persistent:
-// every warp pulls work items (field, band group, packet) from an atomic
-// counter.  The fine phase is the warp-uniform walk of the two-cell march
-// (mc_march_pair.cuh) for mg_steps steps; then every lane continues from its
-// own point on the coarser grids with the reference's position-update march.
-// ---------------------------------------------------------------------------
-// Resident blocks of 256 threads per SM the register allocation must allow
-// (2: up to 128 registers; 3: 85; 4: 64), chosen at build time.
-#ifndef DNSMC_MINB
-#define DNSMC_MINB 4
-#endif
-template <int MODE, bool TRACE>
-__global__ void __launch_bounds__(256, DNSMC_MINB) march_mg_kernel(const MarchParams P) {
-    typedef typename FieldT<MODE>::type VT;
-    const unsigned FULL = 0xffffffffu;
-    const float INF = __int_as_float(0x7f800000);
-    const int lane = threadIdx.x & 31;
-    const int la = lane % P.tile_a, lb = lane / P.tile_a;
-    const int njR = P.ea1 - P.ea0, nkR = P.eb1 - P.eb0;
-    const int plane = P.na * P.nb;
-    unsigned long long my_rays = 0, my_steps = 0;
-    unsigned int flags = 0;
-    const int tid = threadIdx.x;
-    // dynamic shared memory (march_smem, one cell per lane): this warp's copy
-    // of the current ray's table slab (tabulated models), the item's sums as
-    // float pairs [3][threads] and the replicate's shift [threads]
-    extern __shared__ float4 s_dyn[];
-    const int nthr = blockDim.x;
-    float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + (threadIdx.x >> 5) * P.slab_len;
-    const float2 *const sli = slk + P.slab_klen;
-    double *const s_acc = reinterpret_cast<double *>(reinterpret_cast<float2 *>(s_dyn) + ((nthr + 31) >> 5) * P.slab_len);
-    uint4 *const s_shift = reinterpret_cast<uint4 *>(s_acc + 3 * nthr);
-    // each warp's transaction barrier of its slab copies, and its parity
-    __shared__ uint64_t s_bar[8];
-    uint64_t *const sbar = &s_bar[threadIdx.x >> 5];
-    uint32_t sphase = 0;
-    slab_bar_init(sbar, lane);
-    bool dead = false;  // a slab copy did not arrive: this warp stops marching
-
-    for (;;) {
-        long long item;
-        if (TRACE) {
-            if (threadIdx.x >= 32) return;
-            item = ((long long)P.trace_f * P.n_groups + P.trace_g) * P.n_packets + P.trace_p;
-        } else {
-            unsigned int it = 0;
-            if (lane == 0) it = atomicAdd(P.queue, 1u);
-            it = __shfl_sync(FULL, it, 0);
-            if ((long long)it >= P.n_items) break;
-            item = P.item_order ? (long long)__ldg(P.item_order + it) : (long long)it;
-        }
-        const int p = (int)(item % P.n_packets);
-        const long long fg = item / P.n_packets;
-        const int G = (int)(fg % P.n_groups);
-        const int f = (int)(fg / P.n_groups);
-        const int pa = p % P.npa;
-        const int rest = p / P.npa;
-        const int pb = rest % P.npb;
-        const int pw = rest / P.npb;
-        const int w0 = P.ew0 + pw;
-        const int a0 = P.ea0 + pa * P.tile_a + la;
-        const int b0 = P.eb0 + pb * P.tile_b + lb;
-        const bool active = (a0 < P.ea1) && (b0 < P.eb1);
-        const int acl = active ? a0 : P.ea0, bcl = active ? b0 : P.eb0;
-        const int N = P.rays_per_packet ? P.rays_per_packet[G * P.rays_gstride + p] : P.rays;
-        const long long fbase = (long long)f * P.field_stride;
-        const int rowW0 = w0 * plane;
-        // own-cell quantities
-        const VT vown = load_field<MODE>(P, fbase, rowW0 + bcl * P.na + acl);
-        float Ti4 = 0.f, tpos0 = 0.f;
-        int ti_i = 0, ki_i = 0;
-        float ft_i = 0.f, fx_i = 0.f;
-        if constexpr (MODE == MODE_GREY) {
-            const float Ti = vown;
-            if (!(Ti > 0.0f) && active) flags |= DNSMC_STATUS_BAD_FIELD;
-            const float t2 = Ti * Ti;
-            Ti4 = t2 * t2;
-        } else {
-            cell_coords<MODE>(vown, &ki_i, &ti_i, &ft_i, &fx_i);
-            tpos0 = (float)ti_i + ft_i;  // the clamped table coordinate, exactly
-        }
-        const float oW = (__ldg(P.fw + w0) + __ldg(P.fw + w0 + 1)) * 0.5f;
-        // alias table of this packet: band group G of the temperature bin
-        // nearest to lane 0's temperature (one bin when sampling at Tmax)
-        int gs = 0, K = 1;
-        if (MODE != MODE_GREY) {
-            int boff = 0;
-            if (P.n_tbins > 1) {
-                const float tp0 = __shfl_sync(FULL, tpos0, 0);
-                int bin = __float2int_rn(tp0);
-                bin = min(max(bin, 0), P.n_tbins - 1);
-                boff = bin * P.n_groups;
-            }
-            gs = P.group_start[boff + G];
-            K = P.group_start[boff + G + 1] - gs;
-        }
-        const uint32_t ctr2 = (uint32_t)G | ((uint32_t)(f + P.field_base) << 16);
-        const long long tc = ((long long)(w0 - P.ew0) * nkR + (bcl - P.eb0)) * njR + (acl - P.ea0);
-        const long long cell_out = fg * P.region_cells + tc;  // tally index of this lane's cell
-        const int M = P.sampler ? max(1, N / max(1, P.nbatch)) : 1;
-        s_acc[tid] = 0.0; s_acc[nthr + tid] = 0.0; s_acc[2 * nthr + tid] = 0.0;
-        unsigned long long isteps = 0;
-        unsigned int lsteps = 0;  // this lane's active steps in the item
-        int bcur = -1;
-        const int rbeg = TRACE ? P.trace_r : 0;
-        const int rend = TRACE ? P.trace_r + 1 : ((K > 0) ? N : 0);
-        for (int r = rbeg; r < rend; ++r) {
-            int m;
-            const uint4 x = ray_words(P, r, M, p, ctr2, &bcur, &s_shift[tid], &m);
-            if (TRACE && lane == 0) {
-                P.trace_rng[0] = x.x; P.trace_rng[1] = x.y; P.trace_rng[2] = x.z; P.trace_rng[3] = x.w;
-            }
-            float sW, sA, sB;
-            ray_direction(x, &sW, &sA, &sB);
-
-            // spectral sample and ray weight (the ray contributes wk D, D the
-            // net exchange in intensity units)
-            float wk, Ii;
-            int nbnd = 0;
-            if (MODE == MODE_GREY) {
-                Ii = Ti4;
-                wk = P.Wgrey;
-            } else {
-                const int j = (int)__umulhi(x.z, (uint32_t)K);
-                SpecEntry e = P.entries[gs + j];
-                if (!(u24(x.w) < e.prob)) e = P.entries[gs + (int)(e.alias_nb & 0xFFFFu)];
-                nbnd = (int)(e.alias_nb >> 16);
-                if (!load_slab(P, e.koff, slk, lane, sbar, &sphase, &flags)) { dead = true; break; }
-                const float ki = lookup_k<MODE>(slk, ki_i, ft_i, fx_i);
-                Ii = lookup_ib(sli, ti_i, ft_i);
-                wk = e.W * ki;
-            }
-
-            // fine phase: the warp-uniform DDA from the cell centres
-            const float invW = 1.0f / fabsf(sW), invA = 1.0f / fabsf(sA), invB = 1.0f / fabsf(sB);
-            const int dW = sW > 0.f ? 1 : -1, dA = sA > 0.f ? 1 : -1, dB = sB > 0.f ? 1 : -1;
-            int cw = w0, ca = acl, cb = bcl;
-            float tW = (dW > 0 ? (__ldg(P.fw + cw + 1) - oW) : (oW - __ldg(P.fw + cw))) * invW;
-            const float dtA = P.da * invA, dtB = P.db * invB;
-            float tA = 0.5f * dtA, tB = 0.5f * dtB;
-            int nA = 0, nB = 0;
-            float t = 0.0f;
-            int rowW = rowW0, rowB = cb * P.na;
-            float tau = active ? 1.0f : 0.0f;
-            float D = 0.0f;
-            int steps = 0;
-            VT vcur = vown;
-            for (;;) {
-                int axis;
-                float tn;
-                if (tW <= tA && tW <= tB) { axis = 0; tn = tW; }
-                else if (tA <= tB)         { axis = 1; tn = tA; }
-                else                       { axis = 2; tn = tB; }
-                const float ds = tn - t;
-                // next cell of the walk, and its field value fetched now
-                int ncw = cw, nca = ca, ncb = cb, nrowW = rowW, nrowB = rowB;
-                bool wall = false;
-                if (axis == 0) {
-                    ncw = cw + dW;
-                    wall = ncw < 0 || ncw >= P.nw;
-                    nrowW = ncw * plane;
-                } else if (axis == 1) {
-                    nca = ca + dA;
-                    if (nca == P.na) nca = 0; else if (nca < 0) nca = P.na - 1;
-                } else {
-                    ncb = cb + dB;
-                    if (ncb == P.nb) ncb = 0; else if (ncb < 0) ncb = P.nb - 1;
-                    nrowB = ncb * P.na;
-                }
-                VT vnext = vcur;
-                if (!wall && tau > 0.0f) vnext = load_field<MODE>(P, fbase, nrowW + nrowB + nca);
-                if (tau > 0.0f) {
-                    ++lsteps;
-                    float kj, gj;
-                    if constexpr (MODE == MODE_GREY) {
-                        const float t2 = vcur * vcur;
-                        gj = Ti4 - t2 * t2;
-                        kj = P.kappa;
-                    } else {
-                        int kx, tj;
-                        float ftj, fxj;
-                        cell_coords<MODE>(vcur, &kx, &tj, &ftj, &fxj);
-                        kj = lookup_k<MODE>(slk, kx, ftj, fxj);
-                        const float Ibj = lookup_ib(sli, tj, ftj);
-                        gj = Ii - Ibj;
-                    }
-                    const float alpha = -mc_expm1(-(kj * ds));
-                    const float ta = tau * alpha;
-                    D = fmaf(ta, gj, D);
-                    tau = tau - ta;
-                    if (tau < P.toll) { D = fmaf(tau, gj, D); tau = 0.0f; }
-                }
-                if (TRACE && lane == 0 && steps < P.trace_max) {
-                    int *rec = P.trace_rec + 6 * steps;
-                    rec[0] = cw; rec[1] = dA * nA; rec[2] = dB * nB; rec[3] = axis;
-                    rec[4] = __float_as_int(ds); rec[5] = __float_as_int(tau);
-                }
-                t = tn;
-                ++steps;
-                if (axis == 0) {
-                    if (wall) {
-                        const int side = ncw < 0 ? 0 : 1;
-                        const float Iw = (MODE == MODE_GREY) ? P.Tw4[side] : __ldg(P.ibw + side * P.nbands + nbnd);
-                        if (tau > 0.0f) {
-                            D = fmaf(tau, Ii - Iw, D);
-                            tau = 0.0f;
-                        }
-                        break;
-                    }
-                    cw = ncw;
-                    rowW = nrowW;
-                    tW = (dW > 0 ? (__ldg(P.fw + cw + 1) - oW) : (oW - __ldg(P.fw + cw))) * invW;
-                } else if (axis == 1) {
-                    ++nA;
-                    tA = ((float)nA + 0.5f) * dtA;
-                    ca = nca;
-                } else {
-                    ++nB;
-                    tB = ((float)nB + 0.5f) * dtB;
-                    cb = ncb;
-                    rowB = nrowB;
-                }
-                vcur = vnext;
-                if (!__any_sync(FULL, tau > 0.0f)) break;
-                if (steps >= P.mg_steps) break;
-            }
-            {
-                // Coarse grids (the reference's grid switch, code/mc_gpu.cu:193-207):
-                // every lane continues from its own point with the reference's
-                // position-update march; lanes no longer share their cell
-                // faces, but they step in lockstep and leave a level together.
-                if (__any_sync(FULL, tau > 0.0f)) {
-                    const float ua = t / dtA - (float)nA, ub = t / dtB - (float)nB;
-                    const float fa = fminf(fmaxf(dA > 0 ? 0.5f + ua : 0.5f - ua, 0.0f), 1.0f);
-                    const float fb = fminf(fmaxf(dB > 0 ? 0.5f + ub : 0.5f - ub, 0.0f), 1.0f);
-                    float xp = fmaf(sW, t, oW);
-                    float yp = ((float)ca + fa) * P.da;
-                    float zp = ((float)cb + fb) * P.db;
-                    int ic = cw, jc = ca, kc = cb;
-                    const float isx = 1.0f / sW, isy = 1.0f / sA, isz = 1.0f / sB;
-                    int counter = 0, cap = 0;
-                    for (int l = 1; l < P.mg_levels; ++l) {
-                        ic >>= 1; jc >>= 1; kc >>= 1;
-                        const int nwL = P.nw >> l, naL = P.na >> l, nbL = P.nb >> l;
-                        const float *fwL = P.mgfw + P.mg_fwoff[l];
-                        const float daL = P.mg_da[l], dbL = P.mg_db[l];
-                        const float *TL = P.mgT + P.mg_off[l] + (long long)f * nwL * naL * nbL;
-                        cap = (l == P.mg_levels - 1) ? P.max_steps : P.mg_steps;
-                        counter = 0;
-                        while (__any_sync(FULL, tau > 0.0f && counter < cap)) {
-                            float dsr = 0.0f;  // this lane's segment (0 when it idles)
-                            if (tau > 0.0f && counter < cap) {
-                                const float fx = __ldg(fwL + (dW > 0 ? ic + 1 : ic));
-                                const float fy = (float)(dA > 0 ? jc + 1 : jc) * daL;
-                                const float fz = (float)(dB > 0 ? kc + 1 : kc) * dbL;
-                                const float dsx = sW != 0.0f ? (fx - xp) * isx : INF;
-                                const float dsy = sA != 0.0f ? (fy - yp) * isy : INF;
-                                const float dsz = sB != 0.0f ? (fz - zp) * isz : INF;
-                                const float Tc = __ldg(TL + ((long long)ic * nbL + kc) * naL + jc);
-                                float kj, gj;
-                                if constexpr (MODE == MODE_GREY) {
-                                    const float t2 = Tc * Tc;
-                                    gj = Ti4 - t2 * t2;
-                                    kj = P.kappa;
-                                } else {
-                                    float pt = (Tc - P.T0) * P.invdT;
-                                    pt = fminf(fmaxf(pt, 0.0f), (float)(P.nT - 1));
-                                    int tj;
-                                    float ftj;
-                                    pos_split(pt, P.nT, &tj, &ftj);
-                                    kj = lookup_k<MODE_T>(slk, tj, ftj, 0.0f);
-                                    gj = Ii - lookup_ib(sli, tj, ftj);
-                                }
-                                float dmin = dsx;
-                                if (dmin > dsy) dmin = dsy;
-                                if (dmin > dsz) dmin = dsz;
-                                const float ds = fmaxf(dmin, 0.0f);
-                                dsr = ds;
-                                xp = (dmin == dsx) ? fx : fmaf(ds, sW, xp);
-                                yp = (dmin == dsy) ? fy : fmaf(ds, sA, yp);
-                                zp = (dmin == dsz) ? fz : fmaf(ds, sB, zp);
-                                const float alpha = -mc_expm1(-(kj * ds));
-                                const float ta = tau * alpha;
-                                D = fmaf(ta, gj, D);
-                                tau = tau - ta;
-                                if (tau < P.toll) { D = fmaf(tau, gj, D); tau = 0.0f; }
-                                int axis;
-                                if (dsx < dsy) axis = (dsx < dsz) ? 0 : 2;
-                                else axis = (dsy < dsz) ? 1 : 2;
-                                if (axis == 0) {
-                                    ic += dW;
-                                    if (ic < 0 || ic >= nwL) {
-                                        const int side = ic < 0 ? 0 : 1;
-                                        const float Iw = (MODE == MODE_GREY) ? P.Tw4[side]
-                                                                             : __ldg(P.ibw + side * P.nbands + nbnd);
-                                        if (tau > 0.0f) D = fmaf(tau, Ii - Iw, D);
-                                        tau = 0.0f;
-                                        ic = ic < 0 ? 0 : nwL - 1;
-                                    }
-                                } else if (axis == 1) {
-                                    jc += dA;
-                                    if (jc >= naL) { jc = 0; yp = 0.0f; } else if (jc < 0) { jc = naL - 1; yp = P.Ly; }
-                                } else {
-                                    kc += dB;
-                                    if (kc >= nbL) { kc = 0; zp = 0.0f; } else if (kc < 0) { kc = nbL - 1; zp = P.Lz; }
-                                }
-                                ++lsteps;
-                            }
-                            if (TRACE && lane == 0 && steps < P.trace_max) {  // every iteration
-                                int *rec = P.trace_rec + 6 * steps;
-                                rec[0] = ic; rec[1] = jc; rec[2] = kc; rec[3] = 16 + l;
-                                rec[4] = __float_as_int(dsr); rec[5] = __float_as_int(tau);
-                            }
-                            ++counter;
-                            ++steps;
-                        }
-                    }
-                    if (tau > 0.0f) flags |= DNSMC_STATUS_STEP_CAP;
-                }
-            }
-            if (TRACE && lane == 0) *P.trace_n = steps;
-            isteps += (unsigned long long)steps;
-            const float X = wk * D;
-            if (active) {
-                ++my_rays;
-                if (!isfinite(X)) flags |= DNSMC_STATUS_NONFINITE;
-                tally_ray(P, X, m, M, reinterpret_cast<float2 *>(&s_acc[tid]), reinterpret_cast<float2 *>(&s_acc[nthr + tid]),
-                          reinterpret_cast<float2 *>(&s_acc[2 * nthr + tid]));
-            }
-        }
-        if (dead) break;  // the item's sums are incomplete; the solve fails
-        my_steps += lsteps;
-        if (TRACE) return;
-        if (P.item_steps && lane == 0) P.item_steps[item] = isteps;
-        if (active)
-            P.tally[cell_out] = make_double2(ff_value(*reinterpret_cast<const float2 *>(&s_acc[tid])),
-                                             ff_value(*reinterpret_cast<const float2 *>(&s_acc[nthr + tid])));
-    }
-    if (dead) slab_drain(sbar, sphase);
-    // per-warp counters and status
-    for (int o = 16; o > 0; o >>= 1) {
-        my_rays += __shfl_xor_sync(FULL, my_rays, o);
-        my_steps += __shfl_xor_sync(FULL, my_steps, o);
-        flags |= __shfl_xor_sync(FULL, flags, o);
-    }
-    if (lane == 0) {
-        if (my_rays) atomicAdd(P.counters + 0, my_rays);
-        if (my_steps) atomicAdd(P.counters + 1, my_steps);
-        if (flags) atomicOr(P.status, flags);
-    }
 }
 
 // Dynamic shared memory of a march kernel: a kernel whose static plus

@@ -678,7 +678,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
             if (unit_done(P, item, lane)) {
 #pragma unroll
                 for (int k = 0; k < C; ++k)
-                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays(P, rayx + 32 * k, K > 0 ? N : 0, M);
+                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays<64>(P, rayx + 32 * k, K > 0 ? N : 0, M);
             }
             continue;
         }
@@ -1136,7 +1136,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
             if (unit_done(P, item, lane)) {
 #pragma unroll
                 for (int k = 0; k < C; ++k)
-                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays(P, rayx + 32 * k, K > 0 ? N : 0, M);
+                    if (active[k]) P.tally[fg * P.region_cells + tcell[k]] = sum_rays<64>(P, rayx + 32 * k, K > 0 ? N : 0, M);
             }
             continue;
         }

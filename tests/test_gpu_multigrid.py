@@ -17,6 +17,7 @@ import numpy as np
 import pytest
 
 import dnsmc_gb300 as D
+from dnsmc_gb300 import synth
 from oracle import oracle as O
 from tables_io import write_ck_tables, write_particle_tables
 from test_gpu_parity import assert_bitexact, smooth_field
@@ -124,6 +125,36 @@ def test_bitexact_ck_tables_multigrid_stretched(tmp_path, ck_tables):
     T = smooth_field(16, 32, 8, 550, 1000, 8)
     s.set_fields(T)
     s.set_rays(16)
+    assert_bitexact(s, T)
+    assert traces_reach_coarse_levels(s, T) > 0
+    s.close()
+
+
+@pytest.mark.parametrize("per_packet", [False, True])
+@pytest.mark.parametrize("model,shape,levels,steps", [("grey", (16, 24, 12), 3, 2), ("bands", (16, 32, 8), 4, 1),
+                                                      ("bands", (8, 8, 8), 4, 5), ("table", (12, 20, 4), 3, 3)])
+def test_bitexact_whole_and_split_items(model, shape, levels, steps, per_packet):
+    """Uniform rays on small grids go through split items, per-packet rays
+    through whole ones; grey-band tables take their constant absorption
+    coefficient, other tables look it up.  Down to one coarse cell an axis."""
+    ni, nj, nk = shape
+    cfg = dict(imax=ni, jmax=nj, kmax=nk, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=1, T_west=400, T_east=700, seed=21,
+               grid_num=levels, mg_steps=steps, kappa=0.8, nvar=2)
+    if model == "grey":
+        s = D.Solver(D.default_config(model=D.MODEL_GREY, **cfg))
+    elif model == "bands":
+        s = D.Solver(D.default_config(model=D.MODEL_GREY_BANDS, **cfg))
+        s.use_grey_band_tables(60, 30)
+    else:
+        tb = synth.ck_table(nbands=12, nq=4, nT=24, nX=5, seed=6)
+        s = D.Solver(D.default_config(model=D.MODEL_TABLE, n_groups=3, sampler=D.SAMPLER_RQMC, local_sampling=1, **cfg))
+        s.set_table(0.05 * tb["k"][..., 2], tb["wvc"], tb["T0"], tb["dT"], dnu=tb["dnu"], wq=tb["wq"])
+    T = smooth_field(ni, nj, nk, 500, 1300, 4)
+    s.set_fields(T)
+    if per_packet:
+        s.set_rays(0, np.random.default_rng(2).integers(1, 20, s.packet_count()).astype(np.int32) * 2)
+    else:
+        s.set_rays(38)
     assert_bitexact(s, T)
     assert traces_reach_coarse_levels(s, T) > 0
     s.close()
