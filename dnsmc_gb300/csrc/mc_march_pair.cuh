@@ -53,9 +53,11 @@ namespace dnsmc {
 // it knows the cells ahead, so a cell's field value is fetched two steps
 // before it is used.
 // March of the 128^3 correlated-k channel (48 rays): 85.5 -> 66.2 ms; grey 64^3
-// channel at 256 rays: 9.6 -> 4.9 ms.
+// channel at 256 rays: 9.6 -> 4.9 ms.  Chunks of 64 / 96 / 128 / 192 steps:
+// channel 62.5 / 61.9 / 61.6 / 61.7, grey 3.53 / 3.45 / 3.38 / 3.34 ms (longer
+// chunks take more shared memory a warp).
 // ---------------------------------------------------------------------------
-constexpr int kWalkCap = 64;  // steps of a chunk (even)
+constexpr int kWalkCap = 128;  // steps of a chunk (even)
 // words of a warp's walk buffer: a 4-word header whose last word is the cell
 // entered by the chunk's first step, the pairs (one spare), the wall-normal
 // times of the chunk, the state after it (kWalkWords in all)
