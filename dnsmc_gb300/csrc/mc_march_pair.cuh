@@ -311,12 +311,12 @@ __device__ __forceinline__ const typename FieldT<MODE>::type *field_base(const M
 
 // Resident 256-thread blocks per SM.  Tables: 2 (128 registers: the values of
 // four steps of two cells; 3 spill, 66.2 -> 70.1 ms on the 128^3 channel).
-// UNI: 3 (grey) and 4 (band tables): its steps are short, so the walk's
-// generation and the gathers need more warps to hide behind -- grey 64^3
-// 4.32 (2) / 3.51 (3) / 3.62 ms (4), grey bands through the drop-in pair 9.43 /
-// 9.12 / 8.65 ms.  Moments (18 FP64 sums a lane): 2.
-__host__ __device__ constexpr int pair_min_blocks(int mode, bool uni, bool mom) {
-    return uni && !mom ? (mode == MODE_GREY ? 3 : 4) : DNSMC_PAIR_MINB;
+// UNI: 4 (64 registers): its steps are short, so the walk's generation and the
+// gathers need more warps to hide behind -- grey 64^3 4.00 (2) / 3.12 (3) / 2.99
+// ms (4), grey bands through the drop-in pair 8.34 / 7.59 / 7.29 ms.  Moments (18
+// FP64 sums a lane): 2.
+__host__ __device__ constexpr int pair_min_blocks(bool uni, bool mom) {
+    return uni && !mom ? 4 : DNSMC_PAIR_MINB;
 }
 
 // UNI: the absorption coefficient is the same everywhere (grey model, grey
@@ -325,7 +325,7 @@ __host__ __device__ constexpr int pair_min_blocks(int mode, bool uni, bool mom) 
 // gather, one difference and one fused multiply-add.  SPLIT: items in
 // several queue units (MarchParams::parts).
 template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT>
-__global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pair_kernel(const MarchParams P) {
+__global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_kernel(const MarchParams P) {
     typedef typename FieldT<MODE>::type VT;
     constexpr int C = kLaneCells;  // cells per lane
     static_assert(C == 2, "the attenuation goes through a cell pair");
@@ -526,22 +526,23 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
                 // instructions with every sign moved onto an operand whose
                 // negation is exact: e = expm1(k * (t - tn)) = -alpha, nta =
                 // tau e = -ta, D += nta (-g), tau += nta -- the same roundings.
+                auto neg_g = [&](const VT &v, int k) {  // UNI: -g of cell k
+                    if constexpr (MODE == MODE_GREY) {
+                        return v - Ii[k];
+                    } else {
+                        int kx, tj;
+                        float ftj, fxj;
+                        cell_coords<MODE>(v, &kx, &tj, &ftj, &fxj);
+                        return lookup_ib(sli, tj, ftj) - Ii[k];
+                    }
+                };
                 auto step = [&](const VT (&v)[C], float nds, int s) {
                     if constexpr (UNI) {
                         const float nta = tau[0] * nds;  // nds: expm1 of the step
                         float ng[C];
 #pragma unroll
                         for (int k = 0; k < C; ++k) {
-                            float Ibj;
-                            if constexpr (MODE == MODE_GREY) {
-                                Ibj = v[k];
-                            } else {
-                                int kx, tj;
-                                float ftj, fxj;
-                                cell_coords<MODE>(v[k], &kx, &tj, &ftj, &fxj);
-                                Ibj = lookup_ib(sli, tj, ftj);
-                            }
-                            ng[k] = Ibj - Ii[k];
+                            ng[k] = neg_g(v[k], k);
                             D[k] = fmaf(nta, ng[k], D[k]);
                         }
                         tau[0] = tau[0] + nta;
@@ -596,6 +597,18 @@ __global__ void __launch_bounds__(256, pair_min_blocks(MODE, UNI, MOM)) march_pa
                     for (int k = 0; k < C; ++k) v3[k] = __ldg(fp[k] + o3);
                     const float d0 = wc.x, d1 = wc.z;
                     wc = *++wp;
+                    if constexpr (UNI && !TRACE) {
+                        // the two steps at once unless one of them ends the ray (the
+                        // checks of both in one branch: grey 64^3 3.39 -> 3.12 ms)
+                        const float n0 = tau[0] * d0, t0 = tau[0] + n0, n1 = t0 * d1, t1 = t0 + n1;
+                        if (t0 >= P.toll && t1 >= P.toll) {
+#pragma unroll
+                            for (int k = 0; k < C; ++k) D[k] = fmaf(n1, neg_g(v1[k], k), fmaf(n0, neg_g(v0[k], k), D[k]));
+                            tau[0] = t1;
+                            s += 2;
+                            return;
+                        }
+                    }
                     step(v0, d0, steps + s);
                     if (UNI && done) return;
                     step(v1, d1, steps + s + 1);
