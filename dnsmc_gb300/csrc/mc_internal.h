@@ -315,7 +315,7 @@ inline size_t march_smem(const MarchParams &p, int threads, int cells) {
 }
 // of a launch of the gas march: each warp's slab, walk buffer and ray batch, then per
 // thread the sums of its two cells; kPairStaticSmem at most beside it
-constexpr int kWalkWords = 304;  // words of a warp's walk buffer (mc_march_pair.cuh)
+constexpr int kWalkWords = 336;  // words of a warp's walk buffer (mc_march_pair.cuh)
 constexpr size_t kBatchBytes = 1536;  // a warp's ray batch
 constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {

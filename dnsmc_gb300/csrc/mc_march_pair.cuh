@@ -62,7 +62,7 @@ constexpr int kWalkCap = 128;  // steps of a chunk (even)
 // entered by the chunk's first step, the pairs (one spare), the wall-normal
 // times of the chunk, the state after it (kWalkWords in all)
 constexpr int kWalkTimes = 4 + 2 * (kWalkCap + 1);
-constexpr int kWalkState = kWalkTimes + 34;
+constexpr int kWalkState = kWalkTimes + 66;
 static_assert(kWalkState + 7 <= kWalkWords && kWalkWords % 4 == 0, "a warp's walk buffer");
 
 // the float after a non-negative float
@@ -131,7 +131,11 @@ enum WalkEnd { WALK_ON = 0, WALK_WALL = 1, WALK_COL = 2 };
 // before a collision and for unusable faces), *end how the chunk ends.  The
 // state is advanced in shared memory (walk_state reads it back; not written
 // when there are no steps).
-template <bool TRACE, bool COL>
+// TIMES (32 or 64): wall-normal crossings a chunk may reach.  64 for uniform
+// absorption (rays through all planes take one chunk: grey 64^3 2.99 -> 2.90
+// ms, drop-in bands call 7.29 -> 7.12 ms), 32 for the others (64: 128^3 channel
+// 61.6 -> 62.2 ms, with particles at 96^3 11.6 -> 12.0 ms).
+template <bool TRACE, bool COL, int TIMES>
 __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, float aim, int cap, float tcol, float *buf,
                                           int lane, int *end, int step0) {
     const unsigned FULL = 0xffffffffu;
@@ -140,23 +144,28 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     const float *fwn = P.fw + (dW > 0 ? 1 : 0);
     const float dtA = w.dtA, dtB = w.dtB, rA = w.rA, rB = w.rB;
     float *const tw = buf + kWalkTimes;
-    // the next 32 wall-normal crossings
-    const int c = w.cw + dW * lane;
-    const bool in = (unsigned)c < (unsigned)P.nw;
+    // the next TIMES wall-normal crossings
+    const int c = w.cw + dW * lane, c2 = c + dW * 32;
+    const bool in = (unsigned)c < (unsigned)P.nw, in2 = TIMES > 32 && (unsigned)c2 < (unsigned)P.nw;
     const float twl = in ? (__ldg(fwn + c) - w.oW) * w.sinvW : INF;
+    const float twh = in2 ? (__ldg(fwn + c2) - w.oW) * w.sinvW : INF;
     __syncwarp();  // the previous chunk's readers are done
     tw[lane] = twl;
-    const int nv = __popc(__ballot_sync(FULL, in));          // >= 1: the cell is in the grid
-    const float tw0 = __shfl_sync(FULL, twl, 0), twe = __shfl_sync(FULL, twl, nv - 1);
+    int nv = __popc(__ballot_sync(FULL, in));                // >= 1: the cell is in the grid
+    if (TIMES > 32) {
+        tw[32 + lane] = twh;
+        nv += __popc(__ballot_sync(FULL, in2));
+    }
+    const float tw0 = __shfl_sync(FULL, twl, 0), twe = __shfl_sync(FULL, nv > 32 ? twh : twl, (nv - 1) & 31);
     if (lane == 0) {
-        tw[32] = INF;
+        tw[TIMES] = INF;
         buf[kWalkState + 6] = 0.0f;  // (int) 0 steps, unless a lane makes the last one
     }
     // the window: about `aim` crossings at the present rates, no more than
     // the listed wall-normal ones, at least the next crossing
     const float rW = twe < INF ? __fdividef((float)(nv - 1), fmaxf(twe - tw0, 1e-30f)) : 0.0f;
     float te = w.t + __fdividef(aim, rA + rB + rW);
-    te = fminf(te, nv < 32 ? (twe < INF ? next_up(twe) : INF) : twe);
+    te = fminf(te, nv < TIMES ? (twe < INF ? next_up(twe) : INF) : twe);
     const float tmin = fminf(tw0, fminf((w.nA + w.offA) * dtA, (w.nB + w.offB) * dtB));
     te = fmaxf(te, next_up(tmin));
     bool col = false;
@@ -175,7 +184,7 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
         nA = fmaxf(nA, crossings_before(tau, rA, dtA, w.offA));
         nB = fmaxf(nB, crossings_before(tau, rB, dtB, w.offB));
 #pragma unroll
-        for (int h = 16; h; h >>= 1) k += tw[k + h - 1] < tau ? h : 0;
+        for (int h = TIMES / 2; h; h >>= 1) k += tw[k + h - 1] < tau ? h : 0;
         k += tw[k] < tau ? 1 : 0;
     }
     const int mA = (int)(nA - w.nA), mB = (int)(nB - w.nB);
@@ -205,7 +214,7 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
             t = tn;
             if (bW) {
                 hit = (unsigned)(cw + dW) >= (unsigned)P.nw;
-                if (!hit) { cw += dW; k = min(k + 1, 32); tW = tw[k]; }
+                if (!hit) { cw += dW; k = min(k + 1, TIMES); tW = tw[k]; }
             } else if (bA) {
                 nA += 1.0f;
                 tA = (nA + w.offA) * dtA;
@@ -480,7 +489,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
             for (;;) {  // chunks of the walk
                 int end;
                 // a short first chunk where this item's rays have been short
-                const int n = walk_chunk<TRACE, false>(P, w, first && est < 20 ? 28.0f : (float)(kWalkCap - 4),
+                const int n = walk_chunk<TRACE, false, UNI ? 64 : 32>(P, w, first && est < 20 ? 28.0f : (float)(kWalkCap - 4),
                                                        min(kWalkCap, P.max_steps - steps), 0.0f, wbuf, lane, &end, steps);
                 if constexpr (UNI) {
                     // e = expm1(k (t - tn)) of the chunk's steps, a lane each
@@ -951,7 +960,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
             bool first = true;
             for (;;) {  // chunks of the walk
                 int end;
-                const int n = walk_chunk<TRACE, true>(P, w, (float)(kWalkCap - 4), min(kWalkCap, P.max_steps - steps), tcol,
+                const int n = walk_chunk<TRACE, true, 32>(P, w, (float)(kWalkCap - 4), min(kWalkCap, P.max_steps - steps), tcol,
                                                       wbuf, lane, &end, steps);
                 {
                     const unsigned c1 = n ? __float_as_uint(wbuf[3]) : corner;

@@ -162,3 +162,14 @@ def test_general_medium_walks_match_the_replay(kind, size, albedo, kw, region):
     check_bitexact(s, T[None], None if x is None else x[None], fv[None])
     assert status() == (D.STATUS_STEP_CAP if "max_steps" in kw else 0)
     s.close()
+
+
+@pytest.mark.parametrize("model,size,kw", [
+    ("grey", (200, 8, 8), dict(kappa=0.01, max_steps=128)),   # the cap at a chunk's end, and one step on
+    ("grey", (200, 8, 8), dict(kappa=0.01, max_steps=129)),
+    ("grey", (64, 3, 64), dict(kappa=0.02)),                  # as many planes as a chunk lists crossings
+    ("bands", (131, 9, 6), dict(kappa=0.03)),
+    ("T", (150, 5, 8), dict(max_steps=129)),
+])
+def test_walks_at_the_edges_of_a_chunk_match_the_replay(model, size, kw):
+    test_walks_match_the_replay(model, size, kw, None)
