@@ -315,11 +315,13 @@ inline size_t march_smem(const MarchParams &p, int threads, int cells) {
 }
 // of a launch of the gas march: each warp's slab, walk buffer and ray batch, then per
 // thread the sums of its two cells; kPairStaticSmem at most beside it
-constexpr int kWalkWords = 336;  // words of a warp's walk buffer (mc_march_pair.cuh)
+// words of a warp's walk buffer (mc_march_pair.cuh); uni: uniform absorption
+__host__ __device__ constexpr int walk_words(bool uni) { return uni ? 336 : 304; }
 constexpr size_t kBatchBytes = 1536;  // a warp's ray batch
 constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {
-    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kWalkWords * 4u + kBatchBytes) + (size_t)threads * 24u * kLaneCells;
+    const int words = walk_words(p.uni || p.slab_len == 0);  // (no slab: the grey model)
+    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + words * 4u + kBatchBytes) + (size_t)threads * 24u * kLaneCells;
 }
 // ... of the multigrid march: each warp's slab and ray batch, then a thread's sums
 constexpr size_t kMgBatchBytes = 1024;

@@ -59,11 +59,13 @@ namespace dnsmc {
 // ---------------------------------------------------------------------------
 constexpr int kWalkCap = 128;  // steps of a chunk (even)
 // words of a warp's walk buffer: a 4-word header whose last word is the cell
-// entered by the chunk's first step, the pairs (one spare), the wall-normal
-// times of the chunk, the state after it (kWalkWords in all)
-constexpr int kWalkTimes = 4 + 2 * (kWalkCap + 1);
-constexpr int kWalkState = kWalkTimes + 66;
-static_assert(kWalkState + 7 <= kWalkWords && kWalkWords % 4 == 0, "a warp's walk buffer");
+// entered by the chunk's first step, the pairs (one spare), the state after the
+// chunk, its wall-normal times (walk_words in all)
+constexpr int kWalkState = 4 + 2 * (kWalkCap + 1);
+constexpr int kWalkTimes = kWalkState + 7;
+static_assert(kWalkTimes + 32 + 1 <= walk_words(false) && kWalkTimes + 64 + 1 <= walk_words(true) && walk_words(false) % 4 == 0 &&
+                  walk_words(true) % 4 == 0,
+              "a warp's walk buffer");
 
 // the float after a non-negative float
 __device__ __forceinline__ float next_up(float v) { return __uint_as_float(__float_as_uint(v) + 1u); }
@@ -356,9 +358,9 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
     const int warp = threadIdx.x >> 5, nwarp = (nthr + 31) >> 5;
     float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + warp * P.slab_len;
     const float2 *const sli = slk + P.slab_klen;
-    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * kWalkWords;
+    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(UNI);
     RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
-                                                        nwarp * kWalkWords) + warp;
+                                                        nwarp * walk_words(UNI)) + warp;
     float2 *const s_acc = reinterpret_cast<float2 *>(batch - warp + nwarp);
     auto acc = [&](int q, int k) { return s_acc + (q * C + k) * nthr + tid; };
     // each warp's transaction barrier of its slab copies, and its parity
@@ -767,9 +769,9 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
     const int warp = threadIdx.x >> 5, nwarp = (nthr + 31) >> 5;
     float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + warp * P.slab_len;
     const float2 *const sli = slk + P.slab_klen;
-    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * kWalkWords;
+    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(false);
     RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
-                                                        nwarp * kWalkWords) + warp;
+                                                        nwarp * walk_words(false)) + warp;
     float2 *const s_acc = reinterpret_cast<float2 *>(batch - warp + nwarp);
     auto acc = [&](int q, int k) { return s_acc + (q * C + k) * nthr + tid; };
     // each warp's transaction barrier of its slab copies, and its parity
