@@ -329,19 +329,22 @@ inline size_t march_mg_smem(const MarchParams &p, int threads) {
     return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + kMgBatchBytes) + (size_t)threads * 24u;
 }
 // Queue units per item: an item is one warp's serial work over its rays, so
-// with few items the chip idles; units of at least one ray, about 16 per
-// resident warp.  warps: resident warps of the launch; cap_bytes: the most
-// that the rays' contributions may take.
-// 16 per warp leaves the last wave under a tenth of the launch.  Grey 8 x 32 x 4
-// at 32 rays (32 items): march 79 -> 18 us; grey 64^3 at 256 rays (4096
-// items, 1.7 waves of warps): 4.85 -> 4.36 ms.  From 16 items a warp on, one
-// unit per item: the sums stay in shared memory (128^3 with 8 band groups:
-// 262144 items, unchanged).
+// with few items the chip idles.  warps: resident warps of the launch;
+// cap_bytes: the most that the rays' contributions (of `cells` cells) may take.
+// About 16 units per resident warp leave the last wave under a tenth of the
+// launch, but of no fewer than 12 rays each (a unit's first 32 rays are set up
+// together), and 4 per warp whatever that takes.  Grey 8 x 32 x 4 at 32 rays (32 items): march
+// 79 -> 18 us; grey 64^3 at 256 rays (4096 items, 1.7 waves of warps): 4.85 -> 4.36
+// ms; 45 x 60 x 52 tables at 32 rays (10080 items, 4 per warp): 4 units of 8 rays 1.145,
+// 2 of 16 1.090 ms.  From 16 items a warp on, one unit per item: the sums
+// stay in shared memory (128^3 with 8 band groups: 262144 items).
 constexpr long long kRayxBytes = 1LL << 30;
 inline int march_parts(long long n_items, int rays, long long warps, long long cap_bytes, int cells = 64) {
     if (n_items < 1 || rays < 2 || n_items >= 16 * warps) return 1;
     if (n_items * rays > cap_bytes / (cells * (long long)sizeof(float))) return 1;
-    const long long want = (16 * warps + n_items - 1) / n_items;
+    const long long full = (16 * warps + n_items - 1) / n_items, least = (4 * warps + n_items - 1) / n_items;
+    long long want = full < rays / 12 ? full : rays / 12;
+    want = want > least ? want : least;
     return (int)(want < rays ? want : rays);
 }
 int launch_march_gen(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace, bool cv,

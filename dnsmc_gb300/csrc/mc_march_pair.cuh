@@ -371,7 +371,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
     bool dead = false;  // a slab copy did not arrive: this warp stops marching
 
     for (;;) {
-        long long item;
+        long long item;  // below 2^32, as the queue
         int part = 0;
         if (TRACE) {
             if (threadIdx.x >= 32) return;
@@ -387,10 +387,9 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
             }
             item = P.item_order ? (long long)__ldg(P.item_order + it) : (long long)it;
         }
-        const int p = (int)(item % P.n_packets);
-        const long long fg = item / P.n_packets;
-        const int G = (int)(fg % P.n_groups);
-        const int f = (int)(fg / P.n_groups);
+        const unsigned fg = (unsigned)item / (unsigned)P.n_packets;
+        const int p = (int)((unsigned)item - fg * (unsigned)P.n_packets);
+        const int f = (int)(fg / (unsigned)P.n_groups), G = (int)(fg - (unsigned)f * (unsigned)P.n_groups);
         const int pa = p % P.npa;
         const int rest = p / P.npa;
         const int pb = rest % P.npb;
@@ -782,7 +781,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
     bool dead = false;  // a slab copy did not arrive: this warp stops marching
 
     for (;;) {
-        long long item;
+        long long item;  // below 2^32, as the queue
         int part = 0;
         if (TRACE) {
             if (threadIdx.x >= 32) return;
@@ -798,10 +797,9 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
             }
             item = P.item_order ? (long long)__ldg(P.item_order + it) : (long long)it;
         }
-        const int p = (int)(item % P.n_packets);
-        const long long fg = item / P.n_packets;
-        const int G = (int)(fg % P.n_groups);
-        const int f = (int)(fg / P.n_groups);
+        const unsigned fg = (unsigned)item / (unsigned)P.n_packets;
+        const int p = (int)((unsigned)item - fg * (unsigned)P.n_packets);
+        const int f = (int)(fg / (unsigned)P.n_groups), G = (int)(fg - (unsigned)f * (unsigned)P.n_groups);
         const int pa = p % P.npa;
         const int rest = p / P.npa;
         const int pb = rest % P.npb;
