@@ -469,6 +469,19 @@ int ensure_work(dnsmc_cvnet *n, long long rows) {
     return DNSMC_OK;
 }
 
+// A kernel of a training step, placed while the one before it still runs
+// (step_begin).
+template <class... K, class... A>
+cudaError_t launch_step(void (*k)(K...), dim3 grid, int threads, size_t smem, cudaStream_t st, A... args) {
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid; cfg.blockDim = dim3((unsigned)threads); cfg.dynamicSmemBytes = smem; cfg.stream = st;
+    cfg.attrs = &at; cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // Forward, loss, backward (and with `adam` the update) on `rows` rows (a
 // multiple of 128, nvalid real) of X/lab through idx; the tiles' loss sums go
 // to `loss` ([rows / 128][3], device).
@@ -486,8 +499,7 @@ int train_step(dnsmc_cvnet *n, const bf16 *X, const float *lab, int G, const int
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, n->device);
     CK(cudaFuncSetAttribute(train_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TR_SMEM));
     dnsmc::note_launch();
-    train_tile_kernel<<<(unsigned)std::min<long long>(rows / TC_TILE, sms), TR_THREADS, TR_SMEM, n->stream>>>(F);
-    CK(cudaGetLastError());
+    CK(launch_step(train_tile_kernel, dim3((unsigned)std::min<long long>(rows / TC_TILE, sms)), TR_THREADS, TR_SMEM, n->stream, F));
     WgradParams Wp{};
     Wp.rows = rows;
     Wp.splits = (int)std::min<long long>(64, std::max<long long>(1, rows / 256));
@@ -498,8 +510,7 @@ int train_step(dnsmc_cvnet *n, const bf16 *X, const float *lab, int G, const int
     for (int l = 0; l < 4; ++l) { Wp.dZ[l] = dZ[l]; Wp.H[l] = H[l]; }
     CK(cudaFuncSetAttribute(train_wgrad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, WG_SMEM));
     dnsmc::note_launch();
-    train_wgrad_kernel<<<dim3((unsigned)Wp.splits, 4), WG_THREADS, WG_SMEM, n->stream>>>(Wp, n->status.p);
-    CK(cudaGetLastError());
+    CK(launch_step(train_wgrad_kernel, dim3((unsigned)Wp.splits, 4), WG_THREADS, WG_SMEM, n->stream, Wp, n->status.p));
     UpdateParams U{};
     U.part = n->part.p; U.splits = Wp.splits; U.rows = rows;
     for (int l = 0; l < 4; ++l) U.dZ[l] = dZ[l];
@@ -512,8 +523,7 @@ int train_step(dnsmc_cvnet *n, const bf16 *X, const float *lab, int G, const int
         U.c2 = 1.0f - powf(n->cfg.adam_beta2, (float)n->step);
     }
     dnsmc::note_launch();
-    train_update_kernel<<<WU_WBLOCKS + WU_BBLOCKS, WU_THREADS, 0, n->stream>>>(U);
-    CK(cudaGetLastError());
+    CK(launch_step(train_update_kernel, dim3(WU_WBLOCKS + WU_BBLOCKS), WU_THREADS, 0, n->stream, U));
     return DNSMC_OK;
 }
 

@@ -104,7 +104,17 @@ __device__ __forceinline__ void train_loss(const TrainParams &L, const float *y,
     }
 }
 
+// The three kernels of a step follow one another with programmatic dependence
+// (launch_step): each lets the next one's blocks be placed as soon as its own
+// have started, and waits for the one before to have finished before it
+// touches memory.
+__device__ __forceinline__ void step_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __global__ void __launch_bounds__(TR_THREADS, 1) train_tile_kernel(const TrainParams F) {
+    step_begin();
     extern __shared__ __align__(1024) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int row = (warp & 3) * 32 + lane, cg = warp >> 2;  // this thread's tile row and column group
@@ -320,6 +330,7 @@ __device__ __forceinline__ void wg_stage(unsigned char *s, int nrow, const bf16 
 }
 
 __global__ void __launch_bounds__(WG_THREADS, 1) train_wgrad_kernel(const WgradParams G, unsigned int *status) {
+    step_begin();
     extern __shared__ __align__(1024) unsigned char gsm[];
     __shared__ uint64_t bar;
     __shared__ uint32_t tslot;
@@ -439,6 +450,7 @@ __device__ __forceinline__ long long weight_at(long long q, int &l, int &n, int 
 }
 
 __global__ void __launch_bounds__(WU_THREADS) train_update_kernel(const UpdateParams U) {
+    step_begin();
     if (blockIdx.x < WU_WBLOCKS) {
         const long long q = (long long)blockIdx.x * WU_THREADS + threadIdx.x;
         if (q >= NWEIGHT) return;
