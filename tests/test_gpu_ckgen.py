@@ -76,3 +76,28 @@ def test_bins_of_awkward_spectra(n_pwrk):
     ko, ao = O.ck_from_lbl(spec, gq, n_pwrk=n_pwrk)
     np.testing.assert_allclose(kq, ko, rtol=1e-5)
     np.testing.assert_allclose(kavg, ao, rtol=1e-9)
+
+
+@pytest.mark.parametrize("nT,nX", [(5, 3), (3, 1), (1, 14)])
+def test_spectra_copied_in_parts_equal_single_rows(nT, nX):
+    """From 8 MB on the spectra are copied and reduced in parts; every (T, x)
+    row equals the row generated alone, and a bad value in the last part is
+    refused."""
+    per = 9000 if nT * nX > 3 else 88000
+    nb = 9 if nT * nX > 3 else 4
+    n = nb * per + 1
+    assert nT * nX * n * 8 >= 8 << 20 and n * 8 < 8 << 20
+    k = np.exp(np.random.default_rng(nT).normal(-2.0, 2.0, (nT, nX, n)))
+    left = 1000.0 + per * 0.01 * np.arange(nb)
+    spec = dict(kappa=k, wv0=1000.0, dwv=0.01, first=np.arange(nb, dtype=np.int64) * per,
+                count=np.full(nb, per + 1, np.int32), wv_left=left, wv_right=left + per * 0.01)
+    gq = np.array([0.1, 0.5, 0.9])
+    kq, kavg = D.ck_from_lbl(spec, gq, n_pwrk=500)
+    for t in range(nT):
+        for x in range(nX):
+            q1, a1 = D.ck_from_lbl(dict(spec, kappa=k[t:t + 1, x:x + 1]), gq, n_pwrk=500)
+            np.testing.assert_array_equal(kq[..., t, x], q1[..., 0, 0])
+            np.testing.assert_array_equal(kavg[t, x], a1[0, 0])
+    k[-1, -1, -1] = np.nan
+    with pytest.raises(RuntimeError, match="finite"):
+        D.ck_from_lbl(spec, gq, n_pwrk=500)
