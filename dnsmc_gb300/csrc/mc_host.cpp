@@ -266,6 +266,7 @@ struct dnsmc_solver {
     DevBuf<float> d_raw;
     DevBuf<double> d_stat_part;
     DevBuf<double> d_stat_out;
+    PinBuf<double> h_stat;
 
     // region and rays
     int r_i0 = 0, r_i1 = 0, r_j0 = 0, r_j1 = 0, r_k0 = 0, r_k1 = 0;
@@ -276,7 +277,7 @@ struct dnsmc_solver {
     int rays_np = 0;                         // packets the per-packet / per-item rays were set for
     DevBuf<int> d_rays_pp;
     DevBuf<double2> d_rays_rcp;              // (1/N, 1/(N-1)) of d_rays_pp, written by the finalize launch
-    DevBuf<unsigned long long> d_item_steps; // steps per (field, group, packet) of the last solve
+    unsigned long long *item_steps = nullptr; // steps per (field, group, packet) of the last solve (in d_misc)
     DevBuf<unsigned int> d_order, d_order_hist;  // longest-first queue order (per-item ray tables)
     DevBuf<float> d_kP;                      // Planck-mean absorption coefficient on the table grid
 
@@ -334,16 +335,18 @@ struct dnsmc_solver {
 
     // outputs
     DevBuf<double2> d_tally;
-    DevBuf<double> d_Q, d_var, d_sig, d_Qg, d_varg;
-    PinBuf<double> h_Q, h_sig;
+    DevBuf<double> d_Q, d_var, d_Qg, d_varg;  // d_Q: Q, then sigma (one copy brings both)
+    PinBuf<double> h_Q;
     // DNSMC_RESULT_F32: the finalize also writes Q and sqrt(var * sig_scale)
     // as floats and only those cross to the host (8 bytes per cell)
     int result_type = DNSMC_RESULT_F64;
     double sig_scale = 1.0;
-    DevBuf<float> d_Qf, d_sigf;
-    PinBuf<float> h_Qf, h_sigf;
+    DevBuf<float> d_Qf;                       // as d_Q
+    PinBuf<float> h_Qf;
+    size_t nout = 0;                          // values of Q in them
     // [0] queue, [1] status, [4..7] the two 64-bit counters, [8 ...] finished
-    // units per item (split items); the first 8 words come back with the results
+    // units per item (split items), then the items' steps (64-bit); the first 8
+    // words come back with the results
     DevBuf<unsigned int> d_misc;
     PinBuf<unsigned int> h_misc;
     DevBuf<float> d_rayx;         // every ray's contribution (split items), at most kRayxBytes
@@ -1172,8 +1175,12 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     TRY(s->d_tally.ensure((size_t)s->nfields * P.n_groups * P.region_cells));
     P.tally = s->d_tally.p;
-    TRY(s->d_item_steps.ensure((size_t)P.n_items));
-    P.item_steps = s->d_item_steps.p;
+    const size_t done_words = ((size_t)P.n_items + 1) / 2 * 2, misc_words = kMiscWords + done_words + 2 * (size_t)P.n_items;
+    TRY(s->d_misc.ensure(misc_words));
+    P.queue = s->d_misc.p;
+    P.status = s->d_misc.p + 1;
+    P.counters = reinterpret_cast<unsigned long long *>(s->d_misc.p + 4);
+    P.item_steps = s->item_steps = reinterpret_cast<unsigned long long *>(s->d_misc.p + kMiscWords + done_words);
     if (P.rays_per_packet) {  // uneven items: longest first
         TRY(s->d_order.ensure((size_t)P.n_items));
         TRY(s->d_order_hist.ensure(kOrderBuckets));
@@ -1189,11 +1196,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes, cells);
         if (P.parts > 1) {
             TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * cells)));
-            TRY(s->d_misc.ensure((size_t)(kMiscWords + P.n_items)));
             P.rayx = s->d_rayx.p;
-            P.queue = s->d_misc.p;
-            P.status = s->d_misc.p + 1;
-            P.counters = reinterpret_cast<unsigned long long *>(s->d_misc.p + 4);
             P.parts_done = s->d_misc.p + kMiscWords;
         }
     }
@@ -1215,23 +1218,19 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     F.muY = cv ? s->d_muY.p : nullptr;
     F.beta = cv ? P.beta : nullptr;
     const size_t nout = (size_t)s->nfields * P.region_cells;
-    TRY(s->d_Q.ensure(nout));
+    TRY(s->d_Q.ensure(2 * nout));
     TRY(s->d_var.ensure(nout));
-    TRY(s->d_sig.ensure(nout));
     TRY(s->d_Qg.ensure(nout * P.n_groups));
     TRY(s->d_varg.ensure(nout * P.n_groups));
-    F.Q = s->d_Q.p; F.var = s->d_var.p; F.sigma = s->d_sig.p; F.Qg = s->d_Qg.p; F.varg = s->d_varg.p;
+    F.Q = s->d_Q.p; F.var = s->d_var.p; F.sigma = s->d_Q.p + nout; F.Qg = s->d_Qg.p; F.varg = s->d_varg.p;
     F.status = P.status;
     const bool f32 = s->result_type == DNSMC_RESULT_F32;
     if (f32) {
-        TRY(s->d_Qf.ensure(nout));
-        TRY(s->d_sigf.ensure(nout));
-        TRY(s->h_Qf.ensure(nout));
-        TRY(s->h_sigf.ensure(nout));
-        F.Qf = s->d_Qf.p; F.sigf = s->d_sigf.p; F.sig_scale = s->sig_scale;
+        TRY(s->d_Qf.ensure(2 * nout));
+        TRY(s->h_Qf.ensure(2 * nout));
+        F.Qf = s->d_Qf.p; F.sigf = s->d_Qf.p + nout; F.sig_scale = s->sig_scale;
     } else {
-        TRY(s->h_Q.ensure(nout));
-        TRY(s->h_sig.ensure(nout));
+        TRY(s->h_Q.ensure(2 * nout));
     }
 
     // ---- the kernel sequence of a solve (stream-ordered; capturable) -------
@@ -1242,10 +1241,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
             if (rc == 0) rc = launch_cv_mean(cp, s->stream);
             if (rc) return fail(DNSMC_ERR_CUDA, "control-variate launch: %s", cudaGetErrorString((cudaError_t)rc));
         }
-        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, (kMiscWords + (P.parts > 1 ? (size_t)P.n_items : 0)) * sizeof(unsigned int),
-                                 s->stream));
-        if (P.parts > 1 && P.item_steps)
-            CUDA_TRY(cudaMemsetAsync(P.item_steps, 0, (size_t)P.n_items * sizeof(unsigned long long), s->stream));
+        CUDA_TRY(cudaMemsetAsync(s->d_misc.p, 0, (P.parts > 1 ? misc_words : kMiscWords) * sizeof(unsigned int), s->stream));
         if (P.item_order) {
             const int rco = launch_item_order(P.rays_per_packet, P.rays_gstride, P.n_packets, P.n_groups, P.n_items,
                                               std::max(1, c.sampler == DNSMC_SAMPLER_RQMC ? c.nvar : 1),
@@ -1260,13 +1256,9 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         rc = launch_finalize(F, s->stream);
         if (rc) return fail(DNSMC_ERR_CUDA, "finalize launch: %s", cudaGetErrorString((cudaError_t)rc));
         if (f32) {
-            CUDA_TRY(cudaMemcpyAsync(s->h_Qf.p, s->d_Qf.p, nout * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
-            CUDA_TRY(cudaMemcpyAsync(s->h_sigf.p, s->d_sigf.p, nout * sizeof(float), cudaMemcpyDeviceToHost,
-                                     s->stream));
+            CUDA_TRY(cudaMemcpyAsync(s->h_Qf.p, s->d_Qf.p, 2 * nout * sizeof(float), cudaMemcpyDeviceToHost, s->stream));
         } else {
-            CUDA_TRY(cudaMemcpyAsync(s->h_Q.p, s->d_Q.p, nout * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-            CUDA_TRY(cudaMemcpyAsync(s->h_sig.p, s->d_sig.p, nout * sizeof(double), cudaMemcpyDeviceToHost,
-                                     s->stream));
+            CUDA_TRY(cudaMemcpyAsync(s->h_Q.p, s->d_Q.p, 2 * nout * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
         }
         CUDA_TRY(cudaMemcpyAsync(s->h_misc.p, s->d_misc.p, kMiscWords * sizeof(unsigned int), cudaMemcpyDeviceToHost,
                                  s->stream));
@@ -1327,6 +1319,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     s->in_flight = true;
     s->solved = true;
     s->solved_result_type = s->result_type;
+    s->nout = nout;
     return DNSMC_OK;
 }
 
@@ -1501,27 +1494,41 @@ int upload_coarse(dnsmc_solver *s, int nfields, const float *src, int src_step) 
     return DNSMC_OK;
 }
 
-// launch_field_stats of n resident values, its results read back
-int field_stats(dnsmc_solver *s, int kind, const float *v, long long n, double st[4]) {
+// Buffers of the field statistics.
+int stats_buffers(dnsmc_solver *s) {
     TRY(s->d_stat_part.ensure(field_stats_partials()));
+    TRY(s->h_stat.ensure(4));
     if (!s->d_stat_out.p) {
         TRY(s->d_stat_out.ensure(5));
         CUDA_TRY(cudaMemsetAsync(s->d_stat_out.p, 0, 5 * sizeof(double), s->stream));
     }
-    const int rc = launch_field_stats(kind, v, n, s->d_stat_part.p, s->d_stat_out.p, s->stream);
-    if (rc) return fail(DNSMC_ERR_CUDA, "stats launch: %s", cudaGetErrorString((cudaError_t)rc));
-    CUDA_TRY(cudaMemcpyAsync(st, s->d_stat_out.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
-    CUDA_TRY(cudaStreamSynchronize(s->stream));
     return DNSMC_OK;
 }
 
+// The results of the statistics enqueued last, read back.
+int read_stats(dnsmc_solver *s, double st[4]) {
+    CUDA_TRY(cudaMemcpyAsync(s->h_stat.p, s->d_stat_out.p, 4 * sizeof(double), cudaMemcpyDeviceToHost, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    memcpy(st, s->h_stat.p, 4 * sizeof(double));
+    return DNSMC_OK;
+}
+
+// launch_field_stats of n resident values, its results read back
+int field_stats(dnsmc_solver *s, int kind, const float *v, long long n, double st[4]) {
+    TRY(stats_buffers(s));
+    const int rc = launch_field_stats(kind, v, n, s->d_stat_part.p, s->d_stat_out.p, s->stream);
+    if (rc) return fail(DNSMC_ERR_CUDA, "stats launch: %s", cudaGetErrorString((cudaError_t)rc));
+    return read_stats(s, st);
+}
+
 // Tmax / Tmin / sum x over the packed resident fields (code/mc_gpu.cu:470-486),
-// on the device; fails (and drops the fields) when a temperature is not
-// positive and finite.
-int field_stats_checked(dnsmc_solver *s, int nfields, bool with_x, double st[4]) {
+// on the device (done: enqueued with the packing); fails (and drops the fields)
+// when a temperature is not positive and finite.
+int field_stats_checked(dnsmc_solver *s, int nfields, bool with_x, bool done, double st[4]) {
     const dnsmc_config &c = s->cfg;
-    TRY(field_stats(s, with_x ? STATS_TX : STATS_T, with_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p,
-                    (long long)nfields * c.imax * c.jmax * c.kmax, st));
+    if (done) TRY(read_stats(s, st));
+    else TRY(field_stats(s, with_x ? STATS_TX : STATS_T, with_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p,
+                         (long long)nfields * c.imax * c.jmax * c.kmax, st));
     if (st[3] > 0.0 || !(st[1] > 0.0) || !std::isfinite(st[0])) {
         s->nfields = 0;
         return fail(DNSMC_ERR_ARG, "temperature field has non-positive or non-finite values");
@@ -1548,6 +1555,8 @@ int upload_fields_host(dnsmc_solver *s, int nfields, const float *T, const float
     TRY(s->d_raw.ensure((size_t)nsrc * (want_x ? 2 : 1)));
     if (want_x) TRY(s->d_fieldTX.ensure((size_t)nfields * ncell));
     else TRY(s->d_fieldT.ensure((size_t)nfields * ncell));
+    const bool fused = nfields == 1 && ncell <= kPackStatsCells;
+    TRY(stats_buffers(s));
     // each snapshot straight from the caller's arrays into the raw buffer
     // (stream order serialises the buffer's reuse), then packed on the device
     for (int f = 0; f < nfields; ++f) {
@@ -1556,14 +1565,17 @@ int upload_fields_host(dnsmc_solver *s, int nfields, const float *T, const float
             CUDA_TRY(cudaMemcpyAsync(s->d_raw.p + nsrc, x + f * nsrc, nsrc * sizeof(float), cudaMemcpyHostToDevice,
                                      s->stream));
         int rc;
-        if (want_x)
+        if (fused)
+            rc = launch_pack_stats(s->d_raw.p, want_x ? s->d_raw.p + nsrc : nullptr, want_x ? (float *)s->d_fieldTX.p : s->d_fieldT.p, c.imax,
+                                   c.jmax, c.kmax, si, sj, sk, base, s->d_stat_part.p, s->d_stat_out.p, s->stream);
+        else if (want_x)
             rc = launch_pack_TX(s->d_raw.p, s->d_raw.p + nsrc, s->d_fieldTX.p + f * ncell, c.imax, c.jmax, c.kmax, si, sj, sk, base, s->stream);
         else
             rc = launch_pack_T(s->d_raw.p, s->d_fieldT.p + f * ncell, c.imax, c.jmax, c.kmax, si, sj, sk, base, s->stream);
         if (rc) return fail(DNSMC_ERR_CUDA, "pack launch: %s", cudaGetErrorString((cudaError_t)rc));
     }
     double st[4];
-    TRY(field_stats_checked(s, nfields, want_x, st));
+    TRY(field_stats_checked(s, nfields, want_x, fused, st));
     if (c.grid_num > 1)
         TRY(upload_coarse(s, nfields, want_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, want_x ? 2 : 1));
     s->nfields = nfields;
@@ -1623,7 +1635,7 @@ int solver_view(dnsmc_solver *s, SolverView *v) {
         w.last_groups = s->last.n_groups;
         w.moments = (c.control_variate && c.cv_moments) ? s->d_moments.p : nullptr;
         w.varg = s->d_varg.p;
-        w.item_steps = s->d_item_steps.p;
+        w.item_steps = s->item_steps;
         w.rays = s->last.rays;
         w.rays_item = s->last.rays_per_packet;
         w.rays_gstride = s->last.rays_gstride;
@@ -1756,14 +1768,14 @@ int dnsmc_destroy(dnsmc_solver *s) {
     s->d_cv_grp.release(); s->d_cv_sid.release(); s->d_cv_C.release(); s->d_layer.release();
     s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();
-    s->d_stat_part.release(); s->d_stat_out.release(); s->d_rays_pp.release(); s->d_rays_rcp.release(); s->d_item_steps.release(); s->d_kP.release();
+    s->d_stat_part.release(); s->d_stat_out.release(); s->h_stat.release(); s->d_rays_pp.release(); s->d_rays_rcp.release(); s->d_kP.release();
     s->d_order.release(); s->d_order_hist.release();
     s->d_mgT.release(); s->d_mgfw.release(); s->d_mgP.release(); s->d_mgtab.release(); s->d_mgtmp.release(); s->d_mgwork.release();
     s->d_part.release(); s->d_fieldV.release(); s->d_layerV.release();
     s->d_entries.release(); s->d_group_start.release(); s->d_group_empty.release();
-    s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_sig.release(); s->h_sig.release(); s->d_Qg.release(); s->d_varg.release();
+    s->d_tally.release(); s->d_Q.release(); s->d_var.release(); s->d_Qg.release(); s->d_varg.release();
     s->h_Q.release(); s->d_misc.release(); s->d_rayx.release(); s->h_misc.release();
-    s->d_Qf.release(); s->d_sigf.release(); s->h_Qf.release(); s->h_sigf.release();
+    s->d_Qf.release(); s->h_Qf.release();
     if (s->ev_march0) cudaEventDestroy(s->ev_march0);
     if (s->ev_march1) cudaEventDestroy(s->ev_march1);
     if (s->ev_done) cudaEventDestroy(s->ev_done);
@@ -1985,16 +1997,21 @@ int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const
     TRY(wait_done(s, 0));
     if (dx) TRY(s->d_fieldTX.ensure((size_t)nfields * ncell));
     else TRY(s->d_fieldT.ensure((size_t)nfields * ncell));
+    const bool fused = nfields == 1 && ncell <= kPackStatsCells;
+    TRY(stats_buffers(s));
     for (int f = 0; f < nfields; ++f) {
         int rc;
-        if (dx)
+        if (fused)
+            rc = launch_pack_stats(dT, dx, dx ? (float *)s->d_fieldTX.p : s->d_fieldT.p, c.imax, c.jmax, c.kmax, 1, c.imax,
+                                   (long long)c.imax * c.jmax, 0, s->d_stat_part.p, s->d_stat_out.p, s->stream);
+        else if (dx)
             rc = launch_pack_TX(dT + f * ncell, dx + f * ncell, s->d_fieldTX.p + f * ncell, c.imax, c.jmax, c.kmax, 1, c.imax, (long long)c.imax * c.jmax, 0, s->stream);
         else
             rc = launch_pack_T(dT + f * ncell, s->d_fieldT.p + f * ncell, c.imax, c.jmax, c.kmax, 1, c.imax, (long long)c.imax * c.jmax, 0, s->stream);
         if (rc) return fail(DNSMC_ERR_CUDA, "pack launch: %s", cudaGetErrorString((cudaError_t)rc));
     }
     double st[4];
-    TRY(field_stats_checked(s, nfields, dx != nullptr, st));
+    TRY(field_stats_checked(s, nfields, dx != nullptr, fused, st));
     if (c.grid_num > 1)
         TRY(upload_coarse(s, nfields, dx ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, dx ? 2 : 1));
     s->nfields = nfields;
@@ -2301,9 +2318,9 @@ int dnsmc_get_item_steps(dnsmc_solver *s, double *steps) {
     if (!s || !steps) return fail(DNSMC_ERR_ARG, "null argument");
     TRY(wait_done(s, 0));
     const long long n = s->last.n_items;
-    if (n <= 0 || !s->d_item_steps.p) return fail(DNSMC_ERR_STATE, "no solve yet");
+    if (n <= 0 || !s->item_steps) return fail(DNSMC_ERR_STATE, "no solve yet");
     std::vector<unsigned long long> h((size_t)n);
-    CUDA_TRY(cudaMemcpy(h.data(), s->d_item_steps.p, (size_t)n * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemcpy(h.data(), s->item_steps, (size_t)n * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
     for (long long i = 0; i < n; ++i) steps[i] = (double)h[(size_t)i];
     return DNSMC_OK;
 }
@@ -2389,7 +2406,7 @@ int dnsmc_get_results(dnsmc_solver *s, double *Q, double *sigma) {
     if (s->solved_result_type != DNSMC_RESULT_F64)
         return fail(DNSMC_ERR_STATE, "the last solve returned float results: use dnsmc_get_results_float");
     const size_t n = (size_t)std::min(s->nfields, s->last.nfields) * s->last.region_cells;
-    return results_out(s, Q, sigma, s->h_Q.p, s->h_sig.p, s->d_Q.p, s->d_sig.p, n * sizeof(double));
+    return results_out(s, Q, sigma, s->h_Q.p, s->h_Q.p + s->nout, s->d_Q.p, s->d_Q.p + s->nout, n * sizeof(double));
 }
 
 int dnsmc_set_result_type(dnsmc_solver *s, int type) {
@@ -2406,11 +2423,11 @@ int dnsmc_get_results_float(dnsmc_solver *s, float *Q, float *sigma) {
     TRY(wait_done(s, 0));
     const size_t n = (size_t)std::min(s->nfields, s->last.nfields) * s->last.region_cells;
     if (s->solved_result_type == DNSMC_RESULT_F32) {
-        return results_out(s, Q, sigma, s->h_Qf.p, s->h_sigf.p, s->d_Qf.p, s->d_sigf.p, n * sizeof(float));
+        return results_out(s, Q, sigma, s->h_Qf.p, s->h_Qf.p + s->nout, s->d_Qf.p, s->d_Qf.p + s->nout, n * sizeof(float));
     } else {
         for (size_t i = 0; i < n; ++i) {
             if (Q) Q[i] = (float)s->h_Q.p[i];
-            if (sigma) sigma[i] = (float)s->h_sig.p[i];
+            if (sigma) sigma[i] = (float)s->h_Q.p[s->nout + i];
         }
     }
     return DNSMC_OK;
@@ -2696,7 +2713,7 @@ void get_results_(float *resfort, float *varfort) {
     // interior rows of imax floats into the (imax+2)(jl+2)(kmax+2) arrays
     // (code/param.h:110-111 idx_F); ghost cells stay untouched
     scatter_fortran(resfort, g_dropin->h_Qf.p, c.imax, jl, c.kmax);
-    scatter_fortran(varfort, g_dropin->h_sigf.p, c.imax, jl, c.kmax);
+    scatter_fortran(varfort, g_dropin->h_Qf.p + g_dropin->nout, c.imax, jl, c.kmax);
 }
 
 }  // extern "C"

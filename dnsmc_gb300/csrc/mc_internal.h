@@ -401,6 +401,11 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
 enum { STATS_T, STATS_TX, STATS_V };
 int launch_field_stats(int kind, const float *v, long long n, double *partials, double *out, void *stream);
 int field_stats_partials();   // doubles needed in `partials`
+// launch_pack_T (srcX null) or launch_pack_TX of one field of at most
+// kPackStatsCells cells, with its statistics (STATS_T or STATS_TX)
+constexpr long long kPackStatsCells = 1 << 18;
+int launch_pack_stats(const float *srcT, const float *srcX, float *dst, int nw, int na, int nb, long long si, long long sj,
+                      long long sk, long long base, double *partials, double *out, void *stream);
 
 // Control-variate preparation (all stream-ordered).
 struct CvParams {
