@@ -795,29 +795,9 @@ int upload_tables(dnsmc_solver *s) {
     const int nS = t.nbands * t.nq;
     const int klen = t.nX > 1 ? 2 * (t.nT - 1) * (t.nX - 1) : t.nT - 1;
     const int len = (klen + (t.nT - 1) + 1) & ~1;
-    std::vector<float2> sl((size_t)nS * len, make_float2(0.f, 0.f));
-    for (int sid = 0; sid < nS; ++sid) {
-        float2 *o = sl.data() + (size_t)sid * len;
-        if (t.nX > 1) {
-            for (int ti = 0; ti < t.nT - 1; ++ti)
-                for (int xi = 0; xi < t.nX - 1; ++xi) {
-                    const float *r = t.k.data() + ((size_t)sid * t.nT + ti) * t.nX + xi;
-                    const float *r1 = r + t.nX;
-                    const int e = ti * (t.nX - 1) + xi;
-                    o[2 * e] = make_float2(r[0], r[1] - r[0]);
-                    o[2 * e + 1] = make_float2(r1[0], r1[1] - r1[0]);
-                }
-        } else {
-            for (int ti = 0; ti < t.nT - 1; ++ti) {
-                const float *r = t.k.data() + (size_t)sid * t.nT + ti;
-                o[ti] = make_float2(r[0], r[1] - r[0]);
-            }
-        }
-        const float *ib = t.Ib.data() + (size_t)(sid / t.nq) * t.nT;
-        for (int ti = 0; ti < t.nT - 1; ++ti) o[klen + ti] = make_float2(ib[ti], ib[ti + 1] - ib[ti]);
-    }
-    TRY(s->d_slab.ensure(sl.size()));
-    CUDA_TRY(cudaMemcpyAsync(s->d_slab.p, sl.data(), sl.size() * sizeof(float2), cudaMemcpyHostToDevice, s->stream));
+    TRY(s->d_slab.ensure((size_t)nS * len));
+    if (const int rc = launch_slabs(s->d_k.p, s->d_ib.p, s->d_slab.p, nS, t.nq, t.nT, t.nX, klen, len, s->stream))
+        return fail(DNSMC_ERR_CUDA, "slab launch: %s", cudaGetErrorString((cudaError_t)rc));
     s->slab_len = len;
     s->slab_klen = klen;
     CUDA_TRY(cudaStreamSynchronize(s->stream));

@@ -392,6 +392,9 @@ int launch_pack_T4(const float *src, float *dst, int nw, int na, int nb, int pna
 int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
                    int na, int nb, long long si, long long sj, long long sk,
                    long long base, void *stream);
+// The march's table slabs of nS spectral samples, len pairs each, from the
+// tables k [sample][t][x] and Ib [band][t]: klen pairs of k, then Ib (the rest 0).
+int launch_slabs(const float *k, const float *ib, float2 *slab, int nS, int nq, int nT, int nX, int klen, int len, void *stream);
 // Over n cells into out[0..3] (device), deterministic: the largest and
 // smallest value, a sum and a count of refused values -- of temperatures T
 // (STATS_T; not positive or not finite), of (T, x) pairs (STATS_TX; T as

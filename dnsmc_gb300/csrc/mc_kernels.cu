@@ -226,6 +226,32 @@ __global__ void pack_TX_kernel(const float *srcT, const float *srcX, float2 *dst
     }
 }
 
+// Table slabs (launch_slabs), a pair a thread.  On the host this was 60 us of
+// each solve with grey band tables, which depend on the fields' Tmax (1000
+// bands: 0.9 MB of pairs).
+__global__ void slab_kernel(const float *k, const float *ib, float2 *slab, int nS, int nq, int nT, int nX, int klen, int len) {
+    const long long n = (long long)nS * len;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
+        const long long sid = i / len;
+        const int e = (int)(i - sid * len);
+        float a = 0.0f, b = 0.0f;
+        if (e < klen) {
+            const float *r = k + sid * nT * nX;
+            if (nX > 1) {  // pairs 2 c, 2 c + 1 of table cell c: rows t and t + 1
+                const int c = e >> 1, t = c / (nX - 1), x = c - t * (nX - 1);
+                r += (t + (e & 1)) * nX + x;
+            } else {
+                r += e;
+            }
+            a = r[0]; b = r[1];
+        } else if (e < klen + nT - 1) {
+            const float *r = ib + (sid / nq) * nT + (e - klen);
+            a = r[0]; b = r[1];
+        }
+        slab[i] = make_float2(a, b - a);
+    }
+}
+
 // Extremes, sum and count of refused values of n cells (launch_field_stats) in
 // a fixed order (deterministic): a grid-strided
 // share per block, then the block that finishes last reduces the blocks' parts
@@ -1144,6 +1170,12 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw, in
     return (int)cudaGetLastError();
 }
 
+int launch_slabs(const float *k, const float *ib, float2 *slab, int nS, int nq, int nT, int nX, int klen, int len, void *stream) {
+    if (nS <= 0 || len <= 0) return 0;
+    dnsmc::note_launch();
+    slab_kernel<<<grid_for((long long)nS * len, 256), 256, 0, (cudaStream_t)stream>>>(k, ib, slab, nS, nq, nT, nX, klen, len);
+    return (int)cudaGetLastError();
+}
 int launch_pack_stats(const float *srcT, const float *srcX, float *dst, int nw, int na, int nb, long long si, long long sj,
                       long long sk, long long base, double *partials, double *out, void *stream) {
     const unsigned n = (unsigned)((long long)nw * na * nb);
