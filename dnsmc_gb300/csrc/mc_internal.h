@@ -238,7 +238,8 @@ int launch_adaptive_rays(const AdaptParams &a, void *stream);
 // p = clamp((v - v0)/dv, 0, n-1) split into cell i = min((int)p, n-2) and
 // fraction p - i, for T and (MODE_TX) x_H2O.  MODE_TX packs
 // {ti*(nX-1) + xi, ft, fx, ti} into an int4 (fractions as float bits), MODE_T
-// {ti, ft} into an int2, so a march step needs no float-to-int split.
+// {ti, ft} into an int2, so a march step needs no float-to-int split (positions
+// alone, 8 bytes, split in the march: 128^3 channel 61.6 -> 69.8 ms).
 // Queue order of the march's items, longest first: a counting sort of the
 // items by their ray count (n_items = nfields * n_groups * n_packets; rays of
 // item (f, g, p) = rays[g * gstride + p]).  hist needs kOrderBuckets + 1 words.
@@ -307,9 +308,8 @@ int launch_march_ex(int mode, const MarchParams &p, int blocks, int threads, voi
 int march_occupancy_ex(int mode, bool uni, int threads, bool cv, bool mom, bool gen, size_t smem);
 int launch_march_mg(int mode, const MarchParams &p, int blocks, int threads, void *stream, bool trace);
 int march_mg_occupancy(int mode, bool uni, int threads, size_t smem);
-// dynamic shared memory of a march launch with `cells` cells per lane: each
-// warp's table slab (slab_len float2), then per thread and cell the three
-// sums of the item (float pairs, 8 bytes), then per thread the RQMC replicate's shift (uint4)
+// The bound on slabs: a solve is taken when four warps' slabs and 64 bytes a
+// thread fit in shared memory (cells = 2, 128 threads)
 inline size_t march_smem(const MarchParams &p, int threads, int cells) {
     return (size_t)((threads + 31) / 32) * (size_t)p.slab_len * 8u + (size_t)threads * (24u * (size_t)cells + 16u);
 }
@@ -318,10 +318,13 @@ inline size_t march_smem(const MarchParams &p, int threads, int cells) {
 // words of a warp's walk buffer (mc_march_pair.cuh); uni: uniform absorption
 __host__ __device__ constexpr int walk_words(bool uni) { return uni ? 336 : 304; }
 constexpr size_t kBatchBytes = 1536;  // a warp's ray batch
+constexpr size_t kEventBytes = 512;   // a warp's batch of collision events (general medium)
 constexpr size_t kPairStaticSmem = 256;
 inline size_t march_pair_smem(const MarchParams &p, int threads) {
     const int words = walk_words(p.uni || p.slab_len == 0);  // (no slab: the grey model)
-    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + words * 4u + kBatchBytes) + (size_t)threads * 24u * kLaneCells;
+    const size_t events = p.part || p.eps[0] < 1.0f || p.eps[1] < 1.0f ? kEventBytes : 0;  // the general medium's
+    return (size_t)((threads + 31) / 32) * ((size_t)p.slab_len * 8u + words * 4u + kBatchBytes + events) +
+           (size_t)threads * 24u * kLaneCells;
 }
 // ... of the multigrid march: each warp's slab and ray batch, then a thread's sums
 constexpr size_t kMgBatchBytes = 1024;

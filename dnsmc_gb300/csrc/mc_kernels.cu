@@ -2,28 +2,19 @@
 // Monte Carlo radiative-source solver.
 //
 // Replaces kernel_fluid / march_ray / find_band / emiss_ang / kernel_results
-// of the reference (code/mc_gpu.cu:44-438, :813-896, :959-970) with one
-// persistent work-queue kernel built around "packets":
+// of the reference (code/mc_gpu.cu:44-438, :813-896, :959-970) with persistent
+// work-queue kernels built around "packets" (mc_march_pair.cuh on the fine grid,
+// mc_march_mg.cuh with coarse grids): cells of one wall-normal plane that tile
+// the periodic (j, k) plane and are owned by one warp.  Every ray of a packet
+// shares one draw -- direction (reference emiss_ang, code/mc_gpu.cu:813-820) and
+// spectral sample (find_band, :830-896) -- and with it the voxel walk, since the
+// origins differ by whole periodic cells; the lanes do the OERM update of
+// march_ray (:264-276) for their own cells.
 //
-//   * a packet is 32 cells that share the wall-normal index i and tile the
-//     periodic (j, k) plane (tile_a x tile_b, j fastest in memory);
-//   * one warp owns a packet; lane l owns cell l and keeps that cell's FP64
-//     tallies in registers, so no reduction is needed;
-//   * every ray of the packet shares one Philox draw: the isotropic direction
-//     (reference emiss_ang, code/mc_gpu.cu:813-820) and the spectral sample
-//     (band, g) drawn from an alias table (reference find_band, :830-896).
-//     The reference already shares its Sobol direction sequence across all
-//     cells (code/mc_gpu.cu:80-81).  Because the origins differ by whole
-//     periodic cells, the voxel walk (which face is crossed next, and the
-//     segment length) is identical in all 32 lanes: the DDA is warp-uniform,
-//     lanes only offset their (j, k) indices.  Field gathers of the 32 lanes
-//     are contiguous (256 B per step for float2 fields) and the spectral
-//     table slice is the same for the whole warp.
-//   * per segment each lane does the OERM update of march_ray
-//     (code/mc_gpu.cu:264-276): alpha = 1 - exp(-k ds),
-//     D += tau*alpha*(Ib_i - Ib_j)/Ib_i, tau *= 1 - alpha, the remainder is
-//     dumped when tau < toll, black walls add tau*(Ib_i - Ib_w)/Ib_i
-//     (code/mc_gpu.cu:297,314).  The ray contribution is X = W*k_i*Ib_i*D.
+// This file: what surrounds the marches -- packing and statistics of the fields,
+// table coordinates and slabs, the control variate's preparation and means, the
+// queue order, the ray counts by optical thickness, the multigrid march's
+// launch and coarsening, the finalize.
 //
 // Rays are drawn either iid (one Philox4x32-10 call per packet-ray) or as
 // randomised quasi-Monte Carlo: the N rays of a (packet, band group) are
@@ -35,7 +26,7 @@
 // Arithmetic is FP32 with explicit fmaf and the file is compiled with
 // -fmad=false, so the host replay reproduces every ray bit for bit; exp and
 // sin/cos are the project's own polynomial kernels (mc_expm1 / mc_sincos) for
-// the same reason.  Tallies (sum X, sum X^2) are FP64.
+// the same reason.
 #include <atomic>
 
 #include "mc_march_mg.cuh"

@@ -235,9 +235,9 @@ __device__ __forceinline__ float mc_neglog(float u) {
 // uniform in (0, 1) from the top 24 bits
 __device__ __forceinline__ float u24o(uint32_t x) { return ((float)(x >> 8) + 0.5f) * 5.9604644775390625e-8f; }
 
-// Direction scattered by the Henyey-Greenstein phase function (asymmetry g)
-// from (sW, sA, sB): cos(theta) from uc, azimuth 2 pi m / 2^24.
-__device__ __forceinline__ void hg_scatter(float g, uint32_t uc, uint32_t um, float *sW, float *sA, float *sB) {
+// Henyey-Greenstein scattering (asymmetry g): the cosine and sine of the angle
+// from a uniform word, and the new direction from them and the azimuth's.
+__device__ __forceinline__ void hg_angle(float g, uint32_t uc, float *cos_t, float *sin_t) {
     const float u = u24(uc);
     float ct;
     if (fabsf(g) < 1e-6f) {
@@ -247,9 +247,10 @@ __device__ __forceinline__ void hg_scatter(float g, uint32_t uc, uint32_t um, fl
         ct = (1.0f + g * g - tmp * tmp) / (2.0f * g);
     }
     ct = fminf(fmaxf(ct, -1.0f), 1.0f);
-    const float st = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
-    float cph, sph;
-    mc_sincos_turn(um >> 8, &cph, &sph);
+    *cos_t = ct;
+    *sin_t = sqrtf(fmaxf(0.0f, 1.0f - ct * ct));
+}
+__device__ __forceinline__ void hg_turn(float ct, float st, float cph, float sph, float *sW, float *sA, float *sB) {
     const float w = *sW, a = *sA, b = *sB;
     float nw, na, nb;
     if (fabsf(w) > 0.99999f) {

@@ -8,9 +8,8 @@
 // which share their j index and lie 32 / tile_a rows apart in k.  Every ray
 // of the packet shares one direction and one spectral sample, so the voxel
 // walk (which face is crossed next, every segment length) is the same for
-// all 64 cells: it is computed once per lane for two cells, and only the
-// per-cell work (field gather, k and Ib lookups, attenuation, tallies) is
-// done twice.  Every cell's arithmetic is the reference estimator's update
+// all 64 cells: the warp generates it in chunks (walk_chunk), and a lane does
+// the per-cell work (field gather, k and Ib lookups, attenuation, tallies).  Every cell's arithmetic is the reference estimator's update
 // written with explicit fmaf, and the host replay (oracle/mc_oracle.cpp)
 // marches the same 64-cell packets, so it reproduces every cell bit for bit.
 //
@@ -739,10 +738,14 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
 // grey diffuse walls.  The walk restarts at every scattering and wall
 // reflection; its chunks end at the ray's next tentative collision, which is a
 // step of its own.
-// As the gas march it is bound by the L1 gathers and issue; a cell's volume
-// fraction rides in its 16-byte coordinates.  96^3 gas with particles, 8 rays:
-// 19.8 ms with the walk in every lane, 11.6 ms.
+// It is bound by issue and instruction fetches (each collision runs long straight
+// code); a cell's volume fraction rides in its 16-byte coordinates, and the
+// collisions' random words, free paths and angles are set up a lane each.  96^3
+// gas with particles, 8 rays: 19.8 ms with the walk in every lane, 11.5 ms with
+// the events' set-up in every lane, 11.1 ms.
 // ---------------------------------------------------------------------------
+constexpr int kEvents = 16;  // a batch of a ray's collision and reflection events
+static_assert(kEvents * 2 * sizeof(float4) == kEventBytes, "march_pair_smem");
 template <int MODE> struct GenFieldT { typedef int4 type; };
 template <> struct GenFieldT<MODE_GREY> { typedef float2 type; };
 __device__ __forceinline__ float gen_fraction(const int4 &v) { return __int_as_float(v.w); }
@@ -771,7 +774,8 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
     float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(false);
     RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
                                                         nwarp * walk_words(false)) + warp;
-    float2 *const s_acc = reinterpret_cast<float2 *>(batch - warp + nwarp);
+    float4 *const events = reinterpret_cast<float4 *>(batch - warp + nwarp) + warp * 2 * kEvents;
+    float2 *const s_acc = reinterpret_cast<float2 *>(events + (nwarp - warp) * 2 * kEvents);
     auto acc = [&](int q, int k) { return s_acc + (q * C + k) * nthr + tid; };
     // each warp's transaction barrier of its slab copies, and its parity
     __shared__ uint64_t s_bar[8];
@@ -910,16 +914,34 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                 life[k] = active[k] ? 1 << 30 : 0;
             }
             int steps = 0;
-            // scattering events: one Philox word quadruple per event
+            // scattering events: one Philox word quadruple per event, a batch of
+            // kEvents set up a lane each: free path, decision, azimuth; angle of
+            // a scattering and of a reflection
+            const float sigbar = P.fv_max * psc;
             uint32_t ev = 0;
-            uint4 evx = make_uint4(0u, 0u, 0u, 0u);
+            float4 e0 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 *e1 = events;
             auto draw = [&]() {
-                evx = philox4x32_10(make_uint4((uint32_t)r, (uint32_t)p, ctr2, 0x5CA70000u + ev), P.key0, P.key1);
+                const uint32_t q = ev % kEvents;
+                if (q == 0) {
+                    __syncwarp();
+                    if (lane < kEvents) {
+                        const uint4 x = philox4x32_10(make_uint4((uint32_t)r, (uint32_t)p, ctr2, 0x5CA70000u + ev + lane), P.key0, P.key1);
+                        float cp, sp, ct, st;
+                        mc_sincos_turn(x.w >> 8, &cp, &sp);
+                        hg_angle(P.hg_g, x.z, &ct, &st);
+                        const float cmu = sqrtf(u24(x.z));
+                        events[2 * lane] = make_float4(sigbar > 0.0f ? mc_neglog(u24o(x.x)) / sigbar : INF, u24(x.y), cp, sp);
+                        events[2 * lane + 1] = make_float4(ct, st, cmu, sqrtf(fmaxf(0.0f, 1.0f - cmu * cmu)));
+                    }
+                    __syncwarp();
+                }
+                e0 = events[2 * q];
+                e1 = events + 2 * q + 1;
                 ++ev;
             };
-            const float sigbar = P.fv_max * psc;
             float tcol = INF;
-            if (sigbar > 0.0f) { draw(); tcol = mc_neglog(u24o(evx.x)) / sigbar; }
+            if (sigbar > 0.0f) { draw(); tcol = e0.x; }
             // One step of both cells, the same paired update as the gas
             // march's: e = expm1(k * (t - tn)) = -alpha, nta = tau e = -ta,
             // D += nta (-g), tau += nta; a cell already dumped (tau 0) adds
@@ -1042,15 +1064,12 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                     fb0 = fminf(fmaxf(fb0, 0.0f), 1.0f);
                     w.oW = side == 0 ? __ldg(P.fw) : __ldg(P.fw + P.nw);
                     draw();  // this event's words: the reflected direction only
-                    const float cmu = sqrtf(u24(evx.z));
-                    const float smu = sqrtf(fmaxf(0.0f, 1.0f - cmu * cmu));
-                    float cp, sp;
-                    mc_sincos_turn(evx.w >> 8, &cp, &sp);
-                    sW = side == 0 ? cmu : -cmu;
-                    sA = smu * cp;
-                    sB = smu * sp;
+                    const float4 e = *e1;
+                    sW = side == 0 ? e.z : -e.z;
+                    sA = e.w * e0.z;
+                    sB = e.w * e0.w;
                     restart();
-                    if (sigbar > 0.0f) { draw(); tcol = mc_neglog(u24o(evx.x)) / sigbar; }
+                    if (sigbar > 0.0f) { draw(); tcol = e0.x; }
                     if (steps >= P.max_steps) {
                         if (live) flags |= DNSMC_STATUS_STEP_CAP;
                         break;
@@ -1089,7 +1108,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                         pc += __shfl_xor_sync(FULL, pc, o);
                     }
                     const float q = pc > 0.0f ? ps / pc : 0.0f;
-                    const bool scatter = u24(evx.y) < q;
+                    const bool scatter = e0.y < q;
 #pragma unroll
                     for (int k = 0; k < C; ++k)
                         if (tau[k] > 0.0f) {
@@ -1104,12 +1123,13 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                         fa0 = fminf(fmaxf(fa0, 0.0f), 1.0f);
                         fb0 = fminf(fmaxf(fb0, 0.0f), 1.0f);
                         w.oW = fminf(fmaxf(fmaf(sW, w.t, w.oW), __ldg(P.fw + w.cw)), __ldg(P.fw + w.cw + 1));
-                        hg_scatter(P.hg_g, evx.z, evx.w, &sW, &sA, &sB);
+                        const float4 e = *e1;
+                        hg_turn(e.x, e.y, e0.z, e0.w, &sW, &sA, &sB);
                         restart();
                         t0 = 0.0f;
                     }
                     draw();
-                    tcol = t0 + mc_neglog(u24o(evx.x)) / sigbar;
+                    tcol = t0 + e0.x;
                     if (!__any_sync(FULL, tau[0] > 0.0f || tau[1] > 0.0f)) break;
                     if (steps >= P.max_steps) {
                         if (tau[0] > 0.0f || tau[1] > 0.0f) flags |= DNSMC_STATUS_STEP_CAP;

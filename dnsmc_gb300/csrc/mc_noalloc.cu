@@ -155,6 +155,7 @@ extern "C" int dnsmc_solve_grey_noalloc(const dnsmc_config *cfg, const float *xu
     P.rda = 1.0f / P.da; P.rdb = 1.0f / P.db;
     P.n_groups = 1;
     P.n_tbins = 1;
+    P.eps[0] = P.eps[1] = 1.0f;
     P.kappa = c.kappa;
     P.Wgrey = (float)(4.0 * c.kappa * 5.670373e-08);
     P.Tw4[0] = c.T_west * c.T_west * c.T_west * c.T_west;

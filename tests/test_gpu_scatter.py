@@ -234,3 +234,31 @@ def test_control_variate_with_particles_is_unbiased():
     assert math.sqrt(float((zp ** 2).mean())) < 1.6, zp
     assert np.abs(zp).max() < 4.5, zp
     assert (Sc ** 2).mean() < (Sp ** 2).mean()  # the surrogate still helps with scattering
+
+
+@pytest.mark.parametrize("particles", [True, False])
+def test_bitexact_rays_of_many_events(particles):
+    """Rays with more collisions or wall reflections than a batch of events
+    holds (16), several times over, against the replay."""
+    s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=10, jmax=16, kmax=8, Lx=2.0, Ly=3.0, Lz=2.0, stretched_x=0,
+                                  T_west=300, T_east=600, eps_west=0.05, eps_east=0.05, kappa=0.002, seed=6))
+    T = smooth_field(10, 16, 8, 400, 1200, 2)
+    s.set_fields(T)
+    fv = None
+    if particles:
+        fv = (1e-5 * (1 + 0.5 * np.random.default_rng(7).uniform(-1, 1, (8, 16, 10)))).astype(np.float32)
+        s.set_particles(np.array([10.0], np.float32), np.array([8.0e5], np.float32), 0.4)
+        s.set_particle_field(fv)
+    s.set_rays(6)
+    check_bitexact(s, T[None], None, None if fv is None else fv[None])
+    c, keep = O.packet_config(s, T[None], None, fv=None if fv is None else fv[None])
+    events = 0
+    for r in range(6):
+        rec, n, rng = s.trace(0, 0, 3, r, 1 << 15)
+        rec_o, n_o, rng_o = O.packet_trace(c, 0, 0, 3, r, 1 << 15)
+        assert n == n_o and (rng == rng_o).all()
+        np.testing.assert_array_equal(rec, rec_o)
+        edge = (rec[:-1, 3] == 0) & ((rec[:-1, 0] == 0) | (rec[:-1, 0] == 9)) & (rec[1:, 0] == rec[:-1, 0])
+        events = max(events, int((rec[:, 3] == 3).sum() if particles else edge.sum()))
+    assert events > 33
+    s.close()
