@@ -252,6 +252,7 @@ struct dnsmc_solver {
     DevBuf<int2> d_posT;   // per cell (ti, ft) for T-only tables
     DevBuf<int4> d_posTX;  // per cell (ti*(nX-1)+xi, ft, fx, ti)
     DevBuf<float> d_posG;  // per cell T^4 (grey model)
+    DevBuf<float> d_posF;  // per cell the table coordinate (grey band tables)
     DevBuf<float2> d_posVG;  // general medium: (T^4, fv); tables use d_posTX
     int posG_na = 0, posG_nb = 0;  // the padded extents d_posG was written for (0: not written)
     bool tables_dirty = true;
@@ -794,7 +795,7 @@ int upload_tables(dnsmc_solver *s) {
     // per table cell -- (or over [t]), then Ib over [t] of the sample's band
     const int nS = t.nbands * t.nq;
     const int klen = t.nX > 1 ? 2 * (t.nT - 1) * (t.nX - 1) : t.nT - 1;
-    const int len = (klen + (t.nT - 1) + 1) & ~1;
+    const int len = (klen + (t.nT - 1) + (t.grey_bands ? 1 : 0) + 1) & ~1;
     TRY(s->d_slab.ensure((size_t)nS * len));
     if (const int rc = launch_slabs(s->d_k.p, s->d_ib.p, s->d_slab.p, nS, t.nq, t.nT, t.nX, klen, len, s->stream))
         return fail(DNSMC_ERR_CUDA, "slab launch: %s", cudaGetErrorString((cudaError_t)rc));
@@ -1012,12 +1013,15 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     P.pstride = (long long)c.imax * P.pna * P.pnb;
     const long long npos = (long long)s->nfields * P.pstride;
     if (mode == MODE_TX || (mode == MODE_T && gen)) TRY(s->d_posTX.ensure((size_t)npos));
-    if (mode == MODE_T && !gen) TRY(s->d_posT.ensure((size_t)npos));
+    const bool bands = mode == MODE_T && P.uni && !mg && !gen;
+    if (mode == MODE_T && !gen && !bands) TRY(s->d_posT.ensure((size_t)npos));
+    if (bands) TRY(s->d_posF.ensure((size_t)npos));
     if (mode == MODE_GREY && gen) TRY(s->d_posVG.ensure((size_t)npos));
     if (mode == MODE_GREY && !mg && !gen) TRY(grey_positions(s));
     P.fieldP = s->d_posT.p;
     P.fieldPX = s->d_posTX.p;
     P.fieldG = s->d_posG.p;
+    P.fieldF = s->d_posF.p;
     P.fieldVX = s->d_posTX.p;
     P.fieldVG = s->d_posVG.p;
     FieldPos fp{};  // table coordinates of the field for this table (once per solve)
@@ -1029,6 +1033,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         else fp.outVX = s->d_posTX.p;
     } else {
         fp.outP = s->d_posT.p; fp.outPX = s->d_posTX.p;
+        if (bands) fp.outF = s->d_posF.p;
     }
     fp.nfields = s->nfields; fp.nw = c.imax; fp.na = c.jmax; fp.nb = c.kmax; fp.pna = P.pna; fp.pnb = P.pnb;
     fp.T0 = P.T0; fp.invdT = P.invdT; fp.nT = P.nT; fp.X0 = P.X0; fp.invdX = P.invdX; fp.nX = P.nX;
@@ -1744,7 +1749,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     s->d_fw.release(); s->d_k.release(); s->d_ib.release(); s->d_ibw.release();
-    s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posTX.release();
+    s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posF.release(); s->d_posTX.release();
     s->d_cv_grp.release(); s->d_cv_sid.release(); s->d_cv_C.release(); s->d_layer.release();
     s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();

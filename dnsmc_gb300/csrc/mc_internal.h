@@ -62,6 +62,7 @@ struct MarchParams {
     const int2   *fieldP;
     const int4   *fieldPX;
     const float  *fieldG;
+    const float  *fieldF;     // grey band tables on the fine grid: the table coordinate p = ti + ft
     // the general medium's, with the particle volume fraction: tables
     // (ti*(nX-1)+xi | ti << 16, ft, fx, fv), grey (T^4, fv)
     const int4   *fieldVX;
@@ -363,7 +364,7 @@ int upload_sobol_dirs_pair(const uint32_t dirs[4][32]);
 int launch_march(int mode, const MarchParams &p, int blocks, int threads,
                  void *stream, bool trace);
 int launch_finalize(const FinalizeParams &p, void *stream);
-// Table coordinates (outP, outPX or outVX), or T^4 (outG or outVG), of every cell of nfields
+// Table coordinates (outP, outF, outPX or outVX), or T^4 (outG or outVG), of every cell of nfields
 // packed fields [f][i][k][j], into rows of pna values and pnb rows a plane
 // (na <= pna < 2 na, nb <= pnb < 2 nb: continued periodically)
 inline int march_extent(int n, int tile) { return n + (tile < n ? tile : n) - 1; }  // n cells, packets of tile
@@ -377,6 +378,7 @@ struct FieldPos {
     int2 *outP;
     int4 *outPX;
     float *outG;
+    float *outF;
     const float *fV;          // volume fraction (null: 0) for outVX and outVG
     int4 *outVX;
     float2 *outVG;
@@ -396,7 +398,7 @@ int launch_pack_TX(const float *srcT, const float *srcX, float2 *dst, int nw,
                    int na, int nb, long long si, long long sj, long long sk,
                    long long base, void *stream);
 // The march's table slabs of nS spectral samples, len pairs each, from the
-// tables k [sample][t][x] and Ib [band][t]: klen pairs of k, then Ib (the rest 0).
+// tables k [sample][t][x] and Ib [band][t]: klen pairs of k, then Ib and its end point (the rest 0).
 int launch_slabs(const float *k, const float *ib, float2 *slab, int nS, int nq, int nT, int nX, int klen, int len, void *stream);
 // Over n cells into out[0..3] (device), deterministic: the largest and
 // smallest value, a sum and a count of refused values -- of temperatures T

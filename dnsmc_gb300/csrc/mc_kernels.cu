@@ -67,6 +67,10 @@ __global__ void field_pos_kernel(const FieldPos q) {
         } else {
             float pt = (q.fT[src] - q.T0) * q.invdT;
             pt = fminf(fmaxf(pt, 0.0f), (float)(q.nT - 1));
+            if (q.outF) {
+                q.outF[i] = pt;
+                continue;
+            }
             pos_split(pt, q.nT, &ti, &ft);
             if (q.outVX) q.outVX[i] = make_int4(ti | ti << 16, __float_as_int(ft), 0, __float_as_int(fv));
             else q.outP[i] = make_int2(ti, __float_as_int(ft));
@@ -238,6 +242,9 @@ __global__ void slab_kernel(const float *k, const float *ib, float2 *slab, int n
         } else if (e < klen + nT - 1) {
             const float *r = ib + (sid / nq) * nT + (e - klen);
             a = r[0]; b = r[1];
+        } else if (e == klen + nT - 1) {  // the last cell's interpolant at its end
+            const float *r = ib + (sid / nq) * nT + nT - 2;
+            a = b = fmaf(1.0f, r[1] - r[0], r[0]);
         }
         slab[i] = make_float2(a, b - a);
     }

@@ -312,12 +312,40 @@ __device__ __forceinline__ void ray_batch(const MarchParams &P, RayBatch *B, int
 // values, pnb rows a plane: the periodic axes continue past their end by the
 // packet's extent, so a lane's cells lie at fixed offsets from the packet's
 // corner wherever the walk has moved it.
-template <int MODE>
-__device__ __forceinline__ const typename FieldT<MODE>::type *field_base(const MarchParams &P) {
+template <int MODE, bool UNI> struct PairFieldT { typedef typename FieldT<MODE>::type type; };
+template <> struct PairFieldT<MODE_T, true> { typedef float type; };  // the table coordinate
+template <int MODE, bool UNI>
+__device__ __forceinline__ const typename PairFieldT<MODE, UNI>::type *field_base(const MarchParams &P) {
     if constexpr (MODE == MODE_TX) return P.fieldPX;
+    else if constexpr (MODE == MODE_T && UNI) return P.fieldF;
     else if constexpr (MODE == MODE_T) return P.fieldP;
     else return P.fieldG;
 }
+
+// Ib from clamped table coordinates p (uniform absorption: nothing else is
+// looked up).  Adding 2^23 rounded down leaves floor(p) in the low bits of the
+// sum, which the address of the slab's entry takes as it is; the entry past
+// the last cell is the end point's value.  Split as pos_split, bit for bit,
+// the lane's two cells in paired instructions.  4 bytes a cell instead of (index, fraction): the L1 data
+// pipe bounded the band tables' march (86 %), and a gather of 32 four-byte cells takes 2 of
+// its cycles instead of 4.2: drop-in bands call 7.17 -> 6.74 ms.
+struct SlabIb {
+    unsigned ia;  // the address of entry 0, less the bits of 2^23
+    __device__ __forceinline__ explicit SlabIb(const float2 *sli) : ia(smem_addr(sli) - 0x4B000000u * 8u) {}
+    // once a ray's slab has arrived: no lookup of it may move ahead
+    __device__ __forceinline__ void arrived() { asm volatile("" : "+r"(ia)::"memory"); }
+    __device__ __forceinline__ float entry(float s, float f) const {
+        float a, d;
+        asm("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(d) : "r"(__float_as_uint(s) * 8u + ia));
+        return fmaf(f, d, a);
+    }
+    __device__ __forceinline__ float2 lookup(float2 p) const {
+        const float2 sh = make_float2(8388608.0f, 8388608.0f);
+        const float2 s = __fadd2_rd(p, sh);
+        const float2 f = __fadd2_rn(p, __ffma2_rn(s, make_float2(-1.0f, -1.0f), sh));
+        return make_float2(entry(s.x, f.x), entry(s.y, f.y));
+    }
+};
 
 // Resident 256-thread blocks per SM.  Tables: 2 (128 registers: the values of
 // four steps of two cells; 3 spill, 66.2 -> 70.1 ms on the 128^3 channel).
@@ -336,7 +364,8 @@ __host__ __device__ constexpr int pair_min_blocks(bool uni, bool mom) {
 // several queue units (MarchParams::parts).
 template <int MODE, bool UNI, bool TRACE, bool CV, bool MOM, bool SPLIT>
 __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_kernel(const MarchParams P) {
-    typedef typename FieldT<MODE>::type VT;
+    typedef typename PairFieldT<MODE, UNI>::type VT;
+    constexpr bool BANDS = MODE == MODE_T && UNI;
     constexpr int C = kLaneCells;  // cells per lane
     static_assert(C == 2, "the attenuation goes through a cell pair");
     const unsigned FULL = 0xffffffffu;
@@ -367,6 +396,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
     uint64_t *const sbar = &s_bar[warp];
     uint32_t sphase = 0;
     slab_bar_init(sbar, lane);
+    SlabIb tib(sli);  // (used by the band tables)
     bool dead = false;  // a slab copy did not arrive: this warp stops marching
 
     for (;;) {
@@ -403,7 +433,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
             active[k] = ac + la < P.ea1 && bc + lb + k * hb < P.eb1;
             const int a = active[k] ? la : 0, b = active[k] ? lb + k * hb : 0;
             tcell[k] = (pw * nkR + pb * P.tile_b + b) * njR + pa * P.tile_a + a;
-            fp[k] = field_base<MODE>(P) + (long long)f * P.pstride + b * P.pna + a;
+            fp[k] = field_base<MODE, UNI>(P) + (long long)f * P.pstride + b * P.pna + a;
         }
         const unsigned corner = ((unsigned)w0 * P.pnb + bc) * P.pna + ac;
         const int N = P.rays_per_packet ? P.rays_per_packet[G * P.rays_gstride + p] : P.rays;
@@ -421,10 +451,16 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
         } else {
             int boff = 0;
             if (P.n_tbins > 1) {
-                int kx, ti;
-                float ft, fx;
-                cell_coords<MODE>(__ldg(fp[0] + corner), &kx, &ti, &ft, &fx);
-                const float tp0 = __shfl_sync(FULL, (float)ti + ft, 0);
+                float tp;
+                if constexpr (BANDS) {
+                    tp = __ldg(fp[0] + corner);
+                } else {
+                    int kx, ti;
+                    float ft, fx;
+                    cell_coords<MODE>(__ldg(fp[0] + corner), &kx, &ti, &ft, &fx);
+                    tp = (float)ti + ft;
+                }
+                const float tp0 = __shfl_sync(FULL, tp, 0);
                 int bin = __float2int_rn(tp0);
                 bin = min(max(bin, 0), P.n_tbins - 1);
                 boff = bin * P.n_groups;
@@ -505,16 +541,23 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
                     first = false;
                     if constexpr (MODE != MODE_GREY)
                         if (!slab_wait(P, sbar, &sphase, &flags)) { dead = true; break; }
+                    if constexpr (BANDS) {
+                        tib.arrived();
+                        const float2 ib = tib.lookup(make_float2(va[0], va[1]));
+                        Ii[0] = ib.x; Ii[1] = ib.y;
+                    }
 #pragma unroll
                     for (int k = 0; k < C; ++k) {
                         if constexpr (MODE == MODE_GREY) {
                             Ii[k] = va[k];
                             wk[k] = bw.w;
+                        } else if constexpr (BANDS) {
+                            wk[k] = bw.w * P.kappa;
                         } else {
                             int kx, ti;
                             float ft, fx;
                             cell_coords<MODE>(va[k], &kx, &ti, &ft, &fx);
-                            const float ki = UNI ? P.kappa : lookup_k<MODE>(slk, kx, ft, fx);
+                            const float ki = lookup_k<MODE>(slk, kx, ft, fx);
                             Ii[k] = lookup_ib(sli, ti, ft);
                             wk[k] = bw.w * ki;
                         }
@@ -535,25 +578,23 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
                 // instructions with every sign moved onto an operand whose
                 // negation is exact: e = expm1(k * (t - tn)) = -alpha, nta =
                 // tau e = -ta, D += nta (-g), tau += nta -- the same roundings.
-                auto neg_g = [&](const VT &v, int k) {  // UNI: -g of cell k
+                auto neg_g = [&](const VT (&v)[C]) {  // UNI: -g of the cells
                     if constexpr (MODE == MODE_GREY) {
-                        return v - Ii[k];
+                        return make_float2(v[0] - Ii[0], v[1] - Ii[1]);
+                    } else if constexpr (BANDS) {
+                        const float2 ib = tib.lookup(make_float2(v[0], v[1]));
+                        return make_float2(ib.x - Ii[0], ib.y - Ii[1]);
                     } else {
-                        int kx, tj;
-                        float ftj, fxj;
-                        cell_coords<MODE>(v, &kx, &tj, &ftj, &fxj);
-                        return lookup_ib(sli, tj, ftj) - Ii[k];
+                        return make_float2(0.0f, 0.0f);
                     }
                 };
                 auto step = [&](const VT (&v)[C], float nds, int s) {
                     if constexpr (UNI) {
                         const float nta = tau[0] * nds;  // nds: expm1 of the step
-                        float ng[C];
+                        const float2 g = neg_g(v);
+                        const float ng[C] = {g.x, g.y};
 #pragma unroll
-                        for (int k = 0; k < C; ++k) {
-                            ng[k] = neg_g(v[k], k);
-                            D[k] = fmaf(nta, ng[k], D[k]);
-                        }
+                        for (int k = 0; k < C; ++k) D[k] = fmaf(nta, ng[k], D[k]);
                         tau[0] = tau[0] + nta;
                         if (TRACE && lane == 0 && s < P.trace_max)
                             P.trace_rec[6 * s + 5] = __float_as_int(tau[0] < P.toll ? 0.0f : tau[0]);
@@ -611,8 +652,9 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
                         // checks of both in one branch: grey 64^3 3.39 -> 3.12 ms)
                         const float n0 = tau[0] * d0, t0 = tau[0] + n0, n1 = t0 * d1, t1 = t0 + n1;
                         if (t0 >= P.toll && t1 >= P.toll) {
-#pragma unroll
-                            for (int k = 0; k < C; ++k) D[k] = fmaf(n1, neg_g(v1[k], k), fmaf(n0, neg_g(v0[k], k), D[k]));
+                            const float2 g0 = neg_g(v0), g1 = neg_g(v1);
+                            D[0] = fmaf(n1, g1.x, fmaf(n0, g0.x, D[0]));
+                            D[1] = fmaf(n1, g1.y, fmaf(n0, g0.y, D[1]));
                             tau[0] = t1;
                             s += 2;
                             return;

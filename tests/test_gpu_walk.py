@@ -173,3 +173,18 @@ def test_general_medium_walks_match_the_replay(kind, size, albedo, kw, region):
 ])
 def test_walks_at_the_edges_of_a_chunk_match_the_replay(model, size, kw):
     test_walks_match_the_replay(model, size, kw, None)
+
+
+@pytest.mark.parametrize("nT", [2, 3, 4, 55])
+def test_band_tables_that_end_below_the_field_match_the_replay(nT):
+    """With few temperatures the grey band tables end below the field's
+    maximum: cells at the table's end point, and at its first point."""
+    s = D.Solver(D.default_config(model=D.MODEL_GREY_BANDS, imax=14, jmax=12, kmax=9, Lx=1.5, Ly=2.0, Lz=0.7, stretched_x=0,
+                                  T_west=500.0, T_east=700.0, kappa=0.7, seed=12, sampler=D.SAMPLER_RQMC, nvar=2))
+    s.use_grey_band_tables(40, nT, 15000.0, 900.0)
+    T = smooth_field(14, 12, 9, 600, 1500, 3)
+    s.set_fields(T)
+    s.set_rays(14)
+    assert_bitexact(s, T)
+    assert s.status() == 0
+    s.close()
