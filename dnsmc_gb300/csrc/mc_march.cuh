@@ -345,7 +345,7 @@ __device__ __forceinline__ bool slab_bar_wait(const uint64_t *bar, uint32_t pari
 // returns false with the phase unchanged: the warp then takes no further
 // copies or items and calls slab_drain before it exits.  The outcome is
 // the same in every lane of the warp.
-__device__ __forceinline__ void slab_issue(const MarchParams &P, int sid, float2 *slk, int lane, uint64_t *bar) {
+__device__ __forceinline__ void slab_issue(const MarchParams &P, int sid, uint32_t slab, int lane, uint64_t *bar) {
     __syncwarp();
     if (lane == 0) {
         const uint32_t bytes = (uint32_t)P.slab_len * 8u;
@@ -354,7 +354,7 @@ __device__ __forceinline__ void slab_issue(const MarchParams &P, int sid, float2
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                      : "memory");
         asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_addr(slk)),
+                         slab),
                      "l"(src), "r"(bytes), "r"(smem_addr(bar))
                      : "memory");
     }

@@ -161,7 +161,7 @@ __global__ void __launch_bounds__(256, DNSMC_MINB) march_mg_kernel(const MarchPa
                 __syncwarp();
             }
             const float4 bw = batch->walk[rb], br = batch->rates[rb];
-            if constexpr (MODE != MODE_GREY) slab_issue(P, __float_as_int(br.w), slk, lane, sbar);
+            if constexpr (MODE != MODE_GREY) slab_issue(P, __float_as_int(br.w), smem_addr(slk), lane, sbar);
             const float sW = bw.x, sA = bw.y, sB = bw.z;
             const int nbnd = __float_as_int(br.z);
 
