@@ -444,11 +444,28 @@ __device__ __forceinline__ bool unit_done(const MarchParams &P, long long item, 
 }
 
 // Sums of one cell of an item over its N rays in ray order (x: the cell's
-// first contribution, CELLS values a ray), as tally_ray adds them.
+// first contribution, CELLS values a ray), as tally_ray adds them.  Eight rays'
+// values are fetched together; the multigrid march (CELLS = 32), whose steps
+// fill the instruction cache, takes a loop of one ray with four fetched ahead
+// (64^3, five levels: 1.41 -> 1.37 ms; the fine marches lose by it: grey 64^3
+// 2.91 -> 2.98 ms).
 template <int CELLS>
 __device__ __forceinline__ double2 sum_rays(const MarchParams &P, const float *x, int N, int M) {
     float2 sum = make_float2(0.0f, 0.0f), sq = sum, rep = sum;
     int m = 0;
+    if constexpr (CELLS == 32) {
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = q < N ? __ldcg(x + (long long)q * CELLS) : 0.0f;
+#pragma unroll 1
+        for (int r = 0; r < N; ++r) {
+            tally_ray(P, v[0], m, M, &sum, &sq, &rep);
+            m = P.sampler && m == M - 1 ? 0 : m + 1;
+            v[0] = v[1]; v[1] = v[2]; v[2] = v[3];
+            v[3] = r + 4 < N ? __ldcg(x + (long long)(r + 4) * CELLS) : 0.0f;
+        }
+        return make_double2(ff_value(sum), ff_value(sq));
+    }
     for (int r0 = 0; r0 < N; r0 += 8) {
         float v[8];
         const int n = min(8, N - r0);
