@@ -317,7 +317,8 @@ inline size_t march_smem(const MarchParams &p, int threads, int cells) {
 // of a launch of the gas march: each warp's slab, walk buffer and ray batch, then per
 // thread the sums of its two cells; kPairStaticSmem at most beside it
 // words of a warp's walk buffer (mc_march_pair.cuh); uni: uniform absorption
-__host__ __device__ constexpr int walk_words(bool uni) { return uni ? 336 : 304; }
+__host__ __device__ constexpr int walk_cap(bool uni) { return uni ? 192 : 128; }  // steps of a chunk (even)
+__host__ __device__ constexpr int walk_words(bool uni) { return (8 + (uni ? 64 : 32) + 4 + 4 + 2 * (walk_cap(uni) + 1) + 3) / 4 * 4; }
 constexpr size_t kBatchBytes = 1536;  // a warp's ray batch
 constexpr size_t kEventBytes = 512;   // a warp's batch of collision events (general medium)
 constexpr size_t kPairStaticSmem = 256;

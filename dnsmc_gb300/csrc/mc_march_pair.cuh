@@ -41,7 +41,7 @@ namespace dnsmc {
 // A walk is the merge of three sorted sequences: the crossing times of the
 // wall-normal faces and of the two periodic axes, each a closed form of the
 // axis' crossing count (W before A before B where times are equal).  The warp
-// generates it in chunks of at most kWalkCap steps: the chunk's time window
+// generates it in chunks of at most walk_cap steps: the chunk's time window
 // is cut into 31 equal slices, lane l starts slice l from the crossing counts
 // at the slice's start (closed form, corrected by comparing the very products
 // the sequence is made of, so they are exact) and steps through its few
@@ -53,18 +53,15 @@ namespace dnsmc {
 // before it is used.
 // March of the 128^3 correlated-k channel (48 rays): 85.5 -> 66.2 ms; grey 64^3
 // channel at 256 rays: 9.6 -> 4.9 ms.  Chunks of 64 / 96 / 128 / 192 steps:
-// channel 62.5 / 61.9 / 61.6 / 61.7, grey 3.53 / 3.45 / 3.38 / 3.34 ms (longer
-// chunks take more shared memory a warp).
+// channel 62.5 / 61.9 / 61.6 / 61.7 ms (longer chunks take more shared memory a
+// warp).  With uniform absorption, and so with 64 wall-normal crossings listed,
+// 128 / 192 / 256: grey 2.91 / 2.80 / 2.83, drop-in bands call 6.56 / 6.33 / 6.74 ms.
 // ---------------------------------------------------------------------------
-constexpr int kWalkCap = 128;  // steps of a chunk (even)
-// words of a warp's walk buffer: a 4-word header whose last word is the cell
-// entered by the chunk's first step, the pairs (one spare), the state after the
-// chunk, its wall-normal times (walk_words in all)
-constexpr int kWalkState = 4 + 2 * (kWalkCap + 1);
-constexpr int kWalkTimes = kWalkState + 7;
-static_assert(kWalkTimes + 32 + 1 <= walk_words(false) && kWalkTimes + 64 + 1 <= walk_words(true) && walk_words(false) % 4 == 0 &&
-                  walk_words(true) % 4 == 0,
-              "a warp's walk buffer");
+// A warp's walk buffer (walk_words): the state after the chunk (8 words), its
+// wall-normal times (TIMES + 1, rounded up to 4), then -- the pointer the marches
+// hold -- a 4-word header whose last word is the cell entered by the chunk's
+// first step, and the pairs (walk_cap, one spare).
+__host__ __device__ constexpr int walk_times_words(int times) { return times + 4; }
 
 // the float after a non-negative float
 __device__ __forceinline__ float next_up(float v) { return __uint_as_float(__float_as_uint(v) + 1u); }
@@ -127,7 +124,7 @@ __device__ __forceinline__ void walk_direction(const MarchParams &P, Walk &w, fl
 // the tentative collision at time tcol comes next.
 enum WalkEnd { WALK_ON = 0, WALK_WALL = 1, WALK_COL = 2 };
 
-// Generate the next chunk (at most cap steps, cap <= kWalkCap; about `aim` of
+// Generate the next chunk (at most cap steps, cap <= walk_cap; about `aim` of
 // them; none after tcol).  Returns the steps generated (at least one, but
 // before a collision and for unusable faces), *end how the chunk ends.  The
 // state is advanced in shared memory (walk_state reads it back; not written
@@ -144,7 +141,7 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     const int dW = w.dW, dA = w.dA, dB = w.dB;
     const float *fwn = P.fw + (dW > 0 ? 1 : 0);
     const float dtA = w.dtA, dtB = w.dtB, rA = w.rA, rB = w.rB;
-    float *const tw = buf + kWalkTimes;
+    float *const tw = buf - walk_times_words(TIMES), *const st = tw - 8;
     // the next TIMES wall-normal crossings
     const int c = w.cw + dW * lane, c2 = c + dW * 32;
     const bool in = (unsigned)c < (unsigned)P.nw, in2 = TIMES > 32 && (unsigned)c2 < (unsigned)P.nw;
@@ -160,7 +157,7 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     const float tw0 = __shfl_sync(FULL, twl, 0), twe = __shfl_sync(FULL, nv > 32 ? twh : twl, (nv - 1) & 31);
     if (lane == 0) {
         tw[TIMES] = INF;
-        buf[kWalkState + 6] = 0.0f;  // (int) 0 steps, unless a lane makes the last one
+        st[6] = 0.0f;  // (int) 0 steps, unless a lane makes the last one
     }
     // the window: about `aim` crossings at the present rates, no more than
     // the listed wall-normal ones, at least the next crossing
@@ -232,7 +229,6 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
             ++e;
         } while (e < eend && !hit);
         if (e == n0 || hit) {  // this lane made the chunk's last step: the state, and the spare pairs
-            float *st = buf + kWalkState;
             st[0] = t; st[1] = nA; st[2] = nB;
             st[3] = __int_as_float(cw); st[4] = __int_as_float(ca); st[5] = __int_as_float(cb);
             st[6] = __int_as_float(e);
@@ -244,11 +240,12 @@ __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, f
     hit = __any_sync(FULL, hit);
     *end = hit ? WALK_WALL : (col && total <= cap ? WALK_COL : WALK_ON);
     __syncwarp();
-    return __float_as_int(buf[kWalkState + 6]);
+    return __float_as_int(st[6]);
 }
 
+template <int TIMES>
 __device__ __forceinline__ void walk_state(const float *buf, Walk &w) {
-    const float *st = buf + kWalkState;
+    const float *st = buf - walk_times_words(TIMES) - 8;
     w.t = st[0]; w.nA = st[1]; w.nB = st[2];
     w.cw = __float_as_int(st[3]); w.ca = __float_as_int(st[4]); w.cb = __float_as_int(st[5]);
 }
@@ -389,7 +386,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
     const int warp = threadIdx.x >> 5, nwarp = (nthr + 31) >> 5;
     float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + warp * P.slab_len;
     const float2 *const sli = slk + P.slab_klen;
-    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(UNI);
+    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(UNI) + 8 + walk_times_words(UNI ? 64 : 32);
     RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
                                                         nwarp * walk_words(UNI)) + warp;
     float2 *const s_acc = reinterpret_cast<float2 *>(batch - warp + nwarp);
@@ -528,8 +525,8 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
             for (;;) {  // chunks of the walk
                 int end;
                 // a short first chunk where this item's rays have been short
-                const int n = walk_chunk<TRACE, false, UNI ? 64 : 32>(P, w, first && est < 20 ? 28.0f : (float)(kWalkCap - 4),
-                                                       min(kWalkCap, P.max_steps - steps), 0.0f, wbuf, lane, &end, steps);
+                const int n = walk_chunk<TRACE, false, UNI ? 64 : 32>(P, w, first && est < 20 ? 28.0f : (float)(walk_cap(UNI) - 4),
+                                                       min(walk_cap(UNI), P.max_steps - steps), 0.0f, wbuf, lane, &end, steps);
                 if constexpr (UNI) {
                     // e = expm1(k (t - tn)) of the chunk's steps, a lane each
                     for (int q = lane; q < n; q += 32) wbuf[4 + 2 * q] = mc_expm1(P.kappa * wbuf[4 + 2 * q]);
@@ -691,7 +688,7 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
                         flags |= DNSMC_STATUS_STEP_CAP;
                     break;
                 }
-                walk_state(wbuf, w);
+                walk_state<UNI ? 64 : 32>(wbuf, w);
                 {  // the cell the next chunk starts in
                     const unsigned c0 = ((unsigned)w.cw * P.pnb + w.cb) * P.pna + w.ca;
 #pragma unroll
@@ -816,7 +813,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
     const int warp = threadIdx.x >> 5, nwarp = (nthr + 31) >> 5;
     float2 *const slk = reinterpret_cast<float2 *>(s_dyn) + warp * P.slab_len;
     const float2 *const sli = slk + P.slab_klen;
-    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(false);
+    float *const wbuf = reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) + warp * walk_words(false) + 8 + walk_times_words(32);
     RayBatch *const batch = reinterpret_cast<RayBatch *>(reinterpret_cast<float *>(reinterpret_cast<float2 *>(s_dyn) + nwarp * P.slab_len) +
                                                         nwarp * walk_words(false)) + warp;
     float4 *const events = reinterpret_cast<float4 *>(batch - warp + nwarp) + warp * 2 * kEvents;
@@ -1029,7 +1026,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
             bool first = true;
             for (;;) {  // chunks of the walk
                 int end;
-                const int n = walk_chunk<TRACE, true, 32>(P, w, (float)(kWalkCap - 4), min(kWalkCap, P.max_steps - steps), tcol,
+                const int n = walk_chunk<TRACE, true, 32>(P, w, (float)(walk_cap(false) - 4), min(walk_cap(false), P.max_steps - steps), tcol,
                                                       wbuf, lane, &end, steps);
                 {
                     const unsigned c1 = n ? __float_as_uint(wbuf[3]) : corner;
@@ -1081,7 +1078,7 @@ __global__ void __launch_bounds__(256, DNSMC_PAIR_MINB) march_gen_kernel(const M
                         if (done || s >= n) break;
                     }
                     steps += n;
-                    walk_state(wbuf, w);
+                    walk_state<32>(wbuf, w);
                 }
                 if (done) break;  // every cell dumped
                 if (end == WALK_WALL) {

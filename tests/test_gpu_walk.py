@@ -170,6 +170,9 @@ def test_general_medium_walks_match_the_replay(kind, size, albedo, kw, region):
     ("grey", (64, 3, 64), dict(kappa=0.02)),                  # as many planes as a chunk lists crossings
     ("bands", (131, 9, 6), dict(kappa=0.03)),
     ("T", (150, 5, 8), dict(max_steps=129)),
+    ("T", (150, 5, 8), dict(max_steps=128)),
+    ("grey", (300, 8, 8), dict(kappa=0.005, max_steps=192)),  # (uniform absorption takes longer chunks)
+    ("bands", (300, 6, 9), dict(kappa=0.005, max_steps=193)),
 ])
 def test_walks_at_the_edges_of_a_chunk_match_the_replay(model, size, kw):
     test_walks_match_the_replay(model, size, kw, None)
