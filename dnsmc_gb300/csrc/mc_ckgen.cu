@@ -316,7 +316,10 @@ extern "C" int dnsmc_ck_from_lbl(const dnsmc_lbl_desc *d, float *kq, double *kav
     cudaError_t e = mem.alloc(a_kq + (size_t)items * d->nq * 4);
     if (e != cudaSuccess) return report_error(DNSMC_ERR_NOMEM, cudaGetErrorString(e));
     unsigned char *in = mem.p + (size_t)nk * 8;
+    // (the copy of pageable memory may still be under way when cudaMemcpy
+    // returns, and the streams below do not wait for the default stream)
     e = cudaMemcpy(in, small.data(), n_small, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e != cudaSuccess) return report_error(DNSMC_ERR_CUDA, cudaGetErrorString(e));
     unsigned int *bad = (unsigned int *)(in + o_bad);
     CkGenParams P{};
