@@ -334,7 +334,7 @@ extern "C" int dnsmc_ck_from_lbl(const dnsmc_lbl_desc *d, float *kq, double *kav
     }
     // Spectra of 8 MB and more go over in four parts, each with its own stream,
     // so that a part's kernels run while the next is copied.  52 spectra of 80001
-    // points (33 MB): 760 -> 676 us (2 parts 745, 8 parts 740).
+    // points (33 MB): 760 -> 690 us (2 parts 745, 8 parts 740).
     const long long ntx = (long long)d->nT * d->nX;
     const int parts = nk * 8 >= (8 << 20) ? (int)std::min<long long>(Streams::kMax, ntx) : 1;
     Streams st;
