@@ -1024,7 +1024,8 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     P.fieldF = s->d_posF.p;
     P.fieldVX = s->d_posTX.p;
     P.fieldVG = s->d_posVG.p;
-    FieldPos fp{};  // table coordinates of the field for this table (once per solve)
+    FieldPos fp;  // table coordinates of the field for this table (once per solve)
+    memset(&fp, 0, sizeof fp);  // its bytes are part of the graph key too
     fp.fT = mode == MODE_TX ? nullptr : s->d_fieldT.p;
     fp.fTX = mode == MODE_TX ? s->d_fieldTX.p : nullptr;
     if (gen) {
@@ -1256,13 +1257,16 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         // Replay the captured sequence when every parameter it baked in is
         // unchanged; otherwise capture it again.  The march timing then
         // brackets the whole graph.
-        std::vector<unsigned char> key(sizeof P + sizeof cp + sizeof F + 4 * sizeof(long long));
+        // The fields' own arrays are in fp alone, the host's end of the copies in extra.
+        const long long extra[5] = {blocks, threads, (long long)(cv ? 1 : 0) | (mom ? 2 : 0) | ((long long)mode << 2),
+                                    (long long)(uintptr_t)s->stream,
+                                    (long long)(f32 ? (uintptr_t)s->h_Qf.p : (uintptr_t)s->h_Q.p)};
+        std::vector<unsigned char> key(sizeof P + sizeof cp + sizeof F + sizeof fp + sizeof extra);
         unsigned char *k = key.data();
         memcpy(k, &P, sizeof P); k += sizeof P;
         memcpy(k, &cp, sizeof cp); k += sizeof cp;
         memcpy(k, &F, sizeof F); k += sizeof F;
-        const long long extra[4] = {blocks, threads, (long long)(cv ? 1 : 0) | (mom ? 2 : 0) | ((long long)mode << 2),
-                                    (long long)(uintptr_t)s->stream};
+        memcpy(k, &fp, sizeof fp); k += sizeof fp;
         memcpy(k, extra, sizeof extra);
         if (!s->graph_exec || key != s->graph_key) {
             if (s->graph_exec) { cudaGraphExecDestroy(s->graph_exec); s->graph_exec = nullptr; }

@@ -1,0 +1,62 @@
+"""What a solver holds between calls: captured graphs, resident fields and
+buffers across changes of the snapshots' number, refused inputs and short device
+memory."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import dnsmc_gb300 as D
+from dnsmc_gb300 import synth
+
+from test_gpu_parity import smooth_field
+from test_gpu_scatter import particle_table
+
+pytestmark = pytest.mark.gpu
+
+NI, NJ, NK = 12, 40, 9
+
+
+def snapshots(n, seed=1):
+    T = np.stack([smooth_field(NI, NJ, NK, 450, 1600, seed + f) for f in range(n)])
+    rng = np.random.default_rng(seed)
+    x = (0.1 + 0.05 * rng.uniform(-1, 1, T.shape)).astype(np.float32)
+    fv = (1e-5 * rng.uniform(0.2, 1.0, T.shape)).astype(np.float32)
+    fv[:, 0, 0, 0] = 1e-5  # the same largest fraction in every snapshot
+    return T, x, fv
+
+
+def particle_solver(**kw):
+    cfg = dict(model=D.MODEL_TABLE, imax=NI, jmax=NJ, kmax=NK, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=0, T_west=400,
+               T_east=700, n_groups=2, seed=8, local_sampling=1)
+    s = D.Solver(D.default_config(**dict(cfg, **kw)))
+    t = synth.ck_table(nbands=8, nq=4, nT=14, nX=4, seed=5)
+    s.set_table(t["k"], t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"], X0=t["X0"], dX=t["dX"])
+    s.set_particles(*particle_table(8, 2), 0.4)
+    return s
+
+
+def test_graph_is_captured_again_for_other_field_arrays():
+    """Fields of two snapshots take the place of one's arrays; back at one
+    snapshot, nothing else that the solve reads has moved."""
+    T, x, fv = snapshots(2)
+    eager, graph = particle_solver(), particle_solver()
+    graph.set_graph(True)
+    out = []
+    for s in (eager, graph):
+        s.set_rays(16)
+        s.set_fields(T[0], x[0])
+        s.set_particle_field(fv[0])
+        first = s.solve(timeout_s=60)
+        s.set_fields(T, x)
+        s.set_particle_field(fv)
+        s.set_fields(T[0], x[0])
+        s.set_particle_field(fv[0])
+        out.append((first, s.solve(timeout_s=60)))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a[0], b[0])
+        np.testing.assert_array_equal(a[1], b[1])
+    np.testing.assert_array_equal(out[1][0][0], out[1][1][0])
+    assert graph.graph_info() == (2, 2)
+    eager.close()
+    graph.close()
