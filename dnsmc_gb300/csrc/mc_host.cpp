@@ -366,6 +366,21 @@ struct dnsmc_solver {
 
 namespace {
 
+// Host arrays to the device and back, in the order of the solver's stream and
+// complete on return: the default stream is not ordered with that stream, and
+// a copy of pageable memory to the device may still be under way when
+// cudaMemcpy returns.
+int to_device(dnsmc_solver *s, void *dst, const void *src, size_t bytes) {
+    CUDA_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, s->stream));
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    return DNSMC_OK;
+}
+int to_host(dnsmc_solver *s, void *dst, const void *src, size_t bytes) {
+    CUDA_TRY(cudaStreamSynchronize(s->stream));
+    CUDA_TRY(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost));
+    return DNSMC_OK;
+}
+
 // The device side of a solver (stream, events, faces) is created on first
 // use, so table parsing and sampling construction work without a GPU.
 int ensure_device(dnsmc_solver *s) {
@@ -388,11 +403,12 @@ int ensure_device(dnsmc_solver *s) {
         sobol_directions(dirs);
         const int rc = upload_sobol_dirs(dirs);
         if (rc) return fail(DNSMC_ERR_CUDA, "Sobol' table upload: %s", cudaGetErrorString((cudaError_t)rc));
+        CUDA_TRY(cudaStreamSynchronize(0));  // (to_device: these copies are the default stream's)
     }
     if (const int rc = cv_table_allow_smem())
         return fail(DNSMC_ERR_CUDA, "table kernel shared memory: %s", cudaGetErrorString((cudaError_t)rc));
     if (int rc = s->d_fw.ensure(s->fw.size())) return rc;
-    CUDA_TRY(cudaMemcpy(s->d_fw.p, s->fw.data(), s->fw.size() * sizeof(float), cudaMemcpyHostToDevice));
+    TRY(to_device(s, s->d_fw.p, s->fw.data(), s->fw.size() * sizeof(float)));
     return DNSMC_OK;
 }
 
@@ -2037,7 +2053,7 @@ int dnsmc_set_particles(dnsmc_solver *s, int nbands, const float *absorption, co
     }
     TRY(set_device(s));
     TRY(s->d_part.ensure(pp.size()));
-    CUDA_TRY(cudaMemcpy(s->d_part.p, pp.data(), pp.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    TRY(to_device(s, s->d_part.p, pp.data(), pp.size() * sizeof(float2)));
     s->part = pp;
     s->hg_g = hg_g;
     return DNSMC_OK;
@@ -2131,7 +2147,7 @@ int dnsmc_set_rays(dnsmc_solver *s, int rays_per_group, const int *rays_per_pack
         s->rays_pp.assign(rays_per_packet, rays_per_packet + np);
         s->rays_np = np;
         TRY(s->d_rays_pp.ensure(np));
-        CUDA_TRY(cudaMemcpy(s->d_rays_pp.p, s->rays_pp.data(), np * sizeof(int), cudaMemcpyHostToDevice));
+        TRY(to_device(s, s->d_rays_pp.p, s->rays_pp.data(), np * sizeof(int)));
     } else {
         s->rays_pp.clear();
     }
@@ -2158,7 +2174,7 @@ int dnsmc_set_rays_per_item(dnsmc_solver *s, int n_groups, const int *rays) {
     s->rays_dev = false;
     s->rays_np = np;
     TRY(s->d_rays_pp.ensure(n));
-    CUDA_TRY(cudaMemcpy(s->d_rays_pp.p, s->rays_pp.data(), n * sizeof(int), cudaMemcpyHostToDevice));
+    TRY(to_device(s, s->d_rays_pp.p, s->rays_pp.data(), n * sizeof(int)));
     return DNSMC_OK;
 }
 
@@ -2172,9 +2188,7 @@ int dnsmc_get_coarse_field(dnsmc_solver *s, int field, int level, float *T) {
     const int im = c.imax >> level, jm = c.jmax >> level, km = c.kmax >> level;
     const size_t n = (size_t)im * jm * km;
     std::vector<float> h(n);
-    CUDA_TRY(cudaStreamSynchronize(s->stream));  // the coarsening runs on the solver's stream
-    CUDA_TRY(cudaMemcpy(h.data(), s->d_mgT.p + s->mg_off[level] + (long long)field * n, n * sizeof(float),
-                        cudaMemcpyDeviceToHost));
+    TRY(to_host(s, h.data(), s->d_mgT.p + s->mg_off[level] + (long long)field * n, n * sizeof(float)));
     for (int i = 0; i < im; ++i)
         for (int k = 0; k < km; ++k)
             for (int j = 0; j < jm; ++j) T[(size_t)i + (size_t)im * (j + (size_t)jm * k)] = h[((size_t)i * km + k) * jm + j];
@@ -2296,7 +2310,7 @@ int dnsmc_get_rays_per_item(dnsmc_solver *s, int *n_groups, int *rays) {
     const size_t rows = *n_groups > 0 ? (size_t)*n_groups : 1;
     if (s->rays_dev) {
         TRY(set_device(s));
-        CUDA_TRY(cudaMemcpy(rays, s->d_rays_pp.p, rows * np * sizeof(int), cudaMemcpyDeviceToHost));
+        TRY(to_host(s, rays, s->d_rays_pp.p, rows * np * sizeof(int)));
     } else {
         memcpy(rays, s->rays_pp.data(), rows * np * sizeof(int));
     }
@@ -2309,7 +2323,7 @@ int dnsmc_get_item_steps(dnsmc_solver *s, double *steps) {
     const long long n = s->last.n_items;
     if (n <= 0 || !s->item_steps) return fail(DNSMC_ERR_STATE, "no solve yet");
     std::vector<unsigned long long> h((size_t)n);
-    CUDA_TRY(cudaMemcpy(h.data(), s->item_steps, (size_t)n * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
+    TRY(to_host(s, h.data(), s->item_steps, (size_t)n * sizeof(unsigned long long)));
     for (long long i = 0; i < n; ++i) steps[i] = (double)h[(size_t)i];
     return DNSMC_OK;
 }
@@ -2428,8 +2442,8 @@ int dnsmc_get_group_results(dnsmc_solver *s, double *Qg, double *varg) {
     TRY(wait_done(s, 0));
     TRY(set_device(s));
     const size_t n = (size_t)s->nfields * s->last.region_cells * s->last.n_groups;
-    if (Qg) CUDA_TRY(cudaMemcpy(Qg, s->d_Qg.p, n * sizeof(double), cudaMemcpyDeviceToHost));
-    if (varg) CUDA_TRY(cudaMemcpy(varg, s->d_varg.p, n * sizeof(double), cudaMemcpyDeviceToHost));
+    if (Qg) TRY(to_host(s, Qg, s->d_Qg.p, n * sizeof(double)));
+    if (varg) TRY(to_host(s, varg, s->d_varg.p, n * sizeof(double)));
     return DNSMC_OK;
 }
 
@@ -2505,7 +2519,7 @@ int dnsmc_set_cv_beta(dnsmc_solver *s, const float *beta) {
                 }
     TRY(set_device(s));
     TRY(s->d_beta.ensure(tl.size()));
-    CUDA_TRY(cudaMemcpy(s->d_beta.p, tl.data(), tl.size() * sizeof(float2), cudaMemcpyHostToDevice));
+    TRY(to_device(s, s->d_beta.p, tl.data(), tl.size() * sizeof(float2)));
     s->beta_set = true;
     return DNSMC_OK;
 }
@@ -2522,7 +2536,7 @@ int dnsmc_get_cv_beta(dnsmc_solver *s, float *beta) {
     if (s->d_beta.n < n) return fail(DNSMC_ERR_STATE, "coefficients were set for another region");
     std::vector<float2> tl(n);
     TRY(set_device(s));
-    CUDA_TRY(cudaMemcpy(tl.data(), s->d_beta.p, n * sizeof(float2), cudaMemcpyDeviceToHost));
+    TRY(to_host(s, tl.data(), s->d_beta.p, n * sizeof(float2)));
     for (long long fg = 0; fg < (long long)s->nfields * nG; ++fg)
         for (int i = 0; i < ni; ++i)
             for (int k = 0; k < nk; ++k)
@@ -2556,7 +2570,7 @@ int dnsmc_get_cv_moments(dnsmc_solver *s, double *moments) {
     region_dims(s, &ni, &nj, &nk);
     const long long nfg = (long long)s->nfields * s->last.n_groups;
     std::vector<double> tl((size_t)(nfg * ni * nj * nk * 9));
-    CUDA_TRY(cudaMemcpy(tl.data(), s->d_moments.p, tl.size() * sizeof(double), cudaMemcpyDeviceToHost));
+    TRY(to_host(s, tl.data(), s->d_moments.p, tl.size() * sizeof(double)));
     tally_to_dense(tl.data(), moments, nfg, ni, nj, nk, 9);
     return DNSMC_OK;
 }
@@ -2569,7 +2583,7 @@ int dnsmc_get_cv_table(dnsmc_solver *s, float *tab) {
     TRY(wait_done(s, 0));
     TRY(set_device(s));
     const size_t n = (size_t)s->nfields * s->cv_samples * s->cfg.imax * 2 * kSurBins;
-    CUDA_TRY(cudaMemcpy(tab, s->d_surtab.p, n * sizeof(float4), cudaMemcpyDeviceToHost));
+    TRY(to_host(s, tab, s->d_surtab.p, n * sizeof(float4)));
     return DNSMC_OK;
 }
 
@@ -2581,15 +2595,15 @@ int dnsmc_get_cv_data(dnsmc_solver *s, int *n_samples, float *layer, float *sur,
     const int S = s->cv_samples;
     if (n_samples) *n_samples = S;
     const size_t nl = (size_t)s->nfields * s->cfg.imax, ns = nl * S;
-    if (layer) CUDA_TRY(cudaMemcpy(layer, s->d_layer.p, nl * sizeof(float2), cudaMemcpyDeviceToHost));
-    if (sur) CUDA_TRY(cudaMemcpy(sur, s->d_sur.p, ns * sizeof(float2), cudaMemcpyDeviceToHost));
-    if (Jhat) CUDA_TRY(cudaMemcpy(Jhat, s->d_Jhat.p, ns * sizeof(double2), cudaMemcpyDeviceToHost));
+    if (layer) TRY(to_host(s, layer, s->d_layer.p, nl * sizeof(float2)));
+    if (sur) TRY(to_host(s, sur, s->d_sur.p, ns * sizeof(float2)));
+    if (Jhat) TRY(to_host(s, Jhat, s->d_Jhat.p, ns * sizeof(double2)));
     if (muY) {
         int ni, nj, nk;
         region_dims(s, &ni, &nj, &nk);
         const long long nfg = (long long)s->nfields * s->last.n_groups;
         std::vector<double> tl((size_t)(nfg * ni * nj * nk * 2));
-        CUDA_TRY(cudaMemcpy(tl.data(), s->d_muY.p, tl.size() * sizeof(double), cudaMemcpyDeviceToHost));
+        TRY(to_host(s, tl.data(), s->d_muY.p, tl.size() * sizeof(double)));
         tally_to_dense(tl.data(), muY, nfg, ni, nj, nk, 2);
     }
     return DNSMC_OK;

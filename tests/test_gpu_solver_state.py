@@ -60,3 +60,19 @@ def test_graph_is_captured_again_for_other_field_arrays():
     assert graph.graph_info() == (2, 2)
     eager.close()
     graph.close()
+
+
+def test_ray_counts_are_read_after_the_kernel_that_sets_them():
+    """Adaptive counts, read back at once: the kernel runs on the solver's own
+    stream.  (A solve in between must find the same ones.)"""
+    n = 64
+    T = smooth_field(n, n, n, 450, 1600, 3)
+    s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=n, jmax=n, kmax=n, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=0,
+                                  T_west=400, T_east=400, kappa=0.5, seed=2))
+    s.set_fields(T)
+    for per_tau in (40.0, 400.0) * 4:
+        s.set_rays_adaptive(per_tau, 8, 4096)
+        now = s.rays_per_item()
+        s.solve(timeout_s=60)
+        np.testing.assert_array_equal(now, s.rays_per_item())
+    s.close()
