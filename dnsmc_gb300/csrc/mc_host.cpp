@@ -285,6 +285,8 @@ struct dnsmc_solver {
     // multigrid: spline-coarsened temperatures of levels 1..grid_num-1
     DevBuf<float> d_mgT, d_mgfw;
     DevBuf<unsigned char> d_mgtab;           // splines: coefficients, brackets, positions
+    std::vector<unsigned char> mg_tab;       // the sources of d_mgtab and d_mgfw: kept, their copies
+    std::vector<float> mg_faces;             // may be under way when set_fields returns
     DevBuf<float> d_mgtmp;                   // coarsening passes' intermediate fields
     DevBuf<double> d_mgwork;                 // lines too long for shared memory
     DevBuf<int2> d_mgP;                      // their table coordinates (T tables)
@@ -1415,8 +1417,12 @@ int upload_coarse(dnsmc_solver *s, int nfields, const float *src, int src_step) 
         for (int l = 1; l < G; ++l) { oat[l][d] = nat; nat += n[d] >> l; }
     }
     const size_t bat = nco * sizeof(SplineCoef), bpos = bat + nat * sizeof(SplineAt);
-    std::vector<unsigned char> tab(bpos + npos * sizeof(float));
-    std::vector<float> faces, fc, cc;
+    // (the copies of the call before are complete: the statistics of the fields
+    // have been read from the same stream since)
+    std::vector<unsigned char> &tab = s->mg_tab;
+    std::vector<float> &faces = s->mg_faces, fc, cc;
+    tab.assign(bpos + npos * sizeof(float), 0);
+    faces.clear();
     for (int d = 0; d < 3; ++d) {
         centres(u[d], fc);
         spline_coefs(fc, reinterpret_cast<SplineCoef *>(tab.data()) + oco[d]);

@@ -8,6 +8,7 @@ import pytest
 
 import dnsmc_gb300 as D
 from dnsmc_gb300 import synth
+from oracle import oracle as O
 
 from test_gpu_parity import smooth_field
 from test_gpu_scatter import particle_table
@@ -76,3 +77,24 @@ def test_ray_counts_are_read_after_the_kernel_that_sets_them():
         s.solve(timeout_s=60)
         np.testing.assert_array_equal(now, s.rays_per_item())
     s.close()
+
+
+def test_coarse_fields_whatever_follows_the_call():
+    """The coarsening's tables are still being copied when set_fields returns:
+    solvers of other sizes, whose tables would take freed memory of the same
+    kind, must not change them."""
+    sizes = ((24, 16, 8), (40, 8, 24), (16, 32, 16))
+    cfg = [dict(model=D.MODEL_GREY, imax=a, jmax=b, kmax=c, Lx=2.0 + a, Ly=6.28, Lz=3.14, stretched_x=1, grid_num=3,
+                kappa=1.0, T_west=300, T_east=300) for a, b, c in sizes]
+    T = [smooth_field(*n, 450, 1300, 9) for n in sizes]
+    ref = [[O.coarsen(np.pad(t, 1).ravel(), *n, 2.0 + n[0], 6.28, 3.14, 1, 3, lv)[1:-1, 1:-1, 1:-1] for lv in (1, 2)]
+           for n, t in zip(sizes, T)]
+    solvers = [D.Solver(D.default_config(**c)) for c in cfg]
+    for _ in range(10):
+        for s, t in zip(solvers, T):
+            s.set_fields(t)
+        for s, r in zip(solvers, ref):
+            for lv in (1, 2):
+                np.testing.assert_array_equal(s.coarse_field(0, lv), r[lv - 1])
+    for s in solvers:
+        s.close()
