@@ -1987,6 +1987,10 @@ int dnsmc_prepare_sampling(dnsmc_solver *s, float Tmax, float xmean) {
     if (!(Tmax > 0)) return fail(DNSMC_ERR_ARG, "Tmax must be > 0");
     if (s->cfg.model != DNSMC_MODEL_GREY && !s->tab.valid && !s->tab.grey_bands)
         return fail(DNSMC_ERR_STATE, "no tables: load or set tables first");
+    if (s->in_flight) {  // it may still be copying the tables that are rewritten here
+        TRY(set_device(s));
+        CUDA_TRY(cudaEventSynchronize(s->ev_march0));
+    }
     if (s->tab.grey_bands) { build_grey_band_tables(s->tab, Tmax); s->tables_dirty = true; }
     s->tmax_used = Tmax;
     s->sampling_valid = false;  // the host tables now differ from the device's: the next solve rebuilds
@@ -2337,7 +2341,10 @@ int dnsmc_get_item_steps(dnsmc_solver *s, double *steps) {
 int dnsmc_solve_async(dnsmc_solver *s) {
     if (!s) return fail(DNSMC_ERR_ARG, "null solver");
     TRY(wait_done(s, 0));
-    return solve_enqueue(s, false, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr);
+    const int rc = solve_enqueue(s, false, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr);
+    // (copies of the sampling tables may be under way: the next solve rewrites them)
+    if (rc && s->dev_ready && !s->in_flight) cudaStreamSynchronize(s->stream);
+    return rc;
 }
 
 int dnsmc_wait(dnsmc_solver *s, double timeout_s) {

@@ -98,3 +98,23 @@ def test_coarse_fields_whatever_follows_the_call():
                 np.testing.assert_array_equal(s.coarse_field(0, lv), r[lv - 1])
     for s in solvers:
         s.close()
+
+
+def test_sampling_prepared_while_a_solve_is_under_way():
+    """The sampling tables rewritten right after solve_async: the solve has its
+    own copies of them, and the next one builds them again."""
+    T, x, fv = snapshots(1)
+    s = particle_solver()
+    s.set_rays(64)
+    s.set_fields(T, x)
+    s.set_particle_field(fv)
+    Q, S = s.solve(timeout_s=60)
+    for Tmax in (600.0, 1500.0, 900.0):
+        s.prepare_sampling(Tmax, 0.05)  # (the solve that follows uploads its tables)
+        s.solve_async()
+        s.prepare_sampling(Tmax + 50.0, 0.2)
+        s.wait(60)
+        Q1, S1 = s.results()
+        np.testing.assert_array_equal(Q, Q1)
+        np.testing.assert_array_equal(S, S1)
+    s.close()
