@@ -438,6 +438,15 @@ int set_dev(dnsmc_cvnet *n) {
     return DNSMC_OK;
 }
 
+// A host array to the device on the network's stream, complete on return: the
+// default stream is not ordered with that stream, and a copy of pageable
+// memory may still be under way when cudaMemcpy returns.
+int to_device(dnsmc_cvnet *n, void *dst, const void *src, size_t bytes) {
+    CK(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, n->stream));
+    CK(cudaStreamSynchronize(n->stream));
+    return DNSMC_OK;
+}
+
 // The tcgen05 forward (mc_cvnet_tc.cuh): one CTA per SM, persistent.
 int launch_forward_tc(TcParams &F, dnsmc_cvnet *n, cudaStream_t st) {
     static int attr = 0;
@@ -573,9 +582,9 @@ int init_params(dnsmc_cvnet *n) {
         for (int c = NFEAT; c < K0; ++c) h[OFF_W1 + (long long)r * K0 + c] = 0.0f;
     fill(OFF_W2, HID, HID, HID);
     fill(OFF_W3, HID, HID, HID);
-    CK(cudaMemcpy(n->P.p, h.data(), NPARAM * sizeof(float), cudaMemcpyHostToDevice));
-    CK(cudaMemset(n->m.p, 0, NPARAM * sizeof(float)));
-    CK(cudaMemset(n->v.p, 0, NPARAM * sizeof(float)));
+    RTRY(to_device(n, n->P.p, h.data(), NPARAM * sizeof(float)));
+    CK(cudaMemsetAsync(n->m.p, 0, NPARAM * sizeof(float), n->stream));
+    CK(cudaMemsetAsync(n->v.p, 0, NPARAM * sizeof(float), n->stream));
     dnsmc::note_launch();
     weights_to_bf16_kernel<<<grid1(NWEIGHT, 256), 256, 0, n->stream>>>(n->P.p, n->W.p);
     CK(cudaGetLastError());
@@ -623,7 +632,8 @@ int dnsmc_cvnet_create(const dnsmc_cvnet_config *cfg, dnsmc_cvnet **out) {
     if (!rc) rc = n->v.ensure(NPARAM);
     if (!rc) rc = n->W.ensure(NWEIGHT_ALL);  // tensor-core order, then the transposes
     if (!rc) rc = n->status.ensure(1);
-    if (!rc && (e = cudaMemset(n->status.p, 0, sizeof(unsigned int))) != cudaSuccess) rc = cuda_fail("cudaMemset", e);
+    if (!rc && (e = cudaMemsetAsync(n->status.p, 0, sizeof(unsigned int), n->stream)) != cudaSuccess)
+        rc = cuda_fail("cudaMemsetAsync", e);
     if (!rc) rc = init_params(n);
     if (rc) { delete n; return rc; }
     *out = n;
@@ -655,9 +665,9 @@ int dnsmc_cvnet_set_params(dnsmc_cvnet *n, const float *params, const float *sca
     if (params) {
         for (long long e = 0; e < NPARAM; ++e)
             if (!std::isfinite(params[e])) return arg_fail("parameters must be finite");
-        CK(cudaMemcpy(n->P.p, params, NPARAM * sizeof(float), cudaMemcpyHostToDevice));
-        CK(cudaMemset(n->m.p, 0, NPARAM * sizeof(float)));
-        CK(cudaMemset(n->v.p, 0, NPARAM * sizeof(float)));
+        RTRY(to_device(n, n->P.p, params, NPARAM * sizeof(float)));
+        CK(cudaMemsetAsync(n->m.p, 0, NPARAM * sizeof(float), n->stream));
+        CK(cudaMemsetAsync(n->v.p, 0, NPARAM * sizeof(float), n->stream));
         n->step = 0;
         dnsmc::note_launch();
         weights_to_bf16_kernel<<<grid1(NWEIGHT, 256), 256, 0, n->stream>>>(n->P.p, n->W.p);
@@ -840,7 +850,10 @@ int dnsmc_cvnet_eval(dnsmc_cvnet *n, const float *features, long long rows, floa
     CK(cudaMemcpyAsync(n->iX.p, h.data(), h.size() * sizeof(bf16), cudaMemcpyHostToDevice, n->stream));
     TcParams F{};
     F.rows = rows; F.X = n->iX.p; F.out = n->iout.p;
-    RTRY(launch_forward_tc(F, n, n->stream));
+    if (const int rc = launch_forward_tc(F, n, n->stream)) {
+        cudaStreamSynchronize(n->stream);  // (h is still being copied)
+        return rc;
+    }
     CK(cudaMemcpyAsync(out, n->iout.p, (size_t)rows * NOUT * sizeof(float), cudaMemcpyDeviceToHost, n->stream));
     unsigned int st = 0;
     CK(cudaMemcpyAsync(&st, n->status.p, sizeof st, cudaMemcpyDeviceToHost, n->stream));
@@ -861,13 +874,13 @@ int dnsmc_cvnet_gradient(dnsmc_cvnet *n, const float *features, const float *lab
         for (int q = 0; q < NFEAT; ++q) h[(size_t)(r * K0 + q)] = __float2bfloat16(features[r * NFEAT + q]);
     NBuf<bf16> x;
     NBuf<float> lab;
-    RTRY(x.ensure((size_t)R * K0));
-    RTRY(lab.ensure((size_t)rows * n_groups * NLAB));
-    CK(cudaMemcpy(x.p, h.data(), h.size() * sizeof(bf16), cudaMemcpyHostToDevice));
-    CK(cudaMemcpy(lab.p, labels, (size_t)rows * n_groups * NLAB * sizeof(float), cudaMemcpyHostToDevice));
     double l[3] = {0, 0, 0};
     const long long tiles = R / TC_TILE;
-    int rc = n->lpart.ensure((size_t)(tiles * 3));
+    int rc = x.ensure((size_t)R * K0);
+    if (!rc) rc = lab.ensure((size_t)rows * n_groups * NLAB);
+    if (!rc) rc = to_device(n, x.p, h.data(), h.size() * sizeof(bf16));
+    if (!rc) rc = to_device(n, lab.p, labels, (size_t)rows * n_groups * NLAB * sizeof(float));
+    if (!rc) rc = n->lpart.ensure((size_t)(tiles * 3));
     if (!rc) rc = train_step(n, x.p, lab.p, n_groups, nullptr, R, rows, n->lpart.p, false);
     if (!rc) {
         std::vector<double> hl((size_t)(tiles * 3));

@@ -1,0 +1,37 @@
+"""What a network holds between calls: inputs and permutations on their way to
+the device, chained training steps, work buffers shared by several solvers."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+import dnsmc_gb300 as D
+from oracle import cvnet_oracle as NO
+
+from test_gpu_cvnet import make_labels, random_params
+
+pytestmark = pytest.mark.gpu
+
+
+def test_gradients_of_inputs_that_are_still_being_copied():
+    """Calls one after the other on inputs of several megabytes: each has its
+    own inputs complete before its kernels start."""
+    net = D.CvNet(D.cvnet_default_config(ridge=0.05, n_groups=16))
+    scales = np.array([2.0, 1.3, 0.8], np.float32)
+    rng = np.random.default_rng(1)
+    sets = []
+    for seed, rows in ((2, 60000), (3, 3000), (4, 40000)):
+        feats = NO.bf16(rng.uniform(-1, 1, (rows, NO.NFEAT)).astype(np.float32))
+        sets.append((random_params(seed), feats, make_labels(rows, 8, seed)))
+    ref = []
+    for p, f, y in sets:
+        net.set_params(p, scales)
+        net.gradient(f, y)
+        ref.append(net.gradient(f, y))
+    for _ in range(3):
+        for (p, f, y), (g, loss) in zip(sets, ref):
+            net.set_params(p, scales)
+            g1, loss1 = net.gradient(f, y)
+            np.testing.assert_array_equal(g, g1)
+            np.testing.assert_array_equal(loss, loss1)
+    net.close()
