@@ -420,7 +420,14 @@ struct dnsmc_cvnet {
     NBuf<unsigned int> lam_done;     // and its finished-block counter
     NBuf<unsigned int> status;                // DNSMC_STATUS_* bits of the tensor-memory forward
     std::mt19937_64 rng;
+    // the rows' order of a pass, in turn: a pass is shuffled while the one
+    // before runs, and not before the copy of the one before that is complete
+    std::vector<int> perm[2];
+    cudaEvent_t perm_copied[2] = {};
     ~dnsmc_cvnet() {
+        if (stream) cudaStreamSynchronize(stream);
+        for (cudaEvent_t e : perm_copied)
+            if (e) cudaEventDestroy(e);
         P.release(); grad.release(); m.release(); v.release(); W.release(); dX.release(); dlab.release();
         idx.release(); H0.release(); H1.release(); H2.release(); H3.release(); dO.release(); dZ3.release();
         dZ2.release(); dZ1.release(); part.release();
@@ -815,13 +822,18 @@ int dnsmc_cvnet_train(dnsmc_cvnet *n, int epochs, double *loss) {
     RTRY(ensure_work(n, B));
     RTRY(n->idx.ensure((size_t)n->nrows));
     RTRY(n->lpart.ensure((size_t)(steps * tiles * 3)));
-    std::vector<int> perm((size_t)n->nrows);
+    for (cudaEvent_t &e : n->perm_copied)
+        if (!e) CK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     for (int ep = 0; ep < epochs; ++ep) {
+        std::vector<int> &perm = n->perm[ep & 1];
+        CK(cudaEventSynchronize(n->perm_copied[ep & 1]));
+        perm.resize((size_t)n->nrows);
         for (long long i = 0; i < n->nrows; ++i) perm[(size_t)i] = (int)i;
         std::shuffle(perm.begin(), perm.end(), n->rng);
         // the whole pass is enqueued at once; the loss sums of its steps are
         // read at the end (those of the last pass)
         CK(cudaMemcpyAsync(n->idx.p, perm.data(), (size_t)n->nrows * sizeof(int), cudaMemcpyHostToDevice, n->stream));
+        CK(cudaEventRecord(n->perm_copied[ep & 1], n->stream));
         for (long long q = 0; q < steps; ++q)
             RTRY(train_step(n, n->dX.p, n->dlab.p, n->dG, n->idx.p + q * B, B, std::min(B, n->nrows - q * B),
                             n->lpart.p + q * tiles * 3, true));

@@ -8,7 +8,8 @@ import pytest
 import dnsmc_gb300 as D
 from oracle import cvnet_oracle as NO
 
-from test_gpu_cvnet import make_labels, random_params
+from test_gpu_cvnet import make_labels, random_params, small_table, table_solver
+from test_gpu_parity import smooth_field
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +36,31 @@ def test_gradients_of_inputs_that_are_still_being_copied():
             np.testing.assert_array_equal(g, g1)
             np.testing.assert_array_equal(loss, loss1)
     net.close()
+
+
+def training_net(batch, **kw):
+    """A network with the 1536 rows of one small solve."""
+    s = table_solver(small_table(), 12, 32, 4, sampler=D.SAMPLER_RQMC, nvar=4, local_sampling=1, control_variate=1,
+                     cv_moments=1, seed=5)
+    x = (0.1 + 0.05 * np.random.default_rng(3).uniform(-1, 1, (4, 32, 12))).astype(np.float32)
+    s.set_fields(smooth_field(12, 32, 4, 450, 1700, 8), x)
+    s.set_rays(16)
+    s.solve(timeout_s=60)
+    net = D.CvNet(D.cvnet_default_config(n_groups=8, batch=batch, seed=9, **kw))
+    net.add_training_data(s)
+    s.close()
+    return net
+
+
+@pytest.mark.parametrize("batch,passes", [(128, 6), (1024, 3)])
+def test_passes_of_one_call_equal_passes_of_several(batch, passes):
+    """The order of a pass is shuffled while the pass before is still only
+    enqueued; every pass uses its own."""
+    a, b = training_net(batch), training_net(batch)
+    la = a.train(passes)
+    for _ in range(passes):
+        lb = b.train(1)
+    np.testing.assert_array_equal(a.params()[0], b.params()[0])
+    np.testing.assert_array_equal(la, lb)
+    a.close()
+    b.close()
