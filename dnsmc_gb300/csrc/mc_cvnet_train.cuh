@@ -459,8 +459,10 @@ __global__ void __launch_bounds__(WU_THREADS) train_update_kernel(const UpdatePa
         const long long sz = (long long)wg_nout(l) * wg_nin(l);
         const float *p = U.part + wg_part(l, U.splits) + (long long)n * wg_nin(l) + k;
         float s = 0.0f;
+        // (not __ldg: with programmatic dependence the partials are written
+        // while this kernel's blocks are already there)
 #pragma unroll 8
-        for (int z = 0; z < U.splits; ++z) s += __ldg(p + z * sz);
+        for (int z = 0; z < U.splits; ++z) s += __ldcg(p + z * sz);
         U.grad[e] = s;
         if (U.adam) store_weight(U.w, l, n, k, adam_update(U, e, s));
         return;

@@ -9,7 +9,7 @@ import dnsmc_gb300 as D
 from oracle import cvnet_oracle as NO
 
 from test_gpu_cvnet import make_labels, random_params, small_table, table_solver
-from test_gpu_parity import smooth_field
+from test_gpu_parity import packet_index, smooth_field
 
 pytestmark = pytest.mark.gpu
 
@@ -38,8 +38,9 @@ def test_gradients_of_inputs_that_are_still_being_copied():
     net.close()
 
 
-def training_net(batch, **kw):
-    """A network with the 1536 rows of one small solve."""
+def training_net(batch, data=None, **kw):
+    """A network with the 1536 rows of one small solve (data: their features
+    and labels, [rows][67] and [rows][G][8])."""
     s = table_solver(small_table(), 12, 32, 4, sampler=D.SAMPLER_RQMC, nvar=4, local_sampling=1, control_variate=1,
                      cv_moments=1, seed=5)
     x = (0.1 + 0.05 * np.random.default_rng(3).uniform(-1, 1, (4, 32, 12))).astype(np.float32)
@@ -48,6 +49,17 @@ def training_net(batch, **kw):
     s.solve(timeout_s=60)
     net = D.CvNet(D.cvnet_default_config(n_groups=8, batch=batch, seed=9, **kw))
     net.add_training_data(s)
+    if data is not None:
+        rows = lambda a: a.transpose(0, 4, 2, 3, 1, *range(5, a.ndim)).reshape(1536, 4, *a.shape[5:])  # tally order
+        m = rows(s.cv_moments()) / 16
+        var = rows(s.group_results()[1]) * 16
+        pack = packet_index(s).transpose(2, 0, 1).ravel()
+        steps = s.item_steps().reshape(4, -1)[:, pack].T / 16
+        cov = [m[..., 3] - m[..., 0] ** 2, m[..., 4] - m[..., 1] ** 2, m[..., 5] - m[..., 2] ** 2,
+               m[..., 6] - m[..., 0] * m[..., 1], m[..., 7] - m[..., 0] * m[..., 2], m[..., 8] - m[..., 1] * m[..., 2]]
+        for q in range(3):
+            cov[q] = np.maximum(cov[q], 0.0)
+        data += [net.features(s), np.stack(cov + [var, steps], -1).astype(np.float32)]
     s.close()
     return net
 
@@ -64,3 +76,43 @@ def test_passes_of_one_call_equal_passes_of_several(batch, passes):
     np.testing.assert_array_equal(la, lb)
     a.close()
     b.close()
+
+
+def test_chained_steps_are_adam_steps_on_the_gradient():
+    """Steps whose kernels are placed while the ones before still run: the
+    parameters follow Adam on the gradient of the same rows, moments carried
+    along, and both copies of the weights follow the parameters.
+
+    Row order and the labels' last places differ between the two gradients,
+    about 2e-5 of a typical element, so about that share of the elements may
+    step the other way: 2 sqrt(2e-5) = 9e-3 of the step's norm, bound 2e-2."""
+    data = []
+    net = training_net(2048, data, ridge=0.02)
+    feats, lab = data
+    p0 = random_params(9)
+    net.set_params(p0)
+    scales = net.params()[1]
+    other = D.CvNet(D.cvnet_default_config(n_groups=8, ridge=0.02))
+    lr, b1, b2, eps = 1e-3, 0.9, 0.999, 1e-8
+    p, m, v = p0.astype(np.float64), 0.0, 0.0
+    for step in (1, 2, 3):
+        other.set_params(p.astype(np.float32), scales)
+        g = other.gradient(feats, lab)[0].astype(np.float64)
+        m = b1 * m + (1 - b1) * g
+        v = b2 * v + (1 - b2) * g * g
+        upd = lr * (m / (1 - b1 ** step)) / (np.sqrt(v / (1 - b2 ** step)) + eps)
+        net.train(1)
+        now = net.params()[0].astype(np.float64)
+        assert np.linalg.norm(upd) > 0.5 * lr * np.sqrt(upd.size)  # nearly every element steps
+        assert np.linalg.norm((p - now) - upd) <= 2e-2 * np.linalg.norm(upd), step
+        p = now
+    # three steps in one call give what three calls gave
+    again = training_net(2048, None, ridge=0.02)
+    again.set_params(p0)
+    again.train(3)
+    np.testing.assert_array_equal(again.params()[0], net.params()[0])
+    other.set_params(net.params()[0], scales)
+    np.testing.assert_array_equal(again.gradient(feats, lab)[0], other.gradient(feats, lab)[0])
+    np.testing.assert_array_equal(again.eval(feats), other.eval(feats))
+    for n in (net, other, again):
+        n.close()
