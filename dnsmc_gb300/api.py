@@ -231,7 +231,8 @@ class Solver:
 
     def cv_beta(self):
         """Coefficients in effect: (nfields, n_groups, nk, nj, ni, 2) float32."""
-        ng = self.sampling()["n_groups"] if self.cfg.model != _lib.MODEL_GREY else 1
+        # (known before the first solve has built the sampling tables)
+        ng = min(self.cfg.n_groups, max(self.table_info()["nbands"], 1)) if self.cfg.model != _lib.MODEL_GREY else 1
         shp = self._region_shape()
         out = np.zeros((shp[0], ng) + shp[1:] + (2,), np.float32)
         check(self._lib.dnsmc_get_cv_beta(self._h, _fp(out)))

@@ -118,3 +118,15 @@ def test_sampling_prepared_while_a_solve_is_under_way():
         np.testing.assert_array_equal(Q, Q1)
         np.testing.assert_array_equal(S, S1)
     s.close()
+
+
+def test_coefficients_are_read_back_before_the_first_solve():
+    """As many band groups as were set, though no solve has built its sampling
+    tables yet."""
+    T, x, fv = snapshots(1)
+    s = particle_solver(control_variate=1)
+    s.set_fields(T, x)
+    beta = np.random.default_rng(4).normal(size=(1, 2, NK, NJ, NI, 2)).astype(np.float32)
+    s.set_cv_beta(beta)
+    np.testing.assert_array_equal(s.cv_beta(), beta)
+    s.close()
