@@ -418,6 +418,10 @@ struct dnsmc_cvnet {
     NBuf<float> wgt, cost, lam;
     NBuf<double2> lam_part;          // alloc_scale_kernel: per-block partial sums
     NBuf<unsigned int> lam_done;     // and its finished-block counter
+    // after the last dnsmc_cvnet_apply's kernels, which run on its solver's
+    // stream: the next one, of another solver perhaps, takes the same buffers,
+    // and this network's stream changes the weights that they read
+    cudaEvent_t applied = nullptr;
     NBuf<unsigned int> status;                // DNSMC_STATUS_* bits of the tensor-memory forward
     std::mt19937_64 rng;
     // the rows' order of a pass, in turn: a pass is shuffled while the one
@@ -434,6 +438,7 @@ struct dnsmc_cvnet {
         lpart.release(); iX.release(); iout.release(); vc.release(); wgt.release(); cost.release(); lam.release();
         lam_part.release(); lam_done.release();
         status.release();
+        if (applied) cudaEventDestroy(applied);
         if (stream) cudaStreamDestroy(stream);
     }
 };
@@ -633,6 +638,8 @@ int dnsmc_cvnet_create(const dnsmc_cvnet_config *cfg, dnsmc_cvnet **out) {
     if ((e = cudaGetDevice(&n->device)) != cudaSuccess) rc = cuda_fail("cudaGetDevice", e);
     if (!rc && (e = cudaStreamCreateWithFlags(&n->stream, cudaStreamNonBlocking)) != cudaSuccess)
         rc = cuda_fail("cudaStreamCreate", e);
+    if (!rc && (e = cudaEventCreateWithFlags(&n->applied, cudaEventDisableTiming)) != cudaSuccess)
+        rc = cuda_fail("cudaEventCreate", e);
     if (!rc) rc = n->P.ensure(NPARAM);
     if (!rc) rc = n->grad.ensure(NPARAM);
     if (!rc) rc = n->m.ensure(NPARAM);
@@ -945,6 +952,7 @@ int dnsmc_cvnet_apply(dnsmc_cvnet *n, dnsmc_solver *s, int flags, int mean_rays,
     F.apply.vc = n->vc.p; F.apply.region_cells = v.region_cells;
     // the network's weights are written on its own stream
     CK(cudaStreamSynchronize(n->stream));
+    CK(cudaStreamWaitEvent(st, n->applied, 0));
     RTRY(launch_forward_tc(F, n, st));
     if (flags & DNSMC_CVNET_RAYS) {
         const long long items = (long long)G * v.n_packets;
@@ -969,6 +977,8 @@ int dnsmc_cvnet_apply(dnsmc_cvnet *n, dnsmc_solver *s, int flags, int mean_rays,
         alloc_rays_kernel<<<grid1(items, 256), 256, 0, st>>>(n->wgt.p, items, n->lam.p, B, min_rays, max_rays, rays);
         CK(cudaGetLastError());
     }
+    CK(cudaEventRecord(n->applied, st));
+    CK(cudaStreamWaitEvent(n->stream, n->applied, 0));
     return DNSMC_OK;
 }
 

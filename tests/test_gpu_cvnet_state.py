@@ -116,3 +116,36 @@ def test_chained_steps_are_adam_steps_on_the_gradient():
     np.testing.assert_array_equal(again.eval(feats), other.eval(feats))
     for n in (net, other, again):
         n.close()
+
+
+def test_one_network_applied_to_several_solvers():
+    """Applied to two solvers one after the other, each with its own stream, and
+    trained right after: the work buffers and weights of one are not changed
+    under the other."""
+    tb = small_table()
+    net = training_net(128)
+    net.set_params(random_params(13))
+    p0 = net.params()[0]
+
+    def solver(seed):
+        s = table_solver(tb, 48, 64, 32, sampler=D.SAMPLER_RQMC, nvar=4, local_sampling=1, control_variate=1, seed=seed)
+        x = (0.1 + 0.05 * np.random.default_rng(seed).uniform(-1, 1, (32, 64, 48))).astype(np.float32)
+        s.set_fields(smooth_field(48, 64, 32, 450, 1700, seed), x)
+        return s
+
+    solvers = [solver(s) for s in (1, 2)]
+    ref = []
+    for s in solvers:
+        net.apply(s, mean_rays=16, min_rays=4, max_rays=64)
+        ref.append((s.cv_beta(), s.rays_per_item()))
+    for _ in range(5):
+        for s in solvers:
+            net.apply(s, mean_rays=16, min_rays=4, max_rays=64)
+        net.train(1)
+        for s, (beta, rays) in zip(solvers, ref):
+            np.testing.assert_array_equal(s.cv_beta(), beta)
+            np.testing.assert_array_equal(s.rays_per_item(), rays)
+        net.set_params(p0)
+    for s in solvers:
+        s.close()
+    net.close()
