@@ -2086,11 +2086,11 @@ int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
     }
     TRY(set_device(s));
     TRY(wait_done(s, 0));
-    // packed beside the raw values first: a field that is refused leaves the
-    // resident one as it was
+    // packed beside the raw values first, the resident field's array grown and
+    // written when they have been looked over: a field that is refused leaves
+    // the resident one as it was
     const size_t nv = (size_t)s->nfields * ncell;
     TRY(s->d_raw.ensure((size_t)nsrc + nv));
-    TRY(s->d_fieldV.ensure(nv));
     float *const packed = s->d_raw.p + nsrc;
     for (int f = 0; f < s->nfields; ++f) {
         CUDA_TRY(cudaMemcpyAsync(s->d_raw.p, fv + f * nsrc, nsrc * sizeof(float), cudaMemcpyHostToDevice, s->stream));
@@ -2100,6 +2100,8 @@ int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
     double st[4];
     TRY(field_stats(s, STATS_V, packed, (long long)nv, st));
     if (st[3] > 0.0) return fail(DNSMC_ERR_ARG, "volume fractions must be finite and >= 0");
+    s->fv_fields = 0;  // until the new one is in place
+    TRY(s->d_fieldV.ensure(nv));
     CUDA_TRY(cudaMemcpyAsync(s->d_fieldV.p, packed, nv * sizeof(float), cudaMemcpyDeviceToDevice, s->stream));
     CUDA_TRY(cudaStreamSynchronize(s->stream));
     const float vmax = (float)st[0];

@@ -130,3 +130,25 @@ def test_coefficients_are_read_back_before_the_first_solve():
     s.set_cv_beta(beta)
     np.testing.assert_array_equal(s.cv_beta(), beta)
     s.close()
+
+
+def test_refused_fractions_of_more_snapshots_leave_the_resident_field():
+    """The refused field would need a larger array than the resident one has."""
+    T, x, fv = snapshots(3)
+    s = particle_solver()
+    s.set_rays(16)
+    s.set_fields(T[0], x[0])
+    s.set_particle_field(fv[0])
+    Q, S = s.solve(timeout_s=60)
+    s.set_fields(T, x)
+    bad = fv.copy()
+    bad[2, 3, 5, 7] = -1e-6
+    with pytest.raises(RuntimeError, match="volume fractions"):
+        s.set_particle_field(bad)
+    with pytest.raises(RuntimeError, match="particle field"):
+        s.solve(timeout_s=60)  # three snapshots, the resident fractions are one's
+    s.set_fields(T[0], x[0])
+    Q1, S1 = s.solve(timeout_s=60)
+    np.testing.assert_array_equal(Q, Q1)
+    np.testing.assert_array_equal(S, S1)
+    s.close()
