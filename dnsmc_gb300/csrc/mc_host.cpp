@@ -1775,7 +1775,7 @@ int dnsmc_destroy(dnsmc_solver *s) {
     if (s->stream) cudaStreamSynchronize(s->stream);
     if (s->graph_exec) cudaGraphExecDestroy(s->graph_exec);
     s->d_fw.release(); s->d_k.release(); s->d_ib.release(); s->d_ibw.release();
-    s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posF.release(); s->d_posTX.release();
+    s->d_slab.release(); s->d_posT.release(); s->d_posG.release(); s->d_posF.release(); s->d_posTX.release(); s->d_posVG.release();
     s->d_cv_grp.release(); s->d_cv_sid.release(); s->d_cv_C.release(); s->d_layer.release();
     s->d_sur.release(); s->d_surtab.release(); s->d_Jhat.release(); s->d_muY.release(); s->d_cvnodes.release(); s->d_beta.release(); s->d_moments.release();
     s->d_fieldT.release(); s->d_fieldTX.release(); s->d_raw.release();

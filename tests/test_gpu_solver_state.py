@@ -152,3 +152,40 @@ def test_refused_fractions_of_more_snapshots_leave_the_resident_field():
     np.testing.assert_array_equal(Q, Q1)
     np.testing.assert_array_equal(S, S1)
     s.close()
+
+
+@pytest.mark.parametrize("kind", ["grey walls", "grey particles", "bands", "particles cv", "levels"])
+def test_a_closed_solver_leaves_no_device_memory_behind(kind):
+    """Ten solvers one after the other: an array left behind by each (a padded
+    field of these 64^3 cells is 2 MB and more) would show."""
+    torch = pytest.importorskip("torch")
+    n = 64
+    T = smooth_field(n, n, n, 450, 1300, 2)
+
+    def cycle():
+        cfg = dict(imax=n, jmax=n, kmax=n, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=0, T_west=400, T_east=400, kappa=1.0)
+        if kind == "particles cv":
+            s = particle_solver(**dict(cfg, control_variate=1, model=D.MODEL_TABLE))
+            s.set_fields(T, np.full(T.shape, 0.1, np.float32))
+            s.set_particle_field(np.full(T.shape, 1e-6, np.float32))
+        else:
+            s = D.Solver(D.default_config(model=D.MODEL_GREY_BANDS if kind == "bands" else D.MODEL_GREY,
+                                          **dict(cfg, eps_west=0.5 if kind == "grey walls" else 1.0,
+                                                 grid_num=3 if kind == "levels" else 1)))
+            if kind == "bands":
+                s.use_grey_band_tables(40, 12, 15000.0, 500.0)
+            s.set_fields(T)
+            if kind == "grey particles":
+                s.set_particles(np.array([0.5e5], np.float32), np.array([1.0e5], np.float32), 0.3)
+                s.set_particle_field(np.full(T.shape, 1e-6, np.float32))
+        s.set_graph(kind != "levels")
+        s.set_rays(2)
+        s.solve(timeout_s=60)
+        s.close()
+        return torch.cuda.mem_get_info()[0]
+
+    cycle()
+    first = cycle()
+    for _ in range(9):
+        last = cycle()
+    assert first - last < 10 << 20, (first, last)
