@@ -871,6 +871,17 @@ void padded_extents(const dnsmc_solver *s, bool pad, int *pna, int *pnb) {
     *pnb = march_extent(c.kmax, tb);
 }
 
+// The general medium: particles (with their field) and/or grey walls.
+bool general_medium(const dnsmc_solver *s) {
+    return !s->part.empty() || s->cfg.eps_west < 1.0f || s->cfg.eps_east < 1.0f;
+}
+
+// Whether a solve marches the plain grey gas on the fine grid, which reads
+// grey_positions (the general medium has its own array).
+bool reads_grey_positions(const dnsmc_solver *s) {
+    return s->cfg.model == DNSMC_MODEL_GREY && s->cfg.grid_num == 1 && !general_medium(s);
+}
+
 // T^4 of the resident fields for the grey march (after new fields; again
 // when the packet's extent has changed).
 int grey_positions(dnsmc_solver *s) {
@@ -972,11 +983,10 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     P.Wgrey = (float)(4.0 * c.kappa * kSigma);
     P.Tw4[0] = c.T_west * c.T_west * c.T_west * c.T_west;
     P.Tw4[1] = c.T_east * c.T_east * c.T_east * c.T_east;
-    // general medium: particles (with their field) and/or grey walls
     const bool have_part = !s->part.empty();
     if (have_part && s->fv_fields != s->nfields)
         return fail(DNSMC_ERR_STATE, "particles set: set the particle field of the %d resident snapshots", s->nfields);
-    const bool gen = have_part || c.eps_west < 1.0f || c.eps_east < 1.0f;
+    const bool gen = general_medium(s);
     P.part = have_part ? s->d_part.p : nullptr;
     P.fv_max = have_part ? s->fv_max : 0.0f;
     P.hg_g = s->hg_g;
@@ -1035,7 +1045,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     if (mode == MODE_T && !gen && !bands) TRY(s->d_posT.ensure((size_t)npos));
     if (bands) TRY(s->d_posF.ensure((size_t)npos));
     if (mode == MODE_GREY && gen) TRY(s->d_posVG.ensure((size_t)npos));
-    if (mode == MODE_GREY && !mg && !gen) TRY(grey_positions(s));
+    if (reads_grey_positions(s)) TRY(grey_positions(s));
     P.fieldP = s->d_posT.p;
     P.fieldPX = s->d_posTX.p;
     P.fieldG = s->d_posG.p;
@@ -1591,7 +1601,7 @@ int upload_fields_host(dnsmc_solver *s, int nfields, const float *T, const float
         TRY(upload_coarse(s, nfields, want_x ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, want_x ? 2 : 1));
     s->nfields = nfields;
     s->posG_na = 0;
-    if (c.model == DNSMC_MODEL_GREY && c.grid_num == 1 && !want_x) TRY(grey_positions(s));
+    if (!want_x && reads_grey_positions(s)) TRY(grey_positions(s));
     s->have_x = want_x;
     s->tmax_fields = (float)st[0];
     s->tmin_fields = (float)st[1];
@@ -2031,7 +2041,7 @@ int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const
         TRY(upload_coarse(s, nfields, dx ? (const float *)s->d_fieldTX.p : s->d_fieldT.p, dx ? 2 : 1));
     s->nfields = nfields;
     s->posG_na = 0;
-    if (c.model == DNSMC_MODEL_GREY && c.grid_num == 1 && !dx) TRY(grey_positions(s));
+    if (!dx && reads_grey_positions(s)) TRY(grey_positions(s));
     s->have_x = dx != nullptr;
     s->tmax_fields = (float)st[0];
     s->tmin_fields = (float)st[1];

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 import dnsmc_gb300 as D
-from dnsmc_gb300 import synth
+from dnsmc_gb300 import _lib, synth
 from oracle import oracle as O
 
 from test_gpu_parity import smooth_field
@@ -189,3 +189,35 @@ def test_a_closed_solver_leaves_no_device_memory_behind(kind):
     for _ in range(9):
         last = cycle()
     assert first - last < 10 << 20, (first, last)
+
+
+def test_only_the_plain_grey_march_has_its_field_prepared():
+    """Grey walls and particles march on an array of their own: set_fields
+    writes T^4 for black walls and gas alone, and a solve that turns to them
+    afterwards writes it then."""
+    T, _, fv = snapshots(1)
+    T, fv = T[0], fv[0]
+    cfg = dict(model=D.MODEL_GREY, imax=NI, jmax=NJ, kmax=NK, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=0, T_west=400,
+               T_east=700, kappa=0.8, seed=4)
+
+    def launches(s):
+        n0 = _lib.launch_count()
+        s.set_fields(T)
+        return _lib.launch_count() - n0
+
+    black, grey = D.Solver(D.default_config(**cfg)), D.Solver(D.default_config(eps_west=0.5, **cfg))
+    assert launches(black) == 2 and launches(grey) == 1
+    black.set_rays(8)
+    Q, S = black.solve(timeout_s=60)
+    s = D.Solver(D.default_config(**cfg))
+    s.set_rays(8)
+    s.set_particles(np.array([0.5e5], np.float32), np.array([1.0e5], np.float32), 0.3)
+    assert launches(s) == 1
+    s.set_particle_field(fv)
+    s.solve(timeout_s=60)
+    s.set_particles(None, None)
+    Q1, S1 = s.solve(timeout_s=60)
+    np.testing.assert_array_equal(Q, Q1)
+    np.testing.assert_array_equal(S, S1)
+    for s in (s, black, grey):
+        s.close()
