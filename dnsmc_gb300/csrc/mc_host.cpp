@@ -1102,7 +1102,11 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         // beside it; the marches on the fine grid, which keep more, then
         // take fewer warps
         while (pair && threads > 32 && need(threads) > (size_t)smax) threads /= 2;
-        if (march_smem(P, 128, kLaneCells) + 1024 > (size_t)smax)
+        // (grey band tables: not counting their end point's pairs, for which
+        // every march has room beside its smaller share a thread)
+        MarchParams B = P;
+        if (P.uni) B.slab_len = (P.slab_klen + t.nT) & ~1;
+        if (march_smem(B, 128, kLaneCells) + 1024 > (size_t)smax)
             return fail(DNSMC_ERR_TABLE, "a spectral sample's table slab (%d bytes) exceeds the shared memory of the march",
                         P.slab_len * 8);
     }

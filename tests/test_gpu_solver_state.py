@@ -10,7 +10,8 @@ import dnsmc_gb300 as D
 from dnsmc_gb300 import _lib, synth
 from oracle import oracle as O
 
-from test_gpu_parity import smooth_field
+from test_gpu_cv import assert_bitexact_cv
+from test_gpu_parity import assert_bitexact, smooth_field
 from test_gpu_scatter import particle_table
 
 pytestmark = pytest.mark.gpu
@@ -220,4 +221,29 @@ def test_only_the_plain_grey_march_has_its_field_prepared():
     np.testing.assert_array_equal(Q, Q1)
     np.testing.assert_array_equal(S, S1)
     for s in (s, black, grey):
+        s.close()
+
+
+@pytest.mark.parametrize("kw", [dict(), dict(eps_west=0.5), dict(control_variate=1), dict(grid_num=2)],
+                         ids=["gas", "walls", "cv", "levels"])
+def test_the_longest_grey_band_tables(kw):
+    """3489 temperatures: a sample's k and Ib (2 x 3488 pairs) in each of four
+    warps, with 64 bytes a thread and 1 KB beside them, are all of the shared
+    memory; one temperature more is refused."""
+    ni, nj, nk = 8, 16, 8
+    T = smooth_field(ni, nj, nk, 600, 1500, 3)
+    for nT in (3489, 3490):
+        s = D.Solver(D.default_config(model=D.MODEL_GREY_BANDS, imax=ni, jmax=nj, kmax=nk, Lx=1.5, Ly=2.0, Lz=0.7,
+                                      stretched_x=0, T_west=500.0, T_east=700.0, kappa=0.7, seed=12, **kw))
+        s.use_grey_band_tables(3, nT, 15000.0, 500.0)
+        s.set_fields(T)
+        s.set_rays(16)
+        if nT == 3490:
+            with pytest.raises(RuntimeError, match="shared memory"):
+                s.solve(timeout_s=60)
+        elif "grid_num" in kw or "eps_west" in kw:
+            Q, S = s.solve(timeout_s=60)
+            assert np.isfinite(Q).all() and s.status() == 0
+        else:
+            (assert_bitexact_cv if "control_variate" in kw else assert_bitexact)(s, T)
         s.close()
