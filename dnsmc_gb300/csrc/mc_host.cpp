@@ -1097,11 +1097,26 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         const bool pair = !mg;
         const size_t stat = pair ? kPairStaticSmem : 1024;  // the march kernels' static shared memory, at most
         auto need = [&](int th) { return (pair ? march_pair_smem(P, th) : march_smem(P, th, kLaneCells)) + stat; };
-        if (need(threads) > (size_t)smax) threads = 128;
-        // the largest slab is what four warps hold with 64 bytes a thread
-        // beside it; the marches on the fine grid, which keep more, then
-        // take fewer warps
-        while (pair && threads > 32 && need(threads) > (size_t)smax) threads /= 2;
+        if (!pair && need(threads) > (size_t)smax) threads = 128;
+        // The largest slab is what four warps hold with 64 bytes a thread
+        // beside it; the marches on the fine grid keep more.  Where blocks of
+        // 8 warps leave an SM with fewer warps than its registers hold, the
+        // size that leaves most is taken (march of 64^3 cells, 64 x 16 samples
+        // on a 50 x nX grid, 32 rays: nX = 15 4.89 ms with one block of 8 warps,
+        // 3.64 with two of 7; nX = 34 8.27 with one of 4, 5.62 with one of 7).
+        // A block size that the caller chose is kept where it fits.
+        if (pair) {
+            int ssm = smax;
+            (void)cudaDeviceGetAttribute(&ssm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, s->device);
+            // warps that an SM's registers hold (pair_min_blocks blocks of 8)
+            const int full = (P.uni || mode == MODE_GREY) && !gen && !(c.control_variate && c.cv_moments) ? 32 : 16;
+            auto warps = [&](int th) {
+                return need(th) > (size_t)smax ? 0 : std::min(full, (int)((size_t)ssm / (need(th) + 1024)) * (th / 32));
+            };
+            int most = warps(threads);
+            for (int th = 256; most < (c.block_threads ? 1 : full) && th >= 32; th -= 32)
+                if (warps(th) > most) { threads = th; most = warps(th); }
+        }
         // (grey band tables: not counting their end point's pairs, for which
         // every march has room beside its smaller share a thread)
         MarchParams B = P;

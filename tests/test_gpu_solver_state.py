@@ -12,7 +12,7 @@ from oracle import oracle as O
 
 from test_gpu_cv import assert_bitexact_cv
 from test_gpu_parity import assert_bitexact, smooth_field
-from test_gpu_scatter import particle_table
+from test_gpu_scatter import check_bitexact, particle_table
 
 pytestmark = pytest.mark.gpu
 
@@ -247,3 +247,35 @@ def test_the_longest_grey_band_tables(kw):
         else:
             (assert_bitexact_cv if "control_variate" in kw else assert_bitexact)(s, T)
         s.close()
+
+
+@pytest.mark.parametrize("nX,kw", [
+    (14, dict()), (15, dict(control_variate=1, cv_moments=1)),   # two blocks of fewer than 8 warps an SM
+    (34, dict()), (34, dict(block_threads=256)),                 # 8 warps no longer fit
+    (50, dict(control_variate=1)), (71, dict(block_threads=128)),  # down to 3 warps
+])
+def test_table_slabs_that_leave_room_for_fewer_warps(nX, kw):
+    ni, nj, nk = 9, 17, 10
+    s = D.Solver(D.default_config(model=D.MODEL_TABLE, imax=ni, jmax=nj, kmax=nk, Lx=1.5, Ly=2.0, Lz=0.7, stretched_x=0,
+                                  T_west=500.0, T_east=700.0, n_groups=2, local_sampling=1, seed=3,
+                                  sampler=D.SAMPLER_RQMC, nvar=2, **kw))
+    t = synth.ck_table(nbands=4, nq=2, nT=50, nX=nX, seed=5)
+    s.set_table(t["k"], t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"], X0=t["X0"], dX=t["dX"])
+    T = smooth_field(ni, nj, nk, 600, 1500, 3)
+    x = np.random.default_rng(1).uniform(0.05, 0.2, T.shape).astype(np.float32)
+    s.set_fields(T, x)
+    s.set_rays(16)
+    (assert_bitexact_cv if "control_variate" in kw else assert_bitexact)(s, T, x)
+    s.close()
+
+
+def test_particles_and_a_table_slab_that_leaves_room_for_fewer_warps():
+    T, x, fv = snapshots(1)
+    s = particle_solver(nvar=1)
+    t = synth.ck_table(nbands=8, nq=4, nT=50, nX=33, seed=5)
+    s.set_table(t["k"], t["wvc"], t["T0"], t["dT"], dnu=t["dnu"], wq=t["wq"], X0=t["X0"], dX=t["dX"])
+    s.set_fields(T, x)
+    s.set_particle_field(fv)
+    s.set_rays(8)
+    check_bitexact(s, T, x, fv)
+    s.close()
