@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cmath>
 #include <cstdarg>
@@ -192,22 +193,41 @@ void sobol_directions(uint32_t v[4][32]) {
     }
 }
 
+// Device bytes of all solvers, and cudaMalloc: the environment variable
+// DNSMC_TEST_DEVICE_BYTES makes it fail beyond that many, as on a device
+// without the memory, only to test what happens then.
+std::atomic<size_t> g_device_bytes{0};
+cudaError_t device_malloc(void **p, size_t bytes) {
+    const char *ev = getenv("DNSMC_TEST_DEVICE_BYTES");
+    if (ev && *ev && g_device_bytes + bytes > strtoull(ev, nullptr, 10)) return cudaErrorMemoryAllocation;
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaSuccess) g_device_bytes += bytes;
+    else cudaGetLastError();  // reported here; no later launch is to find it
+    return e;
+}
+
 template <class T>
 struct DevBuf {
     T *p = nullptr;
     size_t n = 0;
     int ensure(size_t want) {
         if (want <= n) return DNSMC_OK;
-        if (p) cudaFree(p);
-        p = nullptr;
-        n = 0;
+        release();
         if (want == 0) return DNSMC_OK;
-        cudaError_t e = cudaMalloc((void **)&p, want * sizeof(T));
-        if (e != cudaSuccess) return fail(DNSMC_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want * sizeof(T), cudaGetErrorString(e));
+        cudaError_t e = device_malloc((void **)&p, want * sizeof(T));
+        if (e != cudaSuccess) {
+            p = nullptr;
+            return fail(DNSMC_ERR_NOMEM, "cudaMalloc(%zu bytes): %s", want * sizeof(T), cudaGetErrorString(e));
+        }
         n = want;
         return DNSMC_OK;
     }
-    void release() { if (p) cudaFree(p); p = nullptr; n = 0; }
+    void release() {
+        if (p) cudaFree(p);
+        g_device_bytes -= n * sizeof(T);
+        p = nullptr;
+        n = 0;
+    }
 };
 
 template <class T>
@@ -415,6 +435,16 @@ int ensure_device(dnsmc_solver *s) {
 }
 
 int set_device(dnsmc_solver *s) { return ensure_device(s); }
+
+// f(), and again without the rays' contributions of the last solve (at most
+// kRayxBytes, which a solve can do without) where the device had no memory left.
+template <class F>
+int with_room(dnsmc_solver *s, F f) {
+    const int rc = f();
+    if (rc != DNSMC_ERR_NOMEM || !s->d_rayx.p) return rc;
+    s->d_rayx.release();
+    return f();
+}
 
 int check_config(const dnsmc_config &c) {
     if (c.imax < 1 || c.jmax < 1 || c.kmax < 1) return fail(DNSMC_ERR_ARG, "imax, jmax, kmax must be >= 1");
@@ -1224,15 +1254,6 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     const int occ = mg ? march_mg_occupancy(mode, P.uni != 0, threads, smem)
                        : march_occupancy_ex(mode, P.uni != 0, threads, cv, mom, gen, smem);
     const int blocks = std::max(1, sms * occ);
-    if (!mom && !P.rays_per_packet) {  // few items: their rays in several units
-        const int cells = 32 * lane_cells(s);
-        P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes, cells);
-        if (P.parts > 1) {
-            TRY(s->d_rayx.ensure((size_t)(P.n_items * P.rays * cells)));
-            P.rayx = s->d_rayx.p;
-            P.parts_done = s->d_misc.p + kMiscWords;
-        }
-    }
 
     FinalizeParams F;
     memset(&F, 0, sizeof F);
@@ -1264,6 +1285,17 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         F.Qf = s->d_Qf.p; F.sigf = s->d_Qf.p + nout; F.sig_scale = s->sig_scale;
     } else {
         TRY(s->h_Q.ensure(2 * nout));
+    }
+    if (!mom && !P.rays_per_packet) {  // few items: their rays in several units
+        const int cells = 32 * lane_cells(s);
+        P.parts = march_parts(P.n_items, P.rays, (long long)blocks * (threads / 32), kRayxBytes, cells);
+        // (after all that the solve cannot do without: a device that has no
+        // room for the rays' contributions marches an item as one unit)
+        if (P.parts > 1 && s->d_rayx.ensure((size_t)(P.n_items * P.rays * cells)) != DNSMC_OK) P.parts = 1;
+        if (P.parts > 1) {
+            P.rayx = s->d_rayx.p;
+            P.parts_done = s->d_misc.p + kMiscWords;
+        }
     }
 
     // ---- the kernel sequence of a solve (stream-ordered; capturable) -------
@@ -1689,7 +1721,7 @@ int solver_beta_device(dnsmc_solver *s, float2 **beta, long long *n) {
     TRY(solver_view(s, &v));
     TRY(wait_done(s, 0));
     const long long m = (long long)v.nfields * v.n_groups * v.region_cells;
-    TRY(s->d_beta.ensure((size_t)m));
+    TRY(with_room(s, [&] { return s->d_beta.ensure((size_t)m); }));
     s->beta_set = true;
     *beta = s->d_beta.p;
     *n = m;
@@ -2029,12 +2061,10 @@ int dnsmc_prepare_sampling(dnsmc_solver *s, float Tmax, float xmean) {
 int dnsmc_set_fields(dnsmc_solver *s, int nfields, const float *T, const float *x, int layout) {
     if (!s || !T || nfields < 1) return fail(DNSMC_ERR_ARG, "bad arguments");
     if (nfields > 65535) return fail(DNSMC_ERR_ARG, "at most 65535 fields per solve");
-    return upload_fields_host(s, nfields, T, x, layout);
+    return with_room(s, [&] { return upload_fields_host(s, nfields, T, x, layout); });
 }
 
-int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const float *dx) {
-    if (!s || !dT || nfields < 1) return fail(DNSMC_ERR_ARG, "bad arguments");
-    if (nfields > 65535) return fail(DNSMC_ERR_ARG, "at most 65535 fields per solve");
+static int upload_fields_device(dnsmc_solver *s, int nfields, const float *dT, const float *dx) {
     const dnsmc_config &c = s->cfg;
     const long long ncell = (long long)c.imax * c.jmax * c.kmax;
     TRY(set_device(s));
@@ -2068,6 +2098,12 @@ int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const
     return DNSMC_OK;
 }
 
+int dnsmc_set_fields_device(dnsmc_solver *s, int nfields, const float *dT, const float *dx) {
+    if (!s || !dT || nfields < 1) return fail(DNSMC_ERR_ARG, "bad arguments");
+    if (nfields > 65535) return fail(DNSMC_ERR_ARG, "at most 65535 fields per solve");
+    return with_room(s, [&] { return upload_fields_device(s, nfields, dT, dx); });
+}
+
 int dnsmc_set_particles(dnsmc_solver *s, int nbands, const float *absorption, const float *scattering, float hg_g) {
     if (!s) return fail(DNSMC_ERR_ARG, "null solver");
     TRY(wait_done(s, 0));
@@ -2098,8 +2134,7 @@ int dnsmc_set_particles(dnsmc_solver *s, int nbands, const float *absorption, co
     return DNSMC_OK;
 }
 
-int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
-    if (!s || !fv) return fail(DNSMC_ERR_ARG, "null argument");
+static int upload_particle_field(dnsmc_solver *s, const float *fv, int layout) {
     if (s->nfields < 1) return fail(DNSMC_ERR_STATE, "set the temperature fields first");
     const dnsmc_config &c = s->cfg;
     const long long ncell = (long long)c.imax * c.jmax * c.kmax;
@@ -2139,6 +2174,11 @@ int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
     s->fv_max = vmax;
     s->fv_mean = vsum / ((double)s->nfields * ncell);
     return DNSMC_OK;
+}
+
+int dnsmc_set_particle_field(dnsmc_solver *s, const float *fv, int layout) {
+    if (!s || !fv) return fail(DNSMC_ERR_ARG, "null argument");
+    return with_room(s, [&] { return upload_particle_field(s, fv, layout); });
 }
 
 int dnsmc_set_region(dnsmc_solver *s, int i0, int i1, int j0, int j1, int k0, int k1) {
@@ -2372,7 +2412,7 @@ int dnsmc_get_item_steps(dnsmc_solver *s, double *steps) {
 int dnsmc_solve_async(dnsmc_solver *s) {
     if (!s) return fail(DNSMC_ERR_ARG, "null solver");
     TRY(wait_done(s, 0));
-    const int rc = solve_enqueue(s, false, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr);
+    const int rc = with_room(s, [&] { return solve_enqueue(s, false, 0, 0, 0, 0, 0, nullptr, nullptr, nullptr); });
     // (copies of the sampling tables may be under way: the next solve rewrites them)
     if (rc && s->dev_ready && !s->in_flight) cudaStreamSynchronize(s->stream);
     return rc;
@@ -2562,7 +2602,7 @@ int dnsmc_set_cv_beta(dnsmc_solver *s, const float *beta) {
                     tl[fg * rc_ + ((long long)i * nk + k) * nj + j] = make_float2(b[0], b[1]);
                 }
     TRY(set_device(s));
-    TRY(s->d_beta.ensure(tl.size()));
+    TRY(with_room(s, [&] { return s->d_beta.ensure(tl.size()); }));
     TRY(to_device(s, s->d_beta.p, tl.data(), tl.size() * sizeof(float2)));
     s->beta_set = true;
     return DNSMC_OK;

@@ -279,3 +279,45 @@ def test_particles_and_a_table_slab_that_leaves_room_for_fewer_warps():
     s.set_rays(8)
     check_bitexact(s, T, x, fv)
     s.close()
+
+
+def test_a_split_solve_runs_where_its_contributions_have_no_room(monkeypatch):
+    """32^3 cells, 256 rays: the rays' contributions of the split items are 34
+    MB, all other arrays together under 8 MB.  The sums are the same without."""
+    n = 32
+    T = smooth_field(n, n, n, 450, 1300, 2)
+
+    def solver():
+        s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=n, jmax=n, kmax=n, Lx=2.0, Ly=6.28, Lz=3.14,
+                                      stretched_x=0, T_west=400, T_east=400, kappa=1.0, seed=6))
+        s.set_rays(256)
+        return s
+
+    s = solver()
+    s.set_fields(T)
+    ref = s.solve(timeout_s=60)
+    # 16 snapshots: 0.52 M cells of 68 bytes (fields, tallies, results), 36 MB, in
+    # part where the last solve's contributions were: they are given up
+    monkeypatch.setenv("DNSMC_TEST_DEVICE_BYTES", str(44 << 20))
+    many = np.stack([T] * 16)
+    s.set_fields(many)
+    Q, S = s.solve(timeout_s=60)
+    np.testing.assert_array_equal(Q[0], ref[0][0])
+    s.close()
+    ran = []
+    for mb in (1, 2, 4, 8, 16, 24, 32, 40, 64):
+        monkeypatch.setenv("DNSMC_TEST_DEVICE_BYTES", str(mb << 20))
+        s = solver()
+        try:
+            s.set_fields(T)
+            Q, S = s.solve(timeout_s=60)
+            Q2, S2 = s.solve(timeout_s=60)
+        except RuntimeError as e:
+            assert "cudaMalloc" in str(e)
+        else:
+            ran.append(mb)
+            for a, b in ((Q, ref[0]), (S, ref[1]), (Q2, ref[0]), (S2, ref[1])):
+                np.testing.assert_array_equal(a, b)
+            assert s.status() == 0
+        s.close()
+    assert ran == [8, 16, 24, 32, 40, 64] or ran == [4, 8, 16, 24, 32, 40, 64]
