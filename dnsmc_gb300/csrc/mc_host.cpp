@@ -1179,6 +1179,16 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
         return DNSMC_OK;
     }
     // ---- buffers and kernel parameters (no kernel is enqueued yet) ----------
+    const bool f32 = s->result_type == DNSMC_RESULT_F32;
+    const size_t nout = (size_t)s->nfields * P.region_cells;
+    const size_t done_words = ((size_t)P.n_items + 1) / 2 * 2, misc_words = kMiscWords + done_words + 2 * (size_t)P.n_items;
+    // the last solve's results are in the arrays that have to grow now: gone,
+    // even if this solve fails before it has its own
+    if (s->d_misc.n < misc_words || s->d_Q.n < 2 * nout || s->d_Qg.n < nout * P.n_groups ||
+        (f32 ? s->d_Qf.n < 2 * nout || s->h_Qf.n < 2 * nout : s->h_Q.n < 2 * nout)) {
+        s->solved = false;
+        s->item_steps = nullptr;
+    }
     CvParams cp;
     memset(&cp, 0, sizeof cp);
     if (cv) {
@@ -1238,12 +1248,11 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     TRY(s->d_tally.ensure((size_t)s->nfields * P.n_groups * P.region_cells));
     P.tally = s->d_tally.p;
-    const size_t done_words = ((size_t)P.n_items + 1) / 2 * 2, misc_words = kMiscWords + done_words + 2 * (size_t)P.n_items;
     TRY(s->d_misc.ensure(misc_words));
     P.queue = s->d_misc.p;
     P.status = s->d_misc.p + 1;
     P.counters = reinterpret_cast<unsigned long long *>(s->d_misc.p + 4);
-    P.item_steps = s->item_steps = reinterpret_cast<unsigned long long *>(s->d_misc.p + kMiscWords + done_words);
+    P.item_steps = reinterpret_cast<unsigned long long *>(s->d_misc.p + kMiscWords + done_words);
     if (P.rays_per_packet) {  // uneven items: longest first
         TRY(s->d_order.ensure((size_t)P.n_items));
         TRY(s->d_order_hist.ensure(kOrderBuckets));
@@ -1271,14 +1280,12 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     F.tally = s->d_tally.p;
     F.muY = cv ? s->d_muY.p : nullptr;
     F.beta = cv ? P.beta : nullptr;
-    const size_t nout = (size_t)s->nfields * P.region_cells;
     TRY(s->d_Q.ensure(2 * nout));
     TRY(s->d_var.ensure(nout));
     TRY(s->d_Qg.ensure(nout * P.n_groups));
     TRY(s->d_varg.ensure(nout * P.n_groups));
     F.Q = s->d_Q.p; F.var = s->d_var.p; F.sigma = s->d_Q.p + nout; F.Qg = s->d_Qg.p; F.varg = s->d_varg.p;
     F.status = P.status;
-    const bool f32 = s->result_type == DNSMC_RESULT_F32;
     if (f32) {
         TRY(s->d_Qf.ensure(2 * nout));
         TRY(s->h_Qf.ensure(2 * nout));
@@ -1383,6 +1390,7 @@ int solve_enqueue(dnsmc_solver *s, bool trace, int tf, int tg, int tp, int tr, i
     }
     s->last = P;
     s->lastF = F;
+    s->item_steps = P.item_steps;
     CUDA_TRY(cudaEventRecord(s->ev_done, s->stream));
     s->in_flight = true;
     s->solved = true;

@@ -321,3 +321,50 @@ def test_a_split_solve_runs_where_its_contributions_have_no_room(monkeypatch):
             assert s.status() == 0
         s.close()
     assert ran == [8, 16, 24, 32, 40, 64] or ran == [4, 8, 16, 24, 32, 40, 64]
+
+
+def test_results_after_a_solve_that_did_not_fit(monkeypatch):
+    """Half a grid solved, then the whole one with too little device memory, a
+    little more each time: what is read afterwards are the half's results or an
+    error, never the contents of an array that was being replaced."""
+    n = 64
+    T = smooth_field(n, n, n, 450, 1300, 2)
+    s = D.Solver(D.default_config(model=D.MODEL_GREY, imax=n, jmax=n, kmax=n, Lx=2.0, Ly=6.28, Lz=3.14, stretched_x=0,
+                                  T_west=400, T_east=400, kappa=1.0, seed=6))
+    s.set_fields(T)
+    s.set_rays(2)
+    half, whole = (0, n, 0, n, 0, n // 2), (0, n, 0, n, 0, n)
+    s.set_region(*half)
+    ref = s.solve(timeout_s=60)
+    steps = s.item_steps()
+    seen = []
+    for kb in range(1 << 10, 40 << 10, 1 << 10):  # 0.26 M cells of 68 bytes: 18 MB for the whole grid
+        monkeypatch.setenv("DNSMC_TEST_DEVICE_BYTES", str(kb << 10))
+        s.set_region(*whole)
+        try:
+            full = s.solve(timeout_s=60)
+            break
+        except RuntimeError as e:
+            assert "cudaMalloc" in str(e)
+        s.set_region(*half)
+        try:
+            Q, S = s.results()
+        except RuntimeError as e:
+            assert "no solve" in str(e)
+            with pytest.raises(RuntimeError, match="no solve"):
+                s.item_steps()
+            seen.append("error")
+            continue
+        np.testing.assert_array_equal(Q, ref[0])
+        np.testing.assert_array_equal(S, ref[1])
+        np.testing.assert_array_equal(s.item_steps(), steps)
+        seen.append("results")
+    assert "error" in seen
+    monkeypatch.delenv("DNSMC_TEST_DEVICE_BYTES")
+    other = D.Solver(s.cfg)
+    other.set_fields(T)
+    other.set_rays(2)
+    for a, b in zip(full, other.solve(timeout_s=60)):
+        np.testing.assert_array_equal(a, b)
+    other.close()
+    s.close()
