@@ -201,13 +201,6 @@ __device__ __forceinline__ void cell_coords(const typename FieldT<MODE>::type &v
     }
 }
 
-template <int MODE>
-__device__ __forceinline__ typename FieldT<MODE>::type load_field(const MarchParams &P, long long fbase, int cell) {
-    if constexpr (MODE == MODE_TX) return __ldg(P.fieldPX + fbase + cell);
-    else if constexpr (MODE == MODE_T) return __ldg(P.fieldP + fbase + cell);
-    else return __ldg(P.fieldT + fbase + cell);
-}
-
 // ---------------------------------------------------------------------------
 // -ln(u) for u in (0, 1): u = m 2^e with m in [sqrt(1/2), sqrt(2)),
 // ln m = 2 atanh(s), s = (m - 1)/(m + 1), odd series to s^11 (|s| <= 0.1716,

@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(256, DNSMC_MINB) march_mg_kernel(const MarchPa
     const int lane = threadIdx.x & 31;
     const int la = lane % P.tile_a, lb = lane / P.tile_a;
     const int njR = P.ea1 - P.ea0, nkR = P.eb1 - P.eb0;
-        unsigned long long my_rays = 0, my_steps = 0;
+    unsigned long long my_rays = 0, my_steps = 0;
     unsigned int flags = 0;
     const int tid = threadIdx.x;
     // dynamic shared memory (march_mg_smem): this warp's copy of the current
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(256, DNSMC_MINB) march_mg_kernel(const MarchPa
         const int acl = active ? a0 : P.ea0, bcl = active ? b0 : P.eb0;
         const int N = P.rays_per_packet ? P.rays_per_packet[G * P.rays_gstride + p] : P.rays;
         const long long fbase = (long long)f * P.field_stride;
-                // own-cell quantities
+        // own-cell quantities
         const VT *field;
         if constexpr (MODE == MODE_T) field = P.fieldP + fbase; else field = P.fieldT + fbase;
         const int cell0 = (w0 * P.nb + bcl) * P.na + acl;
