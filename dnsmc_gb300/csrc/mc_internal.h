@@ -338,10 +338,10 @@ inline size_t march_mg_smem(const MarchParams &p, int threads) {
 // cap_bytes: the most that the rays' contributions (of `cells` cells) may take.
 // About 16 units per resident warp leave the last wave under a tenth of the
 // launch, but of no fewer than 12 rays each (a unit's first 32 rays are set up
-// together), and 4 per warp whatever that takes.  Grey 8 x 32 x 4 at 32 rays (32 items): march
-// 79 -> 18 us; grey 64^3 at 256 rays (4096 items, 1.7 waves of warps): 4.85 -> 4.36
-// ms; 45 x 60 x 52 tables at 32 rays (10080 items, 4 per warp): 4 units of 8 rays 1.145,
-// 2 of 16 1.090 ms.  From 16 items a warp on, one unit per item: the sums
+// together), and 4 per warp whatever that takes.  Unsplit and split: grey 8 x 32 x 4 at
+// 32 rays (32 items) march 79 and 18 us; grey 64^3 at 256 rays (4096 items, 1.7 waves of the
+// warps of the time) 4.85 and 4.36 ms; 45 x 60 x 52 tables at 32 rays (10080 items, 4 per
+// warp): 4 units of 8 rays 1.145, 2 of 16 1.090 ms.  From 16 items a warp on, one unit per item: the sums
 // stay in shared memory (128^3 with 8 band groups: 262144 items).
 constexpr long long kRayxBytes = 1LL << 30;
 inline int march_parts(long long n_items, int rays, long long warps, long long cap_bytes, int cells = 64) {

@@ -20,7 +20,8 @@ namespace dnsmc {
 // compiler otherwise computes most of it again in every step).  UNI: the
 // absorption coefficient is the same everywhere (grey model, grey band
 // tables).  The rays are set up a lane each, 32 at a time.  Instructions a
-// coarse step 163 -> 108; 64^3, five levels, 60 rays: 1.93 -> 1.42 ms.
+// coarse step 108 (163 without all this); 64^3, five levels, 60 rays: 1.37 ms
+// (1.93).
 //
 // A value the compiler keeps instead of computing it again in every step.
 __device__ __forceinline__ float keep(float v) { asm volatile("" : "+f"(v)); return v; }
@@ -36,7 +37,8 @@ __device__ __forceinline__ float lookup_ib_at(int ibs, int ti, float ft) {
 }
 
 // Resident blocks of 256 threads per SM the register allocation must allow
-// (2: up to 128 registers; 3: 85; 4: 64): 1.47 / 1.48 / 1.48 ms.
+// (2: up to 128 registers; 3: 85; 4: 64): the march takes 1.47 / 1.48 / 1.48 ms
+// (before the rays were set up together).
 #ifndef DNSMC_MINB
 #define DNSMC_MINB 4
 #endif

@@ -51,11 +51,12 @@ namespace dnsmc {
 // loop loses the face choice, the crossing times and the index updates, and
 // it knows the cells ahead, so a cell's field value is fetched two steps
 // before it is used.
-// March of the 128^3 correlated-k channel (48 rays): 85.5 -> 66.2 ms; grey 64^3
-// channel at 256 rays: 9.6 -> 4.9 ms.  Chunks of 64 / 96 / 128 / 192 steps:
-// channel 62.5 / 61.9 / 61.6 / 61.7 ms (longer chunks take more shared memory a
-// warp).  With uniform absorption, and so with 64 wall-normal crossings listed,
-// 128 / 192 / 256: grey 2.91 / 2.80 / 2.83, drop-in bands call 6.56 / 6.33 / 6.74 ms.
+// Marches with the walk in every lane and now: 128^3 correlated-k channel (48
+// rays) 85.5 and 61.4 ms (4 of them ray_batch's), grey 64^3 channel at 256 rays
+// 9.6 and 2.8 ms.  Chunks of 64 / 96 / 128 / 192 steps: channel 62.5 / 61.9 / 61.6 /
+// 61.7 ms (longer chunks take more shared memory a warp).  With uniform
+// absorption, and so with 64 wall-normal crossings listed, 128 / 192 / 256: grey
+// 2.91 / 2.80 / 2.83, drop-in bands call 6.56 / 6.33 / 6.74 ms.
 // ---------------------------------------------------------------------------
 // A warp's walk buffer (walk_words): the state after the chunk (8 words), its
 // wall-normal times (TIMES + 1, rounded up to 4), then -- the pointer the marches
@@ -130,9 +131,9 @@ enum WalkEnd { WALK_ON = 0, WALK_WALL = 1, WALK_COL = 2 };
 // state is advanced in shared memory (walk_state reads it back; not written
 // when there are no steps).
 // TIMES (32 or 64): wall-normal crossings a chunk may reach.  64 for uniform
-// absorption (rays through all planes take one chunk: grey 64^3 2.99 -> 2.90
-// ms, drop-in bands call 7.29 -> 7.12 ms), 32 for the others (64: 128^3 channel
-// 61.6 -> 62.2 ms, with particles at 96^3 11.6 -> 12.0 ms).
+// absorption (rays through all planes take one chunk: grey 64^3 2.90 ms, with 32
+// 2.99; drop-in bands call 7.21 and 7.31 ms), 32 for the others (128^3 channel
+// 61.6 ms, with 64 62.2; particles at 96^3 11.6 and 12.0 ms).
 template <bool TRACE, bool COL, int TIMES>
 __device__ __forceinline__ int walk_chunk(const MarchParams &P, const Walk &w, float aim, int cap, float tcol, float *buf,
                                           int lane, int *end, int step0) {
@@ -253,8 +254,8 @@ __device__ __forceinline__ void walk_state(const float *buf, Walk &w) {
 // A batch of an item's rays, set up a lane each: words, direction, spectral
 // sample and (control variate) the surrogate of ray r0 + lane go to shared
 // memory, from where the warp takes them ray by ray.
-// Every lane setting up every ray took 250 of its ~3000 instructions: 128^3
-// channel 66.1 -> 62.3 ms, 4 x 96^3 batch 130.1 -> 119.6 ms.
+// Every lane setting up every ray took 250 of its ~3000 instructions (128^3
+// channel 66.1 ms, so 62.3; 4 x 96^3 batch 130.1 and 119.6 ms).
 struct RayBatch {
     float4 walk[32];    // sinvW, dtA and dtB (signed like the direction; general medium: the
                         // direction itself), the sample's weight factor
@@ -783,8 +784,8 @@ __global__ void __launch_bounds__(256, pair_min_blocks(UNI, MOM)) march_pair_ker
 // It is bound by issue and instruction fetches (each collision runs long straight
 // code); a cell's volume fraction rides in its 16-byte coordinates, and the
 // collisions' random words, free paths and angles are set up a lane each.  96^3
-// gas with particles, 8 rays: 19.8 ms with the walk in every lane, 11.5 ms with
-// the events' set-up in every lane, 11.1 ms.
+// gas with particles, 8 rays: 10.95 ms (19.8 with the walk in every lane, 0.4
+// more with the events' set-up in every lane).
 // ---------------------------------------------------------------------------
 constexpr int kEvents = 16;  // a batch of a ray's collision and reflection events
 static_assert(kEvents * 2 * sizeof(float4) == kEventBytes, "march_pair_smem");

@@ -43,7 +43,8 @@ constexpr size_t kMiscBytes = 256;  // [0] queue, [1] status, [2] group flag (ui
 // contribution, as many as the array holds (all that 32^3 cells need up to
 // 256 rays).  One warp per item leaves most of the GPU idle on the grids this
 // entry point serves (32^3 is 512 items for about 3600 resident warps): 32^3 at
-// 60 rays 366 us unsplit, 129 us split.
+// 60 rays 366 us unsplit, 114 us split.  Beyond that room (131072 packet-rays:
+// 48^3 above 75 rays, 64^3 above 32) an item is one unit.
 constexpr long long kMaxSplitItems = 16384;
 constexpr size_t kDoneOff = kMiscOff + kMiscBytes;
 constexpr size_t kRayxOff = kDoneOff + (size_t)kMaxSplitItems * 4;
